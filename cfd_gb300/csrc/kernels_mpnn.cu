@@ -13,6 +13,9 @@
 namespace cfd {
 namespace mpnn {
 
+static_assert((N_PARAMS + 1) % 4 == 0 && L_SIZE % 4 == 0 && LAYER0 % 4 == 0 && L_U % 4 == 0,
+              "float4 accesses to the weights and to the rows of the partial gradients");
+
 // ------------------------------------------------------------------ globals and features
 __device__ __forceinline__ double block_max256(double v, double* red) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -261,224 +264,591 @@ __global__ void k_edge_features(int m, const int* __restrict__ src, const int* _
 }
 
 // ------------------------------------------------------------------ FP32 dense layers
-// Y[n][O] = [X1 | X2][n][I1 + I2] . W^T + b   (W: O x (I1+I2) row-major; b may be null)
-__global__ void __launch_bounds__(128) k_dense(int n, const float* __restrict__ X1, int I1,
-                                               const float* __restrict__ X2, int I2,
-                                               const float* __restrict__ W,
-                                               const float* __restrict__ b, int O,
-                                               float* __restrict__ Y) {
-    __shared__ float xs[DT][2 * HID + 1];
-    const int I = I1 + I2;
-    const int base = blockIdx.x * DT;
-    for (int q = threadIdx.x; q < DT * I; q += blockDim.x) {
-        const int r = q / I, k = q - r * I, node = base + r;
-        float v = 0.f;
-        if (node < n) v = (k < I1) ? X1[(size_t)node * I1 + k] : X2[(size_t)node * I2 + (k - I1)];
-        xs[r][k] = v;
+// The dense products of a training step, n x 64 or n x 128 rows against 64 x 128 weights: a
+// register-tiled FP32 GEMM (kernels below), bound by the FP32 pipe.  A block of 8 or 4
+// warps holds the whole weight matrix in shared memory as [k][column] and a tile of 64 rows
+// of X; a thread forms 8 rows x 4 columns, so that a step of four k takes 8 broadcast and 4
+// vector loads for 128 FMAs.  Each output sums its k in ascending order from the bias.
+// 49,794 nodes: 112-154 us per product before (one output column and 32 rows per thread,
+// the weights re-read from global memory per k), ~20 us now.
+constexpr int GR = 64;  // rows per tile
+// what the product's epilogue does
+enum : int {
+    GE_PLAIN = 0,     // Y = acc
+    GE_RESIDUAL = 1,  // Y = acc (v), Y2 = X + relu(acc) with X the first 64 columns of the input
+    GE_SPLIT = 2,     // columns 64.. divided by the node's degree: [d h | d agg / deg]
+    GE_ACCUM = 3      // Y = (Y + E) + acc, E the first 64 columns of a 128-wide row
+};
+
+// Y[n][N] = X[n][K] . B.  TRANS: B[k][c] = W[c][k] (forward), else W[k][c] (backward).  X is
+// [X1 | X2] in 64-column halves when K = 128 and X2 is given, and masked (X1 where gate > 0,
+// else 0) when gate is given.
+template <int K, int N, bool TRANS, int EPI>
+__global__ void __launch_bounds__(2 * N)
+k_gemm(int n, const float* __restrict__ X1, const float* __restrict__ X2,
+       const float* __restrict__ gate, const float* __restrict__ W, const float* __restrict__ bias,
+       const int* __restrict__ ptr, const float* __restrict__ E, float* __restrict__ Y,
+       float* __restrict__ Y2) {
+    extern __shared__ __align__(16) float gsm[];
+    float* Bs = gsm;          // K x N
+    float* Xs = gsm + K * N;  // GR x K
+    constexpr int T = 2 * N;  // threads: 8 x 4 outputs each
+    const int tid = threadIdx.x;
+    if (TRANS) {
+        for (int q = tid; q < N * K / 4; q += T) {  // lanes over the columns: conflict-free
+            const int c = q % N, k = 4 * (q / N);
+            const float4 w = *reinterpret_cast<const float4*>(W + (size_t)c * K + k);
+            Bs[k * N + c] = w.x;
+            Bs[(k + 1) * N + c] = w.y;
+            Bs[(k + 2) * N + c] = w.z;
+            Bs[(k + 3) * N + c] = w.w;
+        }
+    } else {
+        for (int q = tid; q < K * N / 4; q += T)
+            reinterpret_cast<float4*>(Bs)[q] = reinterpret_cast<const float4*>(W)[q];
     }
-    __syncthreads();
-    for (int o = threadIdx.x; o < O; o += blockDim.x) {
-        float acc[DT];
-        const float bo = b ? b[o] : 0.f;
+    constexpr int CT = N / 4;  // column tiles: the lanes of a warp (N = 128) or half of one
+    const int c0 = 4 * (tid % CT), r0 = 8 * (tid / CT);
+    float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (bias) b4 = *reinterpret_cast<const float4*>(bias + c0);
+    const int ntile = (n + GR - 1) / GR;
+    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+        const int base = tile * GR;
+        __syncthreads();  // the weights are in place; the previous tile has been read
+        for (int q = tid; q < GR * K / 4; q += T) {
+            const int r = q / (K / 4), k = 4 * (q - r * (K / 4)), row = base + r;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row < n) {
+                if (K == 128 && X2)
+                    v = k < 64 ? *reinterpret_cast<const float4*>(X1 + (size_t)row * 64 + k)
+                               : *reinterpret_cast<const float4*>(X2 + (size_t)row * 64 + (k - 64));
+                else
+                    v = *reinterpret_cast<const float4*>(X1 + (size_t)row * K + k);
+                if (gate) {
+                    const float4 g = *reinterpret_cast<const float4*>(gate + (size_t)row * K + k);
+                    v = make_float4(g.x > 0.f ? v.x : 0.f, g.y > 0.f ? v.y : 0.f,
+                                    g.z > 0.f ? v.z : 0.f, g.w > 0.f ? v.w : 0.f);
+                }
+            }
+            *reinterpret_cast<float4*>(Xs + r * K + k) = v;
+        }
+        __syncthreads();
+        float acc[8][4];
 #pragma unroll
-        for (int r = 0; r < DT; ++r) acc[r] = bo;
-        for (int k = 0; k < I; ++k) {
-            const float wv = W[(size_t)o * I + k];
+        for (int i = 0; i < 8; ++i) {
+            acc[i][0] = b4.x;
+            acc[i][1] = b4.y;
+            acc[i][2] = b4.z;
+            acc[i][3] = b4.w;
+        }
+#pragma unroll 2
+        for (int k = 0; k < K; k += 4) {
+            float4 b[4];
 #pragma unroll
-            for (int r = 0; r < DT; ++r) acc[r] += wv * xs[r][k];
+            for (int u = 0; u < 4; ++u)
+                b[u] = *reinterpret_cast<const float4*>(Bs + (k + u) * N + c0);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float4 x = *reinterpret_cast<const float4*>(Xs + (r0 + i) * K + k);
+                const float xv[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    acc[i][0] = fmaf(xv[u], b[u].x, acc[i][0]);
+                    acc[i][1] = fmaf(xv[u], b[u].y, acc[i][1]);
+                    acc[i][2] = fmaf(xv[u], b[u].z, acc[i][2]);
+                    acc[i][3] = fmaf(xv[u], b[u].w, acc[i][3]);
+                }
+            }
         }
 #pragma unroll
-        for (int r = 0; r < DT; ++r)
-            if (base + r < n) Y[(size_t)(base + r) * O + o] = acc[r];
+        for (int i = 0; i < 8; ++i) {
+            const int row = base + r0 + i;
+            if (row >= n) break;
+            float4 o = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+            float4* y = reinterpret_cast<float4*>(Y + (size_t)row * N + c0);
+            if (EPI == GE_RESIDUAL) {
+                const float4 h = *reinterpret_cast<const float4*>(Xs + (r0 + i) * K + c0);
+                *reinterpret_cast<float4*>(Y2 + (size_t)row * N + c0) =
+                    make_float4(h.x + fmaxf(o.x, 0.f), h.y + fmaxf(o.y, 0.f),
+                                h.z + fmaxf(o.z, 0.f), h.w + fmaxf(o.w, 0.f));
+            } else if (EPI == GE_SPLIT) {
+                if (c0 >= 64) {
+                    const float deg = (float)max(ptr[row + 1] - ptr[row], 1);
+                    o = make_float4(o.x / deg, o.y / deg, o.z / deg, o.w / deg);
+                }
+            } else if (EPI == GE_ACCUM) {
+                const float4 d = *y;
+                const float4 e = *reinterpret_cast<const float4*>(E + (size_t)row * 128 + c0);
+                o = make_float4((d.x + e.x) + o.x, (d.y + e.y) + o.y, (d.z + e.z) + o.z,
+                                (d.w + e.w) + o.w);
+            }
+            *y = o;
+        }
     }
 }
 
-// dX[n][I] = dY[n][O] . W   (W: O x I row-major)
-__global__ void __launch_bounds__(128) k_dense_t(int n, const float* __restrict__ dY, int O,
-                                                 const float* __restrict__ W, int I,
-                                                 float* __restrict__ dX) {
-    __shared__ float ys[DT][2 * HID + 1];
-    const int base = blockIdx.x * DT;
-    for (int q = threadIdx.x; q < DT * O; q += blockDim.x) {
-        const int r = q / O, o = q - r * O, node = base + r;
-        ys[r][o] = node < n ? dY[(size_t)node * O + o] : 0.f;
+template <int K, int N, bool TRANS, int EPI>
+static int gemm(cudaStream_t st, int n, const float* X1, const float* X2, const float* gate,
+                const float* W, const float* bias, const int* ptr, const float* E, float* Y,
+                float* Y2) {
+    constexpr int smem = 4 * (K * N + GR * K);
+    // the attribute belongs to a device's copy of the kernel: set once per device
+    static std::atomic<unsigned long long> done{0};
+    int dev = 0;
+    CFD_CUDA(cudaGetDevice(&dev));
+    if (dev > 63 || !(done.load(std::memory_order_relaxed) >> dev & 1ull)) {
+        CFD_CUDA(cudaFuncSetAttribute(k_gemm<K, N, TRANS, EPI>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        if (dev <= 63) done.fetch_or(1ull << dev, std::memory_order_relaxed);
     }
+    // resident blocks by shared memory (4 or 3 per SM); a block loads its weights once
+    const unsigned grid = std::min<unsigned>(blocks_for(n, GR), kTrainChunks * (227 * 1024 / (smem + 1024)));
+    CFD_LAUNCH((k_gemm<K, N, TRANS, EPI>), grid, 2 * N, smem, st, n, X1, X2, gate, W, bias, ptr, E,
+               Y, Y2);
+    return CFD_OK;
+}
+
+int dense_pq(cudaStream_t st, int n, const float* h, const float* W, float* pq) {
+    return gemm<HID, 2 * HID, true, GE_PLAIN>(st, n, h, nullptr, nullptr, W, nullptr, nullptr,
+                                              nullptr, pq, nullptr);
+}
+int dense_update(cudaStream_t st, int n, const float* h, const float* agg, const float* W,
+                 const float* b, float* v, float* h1) {
+    return gemm<2 * HID, HID, true, GE_RESIDUAL>(st, n, h, agg, nullptr, W, b, nullptr, nullptr, v,
+                                                 h1);
+}
+int dense_update_bwd(cudaStream_t st, int n, const float* dh, const float* v, const float* W,
+                     const int* ptr, float* dhc) {
+    return gemm<HID, 2 * HID, false, GE_SPLIT>(st, n, dh, nullptr, v, W, nullptr, ptr, nullptr,
+                                               dhc, nullptr);
+}
+int dense_pq_bwd(cudaStream_t st, int n, const float* dpq, const float* W, const float* dhc,
+                 float* dh) {
+    return gemm<2 * HID, HID, false, GE_ACCUM>(st, n, dpq, nullptr, nullptr, W, nullptr, nullptr,
+                                               dhc, dh, nullptr);
+}
+
+// h0 = relu(W_in f + b_in); h0 > 0 where the argument is, so it is its own backward mask
+__global__ void __launch_bounds__(256) k_encode(int n, const float* __restrict__ f,
+                                                const float* __restrict__ w,
+                                                float* __restrict__ h) {
+    __shared__ float fs[64 * F_IN];
+    const int base = blockIdx.x * 64, o = threadIdx.x & 63;
+    for (int q = threadIdx.x; q < 64 * F_IN; q += 256)
+        fs[q] = base + q / F_IN < n ? f[(size_t)base * F_IN + q] : 0.f;
+    float wr[F_IN];
+#pragma unroll
+    for (int k = 0; k < F_IN; ++k) wr[k] = w[OFF_W_IN + o * F_IN + k];
+    const float b = w[OFF_B_IN + o];
     __syncthreads();
-    for (int k = threadIdx.x; k < I; k += blockDim.x) {
-        float acc[DT];
+    for (int r = threadIdx.x >> 6; r < 64 && base + r < n; r += 4) {
+        float a = b;
 #pragma unroll
-        for (int r = 0; r < DT; ++r) acc[r] = 0.f;
-        for (int o = 0; o < O; ++o) {
-            const float wv = W[(size_t)o * I + k];
-#pragma unroll
-            for (int r = 0; r < DT; ++r) acc[r] += wv * ys[r][o];
-        }
-#pragma unroll
-        for (int r = 0; r < DT; ++r)
-            if (base + r < n) dX[(size_t)(base + r) * I + k] = acc[r];
+        for (int k = 0; k < F_IN; ++k) a = fmaf(wr[k], fs[r * F_IN + k], a);
+        h[(size_t)(base + r) * HID + o] = fmaxf(a, 0.f);
     }
 }
 
-// Weight gradient partials over chunks of WG rows: part[chunk][O*I (+O)] =
-// sum_r dY[r][o] X[r][k] (and sum_r dY[r][o] for the bias)
-__global__ void __launch_bounds__(256) k_wgrad(int n, const float* __restrict__ dY, int O,
-                                               const float* __restrict__ X1, int I1,
-                                               const float* __restrict__ X2, int I2, int with_bias,
-                                               float* __restrict__ part) {
-    extern __shared__ float sm[];
-    const int I = I1 + I2;
-    float* ys = sm;              // WG x O
-    float* xs = sm + WG * O;     // WG x I
-    const int base = blockIdx.x * WG;
-    for (int q = threadIdx.x; q < WG * O; q += blockDim.x) {
-        const int r = q / O, o = q - r * O, row = base + r;
-        ys[q] = row < n ? dY[(size_t)row * O + o] : 0.f;
+// ------------------------------------------------------------------ weight gradients
+// Every weight gradient is a sum over rows, split over kTrainChunks blocks: block c sums its
+// rows' contribution to its slice of the parameters into row c of `part` (kTrainChunks x
+// (N_PARAMS + 1); the last column is the loss), and k_fold adds the rows in order.
+// The fixed chunk count (one block per SM) keeps a step deterministic.
+//
+// dW[O][I] = sum_r dY[r][O] X[r][I] (and the bias sum_r dY[r][O]) for O x I = 64 x 128 or
+// 128 x 64: two groups of 256 threads take alternate rows of a 32-row tile, a thread forms
+// 8 x 4 outputs (3 vector loads for 32 FMAs), the next tile's values are loaded while this
+// one is summed.  49,794 nodes: 128 us + 54 us of fold before (2 shared loads per FMA, 64
+// rows per partial, 779 partials folded by one thread each), ~15 us now.
+template <int O, int I>
+__global__ void __launch_bounds__(512)
+k_wgrad(int n, const float* __restrict__ dY, const float* __restrict__ gate,
+        const float* __restrict__ X1, const float* __restrict__ X2, float* __restrict__ part,
+        int off, int bias_off) {
+    constexpr int R = 32, V = R * (O + I) / 4 / 512;  // float4 per thread and tile
+    __shared__ __align__(16) float ys[R * O], xs[R * I];
+    const int tid = threadIdx.x, grp = tid >> 8, t = tid & 255;
+    constexpr int IT = I / 4;
+    const int i0 = 4 * (t % IT), o0 = 8 * (t / IT);
+    const int rows = (n + kTrainChunks - 1) / kTrainChunks;
+    const int b0 = blockIdx.x * rows, b1 = min(n, b0 + rows);
+    float acc[8][4] = {}, bs[8] = {};
+    float4 pre[V];
+    auto fetch = [&](int base) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const int q = tid + 512 * v;
+            float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (q < R * O / 4) {
+                const int r = q / (O / 4), c = 4 * (q - r * (O / 4)), row = base + r;
+                if (row < b1) {
+                    w = *reinterpret_cast<const float4*>(dY + (size_t)row * O + c);
+                    if (gate) {
+                        const float4 g =
+                            *reinterpret_cast<const float4*>(gate + (size_t)row * O + c);
+                        w = make_float4(g.x > 0.f ? w.x : 0.f, g.y > 0.f ? w.y : 0.f,
+                                        g.z > 0.f ? w.z : 0.f, g.w > 0.f ? w.w : 0.f);
+                    }
+                }
+            } else {
+                const int p = q - R * O / 4, r = p / (I / 4), c = 4 * (p - r * (I / 4)),
+                          row = base + r;
+                if (row < b1)
+                    w = (I == 64 || c < 64)
+                            ? *reinterpret_cast<const float4*>(X1 + (size_t)row * 64 + c)
+                            : *reinterpret_cast<const float4*>(X2 + (size_t)row * 64 + (c - 64));
+            }
+            pre[v] = w;
+        }
+    };
+    fetch(b0);
+    for (int base = b0; base < b1; base += R) {
+        __syncthreads();
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const int q = tid + 512 * v;
+            if (q < R * O / 4) reinterpret_cast<float4*>(ys)[q] = pre[v];
+            else reinterpret_cast<float4*>(xs)[q - R * O / 4] = pre[v];
+        }
+        __syncthreads();
+        if (base + R < b1) fetch(base + R);
+#pragma unroll 4
+        for (int r = grp; r < R; r += 2) {
+            const float4 ya = *reinterpret_cast<const float4*>(ys + r * O + o0);
+            const float4 yb = *reinterpret_cast<const float4*>(ys + r * O + o0 + 4);
+            const float4 x = *reinterpret_cast<const float4*>(xs + r * I + i0);
+            const float y[8] = {ya.x, ya.y, ya.z, ya.w, yb.x, yb.y, yb.z, yb.w};
+#pragma unroll
+            for (int a = 0; a < 8; ++a) {
+                acc[a][0] = fmaf(y[a], x.x, acc[a][0]);
+                acc[a][1] = fmaf(y[a], x.y, acc[a][1]);
+                acc[a][2] = fmaf(y[a], x.z, acc[a][2]);
+                acc[a][3] = fmaf(y[a], x.w, acc[a][3]);
+                bs[a] += y[a];
+            }
+        }
     }
-    for (int q = threadIdx.x; q < WG * I; q += blockDim.x) {
-        const int r = q / I, k = q - r * I, row = base + r;
-        float v = 0.f;
-        if (row < n) v = (k < I1) ? X1[(size_t)row * I1 + k] : X2[(size_t)row * I2 + (k - I1)];
-        xs[q] = v;
+    // group 1 hands its sums to group 0, two output rows at a time (xs holds 256 x 8 floats)
+    float* out = part + (size_t)blockIdx.x * (N_PARAMS + 1);
+    static_assert(R * I >= 256 * 8, "hand-over buffer");
+#pragma unroll
+    for (int a = 0; a < 8; a += 2) {
+        __syncthreads();
+        if (grp == 1) {
+            reinterpret_cast<float4*>(xs)[t] = make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
+            reinterpret_cast<float4*>(xs)[256 + t] =
+                make_float4(acc[a + 1][0], acc[a + 1][1], acc[a + 1][2], acc[a + 1][3]);
+        }
+        __syncthreads();
+        if (grp == 0) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float4 q = reinterpret_cast<const float4*>(xs)[256 * u + t];
+                // 16-byte aligned: N_PARAMS + 1, the slices' offsets and I are multiples of 4
+                *reinterpret_cast<float4*>(out + off + (o0 + a + u) * I + i0) =
+                    make_float4(acc[a + u][0] + q.x, acc[a + u][1] + q.y, acc[a + u][2] + q.z,
+                                acc[a + u][3] + q.w);
+            }
+        }
+    }
+    if (bias_off >= 0 && i0 == 0) {
+        if (grp == 1)
+#pragma unroll
+            for (int a = 0; a < 8; ++a) ys[o0 + a] = bs[a];
     }
     __syncthreads();
-    const int stride = O * I + (with_bias ? O : 0);
-    float* out = part + (size_t)blockIdx.x * stride;
-    for (int q = threadIdx.x; q < O * I; q += blockDim.x) {
-        const int o = q / I, k = q - o * I;
-        float acc = 0.f;
-        for (int r = 0; r < WG; ++r) acc += ys[r * O + o] * xs[r * I + k];
-        out[q] = acc;
-    }
-    if (with_bias)
-        for (int o = threadIdx.x; o < O; o += blockDim.x) {
-            float acc = 0.f;
-            for (int r = 0; r < WG; ++r) acc += ys[r * O + o];
-            out[O * I + o] = acc;
-        }
+    if (bias_off >= 0 && i0 == 0 && grp == 0)
+#pragma unroll
+        for (int a = 0; a < 8; ++a) out[bias_off + o0 + a] = bs[a] + ys[o0 + a];
 }
 
-// out[q] (+)= sum over chunks c (in order) of part[c][q]
-__global__ void k_fold(int nchunk, int stride, const float* __restrict__ part, int accumulate,
-                       float* __restrict__ out) {
+int wgrad_update(cudaStream_t st, int n, const float* dh, const float* v, const float* h,
+                 const float* agg, float* part, int layer) {
+    CFD_LAUNCH((k_wgrad<HID, 2 * HID>), kTrainChunks, 512, 0, st, n, dh, v, h, agg, part,
+               layer_off(layer) + L_U, layer_off(layer) + L_u);
+    return CFD_OK;
+}
+int wgrad_pq(cudaStream_t st, int n, const float* dpq, const float* h, float* part, int layer) {
+    CFD_LAUNCH((k_wgrad<2 * HID, HID>), kTrainChunks, 512, 0, st, n, dpq, (const float*)nullptr, h,
+               (const float*)nullptr, part, layer_off(layer) + L_A, -1);
+    return CFD_OK;
+}
+
+// dW_in, db_in: dh masked by h0 > 0 against the features; thread = output o, rows r mod 4
+__global__ void __launch_bounds__(256) k_wgrad_in(int n, const float* __restrict__ dh,
+                                                  const float* __restrict__ h0,
+                                                  const float* __restrict__ f,
+                                                  float* __restrict__ part) {
+    __shared__ float red[4][64 * (F_IN + 1)];
+    const int o = threadIdx.x & 63, g = threadIdx.x >> 6;
+    const int rows = (n + kTrainChunks - 1) / kTrainChunks;
+    const int b0 = blockIdx.x * rows, b1 = min(n, b0 + rows);
+    float acc[F_IN + 1] = {};
+#pragma unroll 2
+    for (int r = b0 + g; r < b1; r += 4) {
+        const float d = h0[(size_t)r * HID + o] > 0.f ? dh[(size_t)r * HID + o] : 0.f;
+#pragma unroll
+        for (int k = 0; k < F_IN; ++k) acc[k] = fmaf(d, f[(size_t)r * F_IN + k], acc[k]);
+        acc[F_IN] += d;
+    }
+#pragma unroll
+    for (int k = 0; k <= F_IN; ++k) red[g][k * 64 + o] = acc[k];
+    __syncthreads();
+    float* out = part + (size_t)blockIdx.x * (N_PARAMS + 1);
+    for (int q = threadIdx.x; q < 64 * (F_IN + 1); q += 256) {
+        const int k = q >> 6, oo = q & 63;
+        const float s = (red[0][q] + red[1][q]) + (red[2][q] + red[3][q]);
+        out[k < F_IN ? OFF_W_IN + oo * F_IN + k : OFF_B_IN + oo] = s;
+    }
+}
+
+// out[q] = sum over the chunks c, in order, of part[c][q], in four interleaved sums so that
+// four loads are in flight
+__global__ void k_fold(int nq, const float* __restrict__ part, float* __restrict__ out,
+                       float* __restrict__ loss) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= stride) return;
-    float acc = 0.f;
-    for (int c = 0; c < nchunk; ++c) acc += part[(size_t)c * stride + q];
-    out[q] = accumulate ? out[q] + acc : acc;
-}
-
-// ------------------------------------------------------------------ elementwise
-__global__ void k_relu(long n, const float* __restrict__ a, float* __restrict__ h) {
-    const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (i < n) h[i] = fmaxf(a[i], 0.f);
-}
-
-// h1 = h0 + relu(v)
-__global__ void k_residual(long n, const float* __restrict__ h0, const float* __restrict__ v,
-                           float* __restrict__ h1) {
-    const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (i < n) h1[i] = h0[i] + fmaxf(v[i], 0.f);
-}
-
-// d = g * (a > 0)
-__global__ void k_relu_bwd(long n, const float* __restrict__ g, const float* __restrict__ a,
-                           float* __restrict__ d) {
-    const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (i < n) d[i] = a[i] > 0.f ? g[i] : 0.f;
-}
-
-// dh[i][o] = dh[i][o] + dhc[i][o] (first HID of the 2*HID row) + dpq[i][o]
-__global__ void k_add_dh(int n, const float* __restrict__ dhc, const float* __restrict__ dpqh,
-                         float* __restrict__ dh) {
-    const long q = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (q >= (long)n * HID) return;
-    const long i = q / HID, o = q - i * HID;
-    dh[q] = dh[q] + dhc[i * 2 * HID + o] + dpqh[q];
+    if (q >= nq) return;
+    static_assert(kTrainChunks % 4 == 0, "four sums");
+    float a[4] = {};
+    for (int c = 0; c < kTrainChunks; c += 4)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) a[u] += part[(size_t)(c + u) * nq + q];
+    const float s = (a[0] + a[1]) + (a[2] + a[3]);
+    if (q < N_PARAMS) out[q] = s;
+    else *loss = s;
 }
 
 // ------------------------------------------------------------------ message passing
-// z[k][o] = PQ[i][o] + PQ[j][HID+o] + C[o] . e[k] + c[o]   for edge k = (i -> j)
-__global__ void k_edge_fwd(int m, const int* __restrict__ src, const int* __restrict__ nbr,
-                           const float* __restrict__ PQ, const float* __restrict__ e,
-                           const float* __restrict__ C, const float* __restrict__ c,
-                           float* __restrict__ z) {
-    const long q = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (q >= (long)m * HID) return;
-    const long k = q / HID;
-    const int o = (int)(q - k * HID);
-    const int i = src[k], j = nbr[k];
-    const float* ek = e + 3 * k;
-    z[q] = PQ[(size_t)i * 2 * HID + o] + PQ[(size_t)j * 2 * HID + HID + o] +
-           (C[o * 3] * ek[0] + C[o * 3 + 1] * ek[1] + C[o * 3 + 2] * ek[2]) + c[o];
-}
-
-// agg[i][o] = sum over the edges k of i of relu(z[k][o]) / max(deg_i, 1)
-__global__ void k_node_agg(int n, const int* __restrict__ ptr, const float* __restrict__ z,
-                           float* __restrict__ agg) {
-    const long q = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (q >= (long)n * HID) return;
-    const long i = q / HID;
-    const int o = (int)(q - i * HID);
-    const int k0 = ptr[i], k1 = ptr[i + 1];
-    float s = 0.f;
-    for (int k = k0; k < k1; ++k) s += fmaxf(z[(size_t)k * HID + o], 0.f);
-    agg[q] = s / (float)max(k1 - k0, 1);
-}
-
-// dz[k][o] = dhc[i][HID+o] / max(deg_i, 1) * (z[k][o] > 0)  (dhc holds d[h; agg])
-__global__ void k_edge_bwd(int m, const int* __restrict__ src, const int* __restrict__ ptr,
-                           const float* __restrict__ dhc, const float* __restrict__ z,
-                           float* __restrict__ dz) {
-    const long q = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (q >= (long)m * HID) return;
-    const long k = q / HID;
-    const int o = (int)(q - k * HID);
-    const int i = src[k];
-    const int deg = max(ptr[i + 1] - ptr[i], 1);
-    dz[q] = z[q] > 0.f ? dhc[(size_t)i * 2 * HID + HID + o] / (float)deg : 0.f;
-}
-
-// dPQ[i][o] = sum_{k in edges(i)} dz[k][o];  dPQ[i][HID+o] = sum_{k in edges(i)} dz[rev[k]][o]
-__global__ void k_node_dpq(int n, const int* __restrict__ ptr, const int* __restrict__ rev,
-                           const float* __restrict__ dz, float* __restrict__ dPQ) {
-    const long q = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (q >= (long)n * HID) return;
-    const long i = q / HID;
-    const int o = (int)(q - i * HID);
-    float sp = 0.f, sq = 0.f;
-    for (int k = ptr[i]; k < ptr[i + 1]; ++k) {
-        sp += dz[(size_t)k * HID + o];
-        sq += dz[(size_t)rev[k] * HID + o];
-    }
-    dPQ[(size_t)i * 2 * HID + o] = sp;
-    dPQ[(size_t)i * 2 * HID + HID + o] = sq;
-}
-
-// ------------------------------------------------------------------ loss and Adam
-// dy = 2 (y - t) / nfree at free nodes; per-block partial sums of |y - t|^2 (256 threads)
-__global__ void __launch_bounds__(256) k_loss(int n, const float* __restrict__ y,
-                                              const float* __restrict__ t,
-                                              const int* __restrict__ kind, float inv_nfree,
-                                              float* __restrict__ dy, float* __restrict__ part) {
-    __shared__ float red[256];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0.f;
-    if (i < n) {
-        const bool fr = kind[i] == KIND_FREE;
+// 16 lanes per node, four channels each.  Forward: for edge k = (i -> j)
+//     z = P_i + Q_j + C e_k + c,   agg_i = sum_k relu(z) / max(deg_i, 1);
+// z itself is not kept: the backward pass needs its signs only, 64 bits per edge (bit l of
+// plane b: channel 4 l + b), formed by four ballots.  Before, z was written and read back
+// per edge and channel (76 MB per layer at 49,794 nodes: 76 + 22 us against ~20 us now).
+__global__ void __launch_bounds__(256)
+k_edge_fwd(int n, const int* __restrict__ ptr, const int* __restrict__ nbr,
+           const float* __restrict__ PQ, const float* __restrict__ e, const float* __restrict__ C,
+           const float* __restrict__ c, ushort4* __restrict__ mask, float* __restrict__ agg) {
+    const int i = (int)((blockIdx.x * 256u + threadIdx.x) >> 4), l = threadIdx.x & 15;
+    const int half = threadIdx.x & 16;
+    float cw[4][3], cb[4];
 #pragma unroll
-        for (int q = 0; q < OUT; ++q) {
-            const float d = fr ? y[OUT * i + q] - t[OUT * i + q] : 0.f;
-            l += d * d;
-            dy[OUT * i + q] = 2.f * d * inv_nfree;
+    for (int q = 0; q < 4; ++q) {
+        cb[q] = c[4 * l + q];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) cw[q][u] = C[(4 * l + q) * 3 + u];
+    }
+    const bool live = i < n;
+    const int k0 = live ? ptr[i] : 0, k1 = live ? ptr[i + 1] : 0;
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (live) p = *reinterpret_cast<const float4*>(PQ + (size_t)i * 2 * HID + 4 * l);
+    const float pv[4] = {p.x, p.y, p.z, p.w};
+    float s[4] = {};
+    const int deg = k1 - k0, steps = max(deg, __shfl_xor_sync(0xffffffffu, deg, 16));
+    constexpr int B = 4;  // edges whose gathers go out together
+    for (int t0 = 0; t0 < steps; t0 += B) {
+        float4 qv[B];
+        float ev[B][3];
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            const int k = k0 + t0 + u;
+            qv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            ev[u][0] = ev[u][1] = ev[u][2] = 0.f;
+            if (k < k1) {
+                qv[u] = *reinterpret_cast<const float4*>(PQ + (size_t)nbr[k] * 2 * HID + HID + 4 * l);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) ev[u][q] = e[3 * (size_t)k + q];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            if (t0 + u >= steps) break;  // the same in the whole warp
+            const int k = k0 + t0 + u;
+            const float qq[4] = {qv[u].x, qv[u].y, qv[u].z, qv[u].w};
+            unsigned short bits[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float z = pv[q] + qq[q] +
+                                (cw[q][0] * ev[u][0] + cw[q][1] * ev[u][1] + cw[q][2] * ev[u][2]) +
+                                cb[q];
+                const bool on = k < k1 && z > 0.f;
+                s[q] += on ? z : 0.f;
+                bits[q] = (unsigned short)(__ballot_sync(0xffffffffu, on) >> half);
+            }
+            if (l == 0 && k < k1) mask[k] = make_ushort4(bits[0], bits[1], bits[2], bits[3]);
         }
     }
-    red[threadIdx.x] = l;
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+    if (live) {
+        const float d = (float)max(deg, 1);
+        *reinterpret_cast<float4*>(agg + (size_t)i * HID + 4 * l) =
+            make_float4(s[0] / d, s[1] / d, s[2] / d, s[3] / d);
+    }
+}
+
+// Backward of the messages from g = d agg / deg (the second half of the dhc rows) and the
+// signs: with m_k the sign bits of edge k and k' its reverse edge,
+//     dP_i = g_i sum_k m_k,   dQ_i = sum_k m_k' g_nbr(k),
+//     dC += sum_i g_i sum_k m_k e_k,   dc += sum_i g_i sum_k m_k
+// so no per-edge gradient is stored.  kTrainChunks blocks, the nodes interleaved over their
+// half-warps; the block's dC, dc go to its row of `part`.  Before: 95 + 53 + 265 + 28 us per
+// layer (the edge gradients written, read by the weight gradient and the node sums, the
+// partials folded by one block); ~25 us now.
+__global__ void __launch_bounds__(1024)
+k_edge_bwd(int n, const int* __restrict__ ptr, const int* __restrict__ nbr,
+           const int* __restrict__ rev, const ushort4* __restrict__ mask,
+           const float* __restrict__ dhc, const float* __restrict__ e, float* __restrict__ dPQ,
+           float* __restrict__ part, int off) {
+    __shared__ float red[16][4 * HID];
+    const int l = threadIdx.x & 15;
+    float GC[4][3] = {}, Gc[4] = {};
+    const int stride = gridDim.x * 64;
+    for (int i = blockIdx.x * 64 + (threadIdx.x >> 4); i < n; i += stride) {
+        const int k0 = ptr[i], k1 = ptr[i + 1];
+        const float4 g4 = *reinterpret_cast<const float4*>(dhc + (size_t)i * 2 * HID + HID + 4 * l);
+        const float g[4] = {g4.x, g4.y, g4.z, g4.w};
+        float cnt[4] = {}, S[4][3] = {}, dq[4] = {};
+        for (int k = k0; k < k1; ++k) {
+            const ushort4 m = mask[k], mr = mask[rev[k]];
+            const float4 gj =
+                *reinterpret_cast<const float4*>(dhc + (size_t)nbr[k] * 2 * HID + HID + 4 * l);
+            const float e0 = e[3 * (size_t)k], e1 = e[3 * (size_t)k + 1], e2 = e[3 * (size_t)k + 2];
+            const unsigned short mb[4] = {m.x, m.y, m.z, m.w}, rb[4] = {mr.x, mr.y, mr.z, mr.w};
+            const float gv[4] = {gj.x, gj.y, gj.z, gj.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float on = (mb[q] >> l) & 1 ? 1.f : 0.f;
+                cnt[q] += on;
+                S[q][0] = fmaf(on, e0, S[q][0]);
+                S[q][1] = fmaf(on, e1, S[q][1]);
+                S[q][2] = fmaf(on, e2, S[q][2]);
+                dq[q] += (rb[q] >> l) & 1 ? gv[q] : 0.f;
+            }
+        }
+        float4* o = reinterpret_cast<float4*>(dPQ + (size_t)i * 2 * HID + 4 * l);
+        o[0] = make_float4(g[0] * cnt[0], g[1] * cnt[1], g[2] * cnt[2], g[3] * cnt[3]);
+        o[HID / 4] = make_float4(dq[0], dq[1], dq[2], dq[3]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+#pragma unroll
+            for (int u = 0; u < 3; ++u) GC[q][u] = fmaf(g[q], S[q][u], GC[q][u]);
+            Gc[q] = fmaf(g[q], cnt[q], Gc[q]);
+        }
+    }
+    // fold the block's 64 half-warps: the two of a warp by a shuffle, then 16 rows of shared
+    // memory twice, then the rows in order
+    float v[16];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll
+        for (int u = 0; u < 3; ++u) v[3 * q + u] = GC[q][u];
+        v[12 + q] = Gc[q];
+    }
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], 16);
+    const int w = threadIdx.x >> 5;
+    for (int pass = 0; pass < 2; ++pass) {
+        if ((w >> 4) == pass && (threadIdx.x & 31) < 16)
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                float& d = red[w & 15][q < 12 ? (4 * l + q / 3) * 3 + q % 3 : 3 * HID + 4 * l + (q - 12)];
+                d = pass ? d + v[q] : v[q];
+            }
         __syncthreads();
     }
-    if (threadIdx.x == 0) part[blockIdx.x] = red[0];
+    if (threadIdx.x < 4 * HID) {
+        float s = 0.f;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) s += red[r][threadIdx.x];
+        part[(size_t)blockIdx.x * (N_PARAMS + 1) + off + threadIdx.x] = s;  // C (64 x 3), then c
+    }
+}
+
+// ------------------------------------------------------------------ decoder, loss and Adam
+// y = W_out h + b_out, four lanes per node with 16 channels each.  With a target also the
+// loss |y - t|^2 over the free nodes, dy = 2 (y - t) / nfree, dh = W_out^T dy, and the
+// block's share of dW_out, db_out and the loss in its row of `part`.
+__global__ void __launch_bounds__(256)
+k_decode(int n, const float* __restrict__ h, const float* __restrict__ w, float* __restrict__ y,
+         const float* __restrict__ target, const int* __restrict__ kind, float inv_nfree,
+         float* __restrict__ dh, float* __restrict__ part) {
+    __shared__ float red[8][(HID + 1) * OUT + 1];
+    const int l = threadIdx.x & 3;
+    float wo[OUT][16], GW[OUT][16] = {}, gb[OUT] = {}, loss = 0.f;
+#pragma unroll
+    for (int o = 0; o < OUT; ++o)
+#pragma unroll
+        for (int k = 0; k < 16; ++k) wo[o][k] = w[OFF_W_OUT + o * HID + 16 * l + k];
+    const int stride = gridDim.x * 64;
+    // whole warps walk the loop together (the shuffles below)
+    for (int i0 = blockIdx.x * 64 + 8 * (threadIdx.x >> 5); i0 < n; i0 += stride) {
+        const int i = i0 + ((threadIdx.x & 31) >> 2);
+        float hv[16];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i < n) q = *reinterpret_cast<const float4*>(h + (size_t)i * HID + 16 * l + 4 * v);
+            hv[4 * v] = q.x;
+            hv[4 * v + 1] = q.y;
+            hv[4 * v + 2] = q.z;
+            hv[4 * v + 3] = q.w;
+        }
+        float d[OUT];
+#pragma unroll
+        for (int o = 0; o < OUT; ++o) {
+            float a = l == 0 ? w[OFF_B_OUT + o] : 0.f;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) a = fmaf(wo[o][k], hv[k], a);
+            a += __shfl_xor_sync(0xffffffffu, a, 1);
+            a += __shfl_xor_sync(0xffffffffu, a, 2);
+            if (l == 0 && i < n) y[(size_t)OUT * i + o] = a;
+            d[o] = a;
+        }
+        if (!target || i >= n) continue;
+        const bool fr = kind[i] == KIND_FREE;
+        float4 g[4];
+        float* gf = reinterpret_cast<float*>(g);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) gf[k] = 0.f;
+#pragma unroll
+        for (int o = 0; o < OUT; ++o) {
+            const float df = fr ? d[o] - target[(size_t)OUT * i + o] : 0.f;
+            const float dy = 2.f * df * inv_nfree;
+            if (l == 0) {
+                loss += df * df;
+                gb[o] += dy;
+            }
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                gf[k] = fmaf(dy, wo[o][k], gf[k]);
+                GW[o][k] = fmaf(dy, hv[k], GW[o][k]);
+            }
+        }
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+            *reinterpret_cast<float4*>(dh + (size_t)i * HID + 16 * l + 4 * v) = g[v];
+    }
+    if (!target) return;
+    // the eight nodes of a warp, then the eight warps in order
+    const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto fold = [&](float v, int at) {
+        v += __shfl_xor_sync(0xffffffffu, v, 4);
+        v += __shfl_xor_sync(0xffffffffu, v, 8);
+        v += __shfl_xor_sync(0xffffffffu, v, 16);
+        if (lane < 4 && at >= 0) red[wp][at] = v;
+    };
+#pragma unroll
+    for (int o = 0; o < OUT; ++o) {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) fold(GW[o][k], o * HID + 16 * l + k);
+        fold(gb[o], l == 0 ? OUT * HID + o : -1);
+    }
+    fold(loss, l == 0 ? OUT * HID + OUT : -1);
+    __syncthreads();
+    for (int q = threadIdx.x; q < (HID + 1) * OUT + 1; q += 256) {
+        float s = 0.f;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) s += red[r][q];
+        part[(size_t)blockIdx.x * (N_PARAMS + 1) + OFF_W_OUT + q] = s;  // b_out, the loss follow
+    }
 }
 
 __global__ void k_adam(int np, float* __restrict__ w, const float* __restrict__ g,

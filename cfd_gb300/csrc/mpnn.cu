@@ -58,16 +58,13 @@ struct cfd_mpnn_graph {
     double* F = nullptr;
     float *f = nullptr, *e = nullptr, *target = nullptr;
     // forward cache
-    float* a0 = nullptr;                 // n x HID (pre-activation of h0)
     float* h[LAYERS + 1] = {};           // n x HID
     float* agg[LAYERS] = {};             // n x HID
     float* v[LAYERS] = {};               // n x HID
-    float* z[LAYERS] = {};               // m x HID
+    ushort4* mask[LAYERS] = {};          // m (the signs of the messages' 64 channels)
     float *pq = nullptr, *y = nullptr;   // n x 2HID, n x OUT
-    // backward
-    float *dy = nullptr, *dh = nullptr, *dhc = nullptr, *dz = nullptr, *dpq = nullptr,
-          *dpqh = nullptr, *part = nullptr, *lpart = nullptr;
-    size_t part_floats = 0;
+    // backward; part: kTrainChunks rows of every parameter's partial gradient and the loss
+    float *dh = nullptr, *dhc = nullptr, *dpq = nullptr, *part = nullptr, *loss = nullptr;
     // inference (BF16)
     __nv_bfloat16 *hb = nullptr, *pqb = nullptr;
     float* yb = nullptr;
@@ -92,93 +89,48 @@ int arg_err(const char* what) {
 
 inline unsigned nb_of(long n, int t) { return blocks_for(n, t); }
 
-// Y = [X1|X2] W^T + b
-int dense(cudaStream_t st, int n, const float* X1, int I1, const float* X2, int I2,
-          const float* W, const float* b, int O, float* Y) {
-    CFD_LAUNCH(k_dense, nb_of(n, DT), 128, 0, st, n, X1, I1, X2, I2, W, b, O, Y);
-    return CFD_OK;
-}
-
-int dense_t(cudaStream_t st, int n, const float* dY, int O, const float* W, int I, float* dX) {
-    CFD_LAUNCH(k_dense_t, nb_of(n, DT), 128, 0, st, n, dY, O, W, I, dX);
-    return CFD_OK;
-}
-
-// gradient of the weights W (O x (I1+I2)) [and bias] into out (+= when accumulate)
-int wgrad(cudaStream_t st, cfd_mpnn_graph& g, int rows, const float* dY, int O, const float* X1,
-          int I1, const float* X2, int I2, bool bias, float* out) {
-    const int I = I1 + I2;
-    const int nchunk = (int)nb_of(rows, WG);
-    const int stride = O * I + (bias ? O : 0);
-    if ((size_t)nchunk * stride > g.part_floats) {
-        set_last_message("mpnn: gradient partial buffer too small");
-        return CFD_ERR_LIMIT;
-    }
-    const size_t smem = sizeof(float) * WG * (O + I);
-    CFD_LAUNCH(k_wgrad, nchunk, 256, smem, st, rows, dY, O, X1, I1, X2, I2, bias ? 1 : 0, g.part);
-    CFD_LAUNCH(k_fold, nb_of(stride, 256), 256, 0, st, nchunk, stride, (const float*)g.part, 0, out);
-    return CFD_OK;
-}
-
-int forward_fp32(cfd_mpnn& net, cfd_mpnn_graph& g) {
+int forward_fp32(cfd_mpnn& net, cfd_mpnn_graph& g, const float* target = nullptr) {
     cudaStream_t st = g.stream;
-    const int n = g.n, m = g.m;
-    const long nh = (long)n * HID, mh = (long)m * HID;
+    const int n = g.n;
     int rc;
-    if ((rc = dense(st, n, g.f, F_IN, nullptr, 0, net.w + OFF_W_IN, net.w + OFF_B_IN, HID, g.a0)))
-        return rc;
-    CFD_LAUNCH(k_relu, nb_of(nh, 256), 256, 0, st, nh, (const float*)g.a0, g.h[0]);
+    CFD_LAUNCH(k_encode, nb_of(n, 64), 256, 0, st, n, (const float*)g.f, (const float*)net.w, g.h[0]);
     for (int l = 0; l < LAYERS; ++l) {
         const float* W = net.w + layer_off(l);
-        if ((rc = dense(st, n, g.h[l], HID, nullptr, 0, W + L_A, nullptr, 2 * HID, g.pq))) return rc;
-        CFD_LAUNCH(k_edge_fwd, nb_of(mh, 256), 256, 0, st, m, g.src, g.nbr, (const float*)g.pq,
-                   (const float*)g.e, W + L_C, W + L_c, g.z[l]);
-        CFD_LAUNCH(k_node_agg, nb_of(nh, 256), 256, 0, st, n, g.ptr, (const float*)g.z[l], g.agg[l]);
-        if ((rc = dense(st, n, g.h[l], HID, g.agg[l], HID, W + L_U, W + L_u, HID, g.v[l]))) return rc;
-        CFD_LAUNCH(k_residual, nb_of(nh, 256), 256, 0, st, nh, (const float*)g.h[l],
-                   (const float*)g.v[l], g.h[l + 1]);
+        if ((rc = dense_pq(st, n, g.h[l], W + L_A, g.pq))) return rc;
+        CFD_LAUNCH(k_edge_fwd, nb_of(n, 16), 256, 0, st, n, g.ptr, g.nbr, (const float*)g.pq,
+                   (const float*)g.e, W + L_C, W + L_c, g.mask[l], g.agg[l]);
+        if ((rc = dense_update(st, n, g.h[l], g.agg[l], W + L_U, W + L_u, g.v[l], g.h[l + 1])))
+            return rc;
     }
-    return dense(st, n, g.h[LAYERS], HID, nullptr, 0, net.w + OFF_W_OUT, net.w + OFF_B_OUT, OUT, g.y);
+    // with a target (training) the decoder also starts the backward pass
+    CFD_LAUNCH(k_decode, kTrainChunks, 256, 0, st, n, (const float*)g.h[LAYERS], (const float*)net.w,
+               g.y, target, g.kind, 1.f / (float)std::max(g.nfree, 1), g.dh, g.part);
+    return CFD_OK;
 }
 
+// The gradient of every parameter after a forward pass with the target
 int backward_fp32(cfd_mpnn& net, cfd_mpnn_graph& g, float* loss_out) {
     cudaStream_t st = g.stream;
-    const int n = g.n, m = g.m;
-    const long nh = (long)n * HID, mh = (long)m * HID;
+    const int n = g.n;
     int rc;
-    const int nlb = (int)nb_of(n, 256);
-    CFD_LAUNCH(k_loss, nlb, 256, 0, st, n, (const float*)g.y, (const float*)g.target, g.kind,
-               1.f / (float)std::max(g.nfree, 1), g.dy, g.lpart);
-    float* lsum = g.lpart + nlb;
-    CFD_LAUNCH(k_fold, 1, 256, 0, st, nlb, 1, (const float*)g.lpart, 0, lsum);
-    // decoder
-    if ((rc = wgrad(st, g, n, g.dy, OUT, g.h[LAYERS], HID, nullptr, 0, true, net.g + OFF_W_OUT)))
-        return rc;
-    if ((rc = dense_t(st, n, g.dy, OUT, net.w + OFF_W_OUT, HID, g.dh))) return rc;
     for (int l = LAYERS - 1; l >= 0; --l) {
         const float* W = net.w + layer_off(l);
-        float* GW = net.g + layer_off(l);
-        // h_{l+1} = h_l + relu(v): dv = dh * (v > 0)
-        float* dv = g.dpqh;  // scratch n x HID
-        CFD_LAUNCH(k_relu_bwd, nb_of(nh, 256), 256, 0, st, nh, (const float*)g.dh,
-                   (const float*)g.v[l], dv);
-        if ((rc = wgrad(st, g, n, dv, HID, g.h[l], HID, g.agg[l], HID, true, GW + L_U))) return rc;
-        if ((rc = dense_t(st, n, dv, HID, W + L_U, 2 * HID, g.dhc))) return rc;
+        // h_{l+1} = h_l + relu(v), v = U [h; agg] + u
+        if ((rc = wgrad_update(st, n, g.dh, g.v[l], g.h[l], g.agg[l], g.part, l))) return rc;
+        if ((rc = dense_update_bwd(st, n, g.dh, g.v[l], W + L_U, g.ptr, g.dhc))) return rc;
         // agg_i = mean_j relu(z_ij)
-        CFD_LAUNCH(k_edge_bwd, nb_of(mh, 256), 256, 0, st, m, g.src, g.ptr, (const float*)g.dhc,
-                   (const float*)g.z[l], g.dz);
-        if ((rc = wgrad(st, g, m, g.dz, HID, g.e, E_F, nullptr, 0, true, GW + L_C))) return rc;
-        CFD_LAUNCH(k_node_dpq, nb_of(nh, 256), 256, 0, st, n, g.ptr, g.rev, (const float*)g.dz, g.dpq);
-        if ((rc = wgrad(st, g, n, g.dpq, 2 * HID, g.h[l], HID, nullptr, 0, false, GW + L_A))) return rc;
-        if ((rc = dense_t(st, n, g.dpq, 2 * HID, W + L_A, HID, g.dpqh))) return rc;
-        CFD_LAUNCH(k_add_dh, nb_of(nh, 256), 256, 0, st, n, (const float*)g.dhc,
-                   (const float*)g.dpqh, g.dh);
+        CFD_LAUNCH(k_edge_bwd, kTrainChunks, 1024, 0, st, n, g.ptr, g.nbr, g.rev,
+                   (const ushort4*)g.mask[l], (const float*)g.dhc, (const float*)g.e, g.dpq, g.part,
+                   layer_off(l) + L_C);
+        if ((rc = wgrad_pq(st, n, g.dpq, g.h[l], g.part, l))) return rc;
+        if ((rc = dense_pq_bwd(st, n, g.dpq, W + L_A, g.dhc, g.dh))) return rc;
     }
-    float* da0 = g.dpqh;
-    CFD_LAUNCH(k_relu_bwd, nb_of(nh, 256), 256, 0, st, nh, (const float*)g.dh, (const float*)g.a0, da0);
-    if ((rc = wgrad(st, g, n, da0, HID, g.f, F_IN, nullptr, 0, true, net.g + OFF_W_IN))) return rc;
+    CFD_LAUNCH(k_wgrad_in, kTrainChunks, 256, 0, st, n, (const float*)g.dh, (const float*)g.h[0],
+               (const float*)g.f, g.part);
+    CFD_LAUNCH(k_fold, nb_of(N_PARAMS + 1, 128), 128, 0, st, N_PARAMS + 1, (const float*)g.part,
+               net.g, g.loss);
     if (loss_out) {
-        CFD_CUDA(cudaMemcpyAsync(loss_out, lsum, sizeof(float), cudaMemcpyDeviceToHost, st));
+        CFD_CUDA(cudaMemcpyAsync(loss_out, g.loss, sizeof(float), cudaMemcpyDeviceToHost, st));
         CFD_CUDA(cudaStreamSynchronize(st));
         *loss_out /= (float)std::max(g.nfree, 1);
     }
@@ -266,27 +218,20 @@ int graph_build(cfd_mpnn_graph** out, int npoin, const std::vector<int>& rowptr,
     if ((rc = dev_alloc(o, &g->e, (size_t)m * E_F))) return rc;
     if (training) {
         if ((rc = dev_alloc(o, &g->target, n * OUT))) return rc;
-        if ((rc = dev_alloc(o, &g->a0, n * HID))) return rc;
         for (int l = 0; l <= LAYERS; ++l)
             if ((rc = dev_alloc(o, &g->h[l], n * HID))) return rc;
         for (int l = 0; l < LAYERS; ++l) {
             if ((rc = dev_alloc(o, &g->agg[l], n * HID))) return rc;
             if ((rc = dev_alloc(o, &g->v[l], n * HID))) return rc;
-            if ((rc = dev_alloc(o, &g->z[l], (size_t)m * HID))) return rc;
+            if ((rc = dev_alloc(o, &g->mask[l], m))) return rc;
         }
         if ((rc = dev_alloc(o, &g->pq, n * 2 * HID))) return rc;
         if ((rc = dev_alloc(o, &g->y, n * OUT))) return rc;
-        if ((rc = dev_alloc(o, &g->dy, n * OUT))) return rc;
         if ((rc = dev_alloc(o, &g->dh, n * HID))) return rc;
         if ((rc = dev_alloc(o, &g->dhc, n * 2 * HID))) return rc;
-        if ((rc = dev_alloc(o, &g->dz, (size_t)m * HID))) return rc;
         if ((rc = dev_alloc(o, &g->dpq, n * 2 * HID))) return rc;
-        if ((rc = dev_alloc(o, &g->dpqh, n * HID))) return rc;
-        // partials of the largest weight gradient: rows/WG chunks x (128*64 + 128) floats
-        const long rows = std::max<long>(npoin, m);
-        g->part_floats = (size_t)blocks_for(rows, WG) * (2 * HID * HID + 2 * HID);
-        if ((rc = dev_alloc(o, &g->part, g->part_floats))) return rc;
-        if ((rc = dev_alloc(o, &g->lpart, blocks_for(npoin, 256) + 1))) return rc;
+        if ((rc = dev_alloc(o, &g->part, (size_t)kTrainChunks * (N_PARAMS + 1)))) return rc;
+        if ((rc = dev_alloc(o, &g->loss, 1))) return rc;
     }
     g->training = training;
     if ((rc = dev_alloc(o, &g->hb, n * HID))) return rc;
@@ -468,7 +413,7 @@ int cfd_mpnn_graph_set_target(cfd_mpnn_graph* g, const double* phi, const double
 int cfd_mpnn_loss_grad(cfd_mpnn* net, cfd_mpnn_graph* g, float* loss, float* grad) {
     if (!net || !g) return arg_err("null pointer");
     if (!g->training) return arg_err("graph without training buffers");
-    int rc = forward_fp32(*net, *g);
+    int rc = forward_fp32(*net, *g, g->target);
     if (rc) return rc;
     float l = 0.f;
     if ((rc = backward_fp32(*net, *g, &l))) return rc;
@@ -485,7 +430,7 @@ int cfd_mpnn_train_step(cfd_mpnn* net, cfd_mpnn_graph* g, float lr, float* loss)
     if (!net || !g) return arg_err("null pointer");
     if (!(lr > 0.f)) return arg_err("lr");
     if (!g->training) return arg_err("graph without training buffers");
-    int rc = forward_fp32(*net, *g);
+    int rc = forward_fp32(*net, *g, g->target);
     if (rc) return rc;
     float l = 0.f;
     if ((rc = backward_fp32(*net, *g, loss ? &l : nullptr))) return rc;

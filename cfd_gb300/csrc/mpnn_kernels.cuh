@@ -5,8 +5,8 @@
 namespace cfd {
 namespace mpnn {
 
-constexpr int DT = 32;  // nodes per block of the FP32 dense kernels
-constexpr int WG = 64;  // rows per weight-gradient partial
+// row chunks of the weight gradients: one block per SM of the 152
+constexpr int kTrainChunks = 152;
 
 // kernels with a `gate` argument return at once when gate != null and *gate == 0
 __global__ void k_globals(int nb, const int* bnode, const int* bkind, const double* gx,
@@ -23,24 +23,29 @@ __global__ void k_features(int n, const double* X, const double* Y, const int* k
                            const Globals* G, float* f, const int* gate);
 __global__ void k_edge_features(int m, const int* src, const int* nbr, const double* X,
                                 const double* Y, const Globals* G, float* e, const int* gate);
-__global__ void k_dense(int n, const float* X1, int I1, const float* X2, int I2, const float* W,
-                        const float* b, int O, float* Y);
-__global__ void k_dense_t(int n, const float* dY, int O, const float* W, int I, float* dX);
-__global__ void k_wgrad(int n, const float* dY, int O, const float* X1, int I1, const float* X2,
-                        int I2, int with_bias, float* part);
-__global__ void k_fold(int nchunk, int stride, const float* part, int accumulate, float* out);
-__global__ void k_relu(long n, const float* a, float* h);
-__global__ void k_residual(long n, const float* h0, const float* v, float* h1);
-__global__ void k_relu_bwd(long n, const float* g, const float* a, float* d);
-__global__ void k_add_dh(int n, const float* dhc, const float* dpqh, float* dh);
-__global__ void k_edge_fwd(int m, const int* src, const int* nbr, const float* PQ, const float* e,
-                           const float* C, const float* c, float* z);
-__global__ void k_node_agg(int n, const int* ptr, const float* z, float* agg);
-__global__ void k_edge_bwd(int m, const int* src, const int* ptr, const float* dhc, const float* z,
-                           float* dz);
-__global__ void k_node_dpq(int n, const int* ptr, const int* rev, const float* dz, float* dPQ);
-__global__ void k_loss(int n, const float* y, const float* t, const int* kind, float inv_nfree,
-                       float* dy, float* part);
+// FP32 training passes (kernels_mpnn.cu): P|Q = [A; B] h; v = U [h; agg] + u and h1 = h +
+// relu(v); their backward products (dhc = [dh | dagg / deg], dh += its first half + dPQ [A; B])
+int dense_pq(cudaStream_t st, int n, const float* h, const float* W, float* pq);
+int dense_update(cudaStream_t st, int n, const float* h, const float* agg, const float* W,
+                 const float* b, float* v, float* h1);
+int dense_update_bwd(cudaStream_t st, int n, const float* dh, const float* v, const float* W,
+                     const int* ptr, float* dhc);
+int dense_pq_bwd(cudaStream_t st, int n, const float* dpq, const float* W, const float* dhc,
+                 float* dh);
+// weight gradients of layer `layer` into the chunk rows of part
+int wgrad_update(cudaStream_t st, int n, const float* dh, const float* v, const float* h,
+                 const float* agg, float* part, int layer);
+int wgrad_pq(cudaStream_t st, int n, const float* dpq, const float* h, float* part, int layer);
+__global__ void k_encode(int n, const float* f, const float* w, float* h);
+__global__ void k_wgrad_in(int n, const float* dh, const float* h0, const float* f, float* part);
+__global__ void k_fold(int nq, const float* part, float* out, float* loss);
+__global__ void k_edge_fwd(int n, const int* ptr, const int* nbr, const float* PQ, const float* e,
+                           const float* C, const float* c, ushort4* mask, float* agg);
+__global__ void k_edge_bwd(int n, const int* ptr, const int* nbr, const int* rev,
+                           const ushort4* mask, const float* dhc, const float* e, float* dPQ,
+                           float* part, int off);
+__global__ void k_decode(int n, const float* h, const float* w, float* y, const float* target,
+                         const int* kind, float inv_nfree, float* dh, float* part);
 __global__ void k_adam(int np, float* w, const float* g, float* m, float* v, float lr, float b1,
                        float b2, float eps, float bc1, float bc2);
 __global__ void k_targets(int n, const double* phi, const double* psx, const double* psy,

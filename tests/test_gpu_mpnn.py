@@ -64,6 +64,30 @@ def test_forward_and_gradient_match_oracle(gpu_lib):
         assert np.linalg.norm(P[name] - Pr[name]) <= 2e-4 * max(nr, 1e-8), name
 
 
+@pytest.mark.parametrize("nr,nt", [(3, 8), (8, 8), (13, 10), (19, 16), (41, 30)])
+def test_gradient_at_tile_edges(gpu_lib, nr, nt):
+    """Node counts at the edges of the training kernels' tiles: 24 (fewer rows than the 152
+    gradient chunks), 64 (one whole 64-row tile), 130 (a ragged third tile), 304 (two rows
+    per chunk), 1230 (ragged tiles and chunks).  Tolerances as in the test above."""
+    from cfd_gb300 import case as cs, learned
+    k = cs.ogrid_case("edge", nr, nt, cs.flow_params(mach=0.3, re=100.0), body="ellipse",
+                      semi_b=0.2, seed=nr)
+    G, kind, gfull, Gr, (f, i, j, e, deg) = setup(k)
+    rng = np.random.default_rng(nr)
+    w = (M.init_params(5) + 0.05 * rng.normal(size=M.n_params())).astype(np.float32)
+    net = learned.Net(w)
+    t = [0.3 * rng.normal(size=k.npoin) for _ in range(3)]
+    G.set_target(*t)
+    loss, grad = net.loss_grad(G)
+    target = np.stack([t[0], t[1] / Gr["L"], t[2] / Gr["L"]], 1)
+    lref, gref = M.loss_and_grad(w.astype(np.float64), f, i, j, e, deg, target,
+                                 (kind == 0).astype(float))
+    assert abs(loss - lref) <= 1e-5 * lref
+    P, Pr = M.unpack(grad.astype(np.float64)), M.unpack(gref)
+    for name in Pr:
+        assert np.linalg.norm(P[name] - Pr[name]) <= 2e-4 * max(np.linalg.norm(Pr[name]), 1e-8), name
+
+
 def test_adam_step_and_determinism(gpu_lib):
     from cfd_gb300 import learned
     k = small_case(1, scale=12, seed=3)
