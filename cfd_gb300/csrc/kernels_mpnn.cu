@@ -265,13 +265,17 @@ __global__ void k_edge_features(int m, const int* __restrict__ src, const int* _
 
 // ------------------------------------------------------------------ FP32 dense layers
 // The dense products of a training step, n x 64 or n x 128 rows against 64 x 128 weights: a
-// register-tiled FP32 GEMM (kernels below), bound by the FP32 pipe.  A block of 8 or 4
-// warps holds the whole weight matrix in shared memory as [k][column] and a tile of 64 rows
-// of X; a thread forms 8 rows x 4 columns, so that a step of four k takes 8 broadcast and 4
-// vector loads for 128 FMAs.  Each output sums its k in ascending order from the bias.
-// 49,794 nodes: 112-154 us per product before (one output column and 32 rows per thread,
-// the weights re-read from global memory per k), ~20 us now.
-constexpr int GR = 64;  // rows per tile
+// register-tiled FP32 GEMM, bound by the FP32 pipe.  A block holds the whole weight matrix in
+// shared memory as [k][column]; each of its warps walks over row groups of its own (16 rows,
+// private to the warp, so that no block barrier separates one warp's loads from another's
+// FMAs).  A thread forms 8 rows x 8 columns (N = 128; 24 shared wavefronts for 256 FMAs of a
+// step of four k) or 4 x 8 (N = 64).  The lanes of a warp that share columns take adjacent
+// rows of a 4-float padded tile, and a thread's columns come in two groups of four, which
+// keeps every vector load free of bank conflicts.  Each output sums its k in ascending order
+// from the bias.  49,794 nodes: 112-154 us per product with one output column and 32 rows
+// per thread and the weights re-read from global memory, 35-45 us with 8 x 4 outputs in
+// 64-row block tiles, 26-40 us now.
+constexpr int GR = 16;  // rows of a warp's group
 // what the product's epilogue does
 enum : int {
     GE_PLAIN = 0,     // Y = acc
@@ -279,21 +283,33 @@ enum : int {
     GE_SPLIT = 2,     // columns 64.. divided by the node's degree: [d h | d agg / deg]
     GE_ACCUM = 3      // Y = (Y + E) + acc, E the first 64 columns of a 128-wide row
 };
+template <int K, int N>
+struct GemmShape {
+    static constexpr int RT = N / 16;              // rows per thread
+    static constexpr int RG = GR / RT;             // row groups of a warp (2 or 4)
+    static constexpr int L = 32 / RG;              // lanes over the columns
+    static constexpr int KS = K + 4;               // padded row stride
+    static constexpr int WARPS = N == 128 ? 8 : 16;
+    static constexpr int PER_SM = N == 128 ? 2 : 1;
+    static constexpr int SMEM = 4 * (K * N + WARPS * GR * KS);
+    static_assert(8 * L == N && RT * RG == GR, "thread tile");
+};
 
 // Y[n][N] = X[n][K] . B.  TRANS: B[k][c] = W[c][k] (forward), else W[k][c] (backward).  X is
-// [X1 | X2] in 64-column halves when K = 128 and X2 is given, and masked (X1 where gate > 0,
+// [X1 | X2] in 64-column halves when X2 is given (K = 128), and masked (X1 where gate > 0,
 // else 0) when gate is given.
 template <int K, int N, bool TRANS, int EPI>
-__global__ void __launch_bounds__(2 * N)
+__global__ void __launch_bounds__(32 * GemmShape<K, N>::WARPS, GemmShape<K, N>::PER_SM)
 k_gemm(int n, const float* __restrict__ X1, const float* __restrict__ X2,
        const float* __restrict__ gate, const float* __restrict__ W, const float* __restrict__ bias,
        const int* __restrict__ ptr, const float* __restrict__ E, float* __restrict__ Y,
        float* __restrict__ Y2) {
+    typedef GemmShape<K, N> G;
     extern __shared__ __align__(16) float gsm[];
-    float* Bs = gsm;          // K x N
-    float* Xs = gsm + K * N;  // GR x K
-    constexpr int T = 2 * N;  // threads: 8 x 4 outputs each
-    const int tid = threadIdx.x;
+    float* Bs = gsm;  // K x N
+    constexpr int T = 32 * G::WARPS, RT = G::RT, KS = G::KS;
+    const int tid = threadIdx.x, lane = tid & 31;
+    float* Xs = gsm + K * N + (tid >> 5) * GR * KS;  // the warp's rows
     if (TRANS) {
         for (int q = tid; q < N * K / 4; q += T) {  // lanes over the columns: conflict-free
             const int c = q % N, k = 4 * (q / N);
@@ -307,15 +323,20 @@ k_gemm(int n, const float* __restrict__ X1, const float* __restrict__ X2,
         for (int q = tid; q < K * N / 4; q += T)
             reinterpret_cast<float4*>(Bs)[q] = reinterpret_cast<const float4*>(W)[q];
     }
-    constexpr int CT = N / 4;  // column tiles: the lanes of a warp (N = 128) or half of one
-    const int c0 = 4 * (tid % CT), r0 = 8 * (tid / CT);
-    float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (bias) b4 = *reinterpret_cast<const float4*>(bias + c0);
-    const int ntile = (n + GR - 1) / GR;
-    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
-        const int base = tile * GR;
-        __syncthreads();  // the weights are in place; the previous tile has been read
-        for (int q = tid; q < GR * K / 4; q += T) {
+    __syncthreads();
+    const int c0 = 4 * (lane % G::L), c1 = c0 + N / 2, rg = lane / G::L;
+    float4 ba = make_float4(0.f, 0.f, 0.f, 0.f), bb = ba;
+    if (bias) {
+        ba = *reinterpret_cast<const float4*>(bias + c0);
+        bb = *reinterpret_cast<const float4*>(bias + c1);
+    }
+    const int ngroup = (n + GR - 1) / GR;
+    // groups interleaved over the blocks, so that a last partial round spreads over all SMs
+    for (int grp = (tid >> 5) * gridDim.x + blockIdx.x; grp < ngroup; grp += gridDim.x * G::WARPS) {
+        const int base = grp * GR;
+        __syncwarp();  // the previous group has been read
+#pragma unroll 8
+        for (int q = lane; q < GR * K / 4; q += 32) {
             const int r = q / (K / 4), k = 4 * (q - r * (K / 4)), row = base + r;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
             if (row < n) {
@@ -330,59 +351,73 @@ k_gemm(int n, const float* __restrict__ X1, const float* __restrict__ X2,
                                     g.z > 0.f ? v.z : 0.f, g.w > 0.f ? v.w : 0.f);
                 }
             }
-            *reinterpret_cast<float4*>(Xs + r * K + k) = v;
+            *reinterpret_cast<float4*>(Xs + r * KS + k) = v;
         }
-        __syncthreads();
-        float acc[8][4];
+        __syncwarp();
+        float acc[RT][8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            acc[i][0] = b4.x;
-            acc[i][1] = b4.y;
-            acc[i][2] = b4.z;
-            acc[i][3] = b4.w;
+        for (int i = 0; i < RT; ++i) {
+            acc[i][0] = ba.x;
+            acc[i][1] = ba.y;
+            acc[i][2] = ba.z;
+            acc[i][3] = ba.w;
+            acc[i][4] = bb.x;
+            acc[i][5] = bb.y;
+            acc[i][6] = bb.z;
+            acc[i][7] = bb.w;
         }
-#pragma unroll 2
+#pragma unroll 1
         for (int k = 0; k < K; k += 4) {
-            float4 b[4];
+            float4 x[RT];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                b[u] = *reinterpret_cast<const float4*>(Bs + (k + u) * N + c0);
+            for (int i = 0; i < RT; ++i)
+                x[i] = *reinterpret_cast<const float4*>(Xs + (G::RG * i + rg) * KS + k);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float4 x = *reinterpret_cast<const float4*>(Xs + (r0 + i) * K + k);
-                const float xv[4] = {x.x, x.y, x.z, x.w};
+            for (int u = 0; u < 4; ++u) {
+                const float4 b0 = *reinterpret_cast<const float4*>(Bs + (k + u) * N + c0);
+                const float4 b1 = *reinterpret_cast<const float4*>(Bs + (k + u) * N + c1);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    acc[i][0] = fmaf(xv[u], b[u].x, acc[i][0]);
-                    acc[i][1] = fmaf(xv[u], b[u].y, acc[i][1]);
-                    acc[i][2] = fmaf(xv[u], b[u].z, acc[i][2]);
-                    acc[i][3] = fmaf(xv[u], b[u].w, acc[i][3]);
+                for (int i = 0; i < RT; ++i) {
+                    const float xv = u == 0 ? x[i].x : u == 1 ? x[i].y : u == 2 ? x[i].z : x[i].w;
+                    acc[i][0] = fmaf(xv, b0.x, acc[i][0]);
+                    acc[i][1] = fmaf(xv, b0.y, acc[i][1]);
+                    acc[i][2] = fmaf(xv, b0.z, acc[i][2]);
+                    acc[i][3] = fmaf(xv, b0.w, acc[i][3]);
+                    acc[i][4] = fmaf(xv, b1.x, acc[i][4]);
+                    acc[i][5] = fmaf(xv, b1.y, acc[i][5]);
+                    acc[i][6] = fmaf(xv, b1.z, acc[i][6]);
+                    acc[i][7] = fmaf(xv, b1.w, acc[i][7]);
                 }
             }
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int row = base + r0 + i;
+        for (int i = 0; i < RT; ++i) {
+            const int r = G::RG * i + rg, row = base + r;
             if (row >= n) break;
-            float4 o = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-            float4* y = reinterpret_cast<float4*>(Y + (size_t)row * N + c0);
-            if (EPI == GE_RESIDUAL) {
-                const float4 h = *reinterpret_cast<const float4*>(Xs + (r0 + i) * K + c0);
-                *reinterpret_cast<float4*>(Y2 + (size_t)row * N + c0) =
-                    make_float4(h.x + fmaxf(o.x, 0.f), h.y + fmaxf(o.y, 0.f),
-                                h.z + fmaxf(o.z, 0.f), h.w + fmaxf(o.w, 0.f));
-            } else if (EPI == GE_SPLIT) {
-                if (c0 >= 64) {
-                    const float deg = (float)max(ptr[row + 1] - ptr[row], 1);
-                    o = make_float4(o.x / deg, o.y / deg, o.z / deg, o.w / deg);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int c = h ? c1 : c0;
+                float4 o = make_float4(acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2],
+                                       acc[i][4 * h + 3]);
+                float4* y = reinterpret_cast<float4*>(Y + (size_t)row * N + c);
+                if (EPI == GE_RESIDUAL) {
+                    const float4 x = *reinterpret_cast<const float4*>(Xs + r * KS + c);
+                    *reinterpret_cast<float4*>(Y2 + (size_t)row * N + c) =
+                        make_float4(x.x + fmaxf(o.x, 0.f), x.y + fmaxf(o.y, 0.f),
+                                    x.z + fmaxf(o.z, 0.f), x.w + fmaxf(o.w, 0.f));
+                } else if (EPI == GE_SPLIT) {
+                    if (h) {
+                        const float deg = (float)max(ptr[row + 1] - ptr[row], 1);
+                        o = make_float4(o.x / deg, o.y / deg, o.z / deg, o.w / deg);
+                    }
+                } else if (EPI == GE_ACCUM) {
+                    const float4 d = *y;
+                    const float4 e = *reinterpret_cast<const float4*>(E + (size_t)row * 128 + c);
+                    o = make_float4((d.x + e.x) + o.x, (d.y + e.y) + o.y, (d.z + e.z) + o.z,
+                                    (d.w + e.w) + o.w);
                 }
-            } else if (EPI == GE_ACCUM) {
-                const float4 d = *y;
-                const float4 e = *reinterpret_cast<const float4*>(E + (size_t)row * 128 + c0);
-                o = make_float4((d.x + e.x) + o.x, (d.y + e.y) + o.y, (d.z + e.z) + o.z,
-                                (d.w + e.w) + o.w);
+                *y = o;
             }
-            *y = o;
         }
     }
 }
@@ -391,20 +426,20 @@ template <int K, int N, bool TRANS, int EPI>
 static int gemm(cudaStream_t st, int n, const float* X1, const float* X2, const float* gate,
                 const float* W, const float* bias, const int* ptr, const float* E, float* Y,
                 float* Y2) {
-    constexpr int smem = 4 * (K * N + GR * K);
+    typedef GemmShape<K, N> G;
     // the attribute belongs to a device's copy of the kernel: set once per device
     static std::atomic<unsigned long long> done{0};
     int dev = 0;
     CFD_CUDA(cudaGetDevice(&dev));
     if (dev > 63 || !(done.load(std::memory_order_relaxed) >> dev & 1ull)) {
         CFD_CUDA(cudaFuncSetAttribute(k_gemm<K, N, TRANS, EPI>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM));
         if (dev <= 63) done.fetch_or(1ull << dev, std::memory_order_relaxed);
     }
-    // resident blocks by shared memory (4 or 3 per SM); a block loads its weights once
-    const unsigned grid = std::min<unsigned>(blocks_for(n, GR), kTrainChunks * (227 * 1024 / (smem + 1024)));
-    CFD_LAUNCH((k_gemm<K, N, TRANS, EPI>), grid, 2 * N, smem, st, n, X1, X2, gate, W, bias, ptr, E,
-               Y, Y2);
+    // the resident blocks of the 152 SMs (each loads the weights once), fewer for few rows
+    const unsigned grid = std::min<unsigned>(blocks_for(n, GR * G::WARPS), kTrainChunks * G::PER_SM);
+    CFD_LAUNCH((k_gemm<K, N, TRANS, EPI>), grid, 32 * G::WARPS, G::SMEM, st, n, X1, X2, gate, W,
+               bias, ptr, E, Y, Y2);
     return CFD_OK;
 }
 
@@ -574,30 +609,48 @@ int wgrad_pq(cudaStream_t st, int n, const float* dpq, const float* h, float* pa
     return CFD_OK;
 }
 
-// dW_in, db_in: dh masked by h0 > 0 against the features; thread = output o, rows r mod 4
-__global__ void __launch_bounds__(256) k_wgrad_in(int n, const float* __restrict__ dh,
+// dW_in, db_in: dh masked by h0 > 0 against the features; thread = output o, rows r mod 8,
+// eight rows' loads in flight (78 us with one row at a time at 49,794 nodes, 22 us now)
+__global__ void __launch_bounds__(512) k_wgrad_in(int n, const float* __restrict__ dh,
                                                   const float* __restrict__ h0,
                                                   const float* __restrict__ f,
                                                   float* __restrict__ part) {
-    __shared__ float red[4][64 * (F_IN + 1)];
+    constexpr int G = 8, R = 64;
+    __shared__ float fs[R * F_IN];
+    __shared__ float red[G][64 * (F_IN + 1)];
     const int o = threadIdx.x & 63, g = threadIdx.x >> 6;
     const int rows = (n + kTrainChunks - 1) / kTrainChunks;
     const int b0 = blockIdx.x * rows, b1 = min(n, b0 + rows);
     float acc[F_IN + 1] = {};
-#pragma unroll 2
-    for (int r = b0 + g; r < b1; r += 4) {
-        const float d = h0[(size_t)r * HID + o] > 0.f ? dh[(size_t)r * HID + o] : 0.f;
+    for (int base = b0; base < b1; base += R) {
+        __syncthreads();
+        for (int q = threadIdx.x; q < R * F_IN; q += 512)
+            fs[q] = base + q / F_IN < b1 ? f[(size_t)base * F_IN + q] : 0.f;
+        float d[R / G], m[R / G];
 #pragma unroll
-        for (int k = 0; k < F_IN; ++k) acc[k] = fmaf(d, f[(size_t)r * F_IN + k], acc[k]);
-        acc[F_IN] += d;
+        for (int u = 0; u < R / G; ++u) {
+            const int r = base + g + G * u;
+            d[u] = r < b1 ? dh[(size_t)r * HID + o] : 0.f;
+            m[u] = r < b1 ? h0[(size_t)r * HID + o] : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < R / G; ++u) {
+            const float v = m[u] > 0.f ? d[u] : 0.f;
+#pragma unroll
+            for (int k = 0; k < F_IN; ++k) acc[k] = fmaf(v, fs[(g + G * u) * F_IN + k], acc[k]);
+            acc[F_IN] += v;
+        }
     }
 #pragma unroll
     for (int k = 0; k <= F_IN; ++k) red[g][k * 64 + o] = acc[k];
     __syncthreads();
     float* out = part + (size_t)blockIdx.x * (N_PARAMS + 1);
-    for (int q = threadIdx.x; q < 64 * (F_IN + 1); q += 256) {
+    for (int q = threadIdx.x; q < 64 * (F_IN + 1); q += 512) {
         const int k = q >> 6, oo = q & 63;
-        const float s = (red[0][q] + red[1][q]) + (red[2][q] + red[3][q]);
+        float s = 0.f;
+#pragma unroll
+        for (int u = 0; u < G; ++u) s += red[u][q];
         out[k < F_IN ? OFF_W_IN + oo * F_IN + k : OFF_B_IN + oo] = s;
     }
 }

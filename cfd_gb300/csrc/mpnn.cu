@@ -125,7 +125,7 @@ int backward_fp32(cfd_mpnn& net, cfd_mpnn_graph& g, float* loss_out) {
         if ((rc = wgrad_pq(st, n, g.dpq, g.h[l], g.part, l))) return rc;
         if ((rc = dense_pq_bwd(st, n, g.dpq, W + L_A, g.dhc, g.dh))) return rc;
     }
-    CFD_LAUNCH(k_wgrad_in, kTrainChunks, 256, 0, st, n, (const float*)g.dh, (const float*)g.h[0],
+    CFD_LAUNCH(k_wgrad_in, kTrainChunks, 512, 0, st, n, (const float*)g.dh, (const float*)g.h[0],
                (const float*)g.f, g.part);
     CFD_LAUNCH(k_fold, nb_of(N_PARAMS + 1, 128), 128, 0, st, N_PARAMS + 1, (const float*)g.part,
                net.g, g.loss);
