@@ -1104,7 +1104,7 @@ int cfd_bicg_mode(const double* spMtx, const int* spIdx, const int* spRowptr,
     TRY(s.init());
     int *d_rp, *d_col, *d_un, *d_us, *d_it, *d_cv;
     unsigned char* d_isfix;
-    double *d_val, *d_diag, *d_x, *d_b, *d_fv, *d_r, *d_z, *d_y, *d_p0, *d_p1, *d_part, *d_rz;
+    double *d_val, *d_diag, *d_rdiag, *d_x, *d_b, *d_fv, *d_r, *d_z, *d_y, *d_p0, *d_part, *d_rz;
     GridBar* d_bar;
     TRY(s.put(&d_rp, spRowptr, N + 1));
     TRY(s.put(&d_col, col.data(), nnz));
@@ -1116,7 +1116,7 @@ int cfd_bicg_mode(const double* spMtx, const int* spIdx, const int* spRowptr,
     TRY(s.put(&d_fv, NF ? x_fix : (const double*)&tol, NF ? NF : 1));
     TRY(s.put(&d_x, x, N));
     TRY(s.put(&d_b, b, N));
-    for (double** q : {&d_r, &d_z, &d_y, &d_p0, &d_p1}) TRY(s.alloc(q, N));
+    for (double** q : {&d_r, &d_z, &d_y, &d_p0, &d_rdiag}) TRY(s.alloc(q, N));
     const long nc = ((long)N + kChunk - 1) / kChunk;
     TRY(s.alloc(&d_part, 6 * (size_t)nc));
     TRY(s.alloc(&d_bar, 1));
@@ -1131,6 +1131,7 @@ int cfd_bicg_mode(const double* spMtx, const int* spIdx, const int* spRowptr,
     a.col = d_col;
     a.val = d_val;
     a.diag = d_diag;
+    a.rdiag = d_rdiag;
     a.isfix = d_isfix;
     a.nfix = (int)unode.size();
     a.fix_node = d_un;
@@ -1142,7 +1143,6 @@ int cfd_bicg_mode(const double* spMtx, const int* spIdx, const int* spRowptr,
     a.z[0] = a.z[1] = d_z;
     a.y[0] = a.y[1] = d_y;
     a.p[0][0] = a.p[1][0] = d_p0;
-    a.p[0][1] = a.p[1][1] = d_p1;
     a.part = d_part;
     a.bar = d_bar;
     a.tol = tol;
@@ -1152,16 +1152,7 @@ int cfd_bicg_mode(const double* spMtx, const int* spIdx, const int* spRowptr,
     a.rz_out = d_rz;
     a.relres_out = d_rz + 2;
     a.conv_out = d_cv;
-    int dev = 0, nsm = 0, per_sm = 0;
-    CFD_CUDA(cudaGetDevice(&dev));
-    CFD_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    CFD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_fp64, 256, 0));
-    long g = (long)nsm * (per_sm > 0 ? per_sm : 1);
-    if (g > nc) g = nc;
-    if (g < 1) g = 1;
-    void* args[] = {&a};
-    CFD_CUDA(cudaLaunchCooperativeKernel((void*)k_pcg_fp64, dim3((unsigned)g), dim3(256), args, 0, s.stream));
-    g_launches.fetch_add(1, std::memory_order_relaxed);
+    CFD_CUDA(launch_pcg_fp64(s.stream, a));
     int it = 0, cv = 0;
     double rz[4] = {0.0, 0.0, 0.0, 0.0};
     GridBar gb{};

@@ -62,13 +62,17 @@ __device__ __forceinline__ double div3(double x) {
 // x - d*q1 is exact in one FMA and RN(q1 + (x - d*q1)*y) is the correctly rounded x/d
 // (Markstein's theorem: y within half an ulp of 1/d, q1 within an ulp of x/d).  The range
 // check (both exponents and the quotient's) keeps every intermediate normal and finite;
-// other operands (zeros included) take the division.  Bit-identical to x / d (checked on the GPU against the division).
+// other operands take the division.  A zero x (a residual the solve has not reached, a
+// gradient of a uniform flow) with d in range is x*y, the signed zero of x / d.
+// Bit-identical to x / d (checked on the GPU against the division).
 __device__ __forceinline__ double div_rcp(double x, double d, double y) {
     const int ex = (int)((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ff;
     const int ed = (int)((unsigned long long)__double_as_longlong(d) >> 52) & 0x7ff;
     // both exponents in [200, 1800] and the quotient's within 2^+-800
-    if ((unsigned)(ex - 200) > 1600u || (unsigned)(ed - 200) > 1600u || abs(ex - ed) > 800)
+    if ((unsigned)(ex - 200) > 1600u || (unsigned)(ed - 200) > 1600u || abs(ex - ed) > 800) {
+        if (x == 0.0 && (unsigned)(ed - 200) <= 1600u) return x * y;
         return x / d;
+    }
     const double q0 = x * y;
     const double q1 = fma(fma(-d, q0, x), y, q0);
     return fma(fma(-d, q1, x), y, q1);

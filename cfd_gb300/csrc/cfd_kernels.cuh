@@ -370,7 +370,8 @@ struct PcgArgs {
     int* conv_out;               // [2]
 };
 
-__global__ void k_pcg_fp64(PcgArgs a);
+// the FP64 solve on the current device (a.bar zeroed on the stream before)
+cudaError_t launch_pcg_fp64(cudaStream_t st, PcgArgs a);
 __global__ void k_pcg_mixed(PcgArgs a);
 __global__ void k_selftest_waits(GridBar* gb, int* out, long long limit);
 __global__ void k_bicg_fix_mixed(PcgArgs a);

@@ -287,10 +287,14 @@ int Ctx::run_pcg(int nsolve, bool learned, bool fix_done, cudaStream_t sv) {
     }
     CFD_CUDA(cudaMemsetAsync(d_bar, 0, sizeof(GridBar), stream));
     if (mixed && prm.bicg_tol_mode == CFD_BICG_TOL_REL) a.iterated = d_iterated;
-    void* args[] = {&a};
-    CFD_CUDA(cudaLaunchCooperativeKernel(mixed ? (void*)k_pcg_mixed : (void*)k_pcg_fp64, dim3(pcg_grid),
-                                         dim3(256), args, 0, stream));
-    g_launches.fetch_add(1, std::memory_order_relaxed);
+    if (!mixed) {
+        CFD_CUDA(launch_pcg_fp64(stream, a));
+    } else {
+        void* args[] = {&a};
+        CFD_CUDA(cudaLaunchCooperativeKernel((void*)k_pcg_mixed, dim3(pcg_grid), dim3(256), args, 0,
+                                             stream));
+        g_launches.fetch_add(1, std::memory_order_relaxed);
+    }
     if (mixed && prm.bicg_tol_mode == CFD_BICG_TOL_REL) {
         // refinement: the FP32 iterations meet the test on their recursive residual; the
         // precise residual of the solution (against the FP64-assembled matrix) is formed
@@ -864,12 +868,11 @@ int Ctx::create(const cfd_mesh* m, const cfd_params* p, int precision_mode) {
     std::memcpy(h_scal, &sc0, sizeof(sc0));
     CFD_CUDA(cudaMemcpyAsync(d_scal, h_scal, sizeof(StepScal), cudaMemcpyHostToDevice, stream));
     CFD_CUDA(cudaStreamSynchronize(stream));
-    // persistent BiCG grid: co-resident blocks only
+    // persistent mixed BiCG grid: co-resident blocks only
     int dev = 0, per_sm = 0;
     CFD_CUDA(cudaGetDevice(&dev));
     CFD_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    CFD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, prec == CFD_PREC_MIXED ? k_pcg_mixed : k_pcg_fp64, 256, 0));
+    CFD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_mixed, 256, 0));
     long g = (long)nsm * (per_sm > 0 ? per_sm : 1);
     if (g > nc) g = nc;
     pcg_grid = (int)(g > 0 ? g : 1);

@@ -14,293 +14,599 @@
 // Every block folds the chunk partials itself in the fixed order of cfd_common.cuh, so
 // all blocks hold bit-identical scalars and take the same branch.  With --fmad=false the
 // iterates equal the CPU restatement's bit for bit.
+//
+// A block of 1024 threads takes a 1024-row chunk of the dots' order, one row per thread.
+// ON_CHIP (no more chunks than SMs: up to 155,648 rows on 152 SMs): the row's x, r, p and y or
+// z stay in the thread's registers for the whole solve and the matrix rows in shared memory
+// (the first kEll entries; longer rows read the rest from global memory), so an iteration
+// moves p alone through L2; the chunk's rows are dealt to the warps by length, so that a warp
+// runs as many column steps as its rows have entries.  Otherwise a block walks over its
+// chunks with the vectors in global memory, read by the thread that wrote them (p excepted).
+// What bounds an iteration: the FP64 pipe (31 operations per row at 2 per clock and SM) and
+// three barriers with two folds, which one warp per sum does alone: the chunk's products and
+// the partials go from memory straight into the fixed tree, and the scalars' divisions are
+// made once per block.  With 256-thread blocks (four rows per thread, vectors and matrix
+// re-read, every thread dividing the scalars) an iteration took 34.1 us at 147,456 rows,
+// 49.7 at 262,144 and 173 at 1,048,576; now 21.2, 42.5 and 132 us.
 #include "cfd_kernels.cuh"
 
 namespace cfd {
 
-__device__ __forceinline__ double spmv_row(const PcgArgs& a, int i, const double* v) {
-    double dot = 0.0;
-    const int j1 = a.rowptr[i + 1];
-    for (int j = a.rowptr[i]; j < j1; ++j) dot = dot + a.val[j] * v[a.col[j]];
-    return dot;
-}
+constexpr int kEll = 10;              // matrix entries per row kept in shared memory
+constexpr int kPad = kChunk + 32;     // a chunk's products, one pad per 32
+constexpr int kSortLen = 32;          // row-length classes of the deal
+constexpr int kGroup = 4;             // chunks a block takes between two barriers of its own
 
-// Row i of A.v and, in the same column order, the sum over the Dirichlet columns only
-// (the product with x_D, the vector that is v on the Dirichlet rows and 0 elsewhere; a
-// skipped term adds +0, which leaves a sum that starts at +0 unchanged)
-__device__ __forceinline__ double spmv_row_fixcols(const PcgArgs& a, int i, const double* v,
-                                                   double& dfix) {
-    double dot = 0.0, df = 0.0;
-    const int j1 = a.rowptr[i + 1];
-    for (int j = a.rowptr[i]; j < j1; ++j) {
-        const int c = a.col[j];
-        const double t = a.val[j] * v[c];
-        dot = dot + t;
-        if (a.isfix[c]) df = df + t;
+__device__ __forceinline__ int pad32(int i) { return i + (i >> 5); }
+
+// ------------------------------------------------------------------ barrier of one launch
+// gb->arrive counts arrivals from zero (the caller clears it before the launch); a waiter
+// leaves when the count has reached `target` (compared modulo 2^32).  One hop: the last
+// arrival itself releases the waiters.  false: the bounds ran out (gb->err is set).
+__device__ __forceinline__ bool bar_arrive_wait(GridBar* gb, unsigned target) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&gb->arrive) : "memory");
+    unsigned long long t0 = 0;
+    for (long long spins = 0;; ++spins) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&gb->arrive) : "memory");
+        if ((int)(v - target) >= 0) return true;
+        if ((spins & 63) == 63) {
+            const unsigned long long now = globaltimer_ns();
+            if (t0 == 0) t0 = now;
+            if (now - t0 > kWaitNs || spins > kSpinLimit) {
+                atomicExch(&gb->err, (int)CFD_ERR_BARRIER);
+                return false;
+            }
+        }
     }
-    dfix = df;
-    return dot;
 }
 
-__device__ __forceinline__ bool bar_failed(GridBar* gb) {
-    return *((volatile int*)&gb->err) != 0;
+// The 256-lane tree of cfd_common.cuh by one warp, lane 4 w + l taking the eight values of
+// warp w that meet in its (l, l+4) pair: v(t) gives lane t's value.  Sum in lane 0.
+template <class V>
+__device__ __forceinline__ double warp_tree256(V v) {
+    const int lane = threadIdx.x & 31, t = 32 * (lane >> 2) + (lane & 3);
+    const double a0 = v(t), a16 = v(t + 16), a8 = v(t + 8), a24 = v(t + 24), a4 = v(t + 4),
+                 a20 = v(t + 20), a12 = v(t + 12), a28 = v(t + 28);
+    double c = ((a0 + a16) + (a8 + a24)) + ((a4 + a20) + (a12 + a28));
+    c = c + __shfl_down_sync(0xffffffffu, c, 2);
+    c = c + __shfl_down_sync(0xffffffffu, c, 1);
+    c = c + __shfl_down_sync(0xffffffffu, c, 16);
+    c = c + __shfl_down_sync(0xffffffffu, c, 8);
+    c = c + __shfl_down_sync(0xffffffffu, c, 4);
+    return c;
 }
 
-__global__ void __launch_bounds__(256, 3) k_pcg_fp64(PcgArgs a) {
-    __shared__ double red[9];
-    __shared__ double s_thr[2], s_ref2[2];  // relative modes: threshold on r.r, ref.ref
-    const int t = threadIdx.x;
-    const int n = a.n;
-    const int ns = a.nsolve;
+// A chunk's cnt products in shared memory (pad32) -> their sum in the dots' order, by one
+// warp.  A whole chunk takes the branch-free form, whose 32 loads and eight chains of adds
+// overlap.  One copy for all passes (noinline): an iteration runs each pass once, so inlined
+// copies would be fetched anew.
+__device__ __noinline__ double chunk_sum(const double* q, int cnt) {
+    if (cnt == kChunk)
+        return warp_tree256([&](int t) {
+            return ((q[pad32(t)] + q[pad32(t + 256)]) + q[pad32(t + 512)]) + q[pad32(t + 768)];
+        });
+    return warp_tree256([&](int t) {
+        double acc = t < cnt ? q[pad32(t)] : 0.0;
+#pragma unroll
+        for (int k = 1; k < 4; ++k)
+            if (t + 256 * k < cnt) acc = acc + q[pad32(t + 256 * k)];
+        return acc;
+    });
+}
+
+// The nc chunk partials -> their fold (fold_partials's order), by one warp; the loads are
+// clamped, not branched over, so that a lane's eight go out together
+__device__ __noinline__ double chunk_fold(const double* part, long nc) {
+    const int lane = threadIdx.x & 31, t = 32 * (lane >> 2) + (lane & 3);
+    double acc[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        const long c = t + 4 * u;
+        acc[u] = __ldcg(part + min(c, nc - 1));
+        if (c >= nc) acc[u] = 0.0;
+    }
+    for (long base = 256; base < nc; base += 512) {
+        double v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            v[u] = __ldcg(part + min(base + t + 4 * (u & 7) + 256 * (u >> 3), nc - 1));
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            if (base + t + 4 * (u & 7) + 256 * (u >> 3) < nc) acc[u & 7] = acc[u & 7] + v[u];
+    }
+    return warp_tree256([&](int x) { return acc[(x - t) >> 2]; });
+}
+
+// Row i of A times the vectors of the ns solves, the row read from global memory in batches
+// (a batch's columns and values, then its gathers, go out together); sums in column order.
+// FIXC: also the sums over the Dirichlet columns only, the product with x_D, the vector that
+// is v on the Dirichlet rows and 0 elsewhere (a skipped term adds +0, which leaves a sum
+// that starts at +0 unchanged).
+template <bool FIXC>
+__device__ __forceinline__ void row_products(const PcgArgs& a, int j0, int j1, const double* v0,
+                                             const double* v1, double (&dot)[2],
+                                             double (&dfix)[2]) {
+    constexpr int B = 4;
+    double d0 = 0.0, d1 = 0.0, f0 = 0.0, f1 = 0.0;
+    for (int jb = j0; jb < j1; jb += B) {
+        int c[B];
+        double m[B], x0[B], x1[B];
+        bool fx[B];
+#pragma unroll
+        for (int u = 0; u < B; ++u)
+            if (jb + u < j1) {
+                c[u] = a.col[jb + u];
+                m[u] = a.val[jb + u];
+            }
+#pragma unroll
+        for (int u = 0; u < B; ++u)
+            if (jb + u < j1) {
+                if (v0) x0[u] = v0[c[u]];
+                if (v1) x1[u] = v1[c[u]];
+                if (FIXC) fx[u] = a.isfix[c[u]] != 0;
+            }
+#pragma unroll
+        for (int u = 0; u < B; ++u)
+            if (jb + u < j1) {
+                if (v0) {
+                    const double t = m[u] * x0[u];
+                    d0 = d0 + t;
+                    if (FIXC && fx[u]) f0 = f0 + t;
+                }
+                if (v1) {
+                    const double t = m[u] * x1[u];
+                    d1 = d1 + t;
+                    if (FIXC && fx[u]) f1 = f1 + t;
+                }
+            }
+    }
+    dot[0] = d0;
+    dot[1] = d1;
+    dfix[0] = f0;
+    dfix[1] = f1;
+}
+
+// Which partials a pass's sums go to: slot j in byte j, 2 * buffer + solve
+__device__ __forceinline__ int slot_at(unsigned code, int j) { return (int)(code >> (8 * j)) & 0xff; }
+
+// What the block's threads share; prod[g][j]: the products of the group's chunk g, sum j
+template <int G>
+struct PcgShared {
+    double prod[G][4][kPad];
+    double alfa[2], beta[2], err_new[2], err_old[2], rold[2], rr[2], thr[2], ref2[2];
+    int act[2], pend[2], done[2], last[2], fail;
+    int hist[kSortLen];
+    unsigned short perm[kChunk];
+};
+
+template <bool ON_CHIP>
+__global__ void __launch_bounds__(kChunk, 1) k_pcg_fp64(PcgArgs a) {
+    extern __shared__ __align__(16) unsigned char pcg_smem[];
+    constexpr int G = ON_CHIP ? 1 : kGroup;
+    typedef PcgShared<G> Shared;
+    Shared& s = *reinterpret_cast<Shared*>(pcg_smem);
+    double* ellv = reinterpret_cast<double*>(pcg_smem + sizeof(Shared));  // [kEll][kChunk]
+    int* ellc = reinterpret_cast<int*>(ellv + kEll * kChunk);
+    const int t = threadIdx.x, wp = t >> 5, lane = t & 31;
+    const int n = a.n, ns = a.nsolve;
     const long nc = ((long)n + kChunk - 1) / kChunk;
     const unsigned nb = gridDim.x;
-    auto part = [&](int buf, int s) { return a.part + ((long)buf * 2 + s) * nc; };
-    const bool rel = a.tol_mode != CFD_BICG_TOL_ABS;      // r.r per iteration
-    const bool relb = a.tol_mode == CFD_BICG_TOL_REL;     // ||b - A.x_D|| as reference
+    unsigned target = 0;
+    const bool rel = a.tol_mode != CFD_BICG_TOL_ABS;   // r.r per iteration
+    const bool relb = a.tol_mode == CFD_BICG_TOL_REL;  // ||b - A.x_D|| as reference
+    if (t == 0) s.fail = 0;
+
+    // every thread's global writes before, every thread's reads after
+    auto grid_sync = [&]() -> bool {
+        __syncthreads();
+        target += nb;
+        if (t == 0 && !bar_arrive_wait(a.bar, target)) s.fail = 1;
+        __syncthreads();
+        return s.fail == 0;
+    };
+    // the sums of the group of chunks c, c + nb, ... (slot j of chunk g = prod[g][j], into the
+    // partials code names), one warp per sum
+    auto chunk_sums = [&](long c, int m, unsigned code) {
+        __syncthreads();
+        const int g = wp >> 2, j = wp & 3;
+        const long cg = c + (long)g * nb;
+        if (g < G && j < m && cg < nc) {
+            const double v = chunk_sum(s.prod[g][j], (int)min((long)kChunk, n - cg * kChunk));
+            const int q = slot_at(code, j);
+            if (lane == 0) a.part[q * nc + cg] = v;
+        }
+        __syncthreads();  // several warps' partials precede one arrival; prod may be refilled
+    };
+    // the grid's folds of the same slots: warp j arrives for slot j, waits, folds, and hands
+    // the sum to `use` in lane 0; the other warps run `meanwhile`, warps 0..m-1 after their
+    // folds
+    auto fold_sums = [&](int m, unsigned code, auto use, auto meanwhile) -> bool {
+        target += nb * (unsigned)m;
+        if (wp < m) {
+            int ok = 1;
+            if (lane == 0) ok = bar_arrive_wait(a.bar, target) ? 1 : 0;
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (ok) {
+                const int q = slot_at(code, wp);
+                const double v = chunk_fold(a.part + q * nc, nc);
+                if (lane == 0) use(wp, q & 1, v);
+            } else if (lane == 0) {
+                s.fail = 1;
+            }
+        }
+        meanwhile();
+        __syncthreads();
+        return s.fail == 0;
+    };
+    auto nothing = [] {};
 
     // copy1 (biconjGrad.f90:28): x(fix) = x_fix
-    for (int k = blockIdx.x * blockDim.x + t; k < a.nfix; k += gridDim.x * blockDim.x)
-        for (int s = 0; s < ns; ++s) a.x[s][a.fix_node[k]] = 1.0 * a.fixval[s][a.fix_src[k]];
-    grid_barrier(a.bar, nb);
-    if (bar_failed(a.bar)) return;
+    for (int k = blockIdx.x * kChunk + t; k < a.nfix; k += gridDim.x * kChunk)
+        for (int q = 0; q < ns; ++q) a.x[q][a.fix_node[k]] = 1.0 * a.fixval[q][a.fix_src[k]];
+
+    // ON_CHIP: the thread's row (by length class within the chunk) and its matrix entries
+    long row = -1;   // the thread's row; -1: none
+    int slot = 0;    // its position in the chunk (the dots' order)
+    int len = 0, jx = 0;
+    bool fx = false;
+    double d = 1.0, rd = 1.0;
+    double xr[2] = {0.0, 0.0}, rr_[2] = {0.0, 0.0}, pr[2] = {0.0, 0.0}, yz[2] = {0.0, 0.0};
+    if (ON_CHIP) {
+        const long i = (long)blockIdx.x * kChunk + t;
+        int key = 0;
+        if (i < n && !a.isfix[i]) key = min(a.rowptr[i + 1] - a.rowptr[i], kSortLen - 1);
+        if (t < kSortLen) s.hist[t] = 0;
+        __syncthreads();
+        if (i < n) atomicAdd(&s.hist[key], 1);
+        __syncthreads();
+        if (wp == 0) {  // exclusive prefix of the 32 classes
+            const int v = s.hist[lane];
+            int x = v;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, off);
+                if (lane >= off) x += y;
+            }
+            s.hist[lane] = x - v;
+        }
+        __syncthreads();
+        if (i < n) s.perm[atomicAdd(&s.hist[key], 1)] = (unsigned short)t;
+        __syncthreads();
+        if (i < n) {  // as many threads as rows: thread t takes the t-th of the deal
+            slot = s.perm[t];
+            row = (long)blockIdx.x * kChunk + slot;
+            fx = a.isfix[row] != 0;
+            d = a.diag[row];
+            rd = 1.0 / d;
+            if (!fx) {
+                jx = a.rowptr[row];
+                len = a.rowptr[row + 1] - jx;
+#pragma unroll
+                for (int u = 0; u < kEll; ++u)
+                    if (u < len) {
+                        ellv[u * kChunk + t] = a.val[jx + u];
+                        ellc[u * kChunk + t] = a.col[jx + u];
+                    }
+            }
+        }
+    }
+    // ON_CHIP row product with v (global memory), in column order
+    auto chip_row = [&](const double* v) {
+        double dot = 0.0, g[kEll];
+#pragma unroll
+        for (int u = 0; u < kEll; ++u)
+            if (u < len) g[u] = v[ellc[u * kChunk + t]];
+#pragma unroll
+        for (int u = 0; u < kEll; ++u)
+            if (u < len) dot = dot + ellv[u * kChunk + t] * g[u];
+        for (int u = kEll; u < len; ++u) dot = dot + a.val[jx + u] * v[a.col[jx + u]];
+        return dot;
+    };
+    if (a.nfix > 0 && !grid_sync()) return;
 
     // y = A.x; y(fix) = 1e30*x(fix); r = -1*y + b; r(fix) = 0; r.r   (:138-144)
     // CFD_BICG_TOL_REL also forms b - A.x_D (0 on the Dirichlet rows) and its square sum
-    for (long c = blockIdx.x; c < nc; c += gridDim.x) {
-        double acc[2] = {0.0, 0.0}, accb[2] = {0.0, 0.0};
-        for (int k = 0; k < 4; ++k) {
-            const long i = c * kChunk + t + 256L * k;
-            if (i >= n) break;
-            const bool fx = a.isfix[i];
-            for (int s = 0; s < ns; ++s) {
-                double dfix = 0.0;
-                double yi = fx ? 1.0e30 * a.x[s][i]
-                               : (relb ? spmv_row_fixcols(a, (int)i, a.x[s], dfix)
-                                       : spmv_row(a, (int)i, a.x[s]));
-                a.y[s][i] = yi;
-                const double bi = a.b[s] ? a.b[s][i] : 0.0;
-                double ri = -1.0 * yi + bi;
-                if (fx) ri = 0.0;
-                a.r[s][i] = ri;
-                acc[s] = (k == 0) ? ri * ri : acc[s] + ri * ri;
-                if (relb) {
-                    double ei = -1.0 * dfix + bi;
-                    if (fx) ei = 0.0;
-                    accb[s] = (k == 0) ? ei * ei : accb[s] + ei * ei;
-                }
-            }
+    // slots: r.r of the solves (buffer 0), then (relb) the reference norms (buffer 2)
+    const int m0 = (relb ? 2 : 1) * ns;
+    const unsigned code0 = ns > 1 ? 0x05040100u : 0x00000400u;
+    auto first_row = [&](long i, int sl, int g) {
+        const bool f = a.isfix[i] != 0;
+        double dot[2] = {0.0, 0.0}, df[2] = {0.0, 0.0};
+        if (!f) {
+            const int j0 = a.rowptr[i], j1 = a.rowptr[i + 1];
+            const double* v1 = ns > 1 ? a.x[1] : nullptr;
+            if (relb) row_products<true>(a, j0, j1, a.x[0], v1, dot, df);
+            else row_products<false>(a, j0, j1, a.x[0], v1, dot, df);
         }
-        for (int s = 0; s < ns; ++s) {
-            double v = block_tree256(acc[s], red);
-            if (t == 0) part(0, s)[c] = v;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (q >= ns) break;
+            const double xi = a.x[q][i];
+            const double yi = f ? 1.0e30 * xi : dot[q];
+            const double bi = a.b[q] ? a.b[q][i] : 0.0;
+            double ri = -1.0 * yi + bi;
+            if (f) ri = 0.0;
+            if (ON_CHIP) {
+                xr[q] = xi;
+                rr_[q] = ri;
+            } else {
+                a.r[q][i] = ri;
+            }
+            s.prod[g][q][pad32(sl)] = ri * ri;
             if (relb) {
-                v = block_tree256(accb[s], red);
-                if (t == 0) part(2, s)[c] = v;
+                double ei = -1.0 * df[q] + bi;
+                if (f) ei = 0.0;
+                s.prod[g][ns + q][pad32(sl)] = ei * ei;
             }
         }
-    }
-    grid_barrier(a.bar, nb);
-    if (bar_failed(a.bar)) return;
-    bool done[2] = {true, true};
-    double err_old[2] = {0.0, 0.0}, alfa[2] = {0.0, 0.0};
-    // relative modes: r.r of the current residual (rrc), and in shared memory the squared
-    // reference norm and the threshold r.r <= tol^2 * ref.ref
-    double rrc[2] = {0.0, 0.0};
-    for (int s = 0; s < ns; ++s) {
-        double rr = fold_partials(part(0, s), nc, red);
-        if (rel) {
-            const double ref2 = relb ? fold_partials(part(2, s), nc, red) : rr;
-            if (t == 0) {
-                s_ref2[s] = ref2;
-                s_thr[s] = (a.tol * a.tol) * ref2;
-            }
-            __syncthreads();
-            rrc[s] = rr;
-            done[s] = rr <= s_thr[s];
+    };
+    // for (chunk groups) { rows; sums }: row(i, position in the chunk, chunk of the group)
+    auto rows_and_sums = [&](int m, unsigned code, auto on_row) {
+        if (ON_CHIP) {
+            if (row >= 0) on_row(row, slot, 0);
+            chunk_sums(blockIdx.x, m, code);
         } else {
-            done[s] = rr < a.tol;
+            for (long c = blockIdx.x; c < nc; c += (long)G * nb) {
+#pragma unroll 2
+                for (int g = 0; g < G; ++g) {
+                    const long i = (c + (long)g * nb) * kChunk + t;
+                    if (i < n) on_row(i, t, g);
+                }
+                chunk_sums(c, m, code);
+            }
         }
-        if (done[s] && blockIdx.x == 0 && t == 0) {
-            a.iters_out[s] = 0;
-            a.rz_out[s] = rr;
-            a.conv_out[s] = 1;
+    };
+    rows_and_sums(m0, code0, first_row);
+    if (!fold_sums(m0, code0,
+                   [&](int j, int q, double v) {
+                       if (j < ns) s.rr[q] = v;
+                       else s.ref2[q] = v;
+                   },
+                   nothing))
+        return;
+    if (t < ns) {
+        const double rr = s.rr[t];
+        bool done;
+        if (rel) {
+            const double ref2 = relb ? s.ref2[t] : rr;
+            s.ref2[t] = ref2;
+            s.thr[t] = (a.tol * a.tol) * ref2;
+            done = rr <= s.thr[t];
+        } else {
+            done = rr < a.tol;
+        }
+        s.done[t] = done;
+        s.pend[t] = !done;
+        s.last[t] = 0;
+        if (done && blockIdx.x == 0) {
+            a.iters_out[t] = 0;
+            a.rz_out[t] = rr;
+            a.conv_out[t] = 1;
             if (a.relres_out)
-                a.relres_out[s] = (rel && s_ref2[s] > 0.0) ? sqrt(rr / s_ref2[s]) : 0.0;
+                a.relres_out[t] = (rel && s.ref2[t] > 0.0) ? sqrt(rr / s.ref2[t]) : 0.0;
         }
     }
-    if (done[0] && (ns < 2 || done[1])) return;
+    __syncthreads();
+    bool done[2];
+    done[0] = s.done[0] != 0;
+    done[1] = ns < 2 || s.done[1] != 0;
+    if (done[0] && done[1]) return;
+
+    // the slots of the active solves' sums in buffer ba, then (two) in buffer bb
+    auto slots = [&](bool on0, bool on1, bool two, unsigned ba, unsigned bb, unsigned& code) {
+        const unsigned one = on0 ? (on1 ? 0x0100u + 0x0202u * ba : 2u * ba) : 2u * ba + 1u;
+        const int m = (on0 ? 1 : 0) + (on1 ? 1 : 0);
+        code = one;
+        if (!two) return m;
+        const unsigned sec = on0 ? (on1 ? 0x0100u + 0x0202u * bb : 2u * bb) : 2u * bb + 1u;
+        code |= sec << (8 * m);
+        return 2 * m;
+    };
+    unsigned code = 0;
 
     // p = r/diag; err_new = r.p   (:146-147)
-    for (long c = blockIdx.x; c < nc; c += gridDim.x) {
-        double acc[2] = {0.0, 0.0};
-        for (int k = 0; k < 4; ++k) {
-            const long i = c * kChunk + t + 256L * k;
-            if (i >= n) break;
-            const double d = a.diag[i];
-            if (a.rdiag) a.rdiag[i] = 1.0 / d;
-            for (int s = 0; s < ns; ++s) {
-                if (done[s]) continue;
-                double ri = a.r[s][i];
-                double pi = ri / d;
-                a.p[s][0][i] = pi;
-                acc[s] = (k == 0) ? ri * pi : acc[s] + ri * pi;
+    {
+        const int m = slots(!done[0], !done[1], false, 1, 0, code);
+        rows_and_sums(m, code, [&](long i, int sl, int g) {
+            double di = d, rdi = rd;
+            if (!ON_CHIP) {
+                di = a.diag[i];
+                rdi = 1.0 / di;
+                a.rdiag[i] = rdi;
             }
-        }
-        for (int s = 0; s < ns; ++s) {
-            if (done[s]) continue;
-            double v = block_tree256(acc[s], red);
-            if (t == 0) part(1, s)[c] = v;
-        }
-    }
-    grid_barrier(a.bar, nb);
-    if (bar_failed(a.bar)) return;
-    double err_new[2] = {0.0, 0.0};
-    for (int s = 0; s < ns; ++s)
-        if (!done[s]) err_new[s] = fold_partials(part(1, s), nc, red);
-
-    // y = A.p; y(fix) = 1e30*p(fix); py = p.y   (:148-151)
-    for (long c = blockIdx.x; c < nc; c += gridDim.x) {
-        double acc[2] = {0.0, 0.0};
-        for (int k = 0; k < 4; ++k) {
-            const long i = c * kChunk + t + 256L * k;
-            if (i >= n) break;
-            const bool fx = a.isfix[i];
-            for (int s = 0; s < ns; ++s) {
-                if (done[s]) continue;
-                const double* p = a.p[s][0];
-                double yi = fx ? 1.0e30 * p[i] : spmv_row(a, (int)i, p);
-                a.y[s][i] = yi;
-                acc[s] = (k == 0) ? p[i] * yi : acc[s] + p[i] * yi;
+            int j = 0;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                if (done[q]) continue;
+                const double ri = ON_CHIP ? rr_[q] : a.r[q][i];
+                const double pi = div_rcp(ri, di, rdi);
+                a.p[q][0][i] = pi;
+                if (ON_CHIP) pr[q] = pi;
+                s.prod[g][j++][pad32(sl)] = ri * pi;
             }
-        }
-        for (int s = 0; s < ns; ++s) {
-            if (done[s]) continue;
-            double v = block_tree256(acc[s], red);
-            if (t == 0) part(0, s)[c] = v;
-        }
-    }
-    grid_barrier(a.bar, nb);
-    if (bar_failed(a.bar)) return;
-    bool pend[2] = {false, false};
-    int cur[2] = {0, 0};
-    for (int s = 0; s < ns; ++s) {
-        if (done[s]) continue;
-        double py = fold_partials(part(0, s), nc, red);
-        alfa[s] = err_new[s] / py;  // :152
-        err_old[s] = err_new[s];
-        pend[s] = true;  // x = alfa*p + x (:153), applied in the next pass
+        });
+        // p of every block is in place too: the arrivals follow the block's writes of p
+        // (__syncthreads in chunk_sums, the release at the arrival)
+        if (!fold_sums(m, code, [&](int, int q, double v) { s.err_new[q] = v; }, nothing)) return;
     }
 
+    // y = A.p; y(fix) = 1e30*p(fix); py = p.y; alfa = err_new/py   (:148-152), for the solves
+    // with on[q]; x = alfa*p + x (:153) is applied in the next phase 1
     int k = 0;
-    int last_iter[2] = {0, 0};
+    auto product = [&](bool on0, bool on1) -> bool {
+        const int m = slots(on0, on1, false, 0, 0, code);
+        rows_and_sums(m, code, [&](long i, int sl, int g) {
+            int j = 0;
+            if (ON_CHIP) {
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    if (!(q ? on1 : on0)) continue;
+                    const double yi = fx ? 1.0e30 * pr[q] : chip_row(a.p[q][0]);
+                    yz[q] = yi;
+                    s.prod[0][j++][pad32(sl)] = pr[q] * yi;
+                }
+            } else {
+                const bool f = a.isfix[i] != 0;
+                double dot[2] = {0.0, 0.0}, df[2];
+                if (!f)
+                    row_products<false>(a, a.rowptr[i], a.rowptr[i + 1],
+                                        on0 ? a.p[0][0] : nullptr, on1 ? a.p[1][0] : nullptr, dot,
+                                        df);
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    if (!(q ? on1 : on0)) continue;
+                    const double pi = a.p[q][0][i];
+                    const double yi = f ? 1.0e30 * pi : dot[q];
+                    a.y[q][i] = yi;
+                    s.prod[g][j++][pad32(sl)] = pi * yi;
+                }
+            }
+        });
+        return fold_sums(m, code,
+                         [&](int, int q, double py) {
+                             const double e = s.err_new[q];
+                             s.alfa[q] = e / py;
+                             s.err_old[q] = e;
+                             s.pend[q] = 1;
+                             s.last[q] = k;
+                             s.act[q] =
+                                 (rel ? s.rr[q] > s.thr[q] : fabs(e) > a.tol) && k < a.maxit;
+                         },
+                         nothing);
+    };
+    if (!product(!done[0], !done[1])) return;
+
     while (true) {  // :156-170
-        bool act[2] = {false, false};
-        for (int s = 0; s < ns; ++s)
-            act[s] = !done[s] && (rel ? rrc[s] > s_thr[s] : fabs(err_old[s]) > a.tol) &&
-                     k < a.maxit;
+        const bool act[2] = {!done[0] && s.act[0] != 0, !done[1] && s.act[1] != 0};
         if (!act[0] && !act[1]) break;
         k = k + 1;
-        // phase 1
-        for (long c = blockIdx.x; c < nc; c += gridDim.x) {
-            double acc[2] = {0.0, 0.0}, accr[2] = {0.0, 0.0};
-            for (int kk = 0; kk < 4; ++kk) {
-                const long i = c * kChunk + t + 256L * kk;
-                if (i >= n) break;
-                const double d = a.diag[i];
-                const double rd = a.rdiag ? a.rdiag[i] : 0.0;
-                for (int s = 0; s < ns; ++s) {
-                    if (pend[s]) a.x[s][i] = alfa[s] * a.p[s][cur[s]][i] + a.x[s][i];
-                    if (!act[s]) continue;
-                    double ri = (-alfa[s]) * a.y[s][i] + a.r[s][i];
-                    double zi = a.rdiag ? div_rcp(ri, d, rd) : ri / d;
-                    a.r[s][i] = ri;
-                    a.z[s][i] = zi;
-                    acc[s] = (kk == 0) ? ri * zi : acc[s] + ri * zi;
-                    if (rel) accr[s] = (kk == 0) ? ri * ri : accr[s] + ri * ri;
+        // phase 1; 1/err_old for beta's quotient is formed beside it by an idle thread
+        {
+            const bool pend[2] = {!done[0] && s.pend[0] != 0, !done[1] && s.pend[1] != 0};
+            const double alfa[2] = {s.alfa[0], s.alfa[1]};
+            const int m = slots(act[0], act[1], rel, 1, 2, code);
+            const int na = (act[0] ? 1 : 0) + (act[1] ? 1 : 0);
+            if (t >= kChunk - 2) s.rold[t - (kChunk - 2)] = 1.0 / s.err_old[t - (kChunk - 2)];
+            rows_and_sums(m, code, [&](long i, int sl, int g) {
+                double di = d, rdi = rd;
+                if (!ON_CHIP) {
+                    di = a.diag[i];
+                    rdi = a.rdiag[i];
                 }
-            }
-            for (int s = 0; s < ns; ++s) {
-                if (!act[s]) continue;
-                double v = block_tree256(acc[s], red);
-                if (t == 0) part(1, s)[c] = v;
-                if (rel) {
-                    v = block_tree256(accr[s], red);
-                    if (t == 0) part(2, s)[c] = v;
+                int j = 0;
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    if (!ON_CHIP && pend[q]) a.x[q][i] = alfa[q] * a.p[q][0][i] + a.x[q][i];
+                    if (!act[q]) continue;
+                    const double ri = (-alfa[q]) * (ON_CHIP ? yz[q] : a.y[q][i]) +
+                                      (ON_CHIP ? rr_[q] : a.r[q][i]);
+                    const double zi = div_rcp(ri, di, rdi);
+                    if (ON_CHIP) {
+                        rr_[q] = ri;
+                        yz[q] = zi;
+                    } else {
+                        a.r[q][i] = ri;
+                        a.z[q][i] = zi;
+                    }
+                    s.prod[g][j][pad32(sl)] = ri * zi;
+                    if (rel) s.prod[g][na + j][pad32(sl)] = ri * ri;
+                    ++j;
                 }
+            });
+            if (!fold_sums(m, code,
+                           [&](int j, int q, double v) {
+                               if (j >= na) {
+                                   s.rr[q] = v;
+                                   return;
+                               }
+                               s.err_new[q] = v;
+                               s.beta[q] = div_rcp(v, s.err_old[q], s.rold[q]);
+                           },
+                           [&] {  // the deferred x update, under the barrier
+                               if (ON_CHIP && row >= 0)
+#pragma unroll
+                                   for (int q = 0; q < 2; ++q)
+                                       if (pend[q]) xr[q] = alfa[q] * pr[q] + xr[q];
+                           }))
+                return;
+            if (t < 2) {  // read again by the next phase 1 or the end, behind barriers
+                s.pend[t] = 0;
+                if (!(t ? act[1] : act[0])) s.act[t] = 0;
             }
-        }
-        for (int s = 0; s < ns; ++s) pend[s] = false;
-        grid_barrier(a.bar, nb);
-        if (bar_failed(a.bar)) return;
-        double beta[2] = {0.0, 0.0};
-        for (int s = 0; s < ns; ++s) {
-            if (!act[s]) continue;
-            err_new[s] = fold_partials(part(1, s), nc, red);
-            if (rel) rrc[s] = fold_partials(part(2, s), nc, red);
-            beta[s] = err_new[s] / err_old[s];
         }
         // phase 2a: p_new = beta p + z, once per row (the SpMV below reads it; forming it
         // inside every row's column loop would cost two FP64 operations per entry)
-        for (long c = blockIdx.x; c < nc; c += gridDim.x)
-            for (int kk = 0; kk < 4; ++kk) {
-                const long i = c * kChunk + t + 256L * kk;
-                if (i >= n) break;
-                for (int s = 0; s < ns; ++s)
-                    if (act[s]) a.p[s][cur[s] ^ 1][i] = beta[s] * a.p[s][cur[s]][i] + a.z[s][i];
-            }
-        grid_barrier(a.bar, nb);
-        if (bar_failed(a.bar)) return;
-        // phase 2b: y = A p_new, y(fix) = 1e30 p_new(fix), partial p.y
-        for (long c = blockIdx.x; c < nc; c += gridDim.x) {
-            double acc[2] = {0.0, 0.0};
-            for (int kk = 0; kk < 4; ++kk) {
-                const long i = c * kChunk + t + 256L * kk;
-                if (i >= n) break;
-                const bool fx = a.isfix[i];
-                for (int s = 0; s < ns; ++s) {
-                    if (!act[s]) continue;
-                    const double* pn_v = a.p[s][cur[s] ^ 1];
-                    const double pn = pn_v[i];
-                    double yi = fx ? 1.0e30 * pn : spmv_row(a, (int)i, pn_v);
-                    a.y[s][i] = yi;
-                    acc[s] = (kk == 0) ? pn * yi : acc[s] + pn * yi;
+        {
+            const double beta[2] = {s.beta[0], s.beta[1]};
+            if (ON_CHIP) {
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    if (act[q] && row >= 0) {
+                        pr[q] = beta[q] * pr[q] + yz[q];
+                        a.p[q][0][row] = pr[q];
+                    }
+            } else {
+                for (long c = blockIdx.x; c < nc; c += gridDim.x) {
+                    const long i = c * kChunk + t;
+                    if (i < n)
+#pragma unroll
+                        for (int q = 0; q < 2; ++q)
+                            if (act[q]) a.p[q][0][i] = beta[q] * a.p[q][0][i] + a.z[q][i];
                 }
             }
-            for (int s = 0; s < ns; ++s) {
-                if (!act[s]) continue;
-                double v = block_tree256(acc[s], red);
-                if (t == 0) part(0, s)[c] = v;
-            }
         }
-        grid_barrier(a.bar, nb);
-        if (bar_failed(a.bar)) return;
-        for (int s = 0; s < ns; ++s) {
-            if (!act[s]) continue;
-            double py = fold_partials(part(0, s), nc, red);
-            alfa[s] = err_new[s] / py;
-            err_old[s] = err_new[s];
-            cur[s] ^= 1;
-            pend[s] = true;
-            last_iter[s] = k;
-        }
+        if (!grid_sync()) return;
+        // phase 2b: y = A p_new, y(fix) = 1e30 p_new(fix), p.y, alfa
+        if (!product(act[0], act[1])) return;
     }
     // the last deferred x update
-    for (long c = blockIdx.x; c < nc; c += gridDim.x)
-        for (int kk = 0; kk < 4; ++kk) {
-            const long i = c * kChunk + t + 256L * kk;
-            if (i >= n) break;
-            for (int s = 0; s < ns; ++s)
-                if (pend[s]) a.x[s][i] = alfa[s] * a.p[s][cur[s]][i] + a.x[s][i];
+    {
+        const bool pend[2] = {!done[0] && s.pend[0] != 0, !done[1] && s.pend[1] != 0};
+        const double alfa[2] = {s.alfa[0], s.alfa[1]};
+        if (ON_CHIP) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                if (row >= 0 && !done[q])
+                    a.x[q][row] = pend[q] ? alfa[q] * pr[q] + xr[q] : xr[q];
+        } else {
+            for (long c = blockIdx.x; c < nc; c += gridDim.x) {
+                const long i = c * kChunk + t;
+                if (i < n)
+#pragma unroll
+                    for (int q = 0; q < 2; ++q)
+                        if (pend[q]) a.x[q][i] = alfa[q] * a.p[q][0][i] + a.x[q][i];
+            }
         }
-    if (blockIdx.x == 0 && t == 0)
-        for (int s = 0; s < ns; ++s) {
-            if (done[s]) continue;
-            a.iters_out[s] = last_iter[s];
-            a.rz_out[s] = fabs(err_old[s]);
-            a.conv_out[s] = (rel ? rrc[s] > s_thr[s] : fabs(err_old[s]) > a.tol) ? 0 : 1;
-            if (a.relres_out)
-                a.relres_out[s] = (rel && s_ref2[s] > 0.0) ? sqrt(rrc[s] / s_ref2[s]) : 0.0;
-        }
+    }
+    if (blockIdx.x == 0 && t < ns && !s.done[t]) {
+        a.iters_out[t] = s.last[t];
+        a.rz_out[t] = fabs(s.err_old[t]);
+        a.conv_out[t] = (rel ? s.rr[t] > s.thr[t] : fabs(s.err_old[t]) > a.tol) ? 0 : 1;
+        if (a.relres_out)
+            a.relres_out[t] = (rel && s.ref2[t] > 0.0) ? sqrt(s.rr[t] / s.ref2[t]) : 0.0;
+    }
+}
+
+// One solve on the current device (a.bar zeroed before, on the same stream): ON_CHIP when
+// the chunks fit the SMs one each
+cudaError_t launch_pcg_fp64(cudaStream_t st, PcgArgs a) {
+    int dev = 0, nsm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const long nc = ((long)a.n + kChunk - 1) / kChunk;
+    const bool chip = nc <= nsm;
+    if (!chip && !a.rdiag) return cudaErrorInvalidValue;
+    const int smem = chip ? (int)sizeof(PcgShared<1>) + kEll * kChunk * 12 : (int)sizeof(PcgShared<kGroup>);
+    const void* fn = chip ? (const void*)k_pcg_fp64<true> : (const void*)k_pcg_fp64<false>;
+    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
+        return e;
+    const unsigned grid = (unsigned)(chip ? nc : nsm);
+    void* args[] = {&a};
+    e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kChunk), args, (size_t)smem, st);
+    if (e == cudaSuccess) g_launches.fetch_add(1, std::memory_order_relaxed);
+    return e;
 }
 
 // Failure-detection self-test of the two bounded waits (one block): a grid barrier that

@@ -43,9 +43,8 @@ static_assert(sizeof(NoallocCtl) <= kCtlBytes, "control block");
 constexpr int kMaxDevices = 64;
 std::mutex g_mu;
 unsigned char* g_addr[kMaxDevices] = {};
-int g_grid[kMaxDevices] = {};
 
-int scratch_for_current_device(unsigned char** addr, int* grid) {
+int scratch_for_current_device(unsigned char** addr) {
     int dev = 0;
     CFD_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= kMaxDevices) {
@@ -56,14 +55,9 @@ int scratch_for_current_device(unsigned char** addr, int* grid) {
     if (!g_addr[dev]) {
         void* p = nullptr;
         CFD_CUDA(cudaGetSymbolAddress(&p, g_bicg_scratch));
-        int nsm = 0, per_sm = 0;
-        CFD_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        CFD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_fp64, 256, 0));
-        g_grid[dev] = nsm * (per_sm > 0 ? per_sm : 1);
         g_addr[dev] = (unsigned char*)p;
     }
     *addr = g_addr[dev];
-    *grid = g_grid[dev];
     return CFD_OK;
 }
 
@@ -85,14 +79,12 @@ extern "C" int cfd_bicg_device_noalloc(const double* spMtx, const int* col, cons
         return CFD_ERR_LIMIT;
     }
     unsigned char* base = nullptr;
-    int maxgrid = 1;
-    int st = scratch_for_current_device(&base, &maxgrid);
+    int st = scratch_for_current_device(&base);
     if (st) return st;
     cudaStream_t s = (cudaStream_t)stream;
     const long N = npoin;
     double* v = (double*)base;
     NoallocCtl* ctl = (NoallocCtl*)(base + kVecBytes + kPartBytes);
-    const long nc = (N + kChunk - 1) / kChunk;
     PcgArgs a{};
     a.n = npoin;
     a.nsolve = 1;
@@ -118,11 +110,7 @@ extern "C" int cfd_bicg_device_noalloc(const double* spMtx, const int* col, cons
     a.conv_out = ctl->conv;
     // the barrier starts at zero; every other word is written before it is read
     CFD_CUDA(cudaMemsetAsync(&ctl->bar, 0, sizeof(GridBar), s));
-    long g = maxgrid < nc ? maxgrid : nc;
-    if (g < 1) g = 1;
-    void* args[] = {&a};
-    CFD_CUDA(cudaLaunchCooperativeKernel((void*)k_pcg_fp64, dim3((unsigned)g), dim3(256), args, 0, s));
-    g_launches.fetch_add(1, std::memory_order_relaxed);
+    CFD_CUDA(launch_pcg_fp64(s, a));
     NoallocCtl h{};
     CFD_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, s));
     CFD_CUDA(cudaStreamSynchronize(s));

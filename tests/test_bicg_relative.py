@@ -312,3 +312,47 @@ def test_gpu_mesh_motion_matrix_assemblies(gpu_lib, oracle):
         moved = np.abs(gm.state()["Y"] - k.y).max()
         assert moved > 1e-4, moved
         gm.close()
+
+
+def _graph_matrix(n, seed):
+    """A symmetric diagonally dominant matrix in the solver's CSR (1-based, diagonal first):
+    neighbours at +-1 and +-37, and hub rows of 12 and 45 entries (beyond the row entries
+    the solver keeps on chip, and beyond its row-length classes)."""
+    rng = np.random.default_rng(seed)
+    i = np.arange(n)
+    pairs = [(i[:-d], i[d:]) for d in (1, 37) if n > d]
+    for every, width in ((211, 12), (1009, 45)):
+        for h in range(5, n - width - 40, every):
+            pairs.append((np.full(width, h), h + 38 + np.arange(width)))
+    lo = np.concatenate([p[0] for p in pairs]) if pairs else np.zeros(0, int)
+    hi = np.concatenate([p[1] for p in pairs]) if pairs else np.zeros(0, int)
+    key = np.unique(lo.astype(np.int64) * n + hi)
+    lo, hi = key // n, key % n
+    w = -rng.uniform(0.5, 1.5, len(lo))
+    row, col, val = np.concatenate([lo, hi]), np.concatenate([hi, lo]), np.concatenate([w, w])
+    diag = np.bincount(row, weights=-val, minlength=n) + rng.uniform(0.02, 0.1, n)
+    row, col, val = (np.concatenate(p) for p in ((i, row), (i, col), (diag, val)))
+    order = np.lexsort((col, col != row, row))  # the diagonal first in each row
+    rp = np.concatenate([[0], np.cumsum(np.bincount(row, minlength=n))])
+    return val[order], col[order] + 1, rp, diag
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 31, 1023, 1024, 1025, 4500, 155648, 155649, 312000])
+@pytest.mark.parametrize("mode", ["abs", "rel"])
+def test_gpu_solve_at_chunk_edges(gpu_lib, oracle, n, mode):
+    """The FP64 solve's two variants (rows on chip up to a chunk per SM, 155,648 rows on 152
+    SMs; vectors in global memory above) and the edges of its 1024-row chunks against the
+    oracle, bit for bit."""
+    from cfd_gb300 import abi, solver
+    vals, idx, rp, diag = _graph_matrix(n, n)
+    rng = np.random.default_rng(n + 1)
+    fix = (np.array([n // 2 + 1]) if n < 100 else 1 + np.arange(0, n, 500)).astype(np.int32)
+    data = rng.normal(size=len(fix))
+    x0 = 0.1 * rng.normal(size=n)
+    b = rng.normal(size=n)
+    tm = abi.CFD_BICG_TOL_ABS if mode == "abs" else abi.CFD_BICG_TOL_REL
+    xo, io = oracle.bicg(vals, idx, rp, diag, x0, b, data, fix, tol=1e-8, maxit=25, tol_mode=tm)
+    xg, ig = solver.biCG(vals, idx, rp, diag, x0, b, data, fix, tol=1e-8, maxit=25, tol_mode=tm)
+    assert (ig.iters, ig.converged, ig.rz, ig.relres) == (io.iters, io.converged, io.rz, io.relres)
+    assert np.array_equal(xg, xo)
