@@ -300,7 +300,7 @@ int cfd_ctx_upload_state(cfd_ctx* ctx, const double* U, const double* T, const d
                    mx ? c.d_VXf : nullptr, mx ? c.d_VYf : nullptr);
         if (T) {
             CFD_CUDA(cudaMemcpyAsync(c.d_T, T, 8 * N, cudaMemcpyHostToDevice, c.stream));
-            if (mx) TRY(c.narrow_mixed(false, true, false, false, false, false));
+            if (mx) TRY(c.narrow_mixed(false, true, false, false, false));
         }
         CFD_CUDA(cudaStreamSynchronize(c.stream));
         return CFD_OK;
@@ -313,7 +313,7 @@ int cfd_ctx_upload_state(cfd_ctx* ctx, const double* U, const double* T, const d
         CFD_LAUNCH(k_vel_from_U, blocks_for((long)N, 256), 256, 0, c.stream, (int)N, c.d_U,
                    VEL_X ? nullptr : c.d_VX, VEL_Y ? nullptr : c.d_VY);
     if (c.prec == CFD_PREC_MIXED)
-        TRY(c.narrow_mixed(U != nullptr, T != nullptr, VEL_X || U, VEL_Y || U, false, false));
+        TRY(c.narrow_mixed(U != nullptr, T != nullptr, VEL_X || U, VEL_Y || U, false));
     CFD_CUDA(cudaStreamSynchronize(c.stream));
     return CFD_OK;
 }
@@ -334,8 +334,8 @@ int cfd_ctx_upload_mesh(cfd_ctx* ctx, const double* X, const double* Y, const do
             if (k == 0 ? xpos != nullptr : ypos != nullptr)
                 CFD_LAUNCH(k_narrow, blocks_for(c.npoin, 256), 256, 0, c.stream, (long)c.npoin,
                            (const double*)c.d_pos[k], c.d_posf[k]);
-    if (c.prec == CFD_PREC_MIXED && (X || Y || W_X || W_Y))
-        TRY(c.narrow_mixed(false, false, false, false, X || Y, W_X || W_Y));
+    if (c.prec == CFD_PREC_MIXED && (W_X || W_Y))
+        TRY(c.narrow_mixed(false, false, false, false, true));
     if (X || Y) TRY(c.prec == CFD_PREC_MIXED ? c.geometry_mixed(true) : c.geometry(true, true));
     CFD_CUDA(cudaStreamSynchronize(c.stream));
     return c.tcollect();
@@ -359,12 +359,14 @@ int cfd_ctx_set_clock(cfd_ctx* ctx, int iter, double time, double dtmin1, int ba
     CFD_CUDA(cudaMemcpyAsync(c.d_scal, &sc, sizeof(sc), cudaMemcpyHostToDevice, c.stream));
     if (c.d_motion) {  // the structural model's velocities and accelerations are kept
         MotionScal ms{};
-        CFD_CUDA(cudaMemcpyAsync(&ms, c.d_motion, sizeof(ms), cudaMemcpyDeviceToHost, c.stream));
+        CFD_CUDA(cudaMemcpyAsync(&ms, c.d_motion + c.buf, sizeof(ms), cudaMemcpyDeviceToHost,
+                                 c.stream));
         CFD_CUDA(cudaStreamSynchronize(c.stream));
         ms.time = time;
         ms.disn0 = disn1;
         ms.disn1 = disn2;
-        CFD_CUDA(cudaMemcpyAsync(c.d_motion, &ms, sizeof(ms), cudaMemcpyHostToDevice, c.stream));
+        CFD_CUDA(cudaMemcpyAsync(c.d_motion + c.buf, &ms, sizeof(ms), cudaMemcpyHostToDevice,
+                                 c.stream));
     }
     CFD_CUDA(cudaStreamSynchronize(c.stream));
     return CFD_OK;
@@ -514,7 +516,9 @@ int cfd_ctx_download_geometry(cfd_ctx* ctx, double* area, double* dNx, double* d
     Ctx& c = ctx->impl;
     const size_t E = c.nelem;
     if ((dNx || dNy || area) && c.prec == CFD_PREC_MIXED) TRY(c.widen_mixed(4));
-    if (area) CFD_CUDA(cudaMemcpyAsync(area, c.d_area, 8 * E, cudaMemcpyDeviceToHost, c.stream));
+    if (area)
+        CFD_CUDA(cudaMemcpyAsync(area, c.area_put ? c.d_area_old : c.d_area, 8 * E,
+                                 cudaMemcpyDeviceToHost, c.stream));
     if (M) CFD_CUDA(cudaMemcpyAsync(M, c.d_M, 8 * (size_t)c.npoin, cudaMemcpyDeviceToHost, c.stream));
     std::vector<double> g;
     if (dNx || dNy) {

@@ -156,45 +156,46 @@ __device__ __forceinline__ double warp_tree32(double v) {
     return v;  // lane 0
 }
 
-// 256-lane tree; every thread of the block gets the result.  `red` holds >= 9 doubles.
-// The tree: within each warp w of values v[32w .. 32w+31], the shuffle-down pairs
-// (l, l+16), (l, l+8), (l, l+4), (l, l+2), (l, l+1); across the eight warp sums (w, w+4),
-// (w, w+2), (w, w+1).  The same sums are formed by warp 0 alone: lane 4w+l (l < 4) adds the
-// eight values of warp w that meet in its (l, l+4) pair, in the tree's own pairing
-// ((v_l + v_l+16) + (v_l+8 + v_l+24)) + ((v_l+4 + v_l+20) + (v_l+12 + v_l+28)), then the
-// (l, l+2), (l, l+1) levels and the cross-warp levels by shuffles.  12 FP64 warp
-// instructions instead of 43 on GB300's narrow FP64 pipe, the same bits; the values sit in
-// shared memory with one pad per 32 (fewer bank conflicts on the strided reads).
-__device__ __forceinline__ double block_tree256(double v, double* red) {
-    __shared__ double tree_v[256 + 8];
-    const int t = threadIdx.x;
-    tree_v[t + (t >> 5)] = v;
-    __syncthreads();
-    if (t < 32) {
-        const int w = t >> 2, l = t & 3;
-        const double* q = tree_v + 33 * w + l;
-        const double b0 = (q[0] + q[16]) + (q[8] + q[24]);
-        const double b1 = (q[4] + q[20]) + (q[12] + q[28]);
-        double c = b0 + b1;
-        c = c + __shfl_down_sync(0xffffffffu, c, 2);   // (l, l+2)
-        c = c + __shfl_down_sync(0xffffffffu, c, 1);   // (l, l+1): warp w's sum in lane 4w
-        c = c + __shfl_down_sync(0xffffffffu, c, 16);  // (w, w+4)
-        c = c + __shfl_down_sync(0xffffffffu, c, 8);   // (w, w+2)
-        c = c + __shfl_down_sync(0xffffffffu, c, 4);   // (w, w+1)
-        if (t == 0) red[8] = c;
-    }
-    __syncthreads();
-    double r = red[8];
-    __syncthreads();
-    return r;
+// The 256-lane tree by one warp: v(t) gives lane t's value; the sum comes back in lane 0.
+// The tree: within each warp w of values v[32w .. 32w+31], the shuffle-down pairs (l, l+16),
+// (l, l+8), (l, l+4), (l, l+2), (l, l+1); across the eight warp sums (w, w+4), (w, w+2),
+// (w, w+1).  Lane 4w+l (l < 4) adds the eight values of warp w that meet in its (l, l+4) pair,
+// in the tree's own pairing, then the (l, l+2), (l, l+1) levels and the cross-warp levels go
+// by shuffles: 12 FP64 warp instructions instead of the 43 of eight warps on GB300's narrow
+// FP64 pipe, the same bits.
+template <class V>
+__device__ __forceinline__ double warp_tree256(V v) {
+    const int lane = threadIdx.x & 31, t = 32 * (lane >> 2) + (lane & 3);
+    const double a0 = v(t), a16 = v(t + 16), a8 = v(t + 8), a24 = v(t + 24), a4 = v(t + 4),
+                 a20 = v(t + 20), a12 = v(t + 12), a28 = v(t + 28);
+    double c = ((a0 + a16) + (a8 + a24)) + ((a4 + a20) + (a12 + a28));
+    c = c + __shfl_down_sync(0xffffffffu, c, 2);   // (l, l+2)
+    c = c + __shfl_down_sync(0xffffffffu, c, 1);   // (l, l+1): warp w's sum in lane 4w
+    c = c + __shfl_down_sync(0xffffffffu, c, 16);  // (w, w+4)
+    c = c + __shfl_down_sync(0xffffffffu, c, 8);   // (w, w+2)
+    c = c + __shfl_down_sync(0xffffffffu, c, 4);   // (w, w+1)
+    return c;
 }
 
-// Final fold of nc chunk partials (blockDim.x == 256); every thread gets the sum.
-__device__ __forceinline__ double fold_partials(const double* part, long nc, double* red) {
+// index of value i with one pad per 32 (fewer bank conflicts on the tree's strided reads)
+__device__ __forceinline__ int pad32(int i) { return i + (i >> 5); }
+constexpr int kTreePad = kRedThreads + kRedThreads / 32;
+
+// The trees of M sums of a 256-thread block at once, a warp per sum: an FP64 add waits 64
+// clocks here, so that M trees one after the other cost M times a tree's latency.  Every
+// thread reads the sums in out[0..M) afterwards.
+template <int M>
+__device__ __forceinline__ void block_trees(const double (&v)[M], double (*sh)[kTreePad],
+                                            double* out) {
     const int t = threadIdx.x;
-    double acc = (t < nc) ? part[t] : 0.0;
-    for (long c = t + 256; c < nc; c += 256) acc = acc + part[c];
-    return block_tree256(acc, red);
+#pragma unroll
+    for (int j = 0; j < M; ++j) sh[j][pad32(t)] = v[j];
+    __syncthreads();
+    for (int j = t >> 5; j < M; j += 8) {
+        const double r = warp_tree256([&](int i) { return sh[j][pad32(i)]; });
+        if ((t & 31) == 0) out[j] = r;
+    }
+    __syncthreads();
 }
 
 // ------------------------------------------------------------------ bounded waits

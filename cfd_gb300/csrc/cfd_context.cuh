@@ -23,7 +23,7 @@ void graph_free(cfd_mpnn_graph* g);
 int fields_seed(cfd_mpnn_graph* g, cudaStream_t st);
 int fields_guess(cfd_mpnn_graph* g, cudaStream_t st, const double* X, const double* Y,
                  const double* bgx, const double* bgy, const double* x0, const double* x1,
-                 double* c0, double* c1);
+                 double* c0, double* c1, float2* s0, float2* s1);
 int fields_update(cfd_mpnn_graph* g, cudaStream_t st, const double* x0, const double* x1);
 }  // namespace mpnn
 
@@ -32,8 +32,7 @@ __global__ void k_smooth_prep(int n, const double* xpos, const double* ypos, con
                               const double* Y, double* tol, double* xb, double* yb);
 __global__ void k_smooth_w(int n, const double* xpos, const double* ypos, const double* X,
                            const double* Y, const double* xb, const double* yb,
-                           const StepScal* sc, double* WX, double* WY, float2* Wf, float2* Xhi,
-                           float2* Xlo);
+                           const StepScal* sc, double* WX, double* WY, float2* Wf);
 void smoothing_colours(const Adjacency& adj, int npoin, std::vector<int>& order,
                        std::vector<int>& offs);
 int smooth_on_device(cudaStream_t st, int npoin, int nelem, const int4* elem,
@@ -111,12 +110,12 @@ struct Ctx {
     double *d_WX = nullptr, *d_WY = nullptr, *d_M = nullptr, *d_Wxo = nullptr, *d_Wyo = nullptr;
     double *d_area = nullptr, *d_area_old = nullptr, *d_geo = nullptr, *d_DT = nullptr,
            *d_DTL = nullptr;
+    bool area_put = false;  // mixed form: the current area is in d_area_old (putArea), not d_area
     double *d_SHOC = nullptr, *d_TS1 = nullptr, *d_TS2 = nullptr, *d_TS3 = nullptr;
     double *d_contrib = nullptr, *d_contribF = nullptr;
     double* d_einv = nullptr;  // FP64 form: calcRHS's stage-invariant addends (per element)
     // mixed precision: float shadows (FP64 arrays above are widened from them on download)
     float4 *d_Uhi = nullptr, *d_Ulo = nullptr;  // U = hi + lo
-    float2 *d_Xhi = nullptr, *d_Xlo = nullptr;  // (X, Y) = hi + lo
     float2 *d_Wf = nullptr, *d_Wof = nullptr;   // W and the gcl's previous W
     float* d_Tf = nullptr;                      // T
     float2* d_mulam = nullptr;                  // per element: mu, lambda of the RK stage
@@ -189,7 +188,7 @@ struct Ctx {
     int* d_slot_pos = nullptr;
     float4 *d_recInv = nullptr, *d_recVisc = nullptr;  // slot records, element-around-point order
     float4* d_invSum = nullptr;                         // per node: sum of the recInv slots
-    double2* d_gterms = nullptr;  // gcl element terms (FP64)
+    double* d_gterms = nullptr;  // gcl element terms (FP64)
     double estab_eps = 1.0e-3;  // CFD_ESTAB_REGULARIZED relative gradient scale
     double dir[2] = {1.0, 0.0};  // CFD_ESTAB_REGULARIZED freestream direction
     // mesh motion
@@ -219,11 +218,12 @@ struct Ctx {
                        cudaStream_t sv = nullptr);
     void swap_mixed_buffers();
     unsigned branch_grid(long n, int threads, cudaStream_t s) const;
+    unsigned row_grid(long nblk, cudaStream_t s) const;
     int branch_bpsm = 0;
     int node_bulk = 0;          // dynamic smem of the bulk-copy node pass (0: not used)
     int* d_node_err = nullptr;  // its bounded wait's error flag  // mesh-motion branch: blocks per SM of its grid-stride kernels
     void drop_graphs();
-    int narrow_mixed(bool U, bool T, bool VX, bool VY, bool XY, bool W);
+    int narrow_mixed(bool U, bool T, bool VX, bool VY, bool W);
     int widen_mixed(int what);
     int run_pcg(int nsolve, bool learned = false, bool fix_done = false,
                 cudaStream_t sv = nullptr);

@@ -120,6 +120,25 @@ __global__ void k_pack_report(const StepScal* sc, const MotionScal* ms, const in
                               const int* cv, const double* rz, const GridBar* bar,
                               const int* wait_err, StepOut* out);
 
+// CFD_GUESS_EXTRAPOLATED: hist = (dt1, dt2, solutions kept, c1, c2, two kept); the guess's
+// coefficients for a step of dtn, then the history moves on
+__device__ __forceinline__ void guess_history(double dtn, double* hist) {
+    const double dt1 = hist[0], dt2 = hist[1];
+    const bool two = hist[2] >= 2.0;
+    double c1 = 1.0, c2 = 0.0;
+    if (two) {
+        const double h = (dtn + dt1) / (dt1 + dt2);
+        c1 = dtn / dt1 * (1.0 + h);
+        c2 = -(dtn / dt2) * h;
+    }
+    hist[0] = dtn;
+    hist[1] = dt1;
+    hist[2] = hist[2] + 1.0;
+    hist[3] = c1;
+    hist[4] = c2;
+    hist[5] = two ? 1.0 : 0.0;
+}
+
 struct MotionTailArgs {
     int do_motion, do_forces;  // the parts this launch runs (Newmark: both)
     int nset;  // FORCES
@@ -129,7 +148,9 @@ struct MotionTailArgs {
     const double *X, *Y, *xref, *yref;
     int law;  // motion law
     double heave_amp, pitch_amp, freq;
-    MotionScal* m;
+    const MotionScal* m;  // the motion at the step's start ...
+    MotionScal* m_out;    // ... and after it (the other of two buffers: no block waits to store)
+    double* hist;         // null, or the extrapolated guess's history (the motion part)
     int nnmove;  // TRANSF
     const int *fix_node, *fix_set;
     double *xfix_x, *xfix_y;
@@ -160,9 +181,8 @@ cudaError_t launch_force_visc(cudaStream_t st, int form, int nset, const int* se
 
 // ------------------------------------------------------------------ mixed precision
 __global__ void k_narrow_state(int npoin, const double* U, const double* T, const double* VX,
-                               const double* VY, const double* X, const double* Y,
-                               const double* WX, const double* WY, float4* Uhi, float4* Ulo,
-                               float* Tf, float* VXf, float* VYf, float2* Xhi, float2* Xlo,
+                               const double* VY, const double* WX, const double* WY,
+                               float4* Uhi, float4* Ulo, float* Tf, float* VXf, float* VYf,
                                float2* Wf);
 __global__ void k_upload_U(int npoin, const double* hU, double* U, double* VX, double* VY,
                            float4* Uhi, float4* Ulo, float* VXf, float* VYf);
@@ -207,7 +227,7 @@ int node_bulk_smem(const int* esup_ptr_host, int npoin);
 __global__ void k_elem_geometry(int nelem, const int4* elem, const double* X, const double* Y,
                                 int gcl, int literal, const float2* W, const float2* Wold,
                                 int put_area, double* area_old, double* area64, float* areaf,
-                                float4* geo, double2* terms, NormalsArgs nv);
+                                float4* geo, double* terms, NormalsArgs nv);
 constexpr int kGeoNodeBlock = 128;  // block size of k_node_geometry
 __global__ void k_elem_grad64(int nelem, const int4* elem, const double* X, const double* Y,
                               const int* slot_pos, float2* k64);
@@ -215,7 +235,7 @@ __global__ void k_elem_grad64(int nelem, const int4* elem, const double* X, cons
 // from k64 (element-matrix rows as double-float pairs, written as valf + val_lo), not from geo
 cudaError_t launch_node_geometry(bool row64, unsigned grid, cudaStream_t stream, int npoin,
                                  const int* esup_ptr, const int* esup_slot,
-                                 const uchar4* lap_pos, const float4* geo, const double2* terms,
+                                 const uchar4* lap_pos, const float4* geo, const double* terms,
                                  const double* dtp, int gcl, const int* rowptr, float* valf,
                                  double* invdiag, float* invdiagf, double* M, float* invM,
                                  const float2* W, float2* Wold, const float2* k64,
@@ -223,7 +243,7 @@ cudaError_t launch_node_geometry(bool row64, unsigned grid, cudaStream_t stream,
 __global__ void k_widen_geo(int nelem, const float4* geo, double* dN, double* area);
 __global__ void k_motion_update_mixed(int npoin, const double* xpos, const double* ypos,
                                       const StepScal* sc, double* X, double* Y, double* WX,
-                                      double* WY, float2* Xhi, float2* Xlo, float2* Wf);
+                                      double* WY, float2* Wf);
 
 #define ELEM_RHS_ARGS                                                                    \
     int, const int4* __restrict__, const double* __restrict__, const double* __restrict__, \
@@ -370,7 +390,7 @@ struct PcgArgs {
     int* conv_out;               // [2]
 };
 
-// the FP64 solve on the current device (a.bar zeroed on the stream before)
+// the FP64 solve on the current device (a.bar: zeros, and left so)
 cudaError_t launch_pcg_fp64(cudaStream_t st, PcgArgs a);
 __global__ void k_pcg_mixed(PcgArgs a);
 __global__ void k_selftest_waits(GridBar* gb, int* out, long long limit);
@@ -383,8 +403,8 @@ __global__ void k_split_x(PcgArgs a, const double* v0, const double* v1, const i
 __global__ void k_bicg_dir_mixed(PcgArgs a);
 // learned-guess judge: r.z of the candidate (cand[s]) per solve when gflag[0] is set
 __global__ void k_guess_judge(PcgArgs a, const double* cand0, const double* cand1, double* rr);
-__global__ void k_guess_extrapolate(PcgArgs a, const double* dtn_p, double* hist,
-                                    double* xprev0, double* xprev1);
+__global__ void k_guess_extrapolate(PcgArgs a, const double* hist, double* xprev0,
+                                    double* xprev1);
 __global__ void k_guess_extrapolate_hist(const double* dtn_p, double* hist);
 // per solve, the candidate replaces x (and its shadow) when its r.z is the smaller; sets
 // gflag[1]; stats[0..3) += (gate open, solve 0 took it, solve 1 took it)

@@ -128,12 +128,12 @@ int Ctx::geometry(bool masas, bool with_laplace) {
 
 // ------------------------------------------------------------------ PCG launch
 // CFD_GUESS_EXTRAPOLATED: x becomes the last two increments extrapolated to this step's
-// DTMIN (k_guess_extrapolate), then the history moves on
+// DTMIN (k_guess_extrapolate), from the history's coefficients (guess_history)
 int Ctx::guess_extrapolate(const PcgArgs& a, cudaStream_t s, unsigned grid) {
-    const double* dtn = &d_scal->dtmin;
-    CFD_LAUNCH(k_guess_extrapolate, std::min(grid, (unsigned)(4 * nsm)), 256, 0, s, a, dtn, d_xhist,
-               d_xprev[0], d_xprev[1]);
-    CFD_LAUNCH(k_guess_extrapolate_hist, 1, 32, 0, s, dtn, d_xhist);
+    if (prec != CFD_PREC_MIXED)  // the mixed form's k_motion_tail has moved the history on
+        CFD_LAUNCH(k_guess_extrapolate_hist, 1, 32, 0, s, (const double*)&d_scal->dtmin, d_xhist);
+    CFD_LAUNCH(k_guess_extrapolate, std::min(grid, (unsigned)(4 * nsm)), 256, 0, s, a,
+               (const double*)d_xhist, d_xprev[0], d_xprev[1]);
     return CFD_OK;
 }
 
@@ -199,9 +199,7 @@ int Ctx::run_pcg(int nsolve, bool learned, bool fix_done, cudaStream_t sv) {
         if (nufix > 0 && !fix_done)
             CFD_LAUNCH(k_bicg_fix_mixed, blocks_for(nufix, 256), 256, 0, stream, a);
         // beside the RK stages (sv: the branch stream) the row kernels take a smaller grid
-        const unsigned rgrid = (sv && branch_bpsm > 0)
-                                   ? (unsigned)std::min<long>(a.nblk_r, (long)branch_bpsm * nsm)
-                                   : (unsigned)a.nblk_r;
+        const unsigned rgrid = row_grid(a.nblk_r, sv);
         if (extrap_mode()) {
             int st = guess_extrapolate(a, stream, rgrid);
             if (st) return st;
@@ -215,14 +213,12 @@ int Ctx::run_pcg(int nsolve, bool learned, bool fix_done, cudaStream_t sv) {
         const unsigned gsz = std::min((unsigned)a.nblk_r, (unsigned)(4 * nsm));
         PcgArgs ac = a;  // the judge's arguments: the candidates' split
         for (int s = 0; s < 2; ++s) ac.xs[s] = d_xs_c[s];
+        // the candidates and, under the relative tests, their split (ungated: beside the first
+        // pass, which sets the gate, on the branch)
         auto cand_guess = [&](cudaStream_t cs) -> int {
-            int st = mpnn::fields_guess(lgraph, cs, d_X, d_Y, d_xfix[0], d_xfix[1], d_pos[0],
-                                        d_pos[1], d_cand[0], d_cand[1]);
-            if (st) return st;
-            if (split)  // ungated: beside the first pass, which sets the gate, on the branch
-                CFD_LAUNCH(k_split_x, gsz, 256, 0, cs, ac, (const double*)d_cand[0],
-                           (const double*)d_cand[1], (const int*)nullptr);
-            return CFD_OK;
+            return mpnn::fields_guess(lgraph, cs, d_X, d_Y, d_xfix[0], d_xfix[1], d_pos[0],
+                                      d_pos[1], d_cand[0], d_cand[1], split ? d_xs_c[0] : nullptr,
+                                      split ? d_xs_c[1] : nullptr);
         };
         if (side) {
             CFD_CUDA(cudaEventRecord(ev_side[0], stream));
@@ -231,7 +227,7 @@ int Ctx::run_pcg(int nsolve, bool learned, bool fix_done, cudaStream_t sv) {
             if (st) return st;
             CFD_CUDA(cudaEventRecord(ev_side[1], stream3));
         }
-        if (split)
+        if (split && !extrap_mode())  // the extrapolation writes its guess's split itself
             CFD_LAUNCH(k_split_x, rgrid, 256, 0, stream, a, (const double*)d_pos[0],
                        (const double*)d_pos[1], (const int*)nullptr);
         CFD_CUDA(launch_bicg_resid_mixed(rgrid, stream, a));
@@ -285,7 +281,6 @@ int Ctx::run_pcg(int nsolve, bool learned, bool fix_done, cudaStream_t sv) {
         int st = guess_extrapolate(a, stream, blocks_for(npoin, 256));
         if (st) return st;
     }
-    CFD_CUDA(cudaMemsetAsync(d_bar, 0, sizeof(GridBar), stream));
     if (mixed && prm.bicg_tol_mode == CFD_BICG_TOL_REL) a.iterated = d_iterated;
     if (!mixed) {
         CFD_CUDA(launch_pcg_fp64(stream, a));
@@ -304,14 +299,11 @@ int Ctx::run_pcg(int nsolve, bool learned, bool fix_done, cudaStream_t sv) {
         b.only_if = d_iterated;  // nothing to refine where no solve moved from its guess
         b.iterated = nullptr;
         b.accumulate = 1;
-        const unsigned rgrid = (sv && branch_bpsm > 0)
-                                   ? (unsigned)std::min<long>(b.nblk_r, (long)branch_bpsm * nsm)
-                                   : (unsigned)b.nblk_r;
+        const unsigned rgrid = row_grid(b.nblk_r, sv);
         CFD_LAUNCH(k_split_x, rgrid, 256, 0, stream, b, (const double*)d_pos[0],
                    (const double*)d_pos[1], b.only_if);
         CFD_CUDA(launch_bicg_resid_mixed(rgrid, stream, b));
         CFD_LAUNCH(k_bicg_dir_mixed, rgrid, 256, 0, stream, b);
-        CFD_CUDA(cudaMemsetAsync(d_bar, 0, sizeof(GridBar), stream));
         void* bargs[] = {&b};
         CFD_CUDA(cudaLaunchCooperativeKernel((void*)k_pcg_mixed, dim3(pcg_grid), dim3(256), bargs, 0,
                                              stream));
@@ -468,7 +460,6 @@ int Ctx::smooth(int* iters, double* min_quality, bool node_order) {
                           d_sm_flags, iters, min_quality, max_star, node_order);
     if (st) return st;
     if (prec == CFD_PREC_MIXED) {
-        if ((st = narrow_mixed(false, false, false, false, true, false))) return st;
         if ((st = geometry_mixed(true, true))) return st;
     } else {
         if ((st = geometry(true, true))) return st;
@@ -522,8 +513,7 @@ int Ctx::smooth_in_step(cudaStream_t s, double* WX, double* WY, float2* Wf) {
     const bool mixed = prec == CFD_PREC_MIXED;
     CFD_LAUNCH(k_smooth_w, g, 256, 0, s, N, d_pos[0], d_pos[1], d_X, d_Y, d_sm_xb, d_sm_yb,
                (const StepScal*)d_scal,
-               WX, WY, mixed ? Wf : (float2*)nullptr, mixed ? d_Xhi : (float2*)nullptr,
-               mixed ? d_Xlo : (float2*)nullptr);
+               WX, WY, mixed ? Wf : (float2*)nullptr);
     return CFD_OK;
 }
 
@@ -676,7 +666,7 @@ int Ctx::step(int nsteps, cfd_step_report* rep) {
     }
     // the report: one gather on the device, one copy into pinned memory
     CFD_LAUNCH(k_pack_report, 1, 32, 0, stream, (const StepScal*)d_scal,
-               (const MotionScal*)d_motion, (const int*)d_pcg_iters, (const int*)d_pcg_conv,
+               (const MotionScal*)(d_motion ? d_motion + buf : nullptr), (const int*)d_pcg_iters, (const int*)d_pcg_conv,
                (const double*)d_pcg_rz, (const GridBar*)d_bar, (const int*)d_node_err, d_out);
     CFD_CUDA(cudaMemcpyAsync(h_out, d_out, sizeof(StepOut), cudaMemcpyDeviceToHost, stream));
     CFD_CUDA(cudaStreamSynchronize(stream));
@@ -695,6 +685,8 @@ int Ctx::step(int nsteps, cfd_step_report* rep) {
         disn[1] = ms.disn1;
     }
     if (gb.err) {
+        // a barrier that gave up is left mid-count: the next solve starts from a fresh one
+        CFD_CUDA(cudaMemsetAsync(d_bar, 0, sizeof(GridBar), stream));
         set_last_message("a bounded device wait gave up (BiCG grid barrier or node-pass copy)");
         return CFD_ERR_BARRIER;
     }
@@ -847,12 +839,13 @@ int Ctx::create(const cfd_mesh* m, const cfd_params* p, int precision_mode) {
         }
     }
     if (extrap_mode()) {
-        if ((st = dalloc(&d_xhist, 3))) return st;
-        CFD_CUDA(cudaMemsetAsync(d_xhist, 0, 3 * sizeof(double), stream));
+        if ((st = dalloc(&d_xhist, 6))) return st;
+        CFD_CUDA(cudaMemsetAsync(d_xhist, 0, 6 * sizeof(double), stream));
     }
     const long nc = ((long)N + kChunk - 1) / kChunk;
     if ((st = dalloc(&d_part, 6 * (size_t)(nc > 0 ? nc : 1)))) return st;
     if ((st = dalloc(&d_bar, 1))) return st;
+    CFD_CUDA(cudaMemsetAsync(d_bar, 0, sizeof(GridBar), stream));
     if ((st = dalloc(&d_pcg_iters, 2))) return st;
     if ((st = dalloc(&d_pcg_conv, 2))) return st;
     if ((st = dalloc(&d_pcg_rz, 4))) return st;  // |r.z| and ||r||/||ref|| per solve
@@ -902,7 +895,7 @@ int Ctx::create(const cfd_mesh* m, const cfd_params* p, int precision_mode) {
         for (float** q : {&d_Tf, &d_VXf, &d_VYf, &d_RHOf, &d_Ef, &d_Pf, &d_RMACHf,
                           &d_invMf})
             if ((st = dalloc(q, N))) return st;
-        for (float2** q : {&d_Xhi, &d_Xlo, &d_Wf, &d_Wof})
+        for (float2** q : {&d_Wf, &d_Wof})
             if ((st = dalloc(q, N))) return st;
         for (float4** q : {&d_Uhi, &d_Ulo})
             if ((st = dalloc(q, N))) return st;
@@ -943,7 +936,7 @@ int Ctx::create(const cfd_mesh* m, const cfd_params* p, int precision_mode) {
         if ((st = dalloc(&d_recInv, 3 * (size_t)E))) return st;
         if ((st = dalloc(&d_recVisc, 3 * (size_t)E))) return st;
         if ((st = dalloc(&d_invSum, N))) return st;
-        if ((st = dalloc(&d_motion, 1))) return st;
+        if ((st = dalloc(&d_motion, 2))) return st;  // by the parity of the step
         if ((st = dalloc(&d_geo8_n, 2 * (size_t)E))) return st;
         if ((st = dalloc(&d_invMf_n, N))) return st;
         if ((st = dalloc(&d_WX_n, N))) return st;
@@ -964,14 +957,14 @@ int Ctx::create(const cfd_mesh* m, const cfd_params* p, int precision_mode) {
         }
         if ((st = dalloc(&d_tpart, 3 * 10 * kTailBlocks))) return st;
         CFD_CUDA(cudaMemsetAsync(d_tcount, 0, 4 * sizeof(unsigned), stream));
-        CFD_CUDA(cudaMemsetAsync(d_motion, 0, sizeof(MotionScal), stream));
+        CFD_CUDA(cudaMemsetAsync(d_motion, 0, 2 * sizeof(MotionScal), stream));
         graphs_on = !timers_on && !(getenv("CFD_GRAPHS") && atoi(getenv("CFD_GRAPHS")) == 0);
         // 5 blocks per SM measured best at 1M nodes with the current passes (the FP64 gcl
         // areas on the branch; 1000-step runs: 5: 0.557-0.559 ms, 6: 0.561-0.562; 600-step
         // runs, 4, 8, 12: 0.579, 0.568, 0.586); 0 = full grids
         branch_bpsm = getenv("CFD_BRANCH_BLOCKS_PER_SM") ? atoi(getenv("CFD_BRANCH_BLOCKS_PER_SM"))
                                                          : 5;
-        if ((st = narrow_mixed(true, true, true, true, true, true))) return st;
+        if ((st = narrow_mixed(true, true, true, true, true))) return st;
     }
     // setup geometry: NORMALES, DERIV, MASAS, laplace (ns2DComp.ALE.f90:88-100)
     st = (prec == CFD_PREC_MIXED) ? geometry_mixed(true, true) : geometry(true, true);
@@ -984,12 +977,11 @@ int Ctx::create(const cfd_mesh* m, const cfd_params* p, int precision_mode) {
 
 // ------------------------------------------------------------------ mixed precision
 // FP64 arrays -> float shadows, for the arrays the caller replaced (uploads, setup)
-int Ctx::narrow_mixed(bool U, bool T, bool VX, bool VY, bool XY, bool W) {
+int Ctx::narrow_mixed(bool U, bool T, bool VX, bool VY, bool W) {
     const int N = npoin;
     CFD_LAUNCH(k_narrow_state, blocks_for(N, 256), 256, 0, stream, N, U ? d_U : nullptr,
-               T ? d_T : nullptr, VX ? d_VX : nullptr, VY ? d_VY : nullptr, XY ? d_X : nullptr,
-               XY ? d_Y : nullptr, W ? d_WX : nullptr, W ? d_WY : nullptr, d_Uhi, d_Ulo, d_Tf,
-               d_VXf, d_VYf, d_Xhi, d_Xlo, d_Wf);
+               T ? d_T : nullptr, VX ? d_VX : nullptr, VY ? d_VY : nullptr, W ? d_WX : nullptr,
+               W ? d_WY : nullptr, d_Uhi, d_Ulo, d_Tf, d_VXf, d_VYf, d_Wf);
     return CFD_OK;
 }
 
@@ -1002,7 +994,7 @@ int Ctx::widen_mixed(int what) {
     const int nf = (what & 2) ? 7 : ((what & 1) ? 1 : 0);
     for (int i = 0; i < nf; ++i)
         CFD_LAUNCH(k_widen, blocks_for(N, 256), 256, 0, stream, N, src[i], dst[i]);
-    if (what & 4)  // d_area is the FP64 area the element pass keeps
+    if (what & 4)  // the FP64 area is kept by the element pass (area_put)
         CFD_LAUNCH(k_widen_geo, blocks_for(E, 256), 256, 0, stream, (int)E, (const float4*)d_geo8,
                    d_geo, (double*)nullptr);
     return CFD_OK;
@@ -1032,6 +1024,7 @@ int Ctx::geometry_mixed(bool setup, bool put_area, bool to_next, cudaStream_t sv
                0, stream, E, d_elem, d_X, d_Y, gcl ? 1 : 0,
                prm.mass_mode == CFD_MASS_GCL_LITERAL ? 1 : 0, Wn, Wo,
                (gcl || put_area) ? 1 : 0, d_area_old, d_area, d_areaf, geo8, d_gterms, nv);
+    area_put = gcl || put_area;
     tstop(TM_DERIV);
     tstart(TM_LAPLACE);
     if (d_val_lo)  // relative tests: the mesh-motion operator to FP64-class accuracy
@@ -1085,7 +1078,9 @@ int Ctx::enqueue_mixed(bool learned) {
     t.heave_amp = prm.heave_amp;
     t.pitch_amp = prm.pitch_amp;
     t.freq = prm.motion_freq;
-    t.m = d_motion;
+    t.m = d_motion + buf;
+    t.m_out = d_motion + (buf ^ 1);
+    t.hist = extrap_mode() ? d_xhist : nullptr;
     t.nnmove = nnmove;
     t.fix_node = d_fix_node;
     t.fix_set = d_fix_set;
@@ -1121,7 +1116,7 @@ int Ctx::enqueue_mixed(bool learned) {
         if (st) return st;
         tstop(TM_GRAD);
         CFD_LAUNCH(k_motion_update_mixed, branch_grid(N, TB, s), TB, 0, s, N, d_pos[0], d_pos[1],
-                   d_scal, d_X, d_Y, d_WX_n, d_WY_n, d_Xhi, d_Xlo, d_Wf_n);
+                   d_scal, d_X, d_Y, d_WX_n, d_WY_n, d_Wf_n);
         if (smoothing_now && (st = smooth_in_step(s, d_WX_n, d_WY_n, d_Wf_n))) return st;
         if (prm.moving == 1 && (st = geometry_mixed(false, false, true, s))) return st;
         if (side_join) {  // the fields' update on stream3 (it reads this step's solutions)
@@ -1208,12 +1203,27 @@ unsigned Ctx::branch_grid(long n, int threads, cudaStream_t s) const {
     return std::min<unsigned>(full, (unsigned)(branch_bpsm * nsm));
 }
 
+// Grid of the BiCG row kernels (256 threads) over nblk 256-row groups: beside the RK stages, 4
+// blocks per SM.  5, as the other branch kernels have, is more than stay resident with the
+// FP32 kernels' registers, so that every fifth block ran in a second wave of its own
+// (k_bicg_resid_mixed at 1M nodes alone: 49 us on 5, 35 on 4); whole steps on 3, 4, 6: 0.536,
+// 0.535, 0.534 ms at 1M nodes, 1.66, 1.61, 1.72 at 3.1M, 0.591, 0.566, 0.570 at 590k (host
+// coupled).  The relative tests' precise passes stay on branch_bpsm (6.03 against 5.93 ms per
+// 20 steps of 262,144 nodes): the grid is part of the order of their sums, and their long
+// solves amplify its last bit.
+unsigned Ctx::row_grid(long nblk, cudaStream_t s) const {
+    if (!s || branch_bpsm <= 0) return (unsigned)nblk;
+    const int per_sm = prm.bicg_tol_mode == CFD_BICG_TOL_ABS ? 4 : branch_bpsm;
+    return (unsigned)std::min<long>(nblk, (long)per_sm * nsm);
+}
+
 // The next-step buffers become the current ones (after each mixed step)
 void Ctx::swap_mixed_buffers() {
     std::swap(d_WX, d_WX_n);
     std::swap(d_WY, d_WY_n);
     std::swap(d_Wf, d_Wf_n);
     if (prm.moving == 1) {
+        area_put = prm.mass_mode != CFD_MASS_MASAS;  // also of a replayed step
         std::swap(d_geo8, d_geo8_n);
         std::swap(d_invMf, d_invMf_n);
     }

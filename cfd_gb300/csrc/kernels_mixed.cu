@@ -47,15 +47,13 @@ struct Acc {
 __device__ __forceinline__ void split(double v, float& hi, float& lo) { split_bits(v, hi, lo); }
 
 // ------------------------------------------------------------------ float shadows
-// U -> (Uhi, Ulo); T, VX, VY -> float; (X, Y) -> (Xhi, Xlo); W -> Wf.  Any input may be NULL.
+// U -> (Uhi, Ulo); T, VX, VY -> float; W -> Wf.  Any input may be NULL.
 __global__ void k_narrow_state(int npoin, const double* __restrict__ U, const double* __restrict__ T,
                                const double* __restrict__ VX, const double* __restrict__ VY,
-                               const double* __restrict__ X, const double* __restrict__ Y,
                                const double* __restrict__ WX, const double* __restrict__ WY,
                                float4* __restrict__ Uhi, float4* __restrict__ Ulo,
                                float* __restrict__ Tf, float* __restrict__ VXf,
-                               float* __restrict__ VYf, float2* __restrict__ Xhi,
-                               float2* __restrict__ Xlo, float2* __restrict__ Wf) {
+                               float* __restrict__ VYf, float2* __restrict__ Wf) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= npoin) return;
     if (U) {
@@ -67,13 +65,6 @@ __global__ void k_narrow_state(int npoin, const double* __restrict__ U, const do
     if (T) Tf[p] = (float)T[p];
     if (VX) VXf[p] = (float)VX[p];
     if (VY) VYf[p] = (float)VY[p];
-    if (X) {
-        float hx, lx, hy, ly;
-        split(X[p], hx, lx);
-        split(Y[p], hy, ly);
-        Xhi[p] = make_float2(hx, hy);
-        Xlo[p] = make_float2(lx, ly);
-    }
     if (WX) Wf[p] = make_float2((float)WX[p], (float)WY[p]);
 }
 
@@ -158,28 +149,36 @@ __device__ __forceinline__ void refine_one(int e, const int4* __restrict__ elem,
                                            const float* __restrict__ T, const float* __restrict__ VX,
                                            const float* __restrict__ VY, const float2* __restrict__ W,
                                            const float* __restrict__ areaf, float fsafe, float t_inf,
-                                           double m32, StepScal* __restrict__ sc) {
+                                           double m32, double tinf, double itinf,
+                                           unsigned long long& mine) {
     const int4 n = elem[e];
     const float d32 = dtelem_f32(n, T, VX, VY, W, areaf[e], fsafe, t_inf);
     if ((double)d32 > m32 * (1.0 + 1.0e-4)) return;
     const int nn[3] = {n.x, n.y, n.z};
     double vumax = 0.0, vvmax = 0.0;
-    const double T_iel = ((double)T[nn[0]] + (double)T[nn[1]] + (double)T[nn[2]]) / 3.0;
+    const double T_iel = div3((double)T[nn[0]] + (double)T[nn[1]] + (double)T[nn[2]]);
     for (int i = 0; i < 3; ++i) {
         const float2 w = W[nn[i]];
         const double vu = fabs((double)VX[nn[i]] - (double)w.x), vv = fabs((double)VY[nn[i]] - (double)w.y);
         if (vu > vumax) vumax = vu;
         if (vv > vvmax) vvmax = vv;
     }
-    const double tinf = (double)t_inf;
-    const double hh = sqrt(2.0 * (double)areaf[e]);
+    // the reference's expressions and quotients; those by tinf, hh and T + 110 take
+    // reciprocals formed beside the chain (div_rcp: the same bits), for a dependent FP64
+    // operation waits 64 clocks and a division several hundred
+    const double hh = sqrt(2.0 * (double)areaf[e]), ihh = 1.0 / hh;
+    const double t110 = T_iel + 110.0, it110 = 1.0 / t110;
     const double vel = sqrt(vumax * vumax + vvmax * vvmax);
-    const double et = 0.017 * (T_iel / tinf) * sqrt(T_iel / tinf) * (tinf + 110.0) / (T_iel + 110.0);
-    const double alpha = fmin((vel * hh) / (2.0 * et) / 3.0, 1.0);
-    const double deltatu = 1.0 / (4.0 * et / (hh * hh) + alpha * vel / hh);
+    const double r = div_rcp(T_iel, tinf, itinf);
+    const double et = div_rcp(0.017 * r * sqrt(r) * (tinf + 110.0), t110, it110);
+    const double alpha = fmin(div3((vel * hh) / (2.0 * et)), 1.0);
+    const double deltatu = 1.0 / (4.0 * et / (hh * hh) + div_rcp(alpha * vel, hh, ihh));
     const double deltatc = 1.0 / (4.0 * et / (hh * hh));
     const double d = (double)fsafe / (1.0 / deltatc + 1.0 / deltatu);
-    if (d > 0.0 && d < 1.0e20) atomicMin(&sc->dtmin_bits, (unsigned long long)__double_as_longlong(d));
+    if (d > 0.0 && d < 1.0e20) {
+        const unsigned long long b = (unsigned long long)__double_as_longlong(d);
+        mine = b < mine ? b : mine;
+    }
 }
 
 __global__ void k_deltat_refine(int nelem, const int4* __restrict__ elem, const float* __restrict__ T,
@@ -191,6 +190,9 @@ __global__ void k_deltat_refine(int nelem, const int4* __restrict__ elem, const 
     // thread t tests chunk blockIdx.x*256 + t; the block then refines the listed chunks
     __shared__ int list[256];
     __shared__ int nlist;
+    constexpr unsigned long long kNone = 0x7ff0000000000000ull;
+    unsigned long long mine = kNone;
+    const double tinf = (double)t_inf, itinf = 1.0 / tinf;
     const double m32 = __longlong_as_double((long long)sc->dtmin32_bits);
     const double band = m32 * (1.0 + 1.0e-4);
     if (threadIdx.x == 0) nlist = 0;
@@ -201,18 +203,36 @@ __global__ void k_deltat_refine(int nelem, const int4* __restrict__ elem, const 
     __syncthreads();
     for (int k = 0; k < nlist; ++k) {
         const int e = list[k] * 256 + threadIdx.x;
-        if (e < nelem) refine_one(e, elem, T, VX, VY, W, areaf, fsafe, t_inf, m32, sc);
+        if (e < nelem)
+            refine_one(e, elem, T, VX, VY, W, areaf, fsafe, t_inf, m32, tinf, itinf, mine);
     }
-    // the last block to finish forms DTMIN (k_dt_finalize of the FP64 form)
-    __shared__ bool last;
-    __threadfence();
+    // The last block to finish forms DTMIN (k_dt_finalize of the FP64 form).  One thread per
+    // block does the global part: the block's minimum, then the count in an acquire-release
+    // operation that orders it, instead of every element's atomic and two fences.
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const unsigned long long o = __shfl_down_sync(0xffffffffu, mine, off);
+        mine = o < mine ? o : mine;
+    }
+    __shared__ unsigned long long wmin[8];
+    if ((threadIdx.x & 31) == 0) wmin[threadIdx.x >> 5] = mine;
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(count, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (last && threadIdx.x == 0) {
-        __threadfence();
+    if (threadIdx.x != 0) return;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) mine = wmin[w] < mine ? wmin[w] : mine;
+    if (gridDim.x > 1) {
+        if (mine != kNone) atomicMin(&sc->dtmin_bits, mine);
+        unsigned before;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;"
+                     : "=r"(before)
+                     : "l"(count)
+                     : "memory");
+        if (before != gridDim.x - 1) return;
         *count = 0u;
-        dt_finalize_from(sc, atomicExch(&sc->dtmin_bits, 0x7ff0000000000000ull));
+        mine = atomicExch(&sc->dtmin_bits, kNone);
+    }
+    {
+        dt_finalize_from(sc, mine);
         sc->iter += 1;
         if (itlocal) {  // DTFACT of ns2DComp.ALE.f90:160 for this ITER; COTA = 10*DTMIN raw
             sc->dtfact_f = (float)(1.0 - exp(-(sc->iter * 4.6 / itlocal)));
@@ -602,6 +622,11 @@ __device__ __forceinline__ void node_finish(
         RHO[p] = rho; VX[p] = vx; VY[p] = vy; Eo[p] = ee; Po[p] = pp;
         RMACH[p] = sqrtf(fdiv(vel2, tt * g * gf.fr));
     }
+    // of stages 1-3 only T is read, and a fixed T is known without the update
+    if (!LAST && (fl & BC_FIXT)) {
+        Tout[p] = (float)bcval[4 * (size_t)p + 3];
+        return;
+    }
     const double2* u2 = reinterpret_cast<const double2*>(U + 4 * (size_t)p);
     const double2 ua = u2[0], ub = u2[1];
     double u1_0 = ua.x - f2d_bits(d0), u1_1 = ua.y - f2d_bits(d1), u1_2 = ub.x - f2d_bits(d2),
@@ -613,6 +638,10 @@ __device__ __forceinline__ void node_finish(
         const double vel2 = vx * vx + vy * vy;
         const double pp = rho * (gd - 1.0) * (ee - 0.5 * vel2);
         double tt = pp / (rho * FR);
+        if (!LAST) {
+            Tout[p] = (float)tt;
+            return;
+        }
         RMACH[p] = (float)sqrt(vel2 / (tt * gd * FR));
         Po[p] = (float)pp;
         const double2* b2 = reinterpret_cast<const double2*>(bcval + 4 * (size_t)p);
@@ -724,16 +753,18 @@ k_node_mixed(int npoin, const int* __restrict__ esup_ptr, const int* __restrict_
 // the edge vectors truncated to FP32.  The Laplacian weight of mLaplace.f90:28-56: with
 // |grad N_i|^2 = l_i^2/(2a)^2 the quality mu = 2*sqrt(3)*(2a)/sum(l_i^2) of
 // mLaplace.f90:96-108 is sqrt(3)/(a*sum|grad N_i|^2), so q = 1/mu^2 = (a*sum|grad N_i|^2)^2/3;
-// with gcl, the element terms of gcl main (gcl.f90:27-45) divW*area and divW_old*area_old
-// in FP64 (divW itself from the FP32 gradients and W; the node pass applies the 1/3), then
-// putArea.
+// with gcl, the element term of gcl main (gcl.f90:27-45), divW*area + divW_old*area_old, in
+// FP64 (divW itself from the FP32 gradients and W; the node pass sums it over the node's
+// elements and applies the 1/3; the two parts share every weight, so that they are added
+// here once per element and not per node), then putArea.  The FP64 area is written once: to
+// area_old with put_area, else to area64.
 __global__ void k_elem_geometry(int nelem, const int4* __restrict__ elem,
                                 const double* __restrict__ X, const double* __restrict__ Y,
                                 int gcl, int literal, const float2* __restrict__ W,
                                 const float2* __restrict__ Wold, int put_area,
                                 double* __restrict__ area_old, double* __restrict__ area64,
                                 float* __restrict__ areaf, float4* __restrict__ geo,
-                                double2* __restrict__ terms, NormalsArgs nv) {
+                                double* __restrict__ terms, NormalsArgs nv) {
     // the blocks after the elements' do normales (one wall node per thread)
     const int eblocks = (nelem + blockDim.x - 1) / blockDim.x;
     if (nv.nwn > 0 && (int)blockIdx.x >= eblocks) {
@@ -764,7 +795,6 @@ __global__ void k_elem_geometry(int nelem, const int4* __restrict__ elem,
     geo[2 * (size_t)e] = make_float4(gx[0], gx[1], gx[2], gy[0]);
     geo[2 * (size_t)e + 1] = make_float4(gy[1], gy[2], area, q);
     areaf[e] = area;
-    area64[e] = a64;
     if (gcl) {
         const int nn[3] = {n.x, n.y, n.z};
         float divW = 0.f, divWo = 0.f;
@@ -774,9 +804,10 @@ __global__ void k_elem_geometry(int nelem, const int4* __restrict__ elem,
             divW += gx[i] * w.x + gy[i] * (literal ? w.x : w.y);
             divWo += gx[i] * wo.x + gy[i] * (literal ? wo.x : wo.y);
         }
-        terms[e] = make_double2(f2d_bits(divW) * a64, f2d_bits(divWo) * area_old[e]);
+        terms[e] = f2d_bits(divW) * a64 + f2d_bits(divWo) * area_old[e];
     }
-    if (put_area) area_old[e] = a64;
+    if (put_area) area_old[e] = a64;  // putArea; then also the area a download reads
+    else area64[e] = a64;
     }
 }
 
@@ -843,7 +874,7 @@ template <bool ROW64>
 __global__ void __launch_bounds__(kGeoBlock)
 k_node_geometry(int npoin, const int* __restrict__ esup_ptr, const int* __restrict__ esup_slot,
                 const uchar4* __restrict__ lap_pos, const float4* __restrict__ geo,
-                const double2* __restrict__ terms, const double* __restrict__ dtp, int gcl,
+                const double* __restrict__ terms, const double* __restrict__ dtp, int gcl,
                 const int* __restrict__ rowptr, float* __restrict__ valf,
                 double* __restrict__ invdiag, float* __restrict__ invdiagf,
                 double* __restrict__ M, float* __restrict__ invM,
@@ -870,14 +901,14 @@ k_node_geometry(int npoin, const int* __restrict__ esup_ptr, const int* __restri
     }
     Acc m1;
     m1.init();
-    double t1 = 0.0, t2 = 0.0;  // gcl: tot1, tot2 (times 3)
+    double tot = 0.0;  // gcl: (tot1 + tot2) times 3
     // kGeoBatch slots per pass: their loads go out together, the sums stay in slot order
     const int s0 = esup_ptr[p], s1 = esup_ptr[p + 1];
     for (int sb = s0; sb < s1; sb += kGeoBatch) {
         int slot[kGeoBatch];
         uchar4 pos[kGeoBatch];
         float4 ga[kGeoBatch], gb[kGeoBatch];
-        double2 tm[kGeoBatch];
+        double tm[kGeoBatch];
         float2 kr[kGeoBatch][3];
 #pragma unroll
         for (int u = 0; u < kGeoBatch; ++u)
@@ -905,8 +936,7 @@ k_node_geometry(int npoin, const int* __restrict__ esup_ptr, const int* __restri
         for (int u = 0; u < kGeoBatch; ++u) {
             if (sb + u >= s1) break;
             if (gcl) {
-                t1 = t1 + tm[u].x;
-                t2 = t2 + tm[u].y;
+                tot = tot + tm[u];
             } else {
                 m1.add(gb[u].z);
             }
@@ -972,7 +1002,7 @@ k_node_geometry(int npoin, const int* __restrict__ esup_ptr, const int* __restri
     invdiag[p] = f2d_bits(idf);
     double m;
     if (gcl) {
-        m = M[p] + (*dtp) * ((t1 + t2) * (1.0 / 3.0)) * 0.5;
+        m = M[p] + (*dtp) * (tot * (1.0 / 6.0));
         if (Wold) Wold[p] = W[p];  // putW (null: the caller swaps W buffers instead)
     } else {
         m = f2d_bits(m1.value()) * (1.0 / 3.0);
@@ -983,7 +1013,7 @@ k_node_geometry(int npoin, const int* __restrict__ esup_ptr, const int* __restri
 }
 cudaError_t launch_node_geometry(bool row64, unsigned grid, cudaStream_t stream, int npoin,
                                  const int* esup_ptr, const int* esup_slot,
-                                 const uchar4* lap_pos, const float4* geo, const double2* terms,
+                                 const uchar4* lap_pos, const float4* geo, const double* terms,
                                  const double* dtp, int gcl, const int* rowptr, float* valf,
                                  double* invdiag, float* invdiagf, double* M, float* invM,
                                  const float2* W, float2* Wold, const float2* k64,
@@ -1069,12 +1099,11 @@ __global__ void k_widen_geo(int nelem, const float4* __restrict__ geo, double* _
 }
 
 // meshMove.f90:99-126: X += XPOS, W = XPOS/DTMIN (as XPOS*(1/DTMIN), the reciprocal formed
-// once by k_dt_finalize), with the float shadows of (X, Y) and W
+// once by k_dt_finalize), with the float shadow of W
 __global__ void k_motion_update_mixed(int npoin, const double* __restrict__ xpos,
                                       const double* __restrict__ ypos, const StepScal* __restrict__ sc,
                                       double* __restrict__ X, double* __restrict__ Y,
                                       double* __restrict__ WX, double* __restrict__ WY,
-                                      float2* __restrict__ Xhi, float2* __restrict__ Xlo,
                                       float2* __restrict__ Wf) {
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npoin; p += gridDim.x * blockDim.x) {
     const double idt = sc->inv_dtmin;
@@ -1086,11 +1115,6 @@ __global__ void k_motion_update_mixed(int npoin, const double* __restrict__ xpos
     WX[p] = wx;
     WY[p] = wy;
     Wf[p] = make_float2(d2f_trunc(wx), d2f_trunc(wy));
-    float hx, lx, hy, ly;
-    split(x, hx, lx);
-    split(y, hy, ly);
-    Xhi[p] = make_float2(hx, hy);
-    Xlo[p] = make_float2(lx, ly);
     }
 }
 
@@ -1118,13 +1142,12 @@ __device__ MotionScal motion_step(const MotionScal& m, double dt, int law, doubl
     } else {
         d1 = (PI / 8.0) * sin(10.0 * t);
     }
-    const double alpha = d1 - alphav;
     MotionScal o;
     o.time = t;
     o.disn0 = d0;
     o.disn1 = d1;
-    o.ca = cos(alpha);
-    o.sa = sin(alpha);
+    o.ca = d1 - alphav;  // the pitch increment: the caller forms its cosine and sine
+    o.sa = 0.0;
     o.yposr = d0 - yposrv;
     o.dtmin = dt;
     o.veln0 = m.veln0;
@@ -1134,9 +1157,10 @@ __device__ MotionScal motion_step(const MotionScal& m, double dt, int law, doubl
     return o;
 }
 
-// TRANSF into x_fix and the Dirichlet values of the solves, entries k0, k0 + ks, ...
+// TRANSF into x_fix, entries k0, k0 + ks, ..., and the Dirichlet values of the solves,
+// entries f0, f0 + ks, ...
 __device__ __forceinline__ void tail_transf(const MotionTailArgs& a, const MotionScal& mv,
-                                            int k0, int ks);
+                                            int k0, int f0, int ks);
 
 // TRANSF (meshMove.f90:369-392) of moving-list entry k
 __device__ __forceinline__ double2 transf_one(const MotionTailArgs& a, const MotionScal& mv,
@@ -1155,32 +1179,51 @@ __device__ __forceinline__ double2 transf_one(const MotionTailArgs& a, const Mot
 // motion law,
 // TRANSF into x_fix, and the Dirichlet values of the two BiCG solves (biconjGrad.f90:28:
 // x(fix) = x_fix, in x and in its float shadow).  Every block forms the motion from the
-// step-start MotionScal; the last block stores the new one.  The Newmark law runs both
-// parts in one launch: its motion needs the forces.
+// step-start MotionScal; one stores the new one in the other buffer.  The Newmark law runs
+// both parts in one launch: its motion needs the forces.  The launch is latency (a few
+// thousand items, FP64 chains of 64 clocks an operation), and it stands at both ends of a
+// step: the FORCES part 11-16 us of a step before its trees stood side by side and its kinds
+// of items had warps of their own, 8-12 us now.
 __global__ void __launch_bounds__(256) k_motion_tail(MotionTailArgs a) {
     __shared__ MotionScal mv;
-    __shared__ double red[9];
+    __shared__ double sh[3][kTreePad], sums[3];
     __shared__ bool last;
-    if (a.do_motion && threadIdx.x == 0)
+    const int t = threadIdx.x;
+    if (a.do_motion && t == 0)
         mv = motion_step(*a.m, a.sc->dtmin, a.law, a.heave_amp, a.pitch_amp, a.freq);
+    if (a.do_motion && a.hist && t == 96 && blockIdx.x == 0) guess_history(a.sc->dtmin, a.hist);
     __syncthreads();
-    // items interleaved over the blocks (item k in block k % gridDim.x): the FP64 work of a
-    // few thousand items spreads over as many SMs as there are blocks
-    const int gt = threadIdx.x * gridDim.x + blockIdx.x, gs = gridDim.x * blockDim.x;
     const bool structural = a.law == CFD_MOTION_NEWMARK;
-    if (a.do_motion && !structural) tail_transf(a, mv, gt, gs);
+    if (a.do_motion && !structural) {  // the two functions by two warps
+        const double alpha = mv.ca;
+        __syncthreads();
+        if (t == 0) mv.ca = cos(alpha);
+        if (t == 32) mv.sa = sin(alpha);
+        __syncthreads();
+    }
+    // items interleaved over the blocks (item k in block k % gridDim.x): the FP64 work of a
+    // few thousand items spreads over as many SMs as there are blocks, and each kind starts at
+    // a warp of its own (thread w0), so that the kinds' chains of dependent loads and FP64
+    // operations run side by side
+    const int gs = gridDim.x * blockDim.x;
+    auto first = [&](int w0) { return ((t - w0) & 255) * (int)gridDim.x + (int)blockIdx.x; };
+    if (a.do_motion && !structural) tail_transf(a, mv, first(0), first(64), gs);
     if (a.do_forces)  // normales of the moved mesh, for the next step's wall condition
-        for (int k = gt; k < a.nv.nwn; k += gs) normales_node(a.nv, k);
+        for (int k = first(128); k < a.nv.nwn; k += gs) normales_node(a.nv, k);
     if (a.do_motion && a.fgeo)  // the edge geometry FORCES will need, before the mesh moves
-        for (int k = gt; k < a.set_ptr[a.nset]; k += gs) {
+        for (int k = first(128); k < a.set_ptr[a.nset]; k += gs) {
             const int2 ed = a.set_edges[k];
             a.fgeo[k] = make_double4_32a(a.Y[ed.y] - a.Y[ed.x], a.X[ed.x] - a.X[ed.y],
                                      (a.X[ed.x] + a.X[ed.y]) * 0.5, (a.Y[ed.y] + a.Y[ed.x]) * 0.5);
         }
-    for (int s = 0; a.do_forces && s < a.nset; ++s) {
-        double fx = 0.0, fy = 0.0, rm = 0.0;
+    if (!a.do_forces) {  // no sums to fold: the blocks need not find their last one
+        if (blockIdx.x == 0 && t == 0) *a.m_out = mv;
+        return;
+    }
+    for (int s = 0; s < a.nset; ++s) {
+        double f[3] = {0.0, 0.0, 0.0};
         const double xr = a.xref[s], yr = a.yref[s];
-        for (int k = a.set_ptr[s] + gt; k < a.set_ptr[s + 1]; k += gs) {
+        for (int k = a.set_ptr[s] + first(0); k < a.set_ptr[s + 1]; k += gs) {
             const int2 ed = a.set_edges[k];
             const double d_press = ((double)a.P[ed.x] + (double)a.P[ed.y]) * 0.5;
             double4_32a g;  // Y(N2)-Y(N1), X(N1)-X(N2), the edge's midpoint
@@ -1192,34 +1235,29 @@ __global__ void __launch_bounds__(256) k_motion_tail(MotionTailArgs a) {
             }
             const double fa = d_press * g.x;
             const double fb = d_press * g.y;
-            fx += fa;
-            fy += fb;
-            rm += fb * (g.z - xr) - fa * (g.w - yr);
+            f[0] += fa;
+            f[1] += fb;
+            f[2] += fb * (g.z - xr) - fa * (g.w - yr);
         }
-        fx = block_tree256(fx, red);
-        fy = block_tree256(fy, red);
-        rm = block_tree256(rm, red);
-        if (threadIdx.x == 0) {
-            a.part[(3 * s + 0) * gridDim.x + blockIdx.x] = fx;
-            a.part[(3 * s + 1) * gridDim.x + blockIdx.x] = fy;
-            a.part[(3 * s + 2) * gridDim.x + blockIdx.x] = rm;
-        }
+        block_trees(f, sh, sums);
+        if (t < 3) a.part[(3 * s + t) * gridDim.x + blockIdx.x] = sums[t];
     }
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(a.count, 1u) == gridDim.x - 1;
+    if (t == 0) last = atomicAdd(a.count, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!last) return;
     __threadfence();
-    if (a.do_forces)  // the blocks' partials of each sum, folded by a tree in block order
-        for (int j = 0; j < 3 * a.nset; ++j) {
-            double v = (threadIdx.x < gridDim.x) ? __ldcg(a.part + j * gridDim.x + threadIdx.x) : 0.0;
-            v = block_tree256(v, red);
-            if (threadIdx.x == 0) {
-                const int s = j / 3, q = j % 3;
-                (q == 0 ? a.sc->fx : q == 1 ? a.sc->fy : a.sc->rm)[s] = v;
-            }
+    // the blocks' partials of each sum, folded by a tree in block order
+    for (int j = t >> 5; j < 3 * a.nset; j += 8) {
+        const double* pj = a.part + j * gridDim.x;
+        const double v =
+            warp_tree256([&](int i) { return i < (int)gridDim.x ? __ldcg(pj + i) : 0.0; });
+        if ((t & 31) == 0) {
+            const int s = j / 3, q = j % 3;
+            (q == 0 ? a.sc->fx : q == 1 ? a.sc->fy : a.sc->rm)[s] = v;
         }
+    }
     if (a.do_motion && structural) {  // the Newmark step under set 1's load, then TRANSF
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -1245,22 +1283,22 @@ __global__ void __launch_bounds__(256) k_motion_tail(MotionTailArgs a) {
             mv.accn1 = ns.acc[1];
         }
         __syncthreads();
-        tail_transf(a, mv, threadIdx.x, blockDim.x);
+        tail_transf(a, mv, t, t, blockDim.x);
     }
-    if (threadIdx.x == 0) {
-        if (a.do_motion) *a.m = mv;
+    if (t == 0) {
+        if (a.do_motion) *a.m_out = mv;
         *a.count = 0u;
     }
 }
 
 __device__ __forceinline__ void tail_transf(const MotionTailArgs& a, const MotionScal& mv,
-                                            int k0, int ks) {
+                                            int k0, int f0, int ks) {
     for (int k = k0; k < a.nnmove; k += ks) {
         const double2 d = transf_one(a, mv, k);
         a.xfix_x[k] = d.x;
         a.xfix_y[k] = d.y;
     }
-    for (int k = k0; k < a.nufix; k += ks) {
+    for (int k = f0; k < a.nufix; k += ks) {
         const int i = a.ufix_node[k];
         const double2 d = transf_one(a, mv, a.ufix_src[k]);
         a.x0[i] = d.x;

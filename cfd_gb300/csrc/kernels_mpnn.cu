@@ -17,84 +17,107 @@ static_assert((N_PARAMS + 1) % 4 == 0 && L_SIZE % 4 == 0 && LAYER0 % 4 == 0 && L
               "float4 accesses to the weights and to the rows of the partial gradients");
 
 // ------------------------------------------------------------------ globals and features
-__device__ __forceinline__ double block_max256(double v, double* red) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, off));
-    if (lane == 0) red[wid] = v;
-    __syncthreads();
-    if (wid == 0) {
-        double w = lane < 8 ? red[lane] : 0.0;
-#pragma unroll
-        for (int off = 4; off > 0; off >>= 1) w = fmax(w, __shfl_down_sync(0xffffffffu, w, off));
-        if (lane == 0) red[8] = w;
-    }
-    __syncthreads();
-    const double r = red[8];
-    __syncthreads();
-    return r;
-}
-
 // One block of 256 threads.  Boundary nodes are listed in bnode[0..nb) with their kind and
 // prescribed displacement (gx, gy).  Body geometry (c, L, R) and the least-squares affine
 // fit g = t + M d, d = p - c, over the body nodes: since sum d = 0, t = mean g and each row
-// of M solves [Sxx Sxy; Sxy Syy] m = [sum g d_x; sum g d_y].
+// of M solves [Sxx Sxy; Sxy Syy] m = [sum g d_x; sum g d_y].  A launch is latency: a
+// dependent FP64 add waits 64 clocks, so the sums of a pass are formed side by side
+// (block_trees) and a thread's nodes are loaded four at a time (34 us beside a 262,144-node step with one tree after the other, 21 us now).
 __global__ void k_globals(int nb, const int* __restrict__ bnode, const int* __restrict__ bkind,
                           const double* __restrict__ gx, const double* __restrict__ gy,
                           const double* __restrict__ X, const double* __restrict__ Y,
                           Globals* __restrict__ G, const int* __restrict__ gate) {
     if (gate && !*gate) return;
-    __shared__ double red[9];
+    __shared__ double sh[9][kTreePad], out[9];
+    __shared__ double rmax_s;
     const int t = threadIdx.x;
-    double nbody = 0, sx = 0, sy = 0, sgx = 0, sgy = 0, nout = 0;
-    for (int k = t; k < nb; k += 256) {
-        const int p = bnode[k];
-        if (bkind[k] == KIND_BODY) {
-            nbody += 1.0;
-            sx += X[p];
-            sy += Y[p];
-            sgx += gx[k];
-            sgy += gy[k];
-        } else {
-            nout += 1.0;
+    constexpr int B = 4;
+    double a[6] = {};  // body nodes, sum x, sum y, sum gx, sum gy, outer nodes
+    for (int k0 = t; k0 < nb; k0 += 256 * B) {
+        int kd[B], p[B];
+        double x[B], y[B], u[B], v[B];
+#pragma unroll
+        for (int q = 0; q < B; ++q) {
+            const int k = min(k0 + 256 * q, nb - 1);
+            p[q] = bnode[k];
+            kd[q] = bkind[k];
+            u[q] = gx[k];
+            v[q] = gy[k];
+        }
+#pragma unroll
+        for (int q = 0; q < B; ++q) {
+            x[q] = X[p[q]];
+            y[q] = Y[p[q]];
+        }
+#pragma unroll
+        for (int q = 0; q < B; ++q) {
+            if (k0 + 256 * q >= nb) break;
+            if (kd[q] == KIND_BODY) {
+                a[0] += 1.0;
+                a[1] += x[q];
+                a[2] += y[q];
+                a[3] += u[q];
+                a[4] += v[q];
+            } else {
+                a[5] += 1.0;
+            }
         }
     }
-    nbody = block_tree256(nbody, red);
-    sx = block_tree256(sx, red);
-    sy = block_tree256(sy, red);
-    sgx = block_tree256(sgx, red);
-    sgy = block_tree256(sgy, red);
-    nout = block_tree256(nout, red);
+    block_trees(a, sh, out);
+    const double nbody = out[0], nout = out[5];
     const double inb = nbody > 0 ? 1.0 / nbody : 0.0;
-    const double cx = sx * inb, cy = sy * inb;
-    double rmax = 0, rsum = 0, sxx = 0, sxy = 0, syy = 0, gxdx = 0, gxdy = 0, gydx = 0, gydy = 0;
-    for (int k = t; k < nb; k += 256) {
-        const int p = bnode[k];
-        const double dx = X[p] - cx, dy = Y[p] - cy;
-        const double r = sqrt(dx * dx + dy * dy);
-        if (bkind[k] == KIND_BODY) {
-            rmax = fmax(rmax, r);
-            sxx += dx * dx;
-            sxy += dx * dy;
-            syy += dy * dy;
-            gxdx += gx[k] * dx;
-            gxdy += gx[k] * dy;
-            gydx += gy[k] * dx;
-            gydy += gy[k] * dy;
-        } else {
-            rsum += r;
+    const double cx = out[1] * inb, cy = out[2] * inb, sgx = out[3], sgy = out[4];
+    __syncthreads();  // out is written again
+    double rmax = 0, s[8] = {};  // sum r (outer), Sxx, Sxy, Syy, sums of g d
+    for (int k0 = t; k0 < nb; k0 += 256 * B) {
+        int kd[B], p[B];
+        double x[B], y[B], u[B], v[B];
+#pragma unroll
+        for (int q = 0; q < B; ++q) {
+            const int k = min(k0 + 256 * q, nb - 1);
+            p[q] = bnode[k];
+            kd[q] = bkind[k];
+            u[q] = gx[k];
+            v[q] = gy[k];
+        }
+#pragma unroll
+        for (int q = 0; q < B; ++q) {
+            x[q] = X[p[q]];
+            y[q] = Y[p[q]];
+        }
+#pragma unroll
+        for (int q = 0; q < B; ++q) {
+            if (k0 + 256 * q >= nb) break;
+            const double dx = x[q] - cx, dy = y[q] - cy;
+            const double r = sqrt(dx * dx + dy * dy);
+            if (kd[q] == KIND_BODY) {
+                rmax = fmax(rmax, r);
+                s[1] += dx * dx;
+                s[2] += dx * dy;
+                s[3] += dy * dy;
+                s[4] += u[q] * dx;
+                s[5] += u[q] * dy;
+                s[6] += v[q] * dx;
+                s[7] += v[q] * dy;
+            } else {
+                s[0] += r;
+            }
         }
     }
-    rmax = block_max256(rmax, red);
-    rsum = block_tree256(rsum, red);
-    sxx = block_tree256(sxx, red);
-    sxy = block_tree256(sxy, red);
-    syy = block_tree256(syy, red);
-    gxdx = block_tree256(gxdx, red);
-    gxdy = block_tree256(gxdy, red);
-    gydx = block_tree256(gydx, red);
-    gydy = block_tree256(gydy, red);
+    sh[8][t] = rmax;
+    block_trees(s, sh, out);
+    if (t < 32) {
+        double m = sh[8][t];
+#pragma unroll
+        for (int q = 1; q < 8; ++q) m = fmax(m, sh[8][t + 32 * q]);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, off));
+        if (t == 0) rmax_s = m;
+    }
+    __syncthreads();
     if (t == 0) {
+        const double rmax = rmax_s, rsum = out[0], sxx = out[1], sxy = out[2], syy = out[3];
+        const double gxdx = out[4], gxdy = out[5], gydx = out[6], gydy = out[7];
         Globals g;
         g.cx = cx;
         g.cy = cy;
@@ -116,6 +139,15 @@ __global__ void k_globals(int nb, const int* __restrict__ bnode, const int* __re
         const double al = 0.5 * atan2(2.0 * mxy, 2.0 * hx);
         g.ec = cos(al);
         g.es = sin(al);
+        const double a[2][3] = {{g.tx, g.m11, g.m12}, {g.ty, g.m21, g.m22}};
+        double iq[2];
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const double q = a[s][0] * a[s][0] + a[s][1] * a[s][1] + a[s][2] * a[s][2];
+            iq[s] = q > 0.0 ? 1.0 / q : 0.0;
+        }
+        g.iqx = iq[0];
+        g.iqy = iq[1];
         *G = g;
     }
 }
@@ -140,7 +172,8 @@ __global__ void k_fields_seed(int n, const float* __restrict__ y, const int* __r
 __global__ void k_fields_guess(int n, const int* __restrict__ kind, const Globals* __restrict__ G,
                                const double* __restrict__ F, const double* __restrict__ x0,
                                const double* __restrict__ x1, double* __restrict__ c0,
-                               double* __restrict__ c1) {
+                               double* __restrict__ c1, float2* __restrict__ s0,
+                               float2* __restrict__ s1) {
     const Globals g = *G;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double a = x0[i], b = x1[i];
@@ -151,6 +184,13 @@ __global__ void k_fields_guess(int n, const int* __restrict__ kind, const Global
         }
         c0[i] = a;
         c1[i] = b;
+        if (s0) {  // relative tests: hi + lo, the precise product's operand
+            float hi, lo;
+            split_bits(a, hi, lo);
+            s0[i] = make_float2(hi, lo);
+            split_bits(b, hi, lo);
+            s1[i] = make_float2(hi, lo);
+        }
     }
 }
 
@@ -163,12 +203,7 @@ __global__ void k_fields_update(int n, const int* __restrict__ kind, const Globa
                                 double* __restrict__ F) {
     const Globals g = *G;
     const double a[2][3] = {{g.tx, g.m11, g.m12}, {g.ty, g.m21, g.m22}};
-    double iq[2];  // 1/|a_s|^2 (0: the solve has no prescribed motion), once per launch
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-        const double q = a[s][0] * a[s][0] + a[s][1] * a[s][1] + a[s][2] * a[s][2];
-        iq[s] = q > 0.0 ? 1.0 / q : 0.0;
-    }
+    const double iq[2] = {g.iqx, g.iqy};  // formed once, with the fit
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (kind[i] != KIND_FREE) continue;
         double f[3] = {F[i], F[n + i], F[2 * (size_t)n + i]};

@@ -37,12 +37,12 @@ constexpr int kPad = kChunk + 32;     // a chunk's products, one pad per 32
 constexpr int kSortLen = 32;          // row-length classes of the deal
 constexpr int kGroup = 4;             // chunks a block takes between two barriers of its own
 
-__device__ __forceinline__ int pad32(int i) { return i + (i >> 5); }
-
 // ------------------------------------------------------------------ barrier of one launch
-// gb->arrive counts arrivals from zero (the caller clears it before the launch); a waiter
-// leaves when the count has reached `target` (compared modulo 2^32).  One hop: the last
-// arrival itself releases the waiters.  false: the bounds ran out (gb->err is set).
+// gb->arrive counts arrivals from zero; a waiter leaves when the count has reached `target`
+// (compared modulo 2^32).  One hop: the last arrival itself releases the waiters.  false: the
+// bounds ran out (gb->err is set).  The last block to leave a launch that did not fail clears
+// the count for the next one (gb->gen counts the leavers), so that no clearing stands before
+// each launch; after a failure the host clears it.
 __device__ __forceinline__ bool bar_arrive_wait(GridBar* gb, unsigned target) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&gb->arrive) : "memory");
     unsigned long long t0 = 0;
@@ -59,22 +59,6 @@ __device__ __forceinline__ bool bar_arrive_wait(GridBar* gb, unsigned target) {
             }
         }
     }
-}
-
-// The 256-lane tree of cfd_common.cuh by one warp, lane 4 w + l taking the eight values of
-// warp w that meet in its (l, l+4) pair: v(t) gives lane t's value.  Sum in lane 0.
-template <class V>
-__device__ __forceinline__ double warp_tree256(V v) {
-    const int lane = threadIdx.x & 31, t = 32 * (lane >> 2) + (lane & 3);
-    const double a0 = v(t), a16 = v(t + 16), a8 = v(t + 8), a24 = v(t + 24), a4 = v(t + 4),
-                 a20 = v(t + 20), a12 = v(t + 12), a28 = v(t + 28);
-    double c = ((a0 + a16) + (a8 + a24)) + ((a4 + a20) + (a12 + a28));
-    c = c + __shfl_down_sync(0xffffffffu, c, 2);
-    c = c + __shfl_down_sync(0xffffffffu, c, 1);
-    c = c + __shfl_down_sync(0xffffffffu, c, 16);
-    c = c + __shfl_down_sync(0xffffffffu, c, 8);
-    c = c + __shfl_down_sync(0xffffffffu, c, 4);
-    return c;
 }
 
 // A chunk's cnt products in shared memory (pad32) -> their sum in the dots' order, by one
@@ -95,7 +79,7 @@ __device__ __noinline__ double chunk_sum(const double* q, int cnt) {
     });
 }
 
-// The nc chunk partials -> their fold (fold_partials's order), by one warp; the loads are
+// The nc chunk partials -> their fold (256 lanes with stride 256, then the tree), by one warp; the loads are
 // clamped, not branched over, so that a lane's eight go out together
 __device__ __noinline__ double chunk_fold(const double* part, long nc) {
     const int lane = threadIdx.x & 31, t = 32 * (lane >> 2) + (lane & 3);
@@ -197,6 +181,12 @@ __global__ void __launch_bounds__(kChunk, 1) k_pcg_fp64(PcgArgs a) {
     const bool relb = a.tol_mode == CFD_BICG_TOL_REL;  // ||b - A.x_D|| as reference
     if (t == 0) s.fail = 0;
 
+    auto leave = [&] {  // one thread; the block waits no more
+        if (atomicAdd(&a.bar->gen, 1u) == nb - 1) {
+            a.bar->arrive = 0u;
+            a.bar->gen = 0u;
+        }
+    };
     // every thread's global writes before, every thread's reads after
     auto grid_sync = [&]() -> bool {
         __syncthreads();
@@ -391,7 +381,10 @@ __global__ void __launch_bounds__(kChunk, 1) k_pcg_fp64(PcgArgs a) {
     bool done[2];
     done[0] = s.done[0] != 0;
     done[1] = ns < 2 || s.done[1] != 0;
-    if (done[0] && done[1]) return;
+    if (done[0] && done[1]) {
+        if (t == 0) leave();
+        return;
+    }
 
     // the slots of the active solves' sums in buffer ba, then (two) in buffer bb
     auto slots = [&](bool on0, bool on1, bool two, unsigned ba, unsigned bb, unsigned& code) {
@@ -579,6 +572,7 @@ __global__ void __launch_bounds__(kChunk, 1) k_pcg_fp64(PcgArgs a) {
             }
         }
     }
+    if (t == 0) leave();
     if (blockIdx.x == 0 && t < ns && !s.done[t]) {
         a.iters_out[t] = s.last[t];
         a.rz_out[t] = fabs(s.err_old[t]);
@@ -588,7 +582,7 @@ __global__ void __launch_bounds__(kChunk, 1) k_pcg_fp64(PcgArgs a) {
     }
 }
 
-// One solve on the current device (a.bar zeroed before, on the same stream): ON_CHIP when
+// One solve on the current device (a.bar: zeroed once, or left so by the last launch): ON_CHIP when
 // the chunks fit the SMs one each
 cudaError_t launch_pcg_fp64(cudaStream_t st, PcgArgs a) {
     int dev = 0, nsm = 0;
@@ -619,45 +613,63 @@ cudaError_t launch_pcg_fp64(cudaStream_t st, PcgArgs a) {
 //     x = c1 x_{n-1} + c2 x_{n-2},  h = (dt_n + dt1) / (dt1 + dt2),
 //     c1 = dt_n / dt1 (1 + h),  c2 = -(dt_n / dt2) h
 // on the free rows (x_{n-1} is the previous solution, still in x), in the oracle's operation
-// order (--fmad=false: the same bits); x_{n-1} is kept as the next step's x_{n-2}.  hist =
-// (dt1, dt2, solutions kept); with fewer than two kept the guess stays x_{n-1}.  The fixed
-// rows are left to the Dirichlet values (set before, or by the solve).  The float shadow
-// (mixed form) follows x.
-__global__ void k_guess_extrapolate(PcgArgs a, const double* __restrict__ dtn_p,
-                                    double* __restrict__ hist, double* __restrict__ xprev0,
-                                    double* __restrict__ xprev1) {
-    const double dtn = *dtn_p, dt1 = hist[0], dt2 = hist[1];
-    const bool two = hist[2] >= 2.0;
-    double c1 = 1.0, c2 = 0.0;
-    if (two) {
-        const double h = (dtn + dt1) / (dt1 + dt2);
-        c1 = dtn / dt1 * (1.0 + h);
-        c2 = -(dtn / dt2) * h;
-    }
-    double* xprev[2] = {xprev0, xprev1};
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < a.n;
-         i += (long)gridDim.x * blockDim.x) {
-        if (a.isfix[i]) continue;
-        for (int s = 0; s < a.nsolve; ++s) {
-            const double x1 = a.x[s][i];
-            const double xn = two ? c1 * x1 + c2 * xprev[s][i] : x1;
-            xprev[s][i] = x1;
-            if (two) {
-                a.x[s][i] = xn;
-                if (a.xf[s]) a.xf[s][i] = d2f_trunc(xn);
+// order (--fmad=false: the same bits); x_{n-1} is kept as the next step's x_{n-2}; with fewer
+// than two kept the guess stays x_{n-1}.  hist[3..5] = (c1, c2, two kept) from guess_history: a
+// division is ten operations of the FP64 pipe, and a thread takes a node or two.  The fixed
+// rows are left to the Dirichlet values (set before, or by the solve).  The float shadow and,
+// under the relative tests, the hi/lo split (mixed form) follow x.
+__global__ void k_guess_extrapolate(PcgArgs a, const double* __restrict__ hist,
+                                    double* __restrict__ xprev0, double* __restrict__ xprev1) {
+    const double c1 = hist[3], c2 = hist[4];
+    const bool two = hist[5] != 0.0;
+    // two rows and both solves' loads go out together
+    const long step = (long)gridDim.x * blockDim.x;
+    for (long i0 = blockIdx.x * (long)blockDim.x + threadIdx.x; i0 < a.n; i0 += 2 * step) {
+        double x[2][2], xp[2][2];
+        bool fx[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const long i = min(i0 + u * step, (long)a.n - 1);
+            fx[u] = a.isfix[i] != 0;
+#pragma unroll
+            for (int s = 0; s < 2; ++s)
+                if (s < a.nsolve) {
+                    x[u][s] = a.x[s][i];
+                    xp[u][s] = (s ? xprev1 : xprev0)[i];
+                }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const long i = i0 + u * step;
+            if (i >= a.n) break;
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                if (s >= a.nsolve) break;
+                const double x1 = x[u][s];
+                double xn = x1;
+                if (!fx[u]) {
+                    if (two) {
+                        xn = c1 * x1 + c2 * xp[u][s];
+                        a.x[s][i] = xn;
+                        if (a.xf[s]) a.xf[s][i] = d2f_trunc(xn);
+                    }
+                    (s ? xprev1 : xprev0)[i] = x1;
+                }
+                if (a.xs[s]) {  // the precise product's operand (mixed form, relative tests)
+                    float hi, lo;
+                    split_bits(xn, hi, lo);
+                    a.xs[s][i] = make_float2(hi, lo);
+                }
             }
         }
     }
 }
 
-// after k_guess_extrapolate: hist = (dt_n, dt1, solutions kept + 1)
+// before k_guess_extrapolate: guess_history, by one thread (the mixed form's k_motion_tail
+// has it done beside the motion)
 __global__ void k_guess_extrapolate_hist(const double* __restrict__ dtn_p,
                                          double* __restrict__ hist) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        hist[1] = hist[0];
-        hist[0] = *dtn_p;
-        hist[2] = hist[2] + 1.0;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) guess_history(*dtn_p, hist);
 }
 
 // div_rcp against the division x / d over n input pairs: a third raw 64-bit patterns for

@@ -16,15 +16,17 @@
 
 namespace cfd {
 
-// The SpMV rows gather in batches of B entries (8 in the FP32 residual kernel, 4 in the
-// register-limited persistent kernel and in the precise residual, whose 4-entry batches
-// measured 1.29 -> 1.25 ms per 1M-node step against 8): the column indices and values of a batch are loaded
+// The SpMV rows gather in batches of B entries (3 in the FP32 row kernels and the persistent
+// kernel, 4 in the precise residual): the fewer registers of a small batch, and with them the
+// warps in flight, are worth more than long batches (FP32 first pass and direction pass alone
+// at 1M nodes on 760 blocks: 49 + 37 us with 8, 48 + 26 with 5, 35 + 28 with 3; precise: 1.29 ->
+// 1.25 ms per step with 4 against 8).  The column indices and values of a batch are loaded
 // together, then the gathered vector entries, so each batch costs two dependent memory
 // latencies instead of two per entry.  The products are still summed in column order.
 
 // row i of A times (v0, v1): one pass over the row's columns for both right-hand sides;
 // with FIXC also the sums over the Dirichlet columns only (f0, f1: the row of A.x_D)
-template <int NS, bool FIXC = false, int kRowBatch = 8>
+template <int NS, bool FIXC = false, int kRowBatch = 3>
 __device__ __forceinline__ void spmv_row2_f(const PcgArgs& a, int i, const float* v0,
                                             const float* v1, float& d0, float& d1,
                                             float* f0 = nullptr, float* f1 = nullptr) {
@@ -159,7 +161,7 @@ __global__ void k_split_x(PcgArgs a, const double* __restrict__ v0, const double
             }
 }
 
-template <int kRowBatch = 4>
+template <int kRowBatch = 3>
 __device__ __forceinline__ float spmv_row_dir_f(const PcgArgs& a, int i, const float* pf,
                                                 const float* zf, float beta) {
     float dot = 0.f;
@@ -455,7 +457,7 @@ __global__ void __launch_bounds__(256) k_bicg_dir_mixed(PcgArgs a) {
             if (!act[s]) continue;
             const double pi = a.p[s][0][i];
             const double yi =
-                fx ? 1.0e30 * pi : f2d_bits(spmv_row_dir_f<8>(a, (int)i, a.pf[s][0], a.pf[s][0], 0.f));
+                fx ? 1.0e30 * pi : f2d_bits(spmv_row_dir_f(a, (int)i, a.pf[s][0], a.pf[s][0], 0.f));
             a.y[s][i] = yi;
             py[s] += pi * yi;
         }
@@ -798,22 +800,36 @@ __global__ void __launch_bounds__(256, 2) k_pcg_mixed(PcgArgs a) {
             last_iter[s] = k;
         }
     }
-    // last deferred x update; the shadow follows x for the solves that iterated
-    for (long c = blockIdx.x; c < nc; c += gridDim.x)
-        for (int kk = 0; kk < 4; ++kk) {
-            const long i = c * kChunk + t + 256L * kk;
-            if (i >= n) break;
+    // last deferred x update; the shadow follows x for the solves that iterated.  Four rows'
+    // loads go out together (14 -> 11 us of a 1,048,576-node step whose solves stop at once)
+    const long xs = (long)gridDim.x * 256;
 #pragma unroll
-            for (int s = 0; s < 2; ++s) {
-                if (done[s]) continue;
-                double xi = a.x[s][i];
+    for (int s = 0; s < 2; ++s) {
+        if (done[s]) continue;
+        double* __restrict__ x = a.x[s];
+        const double* __restrict__ p = a.p[s][cur[s]];
+        float* __restrict__ xf = a.xf[s];
+        for (long i0 = blockIdx.x * 256L + t; i0 < n; i0 += 4 * xs) {
+            double xv[4], pv[4];
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                const long i = i0 + kk * xs;
+                xv[kk] = i < n ? x[i] : 0.0;
+                pv[kk] = (i < n && pend[s]) ? p[i] : 0.0;
+            }
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                const long i = i0 + kk * xs;
+                if (i >= n) break;
+                double xi = xv[kk];
                 if (pend[s]) {
-                    xi += alfa[s] * a.p[s][cur[s]][i];
-                    a.x[s][i] = xi;
+                    xi += alfa[s] * pv[kk];
+                    x[i] = xi;
                 }
-                a.xf[s][i] = d2f_trunc(xi);
+                xf[i] = d2f_trunc(xi);
             }
         }
+    }
     if (blockIdx.x == 0 && t == 0 && a.iterated) *a.iterated = (last_iter[0] + last_iter[1]) > 0;
     if (blockIdx.x == 0 && t == 0)
 #pragma unroll

@@ -295,11 +295,11 @@ int fields_seed(cfd_mpnn_graph* g, cudaStream_t st) {
 
 int fields_guess(cfd_mpnn_graph* g, cudaStream_t st, const double* X, const double* Y,
                  const double* bgx, const double* bgy, const double* x0, const double* x1,
-                 double* c0, double* c1) {
+                 double* c0, double* c1, float2* s0, float2* s1) {
     const int* ng = nullptr;
     CFD_LAUNCH(k_globals, 1, 256, 0, st, g->nb, g->bnode, g->bkind, bgx, bgy, X, Y, g->G, ng);
     CFD_LAUNCH(k_fields_guess, std::min(blocks_for(g->n, 256), 1216u), 256, 0, st, g->n, g->kind,
-               (const Globals*)g->G, (const double*)g->F, x0, x1, c0, c1);
+               (const Globals*)g->G, (const double*)g->F, x0, x1, c0, c1, s0, s1);
     return CFD_OK;
 }
 

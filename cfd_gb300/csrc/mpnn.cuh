@@ -46,6 +46,7 @@ struct Globals {
     double m11, m12, m21, m22;
     double ea, eb;  // semi-axes of the body's second-moment ellipse (uniform sampling in
     double ec, es;  //   the parametric angle), cos and sin of its major-axis angle
+    double iqx, iqy;  // 1/|(tx, m11, m12)|^2, 1/|(ty, m21, m22)|^2 (0: no prescribed motion)
 };
 
 }  // namespace mpnn

@@ -16,7 +16,8 @@ __global__ void k_scatter_bc(int nb, const int* bnode, const double* gx, const d
                              double* gnx, double* gny, const int* gate);
 __global__ void k_fields_seed(int n, const float* y, const int* kind, const Globals* G, double* F);
 __global__ void k_fields_guess(int n, const int* kind, const Globals* G, const double* F,
-                               const double* x0, const double* x1, double* c0, double* c1);
+                               const double* x0, const double* x1, double* c0, double* c1,
+                               float2* s0, float2* s1);
 __global__ void k_fields_update(int n, const int* kind, const Globals* G, const double* x0,
                                 const double* x1, double* F);
 __global__ void k_features(int n, const double* X, const double* Y, const int* kind,

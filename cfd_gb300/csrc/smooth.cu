@@ -287,13 +287,12 @@ __global__ void k_smooth_prep(int n, const double* __restrict__ xpos,
 
 // ... and after it: W is the whole move of the step over DTMIN (the prescribed displacement
 // plus the smoothing's), so that the geometric conservation law sees the mesh that is
-// used; the mixed form also refreshes its float shadows of W and of (X, Y)
+// used; the mixed form also refreshes its float shadow of W
 __global__ void k_smooth_w(int n, const double* __restrict__ xpos, const double* __restrict__ ypos,
                            const double* __restrict__ X, const double* __restrict__ Y,
                            const double* __restrict__ xb, const double* __restrict__ yb,
                            const StepScal* __restrict__ sc, double* __restrict__ WX,
-                           double* __restrict__ WY, float2* __restrict__ Wf,
-                           float2* __restrict__ Xhi, float2* __restrict__ Xlo) {
+                           double* __restrict__ WY, float2* __restrict__ Wf) {
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         const double x = X[p], y = Y[p];
         const double dx = x - xb[p], dy = y - yb[p];
@@ -304,11 +303,6 @@ __global__ void k_smooth_w(int n, const double* __restrict__ xpos, const double*
             WX[p] = wx;
             WY[p] = wy;
             Wf[p] = make_float2(d2f_trunc(wx), d2f_trunc(wy));
-            float hx, lx, hy, ly;
-            split_bits(x, hx, lx);
-            split_bits(y, hy, ly);
-            Xhi[p] = make_float2(hx, hy);
-            Xlo[p] = make_float2(lx, ly);
         } else {
             WX[p] = mx / sc->dtmin;
             WY[p] = my / sc->dtmin;
