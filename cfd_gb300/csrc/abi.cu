@@ -653,9 +653,7 @@ int cfd_calcrhs(double* rhs, const double* U, const double* theta, const double*
     double* ndo = nullptr;
     CFD_CUDA(launch_elem_rhs(visc, theta != nullptr, s.stream, E, d_el, d_U, d_th, d_T, d_geo,
                              d_area, d_shoc, d_dtl, nd, d_t1, d_t2, d_t3, gc, d_c, nd, nd, ndo));
-    CFD_LAUNCH(k_node_update, blocks_for(N, 256), 256, 0, s.stream, N, d_ptr, d_slot, d_c, nd, nd,
-               nd, 0.0, 0.0, 0.0, (const unsigned char*)nullptr, (const double*)nullptr,
-               (const double2*)nullptr, nd, nd, ndo, ndo, ndo, ndo, ndo, ndo, ndo, ndo, d_rhs, d_rhs);
+    CFD_LAUNCH(k_rhs_gather, blocks_for(N, 256), 256, 0, s.stream, N, d_ptr, d_slot, d_c, d_rhs);
     TRY(s.get(rhs, d_rhs, 4 * (size_t)N));
     return s.sync();
 }
@@ -692,9 +690,7 @@ int cfd_fuente(double* rhs, const double* U, const double* W_X, const double* W_
     double* ndo = nullptr;
     CFD_CUDA(launch_elem_rhs(false, false, s.stream, E, d_el, d_U, nd, nd, d_geo, d_area, nd, d_dtl,
                              nd, nd, nd, nd, gc, ndo, d_wx, d_wy, d_f));
-    CFD_LAUNCH(k_node_update, blocks_for(N, 256), 256, 0, s.stream, N, d_ptr, d_slot, d_f, nd, nd,
-               nd, 0.0, 0.0, 0.0, (const unsigned char*)nullptr, (const double*)nullptr,
-               (const double2*)nullptr, nd, nd, ndo, ndo, ndo, ndo, ndo, ndo, ndo, ndo, d_rhs, d_rhs);
+    CFD_LAUNCH(k_rhs_gather, blocks_for(N, 256), 256, 0, s.stream, N, d_ptr, d_slot, d_f, d_rhs);
     TRY(s.get(rhs, d_rhs, 4 * (size_t)N));
     return s.sync();
 }
@@ -728,10 +724,12 @@ int cfd_estab(const double* U, const double* T, const double* GAMM, const double
     for (int i = 0; i < 4; ++i) TRY(s.alloc(&o[i], E));
     StepScal sc{};
     sc.dtmin = scal5[2];
+    sc.two_dt2 = (2.0 / scal5[2]) * (2.0 / scal5[2]);
     TRY(s.put(&d_sc, &sc, 1));
-    CFD_LAUNCH(k_estab, blocks_for(E, 128), 128, 0, s.stream, E, d_el, d_U, d_T, scal5[0], d_G, d_vx,
-               d_vy, d_wx, d_wy, d_geo, scal5[1], d_sc, scal5[3], scal5[4], (int)CFD_ESTAB_REFERENCE,
-               0.0, 1.0, 0.0, o[0], o[1], o[2], o[3]);
+    CFD_LAUNCH(k_estab, blocks_for(E, 128), 128, 0, s.stream, E, d_el, d_U, d_T, d_G, d_vx, d_vy,
+               d_wx, d_wy, d_geo,
+               estab_args(scal5[0], scal5[1], scal5[3], scal5[4], CFD_ESTAB_REFERENCE, 0.0, 1.0, 0.0),
+               d_sc, o[0], o[1], o[2], o[3]);
     TRY(s.get(SHOC, o[0], E));
     TRY(s.get(T_SUGN1, o[1], E));
     TRY(s.get(T_SUGN2, o[2], E));
@@ -766,7 +764,7 @@ int cfd_deltat(const double* T, const double* VEL_X, const double* VEL_Y, const 
     sc.bandera = 1;
     TRY(s.put(&d_sc, &sc, 1));
     CFD_LAUNCH(k_deltat, blocks_for(E, 256), 256, 0, s.stream, E, d_el, d_T, d_vx, d_vy, d_wx, d_wy, d_a,
-               scal4[0], scal4[3], d_DT, &d_sc->dtmin_bits);
+               scal4[0], make_rcp(scal4[3]), d_DT, &d_sc->dtmin_bits);
     CFD_LAUNCH(k_dt_finalize, 1, 1, 0, s.stream, d_sc);
     CFD_LAUNCH(k_dt_clamp, blocks_for(E, 256), 256, 0, s.stream, E, d_DT, d_sc);
     TRY(s.get(DT, d_DT, E));

@@ -78,6 +78,32 @@ __device__ __forceinline__ double div_rcp(double x, double d, double y) {
     return fma(fma(-d, q1, x), y, q1);
 }
 
+// x / d in a multiply and three FMAs where the reciprocal comes with its remainder, y = RN(1/d)
+// and yl = RN(RN(1 - d*y)*y) (the FMA remainder is exact): q0 = RN(x*y + RN(x*yl)) is within
+// half an ulp and a little of x/d, so one correction by Markstein's theorem (as in div_rcp,
+// which spends its first correction on getting q0 within an ulp) is the correctly rounded
+// quotient.  Same range check and fallback; bit-identical to x / d.
+__host__ __device__ __forceinline__ double rcp_lo(double d, double y) { return fma(-d, y, 1.0) * y; }
+__device__ __forceinline__ double div_rcp2(double x, double d, double y, double yl) {
+    const int ex = (int)((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ff;
+    const int ed = (int)((unsigned long long)__double_as_longlong(d) >> 52) & 0x7ff;
+    if ((unsigned)(ex - 200) > 1600u || (unsigned)(ed - 200) > 1600u || abs(ex - ed) > 800) {
+        if (x == 0.0 && (unsigned)(ed - 200) <= 1600u) return x * y;
+        return x / d;
+    }
+    const double q0 = fma(x, y, x * yl);
+    return fma(fma(-d, q0, x), y, q0);
+}
+// a divisor with its reciprocal, formed once where many threads divide by it
+struct Rcp {
+    double d, y, yl;
+};
+inline Rcp make_rcp(double d) {
+    const double y = 1.0 / d;
+    return Rcp{d, y, rcp_lo(d, y)};
+}
+__device__ __forceinline__ double div_by(double x, const Rcp& r) { return div_rcp2(x, r.d, r.y, r.yl); }
+
 // ------------------------------------------------------------------ FP32 <-> FP64 by bits
 // GB300's FP64 pipe (1/64 of the FP32 rate) also executes the F2F conversions, so the
 // mixed-precision kernels move values between the two formats with integer operations.

@@ -128,6 +128,7 @@ struct Ctx {
     float* d_valf = nullptr;
     float* d_val_lo = nullptr;
     double* d_rdiag = nullptr;   // FP64 form: RN(1/diag) of the BiCG (formed by each solve)
+    double *d_r0 = nullptr, *d_rM = nullptr;  // FP64 form: continuity sum, RN(1/M) of the stages
     double* d_lapq = nullptr;    // FP64 form: the Laplacian weight per element
     double2* d_gcl64 = nullptr;  // FP64 form: the gcl element terms   // relative tests: valf + val_lo = the FP64-assembled matrix
     float2* d_k64 = nullptr;     // relative tests: element-matrix rows (hi, lo), per slot (3 each)

@@ -23,6 +23,7 @@ struct StepScal {
     float pad_f;
     float dtfact_f, cota_f;         // mixed form, ITLOCAL != 0: DTFACT and COTA of DTL
     float pad2_f[2];
+    double two_dt2;                 // FP64 form: (2/DTMIN)^2 (ESTAB)
 };
 
 // DTMIN from the minimum DTELEM (b: its bit pattern, +inf for none) with the 1% hysteresis
@@ -46,6 +47,8 @@ __device__ __forceinline__ void dt_finalize_from(StepScal* sc, unsigned long lon
     sc->dtmin = dtmin;
     sc->cota = 10.0 * sc->dtmin_raw;
     sc->inv_dtmin = 1.0 / dtmin;
+    const double two_dt = 2.0 / dtmin;
+    sc->two_dt2 = two_dt * two_dt;
     sc->dtmin_f = (float)dtmin;
 }
 
@@ -266,16 +269,27 @@ cudaError_t launch_gcl(cudaStream_t st, int npoin, int nelem, const int4* elem,
                        int literal, double2* scratch, double* M);
 __global__ void k_deltat(int nelem, const int4* elem, const double* T, const double* VX,
                          const double* VY, const double* WX, const double* WY,
-                         const double* area, double fsafe, double t_inf, double* DT,
+                         const double* area, double fsafe, Rcp t_inf, double* DT,
                          unsigned long long* dtmin_bits);
 __global__ void k_dt_finalize(StepScal* sc);
 __global__ void k_dtl(int nelem, double* DT, double* DTL, const StepScal* sc, double dtfact);
+// ESTAB's launch constants: what is the same for every element is formed once on the host
+// (GAMM(1:3) averaged when uniform, times FR; the divisors with their reciprocals)
+struct EstabArgs {
+    double gm, gmfr, fr;
+    Rcp rho_inf, t_inf;
+    int mode;
+    double eps, dirx, diry;
+};
+inline EstabArgs estab_args(double gamm, double fr, double rho_inf, double t_inf, int mode,
+                            double eps, double dirx, double diry) {
+    const double gm = (gamm + gamm + gamm) / 3.0;
+    return EstabArgs{gm, gm * fr, fr, make_rcp(rho_inf), make_rcp(t_inf), mode, eps, dirx, diry};
+}
 __global__ void k_estab(int nelem, const int4* elem, const double* U, const double* T,
-                        double gamm, const double* GAMM, const double* VX, const double* VY, const double* WX,
-                        const double* WY, const double* geo, double FR, const StepScal* sc,
-                        double RHOINF, double TINF, int estab_mode, double eps_dir,
-                        double dirx, double diry, double* SHOC, double* TS1, double* TS2,
-                        double* TS3);
+                        const double* GAMM, const double* VX, const double* VY, const double* WX,
+                        const double* WY, const double* geo, EstabArgs c, const StepScal* sc,
+                        double* SHOC, double* TS1, double* TS2, double* TS3);
 __global__ void k_vel_from_U(int npoin, const double* U, double* VX, double* VY);
 // calcRHS split into its stage-invariant part (once per step: the cached addends and
 // factors, FUENTE into contribF; with !viscous the final contributions into contrib) and
@@ -301,14 +315,23 @@ cudaError_t launch_elem_rhs(bool viscous, bool with_theta, cudaStream_t stream, 
                             const double* ts1, const double* ts2, const double* ts3, GasConst gc,
                             double* contrib, const double* WX, const double* WY,
                             double* contribF);
-__global__ void k_node_update(int npoin, const int* esup_ptr, const int* esup_slot,
-                              const double* contrib, const double* contribF, const double* U,
-                              const double* M, double rk_fact, double gamm, double FR,
-                              const unsigned char* bcflag, const double* bcval,
-                              const double2* nrm, const double* WX, const double* WY,
-                              double* U1, double* RHO, double* VX, double* VY, double* Eo,
-                              double* Po, double* To, double* RMACH, const double* rhs_init,
-                              double* rhs_out);
+// drop-in: rhs(4,npoin) += the elements' contributions, in element order
+__global__ void k_rhs_gather(int npoin, const int* esup_ptr, const int* esup_slot,
+                             const double* contrib, double* rhs);
+// one RK stage's node side in the step (kernels_fp64.cu); r0, rM: per-node scratch the first
+// stage fills (the continuity sum, RN(1/M))
+struct NodeStageArgs {
+    int npoin;
+    const int *esup_ptr, *esup_slot;
+    const double *contrib, *contribF, *U, *M;
+    double rk_fact, gamm, gm1, fr;
+    const unsigned char* bcflag;
+    const double* bcval;
+    const double2* nrm;
+    const double *WX, *WY;
+    double *U1, *RHO, *VX, *VY, *E, *P, *T, *RMACH, *r0, *rM;
+};
+cudaError_t launch_node_stage(cudaStream_t stream, int irk, const NodeStageArgs& a);
 __global__ void k_dt_clamp(int nelem, double* DT, const StepScal* sc);
 __global__ void k_min_positive(long n, const double* x, unsigned long long* bits);
 __global__ void k_normales(int nwn, const int* wnode, const int* wptr, const int2* wedge_of,

@@ -536,7 +536,7 @@ int Ctx::step_once() {
     // DELTAT + hysteresis (ns2DComp.ALE.f90:144-156)
     tstart(TM_DELTAT);
     CFD_LAUNCH(k_deltat, blocks_for(E, TB), TB, 0, stream, E, d_elem, d_T, d_VX, d_VY, d_WX, d_WY,
-               d_area, prm.fsafe, prm.t_inf, d_DT, &d_scal->dtmin_bits);
+               d_area, prm.fsafe, make_rcp(prm.t_inf), d_DT, &d_scal->dtmin_bits);
     CFD_LAUNCH(k_dt_finalize, 1, 1, 0, stream, d_scal);
     tstop(TM_DELTAT);
     CFD_CUDA(cudaMemcpyAsync(h_scal, d_scal, sizeof(StepScal), cudaMemcpyDeviceToHost, stream));
@@ -550,10 +550,11 @@ int Ctx::step_once() {
     const double* dtl_scalar = &d_scal->dtmin;
     // RK (subrutinas.f90:645-849): ESTAB once, then 4 stages of calcRHS+FUENTE and update
     tstart(TM_ESTAB);
-    CFD_LAUNCH(k_estab, blocks_for(E, 128), 128, 0, stream, E, d_elem, d_U, d_T, prm.gama,
-               (const double*)nullptr, d_VX,
-               d_VY, d_WX, d_WY, d_geo, prm.fr, d_scal, prm.rho_inf, prm.t_inf, prm.estab_mode,
-               estab_eps, dir[0], dir[1], d_SHOC, d_TS1, d_TS2, d_TS3);
+    CFD_LAUNCH(k_estab, blocks_for(E, 128), 128, 0, stream, E, d_elem, d_U, d_T,
+               (const double*)nullptr, d_VX, d_VY, d_WX, d_WY, d_geo,
+               estab_args(prm.gama, prm.fr, prm.rho_inf, prm.t_inf, prm.estab_mode, estab_eps,
+                          dir[0], dir[1]),
+               d_scal, d_SHOC, d_TS1, d_TS2, d_TS3);
     tstop(TM_ESTAB);
     GasConst gc{prm.fcv, prm.fk, prm.fmu, prm.gama, prm.t_inf, prm.cte, prm.fr};
     const bool viscous = prm.fmu > 2.2250738585072014e-308;
@@ -574,10 +575,12 @@ int Ctx::step_once() {
                                         gc, d_einv, d_contrib));
         tstop(TM_CALCRHS);
         tstart(TM_UPDATE);
-        CFD_LAUNCH(k_node_update, blocks_for(N, TB), TB, 0, stream, N, d_esup_ptr, d_esup_slot,
-                   d_contrib, d_contribF, d_U, d_M, rk_fact, prm.gama, prm.fr, d_bcflag,
-                   (const double*)d_bcval, d_nrm, d_WX, d_WY, d_U1, d_RHO, d_VX, d_VY, d_E,
-                   d_P, d_T, d_RMACH, (const double*)nullptr, (double*)nullptr);
+        const NodeStageArgs na{N,       d_esup_ptr, d_esup_slot, d_contrib, d_contribF, d_U,
+                               d_M,     rk_fact,    prm.gama,    prm.gama - 1.0, prm.fr,
+                               d_bcflag, d_bcval,   d_nrm,       d_WX,      d_WY,       d_U1,
+                               d_RHO,   d_VX,       d_VY,        d_E,       d_P,        d_T,
+                               d_RMACH, d_r0,       d_rM};
+        CFD_CUDA(launch_node_stage(stream, irk, na));
         tstop(TM_UPDATE);
     }
     // fluidStructure (meshMove.f90:28-142) needs TIME: the host reads DTMIN
@@ -781,7 +784,9 @@ int Ctx::create(const cfd_mesh* m, const cfd_params* p, int precision_mode) {
     if ((st = dalloc(&d_val, adj.col.size()))) return st;
     nnz = (long)adj.col.size();
     if ((st = dalloc(&d_diag, N))) return st;
-    if (prec == CFD_PREC_FP64 && (st = dalloc(&d_rdiag, N))) return st;
+    if (prec == CFD_PREC_FP64)
+        for (double** q : {&d_rdiag, &d_r0, &d_rM})
+            if ((st = dalloc(q, N))) return st;
     if (prec == CFD_PREC_FP64 && (st = dalloc(&d_lapq, E))) return st;
     if (prec == CFD_PREC_FP64 && (st = dalloc(&d_gcl64, E))) return st;
     // BC tables

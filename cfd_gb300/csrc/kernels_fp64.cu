@@ -117,7 +117,7 @@ cudaError_t launch_gcl(cudaStream_t st, int npoin, int nelem, const int4* elem,
 __global__ void k_deltat(int nelem, const int4* __restrict__ elem, const double* __restrict__ T,
                          const double* __restrict__ VX, const double* __restrict__ VY,
                          const double* __restrict__ WX, const double* __restrict__ WY,
-                         const double* __restrict__ area, double fsafe, double t_inf,
+                         const double* __restrict__ area, double fsafe, Rcp t_inf,
                          double* __restrict__ DT, unsigned long long* __restrict__ dtmin_bits) {
     int e = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long mybits = 0x7ff0000000000000ull;  // +inf
@@ -135,12 +135,13 @@ __global__ void k_deltat(int nelem, const int4* __restrict__ elem, const double*
         double hh = sqrt(2.0 * area[e]);
         double vel = sqrt(vumax * vumax + vvmax * vvmax);
         const double smu = 110.0;
-        double fmu = 0.017 * pow15(T_iel / t_inf) * (t_inf + smu) / (T_iel + smu);
+        double fmu = 0.017 * pow15(div_by(T_iel, t_inf)) * (t_inf.d + smu) / (T_iel + smu);
         double et = fmu;
         double pe = (vel * hh) / (2.0 * et);
         double alpha = fmin(div3(pe), 1.0);
-        double deltatu = 1.0 / (4.0 * et / (hh * hh) + alpha * vel / hh);
-        double deltatc = 1.0 / (4.0 * et / (hh * hh));
+        const double ac = (4.0 * et) / (hh * hh);
+        double deltatu = 1.0 / (ac + alpha * vel / hh);
+        double deltatc = 1.0 / ac;
         double dtelem = fsafe / (1.0 / deltatc + 1.0 / deltatu);
         DT[e] = dtelem;
         if (dtelem < 1.0e20 && dtelem > 0.0) mybits = (unsigned long long)__double_as_longlong(dtelem);
@@ -183,23 +184,21 @@ __global__ void k_dtl(int nelem, double* __restrict__ DT, double* __restrict__ D
 // ------------------------------------------------------------------ ESTAB
 // subrutinas.f90:346-443 (GAMM is the uniform GAMA for NGAS=0, :78).
 __global__ void k_estab(int nelem, const int4* __restrict__ elem, const double* __restrict__ U,
-                        const double* __restrict__ T, double gamm,
-                        const double* __restrict__ GAMM, const double* __restrict__ VX,
-                        const double* __restrict__ VY, const double* __restrict__ WX,
-                        const double* __restrict__ WY, const double* __restrict__ geo,
-                        double FR, const StepScal* __restrict__ sc, double RHOINF, double TINF,
-                        int estab_mode, double eps_dir, double dirx, double diry,
-                        double* __restrict__ SHOC, double* __restrict__ TS1,
-                        double* __restrict__ TS2, double* __restrict__ TS3) {
+                        const double* __restrict__ T, const double* __restrict__ GAMM,
+                        const double* __restrict__ VX, const double* __restrict__ VY,
+                        const double* __restrict__ WX, const double* __restrict__ WY,
+                        const double* __restrict__ geo, EstabArgs ec,
+                        const StepScal* __restrict__ sc, double* __restrict__ SHOC,
+                        double* __restrict__ TS1, double* __restrict__ TS2,
+                        double* __restrict__ TS3) {
     int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nelem) return;
     const size_t E = (size_t)nelem;
-    const double DTMIN = sc->dtmin;
     int4 n = elem[e];
     const int n1 = n.x, n2 = n.y, n3 = n.z;
     const double DX[3] = {geo[e], geo[E + e], geo[2 * E + e]};
     const double DY[3] = {geo[3 * E + e], geo[4 * E + e], geo[5 * E + e]};
-    double gm = GAMM ? div3(GAMM[n1] + GAMM[n2] + GAMM[n3]) : div3(gamm + gamm + gamm);
+    const double gmfr = GAMM ? div3(GAMM[n1] + GAMM[n2] + GAMM[n3]) * ec.fr : ec.gmfr;
     double tau = 0.0, h_rgne = 0.0, h_rgn = 0.0, h_jgn = 0.0;
     const double r1 = U[4 * (size_t)n1], r2 = U[4 * (size_t)n2], r3 = U[4 * (size_t)n3];
     double rho_elem = div3(r1 + r2 + r3);
@@ -219,7 +218,7 @@ __global__ void k_estab(int nelem, const int4* __restrict__ elem, const double* 
     double dt2 = sqrt(dtx * dtx + dty * dty) + 1.0e-20;
     double dux = vel2 * DX[0] + vel2 * DX[1] + vel2 * DX[2];
     double duy = vel2 * DY[0] + vel2 * DY[1] + vel2 * DY[2];
-    if (estab_mode != CFD_ESTAB_REFERENCE) {
+    if (ec.mode != CFD_ESTAB_REFERENCE) {
         dux = 0.0;
         duy = 0.0;
     }
@@ -227,27 +226,27 @@ __global__ void k_estab(int nelem, const int4* __restrict__ elem, const double* 
     double rtx = dtx / dt2, rty = dty / dt2;
     double rjx = drx / dr2, rjy = dry / dr2;
     double rux = dux / du2, ruy = duy / du2;
-    if (estab_mode == CFD_ESTAB_REGULARIZED) {
+    if (ec.mode == CFD_ESTAB_REGULARIZED) {
         // unit vectors continuous in the state: gradient + eps*scale*G_e along the
         // freestream direction, normalised; the velocity-gradient direction is that d
         double ge = 0.0;
         for (int i = 0; i < 3; ++i) ge += sqrt(DX[i] * DX[i] + DY[i] * DY[i]);
-        const double sr = eps_dir * rho_elem * ge;
-        const double st = eps_dir * (div3(t1 + t2 + t3)) * ge;
-        const double gx = drx + sr * dirx, gy = dry + sr * diry;
-        const double hx = dtx + st * dirx, hy = dty + st * diry;
+        const double sr = ec.eps * rho_elem * ge;
+        const double st = ec.eps * (div3(t1 + t2 + t3)) * ge;
+        const double gx = drx + sr * ec.dirx, gy = dry + sr * ec.diry;
+        const double hx = dtx + st * ec.dirx, hy = dty + st * ec.diry;
         const double gn = sqrt(gx * gx + gy * gy), hn = sqrt(hx * hx + hy * hy);
         rjx = gx / gn;
         rjy = gy / gn;
         rtx = hx / hn;
         rty = hy / hn;
-        rux = dirx;
-        ruy = diry;
+        rux = ec.dirx;
+        ruy = ec.diry;
     }
     double temp = div3(t1 + t2 + t3);
-    double c = sqrt(gm * FR * temp);
+    double c = sqrt(gmfr * temp);
     const double smu = 110.0;
-    double fmu = 0.017 * pow15(temp / TINF) * (TINF + smu) / (temp + smu);
+    double fmu = 0.017 * pow15(div_by(temp, ec.t_inf)) * (ec.t_inf.d + smu) / (temp + smu);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         double term1 = fabs(vx * DX[i] + vy * DY[i]);
@@ -268,12 +267,13 @@ __global__ void k_estab(int nelem, const int4* __restrict__ elem, const double* 
     double tr1 = dr2 * h_jgn / rho_elem;
     double zzz = h_jgn / (2.0 * c);
     SHOC[e] = (tr1 + tr1 * tr1) * 0.5 * (c * c) * zzz;
-    double resumen = 1.0 / (tau * tau) + (2.0 / DTMIN) * (2.0 / DTMIN);
+    double resumen = 1.0 / (tau * tau) + sc->two_dt2;
     double rrr = powm05(resumen);
     double s2 = rrr, s3 = rrr;
     if (fmu != 0.0) {
-        double tau_sung3 = (h_rgn * h_rgn) / (4.0 * fmu / RHOINF);
-        double tau_sung3_e = (h_rgne * h_rgne) / (4.0 * fmu / RHOINF);
+        const double nu4 = div_by((4.0 * fmu), ec.rho_inf);
+        double tau_sung3 = (h_rgn * h_rgn) / nu4;
+        double tau_sung3_e = (h_rgne * h_rgne) / nu4;
         s2 = powm05(resumen + 1.0 / (tau_sung3 * tau_sung3));
         s3 = powm05(resumen + 1.0 / (tau_sung3_e * tau_sung3_e));
     }
@@ -497,19 +497,27 @@ __global__ void k_vel_from_U(int npoin, const double* __restrict__ U, double* __
 // K1, K2 and the sums.  Variable 1 (continuity) has no viscous term: its contribution is
 // final after k_elem_inv.
 //
+// The sum's invariant prefix (the addends of the first quadrature point up to its viscous
+// term) is formed here too, and continuity goes to its place in contrib.
+//
 // Cache planes (kInvPlanes, each nelem doubles, plane-major so a warp's loads coalesce):
-constexpr int kC0 = 0;    // [i]        final continuity contribution of local node i
-constexpr int kA1 = 3;    // [k][q-1]   0.5*AiUi_k(q)
-constexpr int kA2 = 12;   // [i][k][q-1] tau_i*(Nx_i*B1_k(q) + Ny_i*B2_k(q))
-constexpr int kA3 = 39;   // [i][q-1]   nu*(Nx_i*Ux(q) + Ny_i*Uy(q))
-constexpr int kV = 48;    // [k][14]    mu-independent factors of K1_k, K2_k (below)
-constexpr int kVG = 90;   // [4]        Ux(1), Uy(1), 3*Ux(4), 3*Uy(4)
-constexpr int kRc = 94;   // [k][2]     RN(1/rho_k), RN(1/(Cv*rho_k)): the replay's quotients
-                          //            by them take div_rcp (bit-identical, fewer FP64 ops)
+constexpr int kP0 = 0;    // [i][q-1]   the sum before the first point's viscous term
+constexpr int kA1 = 9;    // [k-1][q-1] 0.5*AiUi_k(q), k = 2, 3
+constexpr int kA2 = 15;   // [i][k-1][q-1] tau_i*(Nx_i*B1_k(q) + Ny_i*B2_k(q)), k = 2, 3
+constexpr int kA3 = 33;   // [i][q-1]   nu*(Nx_i*Ux(q) + Ny_i*Uy(q))
+constexpr int kV = 42;    // [k][14]    mu-independent factors of K1_k, K2_k (below)
+constexpr int kVG = 84;   // [4]        Ux(1), Uy(1), 3*Ux(4), 3*Uy(4)
+constexpr int kRc = 88;   // [k][4]     RN(1/rho_k), RN(1/(Cv*rho_k)), each with its remainder: the
+                          //            replay's quotients by them take div_rcp2 (the same bits)
 constexpr int kInvPlanes = 100;
 static_assert(kInvPlanes == kElemInvPlanes, "cache planes");
 // kV + 14*k + m: 0 rho, 1 P11, 2 P12, 3 P13a, 4 P13b, 5 P13c, 6 Ux(2)*v1, 7 3*Ux(3)*v2,
 // 8 Cv*rho, 9 P22, 10 P23a, 11 P23b, 12 3*Uy(2)*v1, 13 Uy(3)*v2
+//
+// Both kernels are bound by the FP64 pipe (85% of it).  Kept out of it: the second product of
+// 0.5*a + 0.5*b (the halves are exact: 0.5*(a + b) has the same bits), the divisions by a
+// shared divisor (div_rcp2), and in the replay the prefix of each sum that no stage changes.
+// 1,048,576 nodes: the replay 1,669 us before, 1,514 now; k_elem_inv 3,912 and 3,875 us.
 
 template <bool VISCOUS>
 __global__ void __launch_bounds__(128)
@@ -563,72 +571,85 @@ k_elem_inv(int nelem, const int4* __restrict__ elem, const double* __restrict__ 
         const int ib = (k == 2) ? 1 : 2;
         double Uk[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) Uk[q] = 0.5 * Un[ia][q] + 0.5 * Un[ib][q];
+        for (int q = 0; q < 4; ++q) Uk[q] = 0.5 * (Un[ia][q] + Un[ib][q]);
         const double rho = Uk[0];
-        const double v1 = Uk[1] / rho, v2 = Uk[2] / rho, ev = Uk[3] / rho;
-        const double V_sq = v1 * v1 + v2 * v2;
+        const double rr = 1.0 / rho, rrl = rcp_lo(rho, rr);
+        const double v1 = div_rcp2(Uk[1], rho, rr, rrl), v2 = div_rcp2(Uk[2], rho, rr, rrl),
+                     ev = div_rcp2(Uk[3], rho, rr, rrl);
+        const double v11 = v1 * v1, v22 = v2 * v2;
+        const double V_sq = v11 + v22;
+        const double d11 = 2.0 * v11, d22 = 2.0 * v22, d_ev = 2.0 * ev;
+        const double hV = 0.5 * V_sq;
         double A[4];
         A[0] = Ux[1] + Uy[2];
-        A[1] = 0.5 * Ux[0] * (V_sq * (g - 1.0) - 2.0 * (v1 * v1)) - Ux[1] * v1 * (g - 3.0) -
+        A[1] = 0.5 * Ux[0] * (V_sq * (g - 1.0) - d11) - Ux[1] * v1 * (g - 3.0) -
                Ux[2] * v2 * (g - 1.0) + Ux[3] * (g - 1.0) - Uy[0] * v1 * v2 + Uy[1] * v2 +
                Uy[2] * v1;
         A[2] = -(Ux[0] * v1 * v2) + Ux[1] * v2 + Ux[2] * v1 +
-               0.5 * Uy[0] * (V_sq * (g - 1.0) - 2.0 * (v2 * v2)) - Uy[1] * v1 * (g - 1.0) -
+               0.5 * Uy[0] * (V_sq * (g - 1.0) - d22) - Uy[1] * v1 * (g - 1.0) -
                Uy[2] * v2 * (g - 3.0) + Uy[3] * (g - 1.0);
         A[3] = Ux[0] * v1 * (V_sq * (g - 1.0) - ev * g) -
-               0.5 * Ux[1] * (V_sq * (g - 1.0) - 2.0 * ev * g + 2.0 * (v1 * v1) * (g - 1.0)) -
+               0.5 * Ux[1] * (V_sq * (g - 1.0) - d_ev * g + d11 * (g - 1.0)) -
                Ux[2] * v1 * v2 * (g - 1.0) + Ux[3] * g * v1 +
                Uy[0] * v2 * (V_sq * (g - 1.0) - ev * g) - Uy[1] * v1 * v2 * (g - 1.0) -
-               0.5 * Uy[2] * (V_sq * (g - 1.0) - 2.0 * ev * g + 2.0 * (v2 * v2) * (g - 1.0)) +
+               0.5 * Uy[2] * (V_sq * (g - 1.0) - d_ev * g + d22 * (g - 1.0)) +
                Uy[3] * g * v2;
         const double* At = A;
         double B1[4], B2[4];
         B1[0] = At[1];
         B1[1] = v1 * (-g + 3.0) * At[1] - v2 * (g - 1.0) * At[2] + (g - 1.0) * At[3] +
-                (0.5 * V_sq * (g - 1.0) - v1 * v1) * At[0];
+                (hV * (g - 1.0) - v11) * At[0];
         B1[2] = -(v1 * v2 * At[0]) + v1 * At[2] + v2 * At[1];
         B1[3] = g * v1 * At[3] - v1 * v2 * (g - 1.0) * At[2] +
                 v1 * (V_sq * (g - 1.0) - ev * g) * At[0] +
-                (-(0.5 * V_sq * (g - 1.0)) + ev * g - v1 * v1 * (g - 1.0)) * At[1];
+                (-(hV * (g - 1.0)) + ev * g - v11 * (g - 1.0)) * At[1];
         B2[0] = At[2];
         B2[1] = B1[2];
         B2[2] = -(v1 * (g - 1.0) * At[1]) + v2 * (-g + 3.0) * At[2] + (g - 1.0) * At[3] +
-                (0.5 * V_sq * (g - 1.0) - v2 * v2) * At[0];
+                (hV * (g - 1.0) - v22) * At[0];
         B2[3] = g * v2 * At[3] - v1 * v2 * (g - 1.0) * At[1] +
                 v2 * (V_sq * (g - 1.0) - ev * g) * At[0] +
-                (-(0.5 * V_sq * (g - 1.0)) + ev * g - v2 * v2 * (g - 1.0)) * At[2];
+                (-(hV * (g - 1.0)) + ev * g - v22 * (g - 1.0)) * At[2];
+        double hA[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) hA[q] = 0.5 * A[q];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const double a2 = tau[i] * (Nx[i] * B1[q] + Ny[i] * B2[q]);
-                if (!VISCOUS || q == 0) {
+                if (!VISCOUS || q == 0 || k == 0) {
                     double t = r[i][q];
-                    if (i != k) t = t + 0.5 * A[q];
+                    if (i != k) t = t + hA[q];
                     r[i][q] = t + a2 + a3[i][q];
+                    if (VISCOUS && q > 0) C(kP0 + 3 * i + (q - 1)) = r[i][q];
                 } else {
-                    C(kA2 + 9 * i + 3 * k + (q - 1)) = a2;
+                    C(kA2 + 6 * i + 3 * (k - 1) + (q - 1)) = a2;
                 }
             }
         if (VISCOUS) {
 #pragma unroll
-            for (int q = 1; q < 4; ++q) C(kA1 + 3 * k + (q - 1)) = 0.5 * A[q];
+            for (int q = 1; q < 4; ++q)
+                if (k > 0) C(kA1 + 3 * (k - 1) + (q - 1)) = hA[q];
             // the mu-independent factors of K1_k, K2_k (calcRHS.f90:119-137), each formed
             // exactly as the full expression forms it
+            const double crho = Cv * rho, rc = 1.0 / crho;
             C(kV + 14 * k + 0) = rho;
             C(kV + 14 * k + 1) = -(2.0 * Ux[0] * v1) + 2.0 * Ux[1] + Uy[0] * v2 - Uy[2];
             C(kV + 14 * k + 2) = -(Ux[0] * v2) + Ux[2] - Uy[0] * v1 + Uy[1];
             C(kV + 14 * k + 3) = -(Uy[0] * v1 * v2) + 3.0 * Uy[1] * v2 - 2.0 * Uy[2] * v1;
-            C(kV + 14 * k + 4) = 3.0 * V_sq + v1 * v1;
+            C(kV + 14 * k + 4) = 3.0 * V_sq + v11;
             C(kV + 14 * k + 5) = V_sq - ev;
             C(kV + 14 * k + 6) = Ux[1] * v1;
             C(kV + 14 * k + 7) = 3.0 * Ux[2] * v2;
-            C(kV + 14 * k + 8) = Cv * rho;
-            C(kRc + 2 * k) = 1.0 / rho;
-            C(kRc + 2 * k + 1) = 1.0 / (Cv * rho);
+            C(kV + 14 * k + 8) = crho;
+            C(kRc + 4 * k) = rr;
+            C(kRc + 4 * k + 1) = rc;
+            C(kRc + 4 * k + 2) = rrl;
+            C(kRc + 4 * k + 3) = rcp_lo(crho, rc);
             C(kV + 14 * k + 9) = Ux[0] * v1 - Ux[1] - 2.0 * Uy[0] * v2 + 2.0 * Uy[2];
             C(kV + 14 * k + 10) = -(Ux[0] * v1 * v2) - 2.0 * Ux[1] * v2 + 3.0 * Ux[2] * v1;
-            C(kV + 14 * k + 11) = 3.0 * V_sq + v2 * v2;
+            C(kV + 14 * k + 11) = 3.0 * V_sq + v22;
             C(kV + 14 * k + 12) = 3.0 * Uy[1] * v1;
             C(kV + 14 * k + 13) = Uy[2] * v2;
         }
@@ -636,7 +657,7 @@ k_elem_inv(int nelem, const int4* __restrict__ elem, const double* __restrict__ 
     if (VISCOUS) {
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            C(kC0 + i) = div3(r[i][0] * ar * dtl);
+            contrib[12 * (size_t)e + 4 * i] = div3(r[i][0] * ar * dtl);
 #pragma unroll
             for (int q = 1; q < 4; ++q) C(kA3 + 3 * i + (q - 1)) = a3[i][q];
         }
@@ -679,77 +700,83 @@ k_elem_inv(int nelem, const int4* __restrict__ elem, const double* __restrict__ 
 
 // One RK stage of the viscous calcRHS from the cache: mu, lambda from this stage's T, the
 // K fluxes (calcRHS.f90:119-137 with the cached factors) and the sums replayed in the order
-// of k_elem_rhs; writes all 12 contributions (continuity copied from the cache).
+// of k_elem_rhs; writes the 9 momentum and energy contributions (k_elem_inv wrote continuity's).
+// the replay's launch constants, formed once on the host
+struct ReplayConst {
+    double cv, cv4, mu_ref, lambda_ref, t110, t194;  // cv4 = 4*Cv, t110 = T_inf + 110, ...
+    Rcp t_inf;
+};
 __global__ void __launch_bounds__(128)
 k_elem_replay(int nelem, const int4* __restrict__ elem, const double* __restrict__ T,
               const double* __restrict__ geo, const double* __restrict__ area,
               const double* __restrict__ dtl_arr, const double* __restrict__ dtl_scalar,
-              GasConst gc, const double* __restrict__ cache, double* __restrict__ contrib) {
+              ReplayConst gc, const double* __restrict__ cache, double* __restrict__ contrib) {
     int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nelem) return;
     const size_t E = (size_t)nelem;
     auto C = [&](int plane) -> double { return __ldcs(cache + (size_t)plane * E + e); };
-    const double Cv = gc.cv, lambda_ref = gc.lambda_ref, mu_ref = gc.mu_ref, T_inf = gc.t_inf;
     const int4 n = elem[e];
     const double T_avg = div3(T[n.x] + T[n.y] + T[n.z]);
-    const double mu = mu_ref * pow15(T_avg / T_inf) * (T_inf + 110.0) / (T_avg + 110.0);
-    const double lambda = lambda_ref * pow15(T_avg / T_inf) * (T_inf + 194.0) / (T_avg + 194.0);
+    const double p15 = pow15(div_by(T_avg, gc.t_inf));
+    const double mu = gc.mu_ref * p15 * gc.t110 / (T_avg + 110.0);
+    const double lambda = gc.lambda_ref * p15 * gc.t194 / (T_avg + 194.0);
     const double Nx[3] = {geo[e], geo[E + e], geo[2 * E + e]};
     const double Ny[3] = {geo[3 * E + e], geo[4 * E + e], geo[5 * E + e]};
     const double dtl = dtl_arr ? dtl_arr[e] : *dtl_scalar;
     const double ar = area[e];
     // the mu, lambda subexpressions as calcRHS.f90:119-137 group them
     const double c23m = 2.0 / 3.0 * mu;
-    const double cm = Cv * mu;
+    const double cm = gc.cv * mu;
     const double l3 = 3.0 * lambda;
-    const double c4m_l3 = 4.0 * Cv * mu - 3.0 * lambda;
-    const double cm_l = Cv * mu - lambda;
+    const double c4m_l3 = gc.cv4 * mu - l3;
+    const double cm_l = cm - lambda;
     const double Ux0 = C(kVG + 0), Uy0 = C(kVG + 1);
     const double t5x = C(kVG + 2) * lambda, t5y = C(kVG + 3) * lambda;
     double r[3][3];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int q = 0; q < 3; ++q) r[i][q] = 0.0;
+        for (int q = 0; q < 3; ++q) r[i][q] = C(kP0 + 3 * i + q);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const int b = kV + 14 * k;
         const double rho = C(b + 0);
         const double P13c = C(b + 5);
         const double crho = C(b + 8);
-        const double rr = C(kRc + 2 * k), rc = C(kRc + 2 * k + 1);
+        const double rr = C(kRc + 4 * k), rc = C(kRc + 4 * k + 1);
+        const double rrl = C(kRc + 4 * k + 2), rcl = C(kRc + 4 * k + 3);
         double K1[3], K2[3];
-        K1[0] = div_rcp(c23m * C(b + 1), rho, rr);
-        K1[1] = div_rcp(mu * C(b + 2), rho, rr);
-        K1[2] = div_rcp(1.0 / 3.0 *
+        K1[0] = div_rcp2(c23m * C(b + 1), rho, rr, rrl);
+        K1[1] = div_rcp2(mu * C(b + 2), rho, rr, rrl);
+        K1[2] = div_rcp2(1.0 / 3.0 *
                             (cm * C(b + 3) - Ux0 * (cm * C(b + 4) - l3 * P13c) +
                              C(b + 6) * c4m_l3 + C(b + 7) * cm_l + t5x),
-                        crho, rc);
+                        crho, rc, rcl);
         K2[0] = K1[1];
-        K2[1] = div_rcp(c23m * C(b + 9), rho, rr);
-        K2[2] = div_rcp(1.0 / 3.0 *
+        K2[1] = div_rcp2(c23m * C(b + 9), rho, rr, rrl);
+        K2[2] = div_rcp2(1.0 / 3.0 *
                             (cm * C(b + 10) - Uy0 * (cm * C(b + 11) - l3 * P13c) +
                              C(b + 12) * cm_l + C(b + 13) * c4m_l3 + t5y),
-                        crho, rc);
+                        crho, rc, rcl);
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
                 double t = r[i][q];
-                if (i != k) t = t + C(kA1 + 3 * k + q);
-                t = t + C(kA2 + 9 * i + 3 * k + q) + C(kA3 + 3 * i + q);
+                if (k > 0) {
+                    if (i != k) t = t + C(kA1 + 3 * (k - 1) + q);
+                    t = t + C(kA2 + 6 * i + 3 * (k - 1) + q) + C(kA3 + 3 * i + q);
+                }
                 r[i][q] = t + (Nx[i] * K1[q] + Ny[i] * K2[q]);
             }
     }
     double* out = contrib + 12 * (size_t)e;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        double2 a, b;
-        a.x = C(kC0 + i);
-        a.y = div3(r[i][0] * ar * dtl);
+        out[4 * i + 1] = div3(r[i][0] * ar * dtl);
+        double2 b;
         b.x = div3(r[i][1] * ar * dtl);
         b.y = div3(r[i][2] * ar * dtl);
-        reinterpret_cast<double2*>(out + 4 * i)[0] = a;
         reinterpret_cast<double2*>(out + 4 * i)[1] = b;
     }
 }
@@ -777,91 +804,154 @@ cudaError_t launch_elem_replay(cudaStream_t stream, int nelem, const int4* elem,
                                const double* geo, const double* area, const double* dtl_arr,
                                const double* dtl_scalar, GasConst gc, const double* cache,
                                double* contrib) {
+    const ReplayConst rc{gc.cv,         4.0 * gc.cv,    gc.mu_ref,       gc.lambda_ref,
+                         gc.t_inf + 110.0, gc.t_inf + 194.0, make_rcp(gc.t_inf)};
     k_elem_replay<<<blocks_for(nelem, 128), 128, 0, stream>>>(nelem, elem, T, geo, area, dtl_arr,
-                                                               dtl_scalar, gc, cache, contrib);
+                                                               dtl_scalar, rc, cache, contrib);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------ RK stage, node side
+// drop-in calls accumulate the elements' contributions into the caller's rhs
+__global__ void k_rhs_gather(int npoin, const int* __restrict__ esup_ptr,
+                             const int* __restrict__ esup_slot, const double* __restrict__ contrib,
+                             double* __restrict__ rhs) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= npoin) return;
+    double2* o = reinterpret_cast<double2*>(rhs + 4 * (size_t)p);
+    double2 ra = o[0], rb = o[1];
+    for (int s = esup_ptr[p]; s < esup_ptr[p + 1]; ++s) {
+        const double2* c = reinterpret_cast<const double2*>(contrib + 4 * (size_t)esup_slot[s]);
+        const double2 a = c[0], b = c[1];
+        ra.x = ra.x + a.x;
+        ra.y = ra.y + a.y;
+        rb.x = rb.x + b.x;
+        rb.y = rb.y + b.y;
+    }
+    o[0] = ra;
+    o[1] = rb;
+}
+
 // subrutinas.f90:680-825 for one stage: RHS = ordered sum of the calcRHS then the FUENTE
 // contributions of the node's elements; U1 = U - rk_fact/M*RHS; primitives; FIXVEL,
 // NORMALVEL, FIX (applied per node: every node's list entries are resolved on the host
 // with the reference's last-write-wins order); U1 rebuilt from the primitives.
-__global__ void k_node_update(int npoin, const int* __restrict__ esup_ptr,
-                              const int* __restrict__ esup_slot, const double* __restrict__ contrib,
-                              const double* __restrict__ contribF, const double* __restrict__ U,
-                              const double* __restrict__ M, double rk_fact, double gamm, double FR,
-                              const unsigned char* __restrict__ bcflag,
-                              const double* __restrict__ bcval, const double2* __restrict__ nrm,
-                              const double* __restrict__ WX, const double* __restrict__ WY,
-                              double* __restrict__ U1, double* __restrict__ RHO,
-                              double* __restrict__ VX, double* __restrict__ VY,
-                              double* __restrict__ Eo, double* __restrict__ Po,
-                              double* __restrict__ To, double* __restrict__ RMACH,
-                              const double* __restrict__ rhs_init, double* __restrict__ rhs_out) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= npoin) return;
+//
+// Every stage starts from the step-start U, and of a stage's results the next one reads T
+// alone (through mu, lambda); so stages 1-3 form T and nothing else, and a node with a fixed
+// T needs no update there.  The continuity sum is the same in every stage: stage 1 keeps it
+// (r0), with RN(1/M) (rM) for the quotients rk_fact/M.  FP64-pipe bound: 342 us per stage at
+// 1,048,576 nodes when every stage did the whole; 249 (stage 1), 204 (2, 3) and 244 us (4)
+// now.  64-thread blocks: 8,192 nodes then spread over 128 SMs instead of 32 (17.5 us per
+// stage before, 14 now).
+constexpr int kStageTB = 64;
+template <bool FIRST, bool LAST>
+__global__ void __launch_bounds__(kStageTB) k_node_stage(NodeStageArgs a) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= a.npoin) return;
+    const unsigned char fl = a.bcflag[p];
+    if (!FIRST && !LAST && (fl & BC_FIXT)) {
+        a.T[p] = a.bcval[4 * (size_t)p + 3];
+        return;
+    }
     double r0 = 0.0, r1 = 0.0, r2 = 0.0, r3 = 0.0;
-    if (rhs_init) {  // drop-in calls accumulate into the caller's rhs
-        const double2* c = reinterpret_cast<const double2*>(rhs_init + 4 * (size_t)p);
-        double2 a = c[0], b = c[1];
-        r0 = a.x; r1 = a.y; r2 = b.x; r3 = b.y;
-    }
-    const int s0 = esup_ptr[p], s1 = esup_ptr[p + 1];
-    for (int s = s0; s < s1; ++s) {
-        const double2* c = reinterpret_cast<const double2*>(contrib + 4 * (size_t)esup_slot[s]);
-        double2 a = c[0], b = c[1];
-        r0 = r0 + a.x; r1 = r1 + a.y; r2 = r2 + b.x; r3 = r3 + b.y;
-    }
-    if (contribF) {
-        for (int s = s0; s < s1; ++s) {
-            const double2* c = reinterpret_cast<const double2*>(contribF + 4 * (size_t)esup_slot[s]);
-            double2 a = c[0], b = c[1];
-            r0 = r0 + a.x; r1 = r1 + a.y; r2 = r2 + b.x; r3 = r3 + b.y;
+    const int s0 = a.esup_ptr[p], s1 = a.esup_ptr[p + 1];
+    // slots in batches whose loads go out together; the sums stay in slot order
+    constexpr int B = 3;
+    auto add = [&](const double* __restrict__ c) {
+        for (int s = s0; s < s1; s += B) {
+            double x[B], y[B];
+            double2 zw[B];
+            int id[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) id[u] = a.esup_slot[min(s + u, s1 - 1)];
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                const double* q = c + 4 * (size_t)id[u];
+                if (FIRST) {
+                    const double2 xy = *reinterpret_cast<const double2*>(q);
+                    x[u] = xy.x;
+                    y[u] = xy.y;
+                } else {
+                    y[u] = q[1];
+                }
+                zw[u] = *reinterpret_cast<const double2*>(q + 2);
+            }
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                if (s + u >= s1) break;
+                if (FIRST) r0 = r0 + x[u];
+                r1 = r1 + y[u];
+                r2 = r2 + zw[u].x;
+                r3 = r3 + zw[u].y;
+            }
         }
+    };
+    add(a.contrib);
+    if (a.contribF) add(a.contribF);
+    double rm;
+    if (FIRST) {
+        rm = 1.0 / a.M[p];
+        a.r0[p] = r0;
+        a.rM[p] = rm;
+        if (!LAST && (fl & BC_FIXT)) {
+            a.T[p] = a.bcval[4 * (size_t)p + 3];
+            return;
+        }
+    } else {
+        r0 = a.r0[p];
+        rm = a.rM[p];
     }
-    if (rhs_out) {
-        double2* o = reinterpret_cast<double2*>(rhs_out + 4 * (size_t)p);
-        o[0] = make_double2(r0, r1);
-        o[1] = make_double2(r2, r3);
-    }
-    if (!U1) return;
-    const double2* u2 = reinterpret_cast<const double2*>(U + 4 * (size_t)p);
-    double2 ua = u2[0], ub = u2[1];
-    const double f = rk_fact / M[p];
+    const double2* u2 = reinterpret_cast<const double2*>(a.U + 4 * (size_t)p);
+    const double2 ua = u2[0], ub = u2[1];
+    const double f = div_rcp(a.rk_fact, a.M[p], rm);
     const double u1_0 = ua.x - f * r0, u1_1 = ua.y - f * r1, u1_2 = ub.x - f * r2, u1_3 = ub.y - f * r3;
     double rho = u1_0;
-    double vx = u1_1 / rho, vy = u1_2 / rho, ee = u1_3 / rho;
-    double vel2 = vx * vx + vy * vy;
-    double pp = rho * (gamm - 1.0) * (ee - 0.5 * vel2);
-    double tt = pp / (rho * FR);
-    RMACH[p] = sqrt(vel2 / (tt * gamm * FR));
-    Po[p] = pp;
-    const unsigned char fl = bcflag[p];
+    const double rr = 1.0 / rho, rrl = rcp_lo(rho, rr);
+    double vx = div_rcp2(u1_1, rho, rr, rrl), vy = div_rcp2(u1_2, rho, rr, rrl),
+           ee = div_rcp2(u1_3, rho, rr, rrl);
+    const double vel2 = vx * vx + vy * vy;
+    const double pp = rho * a.gm1 * (ee - 0.5 * vel2);
+    double tt = pp / (rho * a.fr);
+    if (!LAST) {
+        a.T[p] = tt;
+        return;
+    }
+    a.RMACH[p] = sqrt(vel2 / (tt * a.gamm * a.fr));
+    a.P[p] = pp;
     if (fl) {
-        const double2* b2 = reinterpret_cast<const double2*>(bcval + 4 * (size_t)p);
+        const double2* b2 = reinterpret_cast<const double2*>(a.bcval + 4 * (size_t)p);
         const double2 bva = b2[0], bvb = b2[1];
         const double4_32a bv = {bva.x, bva.y, bvb.x, bvb.y};
         if (fl & BC_FIXV) { vx = bv.x; vy = bv.y; }
         if (fl & BC_NORMAL) {
-            double2 nn = nrm[p];
-            double wx = WX[p], wy = WY[p];
+            double2 nn = a.nrm[p];
+            double wx = a.WX[p], wy = a.WY[p];
             double q = -(nn.y * (vx - wx)) + nn.x * (vy - wy);
             vx = -(nn.y * q) + wx;
             vy = nn.x * q + wy;
         }
         if (fl & BC_FIXRHO) rho = bv.z;
         if (fl & BC_FIXT) {
-            double gm = gamm - 1.0;
+            double gm = a.gm1;
             tt = bv.w;
-            ee = tt * FR / gm + 0.5 * (vx * vx + vy * vy);
+            ee = tt * a.fr / gm + 0.5 * (vx * vx + vy * vy);
         }
     }
-    RHO[p] = rho; VX[p] = vx; VY[p] = vy; Eo[p] = ee; To[p] = tt;
-    double2* o = reinterpret_cast<double2*>(U1 + 4 * (size_t)p);
+    a.RHO[p] = rho; a.VX[p] = vx; a.VY[p] = vy; a.E[p] = ee; a.T[p] = tt;
+    double2* o = reinterpret_cast<double2*>(a.U1 + 4 * (size_t)p);
     o[0] = make_double2(rho, vx * rho);
     o[1] = make_double2(vy * rho, ee * rho);
+}
+
+cudaError_t launch_node_stage(cudaStream_t stream, int irk, const NodeStageArgs& a) {
+    const unsigned grid = blocks_for(a.npoin, kStageTB);
+    if (irk == 1) k_node_stage<true, false><<<grid, kStageTB, 0, stream>>>(a);
+    else if (irk < 4) k_node_stage<false, false><<<grid, kStageTB, 0, stream>>>(a);
+    else k_node_stage<false, true><<<grid, kStageTB, 0, stream>>>(a);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------ normales (gather)

@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(256) k_encode(int n, const float* __restrict__
 // 128 x 64: two groups of 256 threads take alternate rows of a 32-row tile, a thread forms
 // 8 x 4 outputs (3 vector loads for 32 FMAs), the next tile's values are loaded while this
 // one is summed.  49,794 nodes: 128 us + 54 us of fold before (2 shared loads per FMA, 64
-// rows per partial, 779 partials folded by one thread each), ~15 us now.
+// rows per partial, 779 partials folded by one thread each), 26-33 us now.
 template <int O, int I>
 __global__ void __launch_bounds__(512)
 k_wgrad(int n, const float* __restrict__ dY, const float* __restrict__ gate,
@@ -711,7 +711,7 @@ __global__ void k_fold(int nq, const float* __restrict__ part, float* __restrict
 //     z = P_i + Q_j + C e_k + c,   agg_i = sum_k relu(z) / max(deg_i, 1);
 // z itself is not kept: the backward pass needs its signs only, 64 bits per edge (bit l of
 // plane b: channel 4 l + b), formed by four ballots.  Before, z was written and read back
-// per edge and channel (76 MB per layer at 49,794 nodes: 76 + 22 us against ~20 us now).
+// per edge and channel (76 MB per layer at 49,794 nodes: 76 + 22 us against 33 us now).
 __global__ void __launch_bounds__(256)
 k_edge_fwd(int n, const int* __restrict__ ptr, const int* __restrict__ nbr,
            const float* __restrict__ PQ, const float* __restrict__ e, const float* __restrict__ C,
@@ -779,7 +779,7 @@ k_edge_fwd(int n, const int* __restrict__ ptr, const int* __restrict__ nbr,
 // so no per-edge gradient is stored.  kTrainChunks blocks, the nodes interleaved over their
 // half-warps; the block's dC, dc go to its row of `part`.  Before: 95 + 53 + 265 + 28 us per
 // layer (the edge gradients written, read by the weight gradient and the node sums, the
-// partials folded by one block); ~25 us now.
+// partials folded by one block); 26 us now.
 __global__ void __launch_bounds__(1024)
 k_edge_bwd(int n, const int* __restrict__ ptr, const int* __restrict__ nbr,
            const int* __restrict__ rev, const ushort4* __restrict__ mask,

@@ -672,11 +672,11 @@ __global__ void k_guess_extrapolate_hist(const double* __restrict__ dtn_p,
     if (blockIdx.x == 0 && threadIdx.x == 0) guess_history(*dtn_p, hist);
 }
 
-// div_rcp against the division x / d over n input pairs: a third raw 64-bit patterns for
+// div_rcp and div_rcp2 against the division x / d over n input pairs: a third raw 64-bit patterns for
 // both (splitmix64: every exponent and sign, zeros, subnormals, infinities, NaNs), a third
 // with both of magnitude 2^-60 .. 2^60, a third with x = d * m for a random significand m
 // moved by up to +-2^12 ulps (quotients next to binade edges and to halfway cases).  Counts
-// the pairs whose results differ in any bit (two NaNs count as equal).
+// the pairs whose results differ in any bit (NaNs count as equal).
 __device__ __forceinline__ unsigned long long splitmix(unsigned long long z) {
     z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
     z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
@@ -704,7 +704,11 @@ __global__ void k_selftest_divrcp(long long n, unsigned long long seed,
         const double x = __longlong_as_double((long long)bx), d = __longlong_as_double((long long)bd);
         const double y = 1.0 / d;
         const double a = div_rcp(x, d, y), b = x / d;
-        if (__double_as_longlong(a) != __double_as_longlong(b) && !(a != a && b != b)) ++local;
+        const double c = div_rcp2(x, d, y, rcp_lo(d, y));
+        const bool nan = a != a && b != b && c != c;
+        if ((__double_as_longlong(a) != __double_as_longlong(b) ||
+             __double_as_longlong(c) != __double_as_longlong(b)) && !nan)
+            ++local;
     }
     if (local) atomicAdd(bad, local);
 }
