@@ -25,6 +25,7 @@ UNITS = [
     ("kernels_pcg_mixed.cu", []),
     ("context.cu", ["--fmad=false"]),
     ("abi.cu", ["--fmad=false"]),
+    ("hostmesh.cu", []),
     ("noalloc.cu", ["--fmad=false"]),
     ("kernels_mpnn.cu", []),
     ("mpnn.cu", []),

@@ -4,6 +4,8 @@
 // same kernels the resident context uses and copy the results back.  Every call checks
 // its arguments and returns a status; nothing here falls back to the CPU.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <cmath>
 #include <cstring>
@@ -17,39 +19,85 @@ using namespace cfd;
 
 namespace {
 
-// device buffers freed at scope exit
+constexpr int kPopulateWrite = 23;  // MADV_POPULATE_WRITE, which older headers lack
+
+// A call's device buffers, freed at scope exit.  init(bytes) takes them as one allocation, which
+// alloc() cuts up (a cudaMalloc and its cudaFree cost ~70 us together on GB300, and a call has up
+// to 17 buffers: 1.0 ms of them in calcRHS at 262,144 nodes, 0.12 ms as one); what does not fit
+// takes an allocation of its own.
 struct Scratch {
     std::vector<void*> ptrs;
-    cudaStream_t stream = nullptr;
+    cudaStream_t stream = nullptr, stream2 = nullptr;  // stream2: fork()
+    cudaEvent_t ev = nullptr;
+    char* at = nullptr;
+    size_t left = 0;
     ~Scratch() {
-        if (stream) {
-            cudaStreamSynchronize(stream);
-            cudaStreamDestroy(stream);
-        }
+        for (cudaStream_t q : {stream, stream2})
+            if (q) {
+                cudaStreamSynchronize(q);
+                cudaStreamDestroy(q);
+            }
+        if (ev) cudaEventDestroy(ev);
         for (void* p : ptrs) cudaFree(p);
     }
-    int init() {
+    int init(size_t bytes = 0) {
         CFD_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        if (bytes) {
+            bytes += 32 * 256;  // the roundings of up to 32 buffers
+            CFD_CUDA(cudaMalloc((void**)&at, bytes));
+            ptrs.push_back(at);
+            left = bytes;
+        }
         return CFD_OK;
     }
     template <class T>
     int alloc(T** p, size_t n) {
+        const size_t bytes = ((n ? n : 1) * sizeof(T) + 255) / 256 * 256;
+        if (bytes <= left) {
+            *p = (T*)at;
+            at += bytes;
+            left -= bytes;
+            return CFD_OK;
+        }
         void* v = nullptr;
-        CFD_CUDA(cudaMalloc(&v, (n ? n : 1) * sizeof(T)));
+        CFD_CUDA(cudaMalloc(&v, bytes));
         ptrs.push_back(v);
         *p = (T*)v;
         return CFD_OK;
     }
     template <class T>
-    int put(T** p, const T* h, size_t n) {
-        int st = alloc(p, n);
-        if (st) return st;
-        if (n) CFD_CUDA(cudaMemcpyAsync(*p, h, n * sizeof(T), cudaMemcpyHostToDevice, stream));
+    int copy(T* d, const T* h, size_t n) {
+        if (n) CFD_CUDA(cudaMemcpyAsync(d, h, n * sizeof(T), cudaMemcpyHostToDevice, stream));
         return CFD_OK;
     }
     template <class T>
+    int put(T** p, const T* h, size_t n) {
+        int st = alloc(p, n);
+        return st ? st : copy(*p, h, n);
+    }
+    // A large result's pages are mapped first (contents kept; a kernel that does not know the
+    // advice refuses it, which changes nothing): the device's copy into pages that the host has
+    // not touched yet, a fresh calloc's, faults on each of them (four arrays of 4 MB: 12 ms, 0.6 ms now).
+    template <class T>
     int get(T* h, const T* d, size_t n) {
+        const uintptr_t page = sysconf(_SC_PAGESIZE), a = (uintptr_t)h / page * page, b = (uintptr_t)(h + n);
+        if (n * sizeof(T) >= 16 * page) (void)madvise((void*)a, (b - a + page - 1) / page * page, kPopulateWrite);
         if (n) CFD_CUDA(cudaMemcpyAsync(h, d, n * sizeof(T), cudaMemcpyDeviceToHost, stream));
+        return CFD_OK;
+    }
+    // stream2 goes on after what stream has been given so far / the other way round
+    int fork() {
+        if (!stream2) {
+            CFD_CUDA(cudaStreamCreateWithFlags(&stream2, cudaStreamNonBlocking));
+            CFD_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        }
+        CFD_CUDA(cudaEventRecord(ev, stream));
+        CFD_CUDA(cudaStreamWaitEvent(stream2, ev, 0));
+        return CFD_OK;
+    }
+    int join() {
+        CFD_CUDA(cudaEventRecord(ev, stream2));
+        CFD_CUDA(cudaStreamWaitEvent(stream, ev, 0));
         return CFD_OK;
     }
     int sync() {
@@ -108,15 +156,67 @@ void make_esup(const int* inpoel, int nelem, int npoin, std::vector<int>& ptr, s
         for (int i = 0; i < 3; ++i) slot[fill[inpoel[3 * e + i] - 1]++] = (int)(3 * e + i);
 }
 
-// dNx(3,nelem), dNy(3,nelem) -> [dNx1|dNx2|dNx3|dNy1|dNy2|dNy3]
-std::vector<double> to_geo(const double* dNx, const double* dNy, int nelem) {
-    std::vector<double> g(6 * (size_t)nelem);
-    for (int e = 0; e < nelem; ++e)
-        for (int i = 0; i < 3; ++i) {
-            g[i * (size_t)nelem + e] = dNx[3 * e + i];
-            g[(3 + i) * (size_t)nelem + e] = dNy[3 * e + i];
+// A host caller's inpoel on the device: the element table, and with `around` the elements around
+// each point.  begin() queues the work; check() waits for it and refuses an index outside
+// 1..npoin, so it comes before the first kernel that reads the tables and before any result is
+// copied out.
+struct HostMesh {
+    int4* el = nullptr;
+    int *ptr = nullptr, *slot = nullptr;
+
+    static size_t bytes(int nelem, int npoin, bool around) {
+        size_t n = (12 + 16) * (size_t)nelem;
+        if (around) n += 24 * (size_t)nelem + 8 * (size_t)npoin + 4 * (size_t)esup_scan_blocks(npoin);
+        return n;
+    }
+    int begin(Scratch& s, const int* inpoel, int nelem, int npoin, bool around) {
+        int *d_in, *deg = nullptr, *rank = nullptr, *sums;
+        TRY(s.alloc(&flags, 2));
+        CFD_CUDA(cudaMemsetAsync(flags, 0xff, 2 * sizeof(unsigned), s.stream));
+        TRY(s.put(&d_in, inpoel, 3 * (size_t)nelem));
+        TRY(s.alloc(&el, nelem));
+        if (around) {
+            TRY(s.alloc(&deg, npoin));
+            TRY(s.alloc(&rank, 3 * (size_t)nelem));
+            TRY(s.alloc(&ptr, npoin + 1));
+            TRY(s.alloc(&slot, 3 * (size_t)nelem));
+            TRY(s.alloc(&sums, esup_scan_blocks(npoin)));
+            CFD_CUDA(cudaMemsetAsync(deg, 0, sizeof(int) * npoin, s.stream));
         }
-    return g;
+        CFD_CUDA(launch_elem_table(s.stream, nelem, npoin, d_in, el, deg, rank, flags));
+        if (around)
+            CFD_CUDA(launch_esup(s.stream, nelem, npoin, el, deg, rank, sums, ptr, slot, flags));
+        return CFD_OK;
+    }
+    int check(Scratch& s, const int* inpoel, int nelem, int npoin) {
+        unsigned f[2];
+        TRY(s.get(f, flags, 2));
+        TRY(s.sync());
+        if (f[0] != ~0u) {
+            set_last_message("inpoel(:," + std::to_string((long)f[0] + 1) + ") outside 1..npoin");
+            return CFD_ERR_MESH;
+        }
+        if (slot && ~f[1] > (unsigned)kEsupSortMax) {  // a fan: one thread would sort for long
+            std::vector<int> hp, hs;
+            make_esup(inpoel, nelem, npoin, hp, hs);
+            TRY(s.copy(slot, hs.data(), hs.size()));
+            TRY(s.sync());
+        }
+        return CFD_OK;
+    }
+
+private:
+    unsigned* flags = nullptr;
+};
+
+// dNx(3,nelem), dNy(3,nelem) in the kernels' planes
+int put_geo(Scratch& s, double** geo, const double* dNx, const double* dNy, int nelem) {
+    double *dx, *dy;
+    TRY(s.put(&dx, dNx, 3 * (size_t)nelem));
+    TRY(s.put(&dy, dNy, 3 * (size_t)nelem));
+    TRY(s.alloc(geo, 6 * (size_t)nelem));
+    CFD_LAUNCH(k_geo_planes, blocks_for(nelem, 256), 256, 0, s.stream, 0, nelem, nelem, dx, dy, *geo);
+    return CFD_OK;
 }
 
 bool bad_sizes(const int* nelem, const int* npoin) {
@@ -613,6 +713,11 @@ int cfd_laplace_pattern(const int* inpoel, const int* nelem, const int* npoin, i
 }
 
 // ------------------------------------------------------------------ drop-in routines
+// calcRHS's smallest piece, in elements.  A copy costs ~10 us whatever its size, eight of them a
+// piece: at 523,264 elements four pieces take 2.2 ms, eight 2.3, sixteen 2.4, and one after
+// the other without pieces ~2.6.
+constexpr int kRhsPiece = 1 << 16;
+
 int cfd_calcrhs(double* rhs, const double* U, const double* theta, const double* dNx,
                 const double* dNy, const double* area, const double* shoc, const double* dtl,
                 const double* t_sugn1, const double* t_sugn2, const double* t_sugn3,
@@ -622,38 +727,44 @@ int cfd_calcrhs(double* rhs, const double* U, const double* theta, const double*
         !t_sugn3 || !inpoel || !T || !gas6 || bad_sizes(nelem, npoin))
         return arg_error("cfd_calcrhs");
     const int E = *nelem, N = *npoin;
-    std::vector<int4> el;
-    TRY(make_elems(inpoel, E, N, el));
-    std::vector<int> ptr, slot;
-    make_esup(inpoel, E, N, ptr, slot);
-    std::vector<double> geo = to_geo(dNx, dNy, E);
     Scratch s;
-    TRY(s.init());
-    int4* d_el; int *d_ptr, *d_slot;
-    double *d_U, *d_th = nullptr, *d_geo, *d_area, *d_shoc, *d_dtl, *d_t1, *d_t2, *d_t3, *d_T,
-           *d_rhs, *d_c;
-    TRY(s.put(&d_el, el.data(), E));
-    TRY(s.put(&d_ptr, ptr.data(), N + 1));
-    TRY(s.put(&d_slot, slot.data(), 3 * (size_t)E));
+    TRY(s.init(HostMesh::bytes(E, N, true) + 8 * (30 * (size_t)E + (theta ? 13 : 9) * (size_t)N)));
+    HostMesh m;
+    TRY(m.begin(s, inpoel, E, N, true));
+    double *d_U, *d_th = nullptr, *d_dnx, *d_dny, *d_geo, *d_T, *d_rhs, *d_c;
     TRY(s.put(&d_U, U, 4 * (size_t)N));
     if (theta) TRY(s.put(&d_th, theta, 4 * (size_t)N));
-    TRY(s.put(&d_geo, geo.data(), 6 * (size_t)E));
-    TRY(s.put(&d_area, area, E));
-    TRY(s.put(&d_shoc, shoc, E));
-    TRY(s.put(&d_dtl, dtl, E));
-    TRY(s.put(&d_t1, t_sugn1, E));
-    TRY(s.put(&d_t2, t_sugn2, E));
-    TRY(s.put(&d_t3, t_sugn3, E));
     TRY(s.put(&d_T, T, N));
-    TRY(s.put(&d_rhs, rhs, 4 * (size_t)N));
+    TRY(m.check(s, inpoel, E, N));
+    TRY(s.alloc(&d_dnx, 3 * (size_t)E));
+    TRY(s.alloc(&d_dny, 3 * (size_t)E));
+    TRY(s.alloc(&d_geo, 6 * (size_t)E));
     TRY(s.alloc(&d_c, 12 * (size_t)E));
+    const double* h[6] = {area, shoc, dtl, t_sugn1, t_sugn2, t_sugn3};
+    double* d[6];
+    for (double*& q : d) TRY(s.alloc(&q, E));
     GasConst gc{gas6[0], gas6[1], gas6[2], gas6[3], gas6[4], gas6[5]};
     const bool visc = gc.mu_ref > 2.2250738585072014e-308;
     const double* nd = nullptr;
     double* ndo = nullptr;
-    CFD_CUDA(launch_elem_rhs(visc, theta != nullptr, s.stream, E, d_el, d_U, d_th, d_T, d_geo,
-                             d_area, d_shoc, d_dtl, nd, d_t1, d_t2, d_t3, gc, d_c, nd, nd, ndo));
-    CFD_LAUNCH(k_rhs_gather, blocks_for(N, 256), 256, 0, s.stream, N, d_ptr, d_slot, d_c, d_rhs);
+    // The element arrays come over in pieces, and a piece's element pass runs on stream2 while the
+    // next is copied (a copy from pageable memory returns when it is done).  The first is half as
+    // large: nothing runs beside its copy.
+    const int piece = std::max(kRhsPiece, (E + 3) / 4);
+    for (int e0 = 0, e1; e0 < E; e0 = e1) {
+        const int n = std::min(e0 ? piece : piece / 2, E - e0);
+        e1 = e0 + n;
+        TRY(s.copy(d_dnx + 3 * (size_t)e0, dNx + 3 * (size_t)e0, 3 * (size_t)n));
+        TRY(s.copy(d_dny + 3 * (size_t)e0, dNy + 3 * (size_t)e0, 3 * (size_t)n));
+        for (int k = 0; k < 6; ++k) TRY(s.copy(d[k] + e0, h[k] + e0, n));
+        TRY(s.fork());
+        CFD_LAUNCH(k_geo_planes, blocks_for(n, 256), 256, 0, s.stream2, e0, e1, E, d_dnx, d_dny, d_geo);
+        CFD_CUDA(launch_elem_rhs(visc, theta != nullptr, s.stream2, e0, e1, E, m.el, d_U, d_th, d_T,
+                                 d_geo, d[0], d[1], d[2], nd, d[3], d[4], d[5], gc, d_c, nd, nd, ndo));
+    }
+    TRY(s.put(&d_rhs, rhs, 4 * (size_t)N));
+    TRY(s.join());
+    CFD_LAUNCH(k_rhs_gather, blocks_for(N, 256), 256, 0, s.stream, N, m.ptr, m.slot, d_c, d_rhs);
     TRY(s.get(rhs, d_rhs, 4 * (size_t)N));
     return s.sync();
 }
@@ -665,32 +776,26 @@ int cfd_fuente(double* rhs, const double* U, const double* W_X, const double* W_
         bad_sizes(nelem, npoin))
         return arg_error("cfd_fuente");
     const int E = *nelem, N = *npoin;
-    std::vector<int4> el;
-    TRY(make_elems(inpoel, E, N, el));
-    std::vector<int> ptr, slot;
-    make_esup(inpoel, E, N, ptr, slot);
-    std::vector<double> geo = to_geo(dNx, dNy, E);
     Scratch s;
-    TRY(s.init());
-    int4* d_el; int *d_ptr, *d_slot;
+    TRY(s.init(HostMesh::bytes(E, N, true) + 8 * (26 * (size_t)E + 10 * (size_t)N)));
+    HostMesh m;
+    TRY(m.begin(s, inpoel, E, N, true));
     double *d_U, *d_wx, *d_wy, *d_geo, *d_area, *d_dtl, *d_rhs, *d_f;
-    TRY(s.put(&d_el, el.data(), E));
-    TRY(s.put(&d_ptr, ptr.data(), N + 1));
-    TRY(s.put(&d_slot, slot.data(), 3 * (size_t)E));
     TRY(s.put(&d_U, U, 4 * (size_t)N));
     TRY(s.put(&d_wx, W_X, N));
     TRY(s.put(&d_wy, W_Y, N));
-    TRY(s.put(&d_geo, geo.data(), 6 * (size_t)E));
+    TRY(put_geo(s, &d_geo, dNx, dNy, E));
     TRY(s.put(&d_area, area, E));
     TRY(s.put(&d_dtl, dtl, E));
     TRY(s.put(&d_rhs, rhs, 4 * (size_t)N));
     TRY(s.alloc(&d_f, 12 * (size_t)E));
+    TRY(m.check(s, inpoel, E, N));
     GasConst gc{};
     const double* nd = nullptr;
     double* ndo = nullptr;
-    CFD_CUDA(launch_elem_rhs(false, false, s.stream, E, d_el, d_U, nd, nd, d_geo, d_area, nd, d_dtl,
+    CFD_CUDA(launch_elem_rhs(false, false, s.stream, 0, E, E, m.el, d_U, nd, nd, d_geo, d_area, nd, d_dtl,
                              nd, nd, nd, nd, gc, ndo, d_wx, d_wy, d_f));
-    CFD_LAUNCH(k_rhs_gather, blocks_for(N, 256), 256, 0, s.stream, N, d_ptr, d_slot, d_f, d_rhs);
+    CFD_LAUNCH(k_rhs_gather, blocks_for(N, 256), 256, 0, s.stream, N, m.ptr, m.slot, d_f, d_rhs);
     TRY(s.get(rhs, d_rhs, 4 * (size_t)N));
     return s.sync();
 }
@@ -704,15 +809,12 @@ int cfd_estab(const double* U, const double* T, const double* GAMM, const double
         !scal5 || !SHOC || !T_SUGN1 || !T_SUGN2 || !T_SUGN3 || bad_sizes(nelem, npoin))
         return arg_error("cfd_estab");
     const int E = *nelem, N = *npoin;
-    std::vector<int4> el;
-    TRY(make_elems(inpoel, E, N, el));
-    std::vector<double> geo = to_geo(dNx, dNy, E);
     Scratch s;
-    TRY(s.init());
-    int4* d_el;
+    TRY(s.init(HostMesh::bytes(E, N, false) + 8 * (16 * (size_t)E + 10 * (size_t)N)));
+    HostMesh m;
+    TRY(m.begin(s, inpoel, E, N, false));
     double *d_U, *d_T, *d_G, *d_vx, *d_vy, *d_wx, *d_wy, *d_geo, *o[4];
     StepScal* d_sc;
-    TRY(s.put(&d_el, el.data(), E));
     TRY(s.put(&d_U, U, 4 * (size_t)N));
     TRY(s.put(&d_T, T, N));
     TRY(s.put(&d_G, GAMM, N));
@@ -720,13 +822,14 @@ int cfd_estab(const double* U, const double* T, const double* GAMM, const double
     TRY(s.put(&d_vy, VEL_Y, N));
     TRY(s.put(&d_wx, W_X, N));
     TRY(s.put(&d_wy, W_Y, N));
-    TRY(s.put(&d_geo, geo.data(), 6 * (size_t)E));
+    TRY(put_geo(s, &d_geo, dNx, dNy, E));
     for (int i = 0; i < 4; ++i) TRY(s.alloc(&o[i], E));
+    TRY(m.check(s, inpoel, E, N));
     StepScal sc{};
     sc.dtmin = scal5[2];
     sc.two_dt2 = (2.0 / scal5[2]) * (2.0 / scal5[2]);
     TRY(s.put(&d_sc, &sc, 1));
-    CFD_LAUNCH(k_estab, blocks_for(E, 128), 128, 0, s.stream, E, d_el, d_U, d_T, d_G, d_vx, d_vy,
+    CFD_LAUNCH(k_estab, blocks_for(E, 128), 128, 0, s.stream, E, m.el, d_U, d_T, d_G, d_vx, d_vy,
                d_wx, d_wy, d_geo,
                estab_args(scal5[0], scal5[1], scal5[3], scal5[4], CFD_ESTAB_REFERENCE, 0.0, 1.0, 0.0),
                d_sc, o[0], o[1], o[2], o[3]);
@@ -744,14 +847,12 @@ int cfd_deltat(const double* T, const double* VEL_X, const double* VEL_Y, const 
         bad_sizes(nelem, npoin))
         return arg_error("cfd_deltat");
     const int E = *nelem, N = *npoin;
-    std::vector<int4> el;
-    TRY(make_elems(inpoel, E, N, el));
     Scratch s;
-    TRY(s.init());
-    int4* d_el;
+    TRY(s.init(HostMesh::bytes(E, N, false) + 8 * (2 * (size_t)E + 5 * (size_t)N)));
+    HostMesh m;
+    TRY(m.begin(s, inpoel, E, N, false));
     double *d_T, *d_vx, *d_vy, *d_wx, *d_wy, *d_a, *d_DT;
     StepScal* d_sc;
-    TRY(s.put(&d_el, el.data(), E));
     TRY(s.put(&d_T, T, N));
     TRY(s.put(&d_vx, VEL_X, N));
     TRY(s.put(&d_vy, VEL_Y, N));
@@ -763,7 +864,8 @@ int cfd_deltat(const double* T, const double* VEL_X, const double* VEL_Y, const 
     sc.dtmin_bits = 0x7ff0000000000000ull;
     sc.bandera = 1;
     TRY(s.put(&d_sc, &sc, 1));
-    CFD_LAUNCH(k_deltat, blocks_for(E, 256), 256, 0, s.stream, E, d_el, d_T, d_vx, d_vy, d_wx, d_wy, d_a,
+    TRY(m.check(s, inpoel, E, N));
+    CFD_LAUNCH(k_deltat, blocks_for(E, 256), 256, 0, s.stream, E, m.el, d_T, d_vx, d_vy, d_wx, d_wy, d_a,
                scal4[0], make_rcp(scal4[3]), d_DT, &d_sc->dtmin_bits);
     CFD_LAUNCH(k_dt_finalize, 1, 1, 0, s.stream, d_sc);
     CFD_LAUNCH(k_dt_clamp, blocks_for(E, 256), 256, 0, s.stream, E, d_DT, d_sc);
@@ -909,14 +1011,12 @@ int cfd_deriv(const double* X, const double* Y, const int* inpoel, const int* ne
         bad_sizes(nelem, npoin))
         return arg_error("cfd_deriv");
     const int E = *nelem, N = *npoin;
-    std::vector<int4> el;
-    TRY(make_elems(inpoel, E, N, el));
     Scratch s;
-    TRY(s.init());
-    int4* d_el;
-    double *d_X, *d_Y, *d_a, *d_geo, *d_hh, *d_hx, *d_hy;
+    TRY(s.init(HostMesh::bytes(E, N, false) + 8 * (16 * (size_t)E + 2 * (size_t)N)));
+    HostMesh m;
+    TRY(m.begin(s, inpoel, E, N, false));
+    double *d_X, *d_Y, *d_a, *d_geo, *d_hh, *d_hx, *d_hy, *d_dnx, *d_dny;
     unsigned long long* d_bits;
-    TRY(s.put(&d_el, el.data(), E));
     TRY(s.put(&d_X, X, N));
     TRY(s.put(&d_Y, Y, N));
     TRY(s.alloc(&d_a, E));
@@ -924,24 +1024,23 @@ int cfd_deriv(const double* X, const double* Y, const int* inpoel, const int* ne
     TRY(s.alloc(&d_hh, E));
     TRY(s.alloc(&d_hx, E));
     TRY(s.alloc(&d_hy, E));
+    TRY(s.alloc(&d_dnx, 3 * (size_t)E));
+    TRY(s.alloc(&d_dny, 3 * (size_t)E));
     unsigned long long inf = 0x7ff0000000000000ull;
     TRY(s.put(&d_bits, &inf, 1));
-    CFD_LAUNCH(k_deriv, blocks_for(E, 256), 256, 0, s.stream, E, d_el, d_X, d_Y, d_a, d_geo, d_hh, d_hx, d_hy);
+    TRY(m.check(s, inpoel, E, N));
+    CFD_LAUNCH(k_deriv, blocks_for(E, 256), 256, 0, s.stream, E, m.el, d_X, d_Y, d_a, d_geo, d_hh, d_hx, d_hy);
     CFD_LAUNCH(k_min_positive, 152, 256, 0, s.stream, (long)E, d_hh, d_bits);
-    std::vector<double> geo(6 * (size_t)E);
+    CFD_LAUNCH(k_geo_rows, blocks_for(E, 256), 256, 0, s.stream, E, d_geo, d_dnx, d_dny);
     TRY(s.get(area, d_a, E));
-    TRY(s.get(geo.data(), d_geo, 6 * (size_t)E));
+    TRY(s.get(dNx, d_dnx, 3 * (size_t)E));
+    TRY(s.get(dNy, d_dny, 3 * (size_t)E));
     TRY(s.get(HH, d_hh, E));
     TRY(s.get(HHX, d_hx, E));
     TRY(s.get(HHY, d_hy, E));
     unsigned long long bits = 0;
     TRY(s.get(&bits, d_bits, 1));
     TRY(s.sync());
-    for (int e = 0; e < E; ++e)
-        for (int i = 0; i < 3; ++i) {
-            dNx[3 * e + i] = geo[i * (size_t)E + e];
-            dNy[3 * e + i] = geo[(3 + i) * (size_t)E + e];
-        }
     double h;
     std::memcpy(&h, &bits, sizeof(h));
     if (h > 1.0e10) h = 1.0e10;  // subrutinas.f90:125 (also when no element is positive)
@@ -952,19 +1051,15 @@ int cfd_deriv(const double* X, const double* Y, const int* inpoel, const int* ne
 int cfd_masas(const double* area, const int* inpoel, const int* nelem, const int* npoin, double* M) {
     if (!area || !inpoel || !M || bad_sizes(nelem, npoin)) return arg_error("cfd_masas");
     const int E = *nelem, N = *npoin;
-    std::vector<int4> el;
-    TRY(make_elems(inpoel, E, N, el));
-    std::vector<int> ptr, slot;
-    make_esup(inpoel, E, N, ptr, slot);
     Scratch s;
-    TRY(s.init());
-    int *d_ptr, *d_slot;
+    TRY(s.init(HostMesh::bytes(E, N, true) + 8 * ((size_t)E + (size_t)N)));
+    HostMesh m;
+    TRY(m.begin(s, inpoel, E, N, true));
     double *d_a, *d_M;
-    TRY(s.put(&d_ptr, ptr.data(), N + 1));
-    TRY(s.put(&d_slot, slot.data(), 3 * (size_t)E));
     TRY(s.put(&d_a, area, E));
     TRY(s.alloc(&d_M, N));
-    CFD_LAUNCH(k_mass, blocks_for(N, 256), 256, 0, s.stream, N, d_ptr, d_slot, d_a, d_M);
+    TRY(m.check(s, inpoel, E, N));
+    CFD_LAUNCH(k_mass, blocks_for(N, 256), 256, 0, s.stream, N, m.ptr, m.slot, d_a, d_M);
     TRY(s.get(M, d_M, N));
     return s.sync();
 }
@@ -978,30 +1073,24 @@ int cfd_gcl(double* M, const double* W_x, const double* W_y, const double* W_x_o
         return arg_error("cfd_gcl");
     if (mode != CFD_MASS_GCL_LITERAL && mode != CFD_MASS_GCL_CORRECTED) return arg_error("mode");
     const int E = *nelem, N = *npoin;
-    std::vector<int4> el;
-    TRY(make_elems(inpoel, E, N, el));
-    std::vector<int> ptr, slot;
-    make_esup(inpoel, E, N, ptr, slot);
-    std::vector<double> geo = to_geo(dNx, dNy, E);
     Scratch s;
-    TRY(s.init());
-    int4* d_el; int *d_ptr, *d_slot;
+    TRY(s.init(HostMesh::bytes(E, N, true) + 8 * (16 * (size_t)E + 5 * (size_t)N)));
+    HostMesh m;
+    TRY(m.begin(s, inpoel, E, N, true));
     double *d_M, *d_wx, *d_wy, *d_wxo, *d_wyo, *d_geo, *d_a, *d_ao, *d_dt;
-    TRY(s.put(&d_el, el.data(), E));
-    TRY(s.put(&d_ptr, ptr.data(), N + 1));
-    TRY(s.put(&d_slot, slot.data(), 3 * (size_t)E));
     TRY(s.put(&d_M, M, N));
     TRY(s.put(&d_wx, W_x, N));
     TRY(s.put(&d_wy, W_y, N));
     TRY(s.put(&d_wxo, W_x_old, N));
     TRY(s.put(&d_wyo, W_y_old, N));
-    TRY(s.put(&d_geo, geo.data(), 6 * (size_t)E));
+    TRY(put_geo(s, &d_geo, dNx, dNy, E));
     TRY(s.put(&d_a, area, E));
     TRY(s.put(&d_ao, area_old, E));
     TRY(s.put(&d_dt, dt, 1));
     double2* d_terms;
     TRY(s.alloc(&d_terms, E));
-    CFD_CUDA(launch_gcl(s.stream, N, E, d_el, d_ptr, d_slot, d_geo, d_a, d_ao, d_wx, d_wy, d_wxo,
+    TRY(m.check(s, inpoel, E, N));
+    CFD_CUDA(launch_gcl(s.stream, N, E, m.el, m.ptr, m.slot, d_geo, d_a, d_ao, d_wx, d_wy, d_wxo,
                         d_wyo, d_dt, mode == CFD_MASS_GCL_LITERAL ? 1 : 0, d_terms, d_M));
     TRY(s.get(M, d_M, N));
     return s.sync();
@@ -1041,10 +1130,9 @@ int cfd_laplace(const int* inpoel, const double* area, const double* dNx, const 
             pos[s2] = make_uchar4(o[0], o[1], o[2], 0);
         }
     }
-    std::vector<double> geo = to_geo(dNx, dNy, E);
     const int nnz = lap_rowptr[N];
     Scratch s;
-    TRY(s.init());
+    TRY(s.init(8 * (23 * (size_t)E + 4 * (size_t)N + (size_t)nnz)));
     int4* d_el; int *d_ptr, *d_slot, *d_rp;
     uchar4* d_pos;
     double *d_geo, *d_X, *d_Y, *d_v, *d_d;
@@ -1053,7 +1141,7 @@ int cfd_laplace(const int* inpoel, const double* area, const double* dNx, const 
     TRY(s.put(&d_slot, slot.data(), 3 * (size_t)E));
     TRY(s.put(&d_pos, pos.data(), 3 * (size_t)E));
     TRY(s.put(&d_rp, lap_rowptr, N + 1));
-    TRY(s.put(&d_geo, geo.data(), 6 * (size_t)E));
+    TRY(put_geo(s, &d_geo, dNx, dNy, E));
     TRY(s.put(&d_X, X, N));
     TRY(s.put(&d_Y, Y, N));
     TRY(s.alloc(&d_v, nnz));
@@ -1078,14 +1166,6 @@ int cfd_bicg_mode(const double* spMtx, const int* spIdx, const int* spRowptr,
     const int N = *npoin, NF = *nfix;
     const int nnz = spRowptr[N];
     if (spRowptr[0] != 0 || nnz < 0) return arg_error("spRowptr");
-    std::vector<int> col(nnz);
-    for (int k = 0; k < nnz; ++k) {
-        if (spIdx[k] < 1 || spIdx[k] > N) {
-            set_last_message("spIdx outside 1..npoin");
-            return CFD_ERR_MESH;
-        }
-        col[k] = spIdx[k] - 1;
-    }
     std::vector<unsigned char> isfix(N, 0);
     std::vector<int> last(N, -1);
     for (int k = 0; k < NF; ++k) {
@@ -1103,13 +1183,21 @@ int cfd_bicg_mode(const double* spMtx, const int* spIdx, const int* spRowptr,
             usrc.push_back(last[p]);
         }
     Scratch s;
-    TRY(s.init());
-    int *d_rp, *d_col, *d_un, *d_us, *d_it, *d_cv;
+    const long nc = ((long)N + kChunk - 1) / kChunk;
+    TRY(s.init(16 * (size_t)nnz + 73 * (size_t)N + 16 * (size_t)NF + 48 * (size_t)nc + 4096));
+    int *d_rp, *d_in, *d_col, *d_un, *d_us, *d_it, *d_cv;
+    unsigned *d_bad, bad;
     unsigned char* d_isfix;
     double *d_val, *d_diag, *d_rdiag, *d_x, *d_b, *d_fv, *d_r, *d_z, *d_y, *d_p0, *d_part, *d_rz;
     GridBar* d_bar;
     TRY(s.put(&d_rp, spRowptr, N + 1));
-    TRY(s.put(&d_col, col.data(), nnz));
+    TRY(s.put(&d_in, spIdx, nnz));
+    TRY(s.alloc(&d_col, nnz));
+    TRY(s.alloc(&d_bad, 1));
+    CFD_CUDA(cudaMemsetAsync(d_bad, 0xff, sizeof(unsigned), s.stream));
+    if (nnz > 0)
+        CFD_LAUNCH(k_index_list, blocks_for(nnz, 256), 256, 0, s.stream, nnz, N, d_in, d_col, d_bad);
+    TRY(s.get(&bad, d_bad, 1));
     TRY(s.put(&d_val, spMtx, nnz));
     TRY(s.put(&d_diag, diagMtx, N));
     TRY(s.put(&d_isfix, isfix.data(), N));
@@ -1119,12 +1207,16 @@ int cfd_bicg_mode(const double* spMtx, const int* spIdx, const int* spRowptr,
     TRY(s.put(&d_x, x, N));
     TRY(s.put(&d_b, b, N));
     for (double** q : {&d_r, &d_z, &d_y, &d_p0, &d_rdiag}) TRY(s.alloc(q, N));
-    const long nc = ((long)N + kChunk - 1) / kChunk;
     TRY(s.alloc(&d_part, 6 * (size_t)nc));
     TRY(s.alloc(&d_bar, 1));
     TRY(s.alloc(&d_it, 2));
     TRY(s.alloc(&d_cv, 2));
     TRY(s.alloc(&d_rz, 4));
+    TRY(s.sync());
+    if (bad != ~0u) {
+        set_last_message("spIdx outside 1..npoin");
+        return CFD_ERR_MESH;
+    }
     CFD_CUDA(cudaMemsetAsync(d_bar, 0, sizeof(GridBar), s.stream));
     PcgArgs a{};
     a.n = N;

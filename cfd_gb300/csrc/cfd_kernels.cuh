@@ -308,13 +308,27 @@ cudaError_t launch_elem_replay(cudaStream_t stream, int nelem, const int4* elem,
                                const double* dtl_scalar, GasConst gc, const double* cache,
                                double* contrib);
 // calcRHS (+ FUENTE when contribF != NULL) element kernel; contrib may be NULL (FUENTE only)
-cudaError_t launch_elem_rhs(bool viscous, bool with_theta, cudaStream_t stream, int nelem,
-                            const int4* elem, const double* U, const double* theta,
+// elements [e0, e1) of nelem
+cudaError_t launch_elem_rhs(bool viscous, bool with_theta, cudaStream_t stream, int e0, int e1,
+                            int nelem, const int4* elem, const double* U, const double* theta,
                             const double* T, const double* geo, const double* area,
                             const double* shoc, const double* dtl_arr, const double* dtl_scalar,
                             const double* ts1, const double* ts2, const double* ts3, GasConst gc,
                             double* contrib, const double* WX, const double* WY,
                             double* contribF);
+// a host caller's mesh on the device (hostmesh.cu).  flags[2] all ones at the start: flags[0]
+// becomes the first element with a node out of range, flags[1] the complement of the largest
+// number of elements around a point; a point of more than kEsupSortMax has unsorted lists
+constexpr int kEsupSortMax = 64;
+long esup_scan_blocks(long npoin);
+cudaError_t launch_elem_table(cudaStream_t st, int nelem, int npoin, const int* inpoel, int4* elem,
+                              int* deg, int* rank, unsigned* flags);
+cudaError_t launch_esup(cudaStream_t st, int nelem, int npoin, const int4* elem, const int* deg,
+                        const int* rank, int* sums, int* ptr, int* slot, unsigned* flags);
+__global__ void k_index_list(int n, int npoin, const int* in, int* out, unsigned* flag);
+__global__ void k_geo_planes(int e0, int e1, int nelem, const double* dnx, const double* dny,
+                             double* geo);
+__global__ void k_geo_rows(int nelem, const double* geo, double* dnx, double* dny);
 // drop-in: rhs(4,npoin) += the elements' contributions, in element order
 __global__ void k_rhs_gather(int npoin, const int* esup_ptr, const int* esup_slot,
                              const double* contrib, double* rhs);

@@ -290,16 +290,16 @@ __global__ void k_estab(int nelem, const int4* __restrict__ elem, const double* 
 // add a signed zero, which leaves every sum's value unchanged.
 template <bool VISCOUS, bool THETA>
 __global__ void __launch_bounds__(128)
-k_elem_rhs(int nelem, const int4* __restrict__ elem, const double* __restrict__ U,
+k_elem_rhs(int e0, int e1, int nelem, const int4* __restrict__ elem, const double* __restrict__ U,
            const double* __restrict__ theta, const double* __restrict__ T,
            const double* __restrict__ geo, const double* __restrict__ area,
            const double* __restrict__ shoc, const double* __restrict__ dtl_arr,
            const double* __restrict__ dtl_scalar, const double* __restrict__ ts1,
-           const double* __restrict__ ts2, const double* __restrict__ ts3, GasConst gc,
+           const double* __restrict__ ts2, const double* __restrict__ ts3, GasConst gc, Rcp t_inf,
            double* __restrict__ contrib, const double* __restrict__ WX,
            const double* __restrict__ WY, double* __restrict__ contribF) {
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nelem) return;
+    int e = e0 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= e1) return;
     const size_t E = (size_t)nelem;
     const double Cv = gc.cv, lambda_ref = gc.lambda_ref, mu_ref = gc.mu_ref, g = gc.gamma;
     const double T_inf = gc.t_inf, cte = gc.cte;
@@ -328,14 +328,18 @@ k_elem_rhs(int nelem, const int4* __restrict__ elem, const double* __restrict__ 
     double mu = 0.0, lambda = 0.0;
     if (VISCOUS) {
         const double T_avg = div3(T[p[0]] + T[p[1]] + T[p[2]]);
-        mu = mu_ref * pow15(T_avg / T_inf) * (T_inf + 110.0) / (T_avg + 110.0);
-        lambda = lambda_ref * pow15(T_avg / T_inf) * (T_inf + 194.0) / (T_avg + 194.0);
+        const double p15 = pow15(div_by(T_avg, t_inf));
+        mu = mu_ref * p15 * (T_inf + 110.0) / (T_avg + 110.0);
+        lambda = lambda_ref * p15 * (T_inf + 194.0) / (T_avg + 194.0);
     }
-    double r[3][4];
+    double r[3][4], a3[3][4];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) r[i][q] = 0.0;
+        for (int q = 0; q < 4; ++q) {
+            r[i][q] = 0.0;
+            a3[i][q] = nu * (Nx[i] * Ux[q] + Ny[i] * Uy[q]);
+        }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         // U_k = N(1,k) U1 + N(2,k) U2 + N(3,k) U3 with N(k,k) = 0: the two 0.5 terms in order
@@ -343,9 +347,11 @@ k_elem_rhs(int nelem, const int4* __restrict__ elem, const double* __restrict__ 
         const int ib = (k == 2) ? 1 : 2;
         double Uk[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) Uk[q] = 0.5 * Un[ia][q] + 0.5 * Un[ib][q];
+        for (int q = 0; q < 4; ++q) Uk[q] = 0.5 * (Un[ia][q] + Un[ib][q]);
         const double rho = Uk[0];
-        const double v1 = Uk[1] / rho, v2 = Uk[2] / rho, ev = Uk[3] / rho;
+        const double rr = 1.0 / rho, rrl = rcp_lo(rho, rr);
+        const double v1 = div_rcp2(Uk[1], rho, rr, rrl), v2 = div_rcp2(Uk[2], rho, rr, rrl),
+                     ev = div_rcp2(Uk[3], rho, rr, rrl);
         const double V_sq = v1 * v1 + v2 * v2;
         double A[4];
         A[0] = Ux[1] + Uy[2];
@@ -393,27 +399,29 @@ k_elem_rhs(int nelem, const int4* __restrict__ elem, const double* __restrict__ 
             for (int q = 0; q < 4; ++q) {
                 double t = r[i][q];
                 if (i != k) t = t + 0.5 * A[q];
-                r[i][q] = t + tau[i] * (Nx[i] * B1[q] + Ny[i] * B2[q]) +
-                          nu * (Nx[i] * Ux[q] + Ny[i] * Uy[q]);
+                r[i][q] = t + tau[i] * (Nx[i] * B1[q] + Ny[i] * B2[q]) + a3[i][q];
             }
         if (VISCOUS) {
+            const double crho = Cv * rho, rc = 1.0 / crho, rcl = rcp_lo(crho, rc);
             double K1[4], K2[4];
-            K1[1] = 2.0 / 3.0 * mu * (-(2.0 * Ux[0] * v1) + 2.0 * Ux[1] + Uy[0] * v2 - Uy[2]) / rho;
-            K1[2] = mu * (-(Ux[0] * v2) + Ux[2] - Uy[0] * v1 + Uy[1]) / rho;
-            K1[3] = 1.0 / 3.0 *
+            K1[1] = div_rcp2(2.0 / 3.0 * mu * (-(2.0 * Ux[0] * v1) + 2.0 * Ux[1] + Uy[0] * v2 - Uy[2]),
+                             rho, rr, rrl);
+            K1[2] = div_rcp2(mu * (-(Ux[0] * v2) + Ux[2] - Uy[0] * v1 + Uy[1]), rho, rr, rrl);
+            K1[3] = div_rcp2(1.0 / 3.0 *
                     (Cv * mu * (-(Uy[0] * v1 * v2) + 3.0 * Uy[1] * v2 - 2.0 * Uy[2] * v1) -
                      Ux[0] * (Cv * mu * (3.0 * V_sq + v1 * v1) - 3.0 * lambda * (V_sq - ev)) +
                      Ux[1] * v1 * (4.0 * Cv * mu - 3.0 * lambda) +
-                     3.0 * Ux[2] * v2 * (Cv * mu - lambda) + 3.0 * Ux[3] * lambda) /
-                    (Cv * rho);
+                     3.0 * Ux[2] * v2 * (Cv * mu - lambda) + 3.0 * Ux[3] * lambda),
+                    crho, rc, rcl);
             K2[1] = K1[2];
-            K2[2] = 2.0 / 3.0 * mu * (Ux[0] * v1 - Ux[1] - 2.0 * Uy[0] * v2 + 2.0 * Uy[2]) / rho;
-            K2[3] = 1.0 / 3.0 *
+            K2[2] = div_rcp2(2.0 / 3.0 * mu * (Ux[0] * v1 - Ux[1] - 2.0 * Uy[0] * v2 + 2.0 * Uy[2]),
+                             rho, rr, rrl);
+            K2[3] = div_rcp2(1.0 / 3.0 *
                     (Cv * mu * (-(Ux[0] * v1 * v2) - 2.0 * Ux[1] * v2 + 3.0 * Ux[2] * v1) -
                      Uy[0] * (Cv * mu * (3.0 * V_sq + v2 * v2) - 3.0 * lambda * (V_sq - ev)) +
                      3.0 * Uy[1] * v1 * (Cv * mu - lambda) +
-                     Uy[2] * v2 * (4.0 * Cv * mu - 3.0 * lambda) + 3.0 * Uy[3] * lambda) /
-                    (Cv * rho);
+                     Uy[2] * v2 * (4.0 * Cv * mu - 3.0 * lambda) + 3.0 * Uy[3] * lambda),
+                    crho, rc, rcl);
 #pragma unroll
             for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -453,16 +461,17 @@ k_elem_rhs(int nelem, const int4* __restrict__ elem, const double* __restrict__ 
     }
 }
 
-cudaError_t launch_elem_rhs(bool viscous, bool with_theta, cudaStream_t stream, int nelem,
-                            const int4* elem, const double* U, const double* theta,
+cudaError_t launch_elem_rhs(bool viscous, bool with_theta, cudaStream_t stream, int e0, int e1,
+                            int nelem, const int4* elem, const double* U, const double* theta,
                             const double* T, const double* geo, const double* area,
                             const double* shoc, const double* dtl_arr, const double* dtl_scalar,
                             const double* ts1, const double* ts2, const double* ts3, GasConst gc,
                             double* contrib, const double* WX, const double* WY,
                             double* contribF) {
-    const unsigned grid = blocks_for(nelem, 128);
-#define CFD_ELEM_ARGS nelem, elem, U, theta, T, geo, area, shoc, dtl_arr, dtl_scalar, ts1, ts2, \
-                      ts3, gc, contrib, WX, WY, contribF
+    const unsigned grid = blocks_for(e1 - e0, 128);
+    const Rcp ti = make_rcp(gc.t_inf);
+#define CFD_ELEM_ARGS e0, e1, nelem, elem, U, theta, T, geo, area, shoc, dtl_arr, dtl_scalar, ts1, \
+                      ts2, ts3, gc, ti, contrib, WX, WY, contribF
     if (viscous && with_theta) k_elem_rhs<true, true><<<grid, 128, 0, stream>>>(CFD_ELEM_ARGS);
     else if (viscous) k_elem_rhs<true, false><<<grid, 128, 0, stream>>>(CFD_ELEM_ARGS);
     else if (with_theta) k_elem_rhs<false, true><<<grid, 128, 0, stream>>>(CFD_ELEM_ARGS);
