@@ -4,8 +4,6 @@
 // same kernels the resident context uses and copy the results back.  Every call checks
 // its arguments and returns a status; nothing here falls back to the CPU.
 #include <cuda_runtime.h>
-#include <sys/mman.h>
-#include <unistd.h>
 
 #include <cmath>
 #include <cstring>
@@ -18,8 +16,6 @@
 using namespace cfd;
 
 namespace {
-
-constexpr int kPopulateWrite = 23;  // MADV_POPULATE_WRITE, which older headers lack
 
 // A call's device buffers, freed at scope exit.  init(bytes) takes them as one allocation, which
 // alloc() cuts up (a cudaMalloc and its cudaFree cost ~70 us together on GB300, and a call has up
@@ -75,13 +71,9 @@ struct Scratch {
         int st = alloc(p, n);
         return st ? st : copy(*p, h, n);
     }
-    // A large result's pages are mapped first (contents kept; a kernel that does not know the
-    // advice refuses it, which changes nothing): the device's copy into pages that the host has
-    // not touched yet, a fresh calloc's, faults on each of them (four arrays of 4 MB: 12 ms, 0.6 ms now).
     template <class T>
     int get(T* h, const T* d, size_t n) {
-        const uintptr_t page = sysconf(_SC_PAGESIZE), a = (uintptr_t)h / page * page, b = (uintptr_t)(h + n);
-        if (n * sizeof(T) >= 16 * page) (void)madvise((void*)a, (b - a + page - 1) / page * page, kPopulateWrite);
+        map_result(h, n * sizeof(T));
         if (n) CFD_CUDA(cudaMemcpyAsync(h, d, n * sizeof(T), cudaMemcpyDeviceToHost, stream));
         return CFD_OK;
     }

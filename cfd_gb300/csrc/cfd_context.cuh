@@ -1,5 +1,9 @@
 // cfd_context.cuh — the resident context (one mesh, its state and every work array in HBM).
 #pragma once
+#include <sys/mman.h>
+#include <unistd.h>
+
+#include <cstdint>
 #include <string>
 #include <vector>
 
@@ -45,6 +49,17 @@ int smooth_on_device(cudaStream_t st, int npoin, int nelem, const int4* elem,
 
 enum { TM_DELTAT, TM_ESTAB, TM_CALCRHS, TM_FUENTE, TM_UPDATE, TM_FORCES, TM_TRANSF, TM_GRAD,
        TM_NORMALES, TM_DERIV, TM_MASAS, TM_LAPLACE, TM_N };
+
+// A large result's host pages are mapped before the device copies into it (contents kept; a
+// kernel that does not know the advice refuses it, which changes nothing): a copy into pages that
+// the host has not touched yet, a fresh calloc's, faults on each of them (four arrays of 4 MB:
+// 12 ms, 0.6 ms so).
+inline void map_result(void* p, size_t bytes) {
+    const uintptr_t page = sysconf(_SC_PAGESIZE), a = (uintptr_t)p / page * page,
+                    b = (uintptr_t)p + bytes;
+    constexpr int populate_write = 23;  // MADV_POPULATE_WRITE, which older headers lack
+    if (bytes >= 16 * page) (void)madvise((void*)a, (b - a + page - 1) / page * page, populate_write);
+}
 
 void set_last_message(const std::string& m);
 std::string last_message();

@@ -7,6 +7,7 @@
 // Reductions over nodes or edges (weight gradients, loss) go through per-block partials
 // folded in a fixed order, so a training step is deterministic.
 #include <algorithm>
+#include <type_traits>
 
 #include "mpnn_kernels.cuh"
 
@@ -1280,6 +1281,15 @@ __global__ void __launch_bounds__(32 * IW, 2) k_infer_layer(
 // the accumulator with tcgen05.ld for the epilogue.  The update GEMM (N = 64, K = 128) and
 // the next layer's P|Q GEMM (N = 128, K = 64) use the same 128 tensor-memory columns one
 // after the other.
+//
+// The gather bounds a layer, by the latency of its loads (row pointer, neighbour, neighbour's
+// Q row) as long as few of them are in flight.  So the tile's neighbours and edge features,
+// contiguous in both arrays, come by cp.async.bulk while the block finishes the tile before;
+// eight lanes take a node (eight channels each, C's 24 coefficients in registers) and have
+// the Q rows of up to eight edges in flight; and every global row goes out through shared
+// memory, so that a warp writes whole lines.  1,048,576 nodes, 6.3 M edges: 480 us a layer
+// with one edge in flight per lane and rows stored by their owner threads, 312 us now; the
+// encoder pass 194 us, 118 us now.
 namespace tc {
 constexpr int TM = 128;          // nodes per tile
 constexpr int NTHR = 256;        // 8 warps
@@ -1287,26 +1297,35 @@ constexpr unsigned TMEM_COLS = 128;
 // K-major operands in the no-swizzle core-matrix layout: a core matrix is 8 rows x 16
 // bytes (128 contiguous bytes); the core matrices of one 8-row group lie along K, 128 B
 // apart (the descriptor's leading byte offset); the 8-row groups lie SBO bytes apart.
+// The tile's core matrices lie 144 B apart: lanes that write one row's chunks hit different banks.
 constexpr int LBO = 128;
-constexpr int SBO_X = 16 * 2 * HID;  // the tile, 128 rows x K = 128 (h, then agg)
+constexpr int LBO_X = 144;
+constexpr int SBO_X = LBO_X * 2 * HID / 8;  // the tile, 128 rows x K = 128 (h, then agg)
 constexpr int SBO_U = 16 * 2 * HID;  // U: N = 64 rows x K = 128
 constexpr int SBO_W = 16 * HID;      // [A; B]: N = 128 rows x K = 64
-constexpr int X_BYTES = TM * 2 * HID * 2;
+constexpr int X_BYTES = TM / 8 * SBO_X;
+constexpr int PQ_ROW = 2 * 2 * HID + 16;  // a staged P|Q row (padded: rows in different banks)
+constexpr int PQ_BLK = X_BYTES / 4;       // 32 of them: the rows of one quarter of the tile
+static_assert(32 * PQ_ROW <= PQ_BLK, "staged P|Q rows");
+constexpr int GB = 3;                     // edges of a batch
+constexpr int EC = 1024;                  // staged edges (a tile of more reads global memory)
 constexpr int U_BYTES = HID * 2 * HID * 2;
 constexpr int W_BYTES = 2 * HID * HID * 2;
 constexpr int F_FLOATS = HID * F_IN + HID;  // the largest float table (W_in, b_in)
 static_assert(HID * E_F + 2 * HID + OUT * HID + OUT <= F_FLOATS, "float tables");
-constexpr int SMEM = X_BYTES + U_BYTES + W_BYTES + 4 * F_FLOATS + 16;
+static_assert(F_FLOATS % 4 == 0 && EC % 4 == 0, "16-byte offsets");
+constexpr int SMEM = X_BYTES + U_BYTES + W_BYTES + 4 * F_FLOATS + 16 * EC + 32;
 
-__host__ __device__ constexpr int cm_off(int r, int k, int sbo) {
-    return (r >> 3) * sbo + (k >> 3) * LBO + (r & 7) * 16 + (k & 7) * 2;
+__host__ __device__ constexpr int cm_off(int r, int k, int sbo, int lbo = LBO) {
+    return (r >> 3) * sbo + (k >> 3) * lbo + (r & 7) * 16 + (k & 7) * 2;
 }
+__host__ __device__ constexpr int x_off(int r, int k) { return cm_off(r, k, SBO_X, LBO_X); }
 
 // shared-memory matrix descriptor: start address, leading and stride byte offsets (all
 // >> 4), the descriptor version 1 at bit 46, base offset 0, no swizzle
-__device__ __forceinline__ unsigned long long sdesc(unsigned saddr, unsigned sbo) {
+__device__ __forceinline__ unsigned long long sdesc(unsigned saddr, unsigned sbo, unsigned lbo) {
     return (unsigned long long)((saddr & 0x3FFFFu) >> 4) |
-           ((unsigned long long)(LBO >> 4) << 16) | ((unsigned long long)(sbo >> 4) << 32) |
+           ((unsigned long long)(lbo >> 4) << 16) | ((unsigned long long)(sbo >> 4) << 32) |
            (1ull << 46);
 }
 
@@ -1390,8 +1409,67 @@ __device__ __forceinline__ unsigned pack2(float a, float b) {
     return *reinterpret_cast<const unsigned*>(&h);
 }
 
+__device__ __forceinline__ void cp_async16(unsigned dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_copy(unsigned dst, const void* src, unsigned bytes, unsigned mbar) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
+            "r"(dst), "l"(src), "r"(bytes), "r"(mbar)
+        : "memory");
+}
+// the two warps that share a quarter of the tile
+__device__ __forceinline__ void pair_sync(int q4) {
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + q4) : "memory");
+}
+__device__ __forceinline__ void unpack8(const uint4 v, float (&x)[8]) {
+    const unsigned w4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const float2 f2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w4[u]));
+        x[2 * u] = f2.x;
+        x[2 * u + 1] = f2.y;
+    }
+}
+// two FP32 operations in one instruction, each rounded as the single one
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpair(f32x2 p) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// a BF16 pair as two floats
+__device__ __forceinline__ f32x2 widen2(unsigned v) {
+    return pair(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+}
+__device__ __forceinline__ uint4 pack8(const float (&x)[8]) {
+    return make_uint4(pack2(x[0], x[1]), pack2(x[2], x[3]), pack2(x[4], x[5]), pack2(x[6], x[7]));
+}
+
 // ENC: h0 = relu(W_in f + b_in), then P|Q of layer 0.  Otherwise layer l: aggregation,
-// update GEMM, residual, then P|Q of layer l+1 (has_next) or the decoder.
+// update GEMM, residual, then P|Q of layer l+1 (has_next) or the decoder.  nbr and e are
+// readable up to the next 16-byte boundary.
 template <bool ENC>
 __global__ void __launch_bounds__(NTHR, 2) k_infer_tc(
     int n, int l, const int* __restrict__ ptr, const int* __restrict__ nbr,
@@ -1405,15 +1483,19 @@ __global__ void __launch_bounds__(NTHR, 2) k_infer_tc(
     unsigned char* Us = Xs + X_BYTES;
     unsigned char* Ws = Us + U_BYTES;
     float* fl = reinterpret_cast<float*>(Ws + W_BYTES);
-    unsigned long long* mbar = reinterpret_cast<unsigned long long*>(fl + F_FLOATS);
-    unsigned* tslot = reinterpret_cast<unsigned*>(mbar + 1);
+    int* sn = reinterpret_cast<int*>(fl + F_FLOATS);       // the tile's neighbours ..
+    float* se = reinterpret_cast<float*>(sn + EC);          // .. and edge features
+    unsigned long long* mbar = reinterpret_cast<unsigned long long*>(se + 3 * EC);
+    unsigned* tslot = reinterpret_cast<unsigned*>(mbar + 2);
     int* abort_flag = reinterpret_cast<int*>(tslot + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // float tables: ENC W_in, b_in; layers C, c, u, W_out, b_out
+    // float tables: ENC W_in (transposed), b_in; layers C, c, u, W_out, b_out
     float *Cs = fl, *cs = fl + HID * E_F, *us = cs + HID, *wo = us + HID;
     const int has_pq = ENC || has_next;
     if (ENC) {
-        for (int q = tid; q < F_FLOATS; q += NTHR) fl[q] = w[OFF_W_IN + q];
+        for (int q = tid; q < HID * F_IN; q += NTHR)
+            fl[(q % F_IN) * HID + q / F_IN] = w[OFF_W_IN + q];
+        for (int q = tid; q < HID; q += NTHR) fl[HID * F_IN + q] = w[OFF_W_IN + HID * F_IN + q];
     } else {
         const float* W = w + layer_off(l);
         load_cm(Us, SBO_U, wb + layer_off(l) + L_U, HID, 2 * HID);
@@ -1426,10 +1508,11 @@ __global__ void __launch_bounds__(NTHR, 2) k_infer_tc(
             for (int q = tid; q < OUT * HID + OUT; q += NTHR) wo[q] = w[OFF_W_OUT + q];
     }
     if (has_pq) load_cm(Ws, SBO_W, wb + layer_off(ENC ? 0 : l + 1) + L_A, 2 * HID, HID);
-    const unsigned ubar = su32(mbar);
+    const unsigned ubar = su32(mbar), sbar = su32(mbar + 1);  // the MMAs, the staged edges
     if (tid == 0) {
         *abort_flag = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ubar) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sbar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -1447,107 +1530,194 @@ __global__ void __launch_bounds__(NTHR, 2) k_infer_tc(
     const unsigned tbase = *tslot;
     const unsigned xa = su32(Xs), ua = su32(Us), wa = su32(Ws);
     // epilogue geometry: warp w reads tensor-memory lanes 32 (w % 4) .. (its 32 rows) and
-    // half w / 4 of the accumulator's columns
+    // half w / 4 of the accumulator's columns; it writes the rows 16 (w / 4) .. of them out
     const int q4 = warp & 3, half = warp >> 2;
     const int erow = 32 * q4 + lane;
     const unsigned tlane = tbase + ((unsigned)(32 * q4) << 16);
-    unsigned phase = 0;
-    bool pending = false;  // a commit that this block has not seen arrive
-    float acc_hi[8];
+    // gather geometry: lane l takes node l / 8 of the pass and the channels 8 (l % 8) ..
+    const int sub = lane >> 3, f0 = 8 * (lane & 7);
+    unsigned phase = 0, sphase = 0;
+    bool pending = false;   // a commit that this block has not seen arrive
+    bool spending = false;  // staged edges that this thread has not seen arrive
+    f32x2 C0[4], C1[4], C2[4];
+    if (!ENC)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float* c = Cs + 3 * (f0 + 2 * i);
+            C0[i] = pair(c[0], c[3]);
+            C1[i] = pair(c[1], c[4]);
+            C2[i] = pair(c[2], c[5]);
+        }
     const int ntile = (n + TM - 1) / TM;
+    // the row pointers of a tile: its first and last edge, and this warp's nodes (lanes 0..16)
+    int tk0 = 0, tk1 = 0, pv = 0;
+    auto pointers = [&](int tile, int& k0, int& k1, int& v) {
+        const int tb = tile * TM;
+        k0 = ptr[tb];
+        k1 = ptr[min(tb + TM, n)];
+        v = ptr[min(tb + 16 * warp + min(lane, 16), n)];
+    };
+    // edges [tk0, tk1) into shared memory, from the 16-byte boundary before the first
+    auto stage = [&]() {
+        const int ka = tk0 & ~3, cnt = tk1 - ka;
+        spending = tk1 > tk0 && cnt <= EC;
+        if (spending && tid == NTHR - 32) {
+            const unsigned nbytes = (4u * cnt + 15u) & ~15u, ebytes = (12u * cnt + 15u) & ~15u;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sbar),
+                         "r"(nbytes + ebytes)
+                         : "memory");
+            bulk_copy(su32(sn), nbr + ka, nbytes, sbar);
+            bulk_copy(su32(se), e + 3 * (size_t)ka, ebytes, sbar);
+        }
+    };
+    if (!ENC && (int)blockIdx.x < ntile) {
+        pointers(blockIdx.x, tk0, tk1, pv);
+        stage();
+    }
     for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
         const int tb = tile * TM;
+        const bool more = tile + (int)gridDim.x < ntile;
+        int nk0 = 0, nk1 = 0, nv = 0;
+        if (!ENC && more) pointers(tile + gridDim.x, nk0, nk1, nv);
         if (ENC) {
-            // lane l of warp w owns row 16 w + l / 2 and the outputs [32 (l % 2), +32)
-            const int r = 16 * warp + (lane >> 1), o0 = 32 * (lane & 1), node = tb + r;
+            // lane l of warp w owns row 16 w + l / 2 and every other chunk of eight outputs
+            const int r = 16 * warp + (lane >> 1), node = tb + r;
             float fi[F_IN];
+            static_assert(F_IN % 2 == 0, "float2 rows");
 #pragma unroll
-            for (int k = 0; k < F_IN; ++k) fi[k] = node < n ? f[(size_t)node * F_IN + k] : 0.f;
-            unsigned w16[16];
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                float hv[2];
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int o = o0 + 2 * q + u;
-                    float a = fl[HID * F_IN + o];
-#pragma unroll
-                    for (int k = 0; k < F_IN; ++k) a += fl[o * F_IN + k] * fi[k];
-                    hv[u] = node < n ? fmaxf(a, 0.f) : 0.f;
-                }
-                w16[q] = pack2(hv[0], hv[1]);
+            for (int k = 0; k < F_IN; k += 2) {
+                const float2 v = node < n ? *reinterpret_cast<const float2*>(f + (size_t)node * F_IN + k)
+                                          : make_float2(0.f, 0.f);
+                fi[k] = v.x;
+                fi[k + 1] = v.y;
             }
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                const uint4 wv = make_uint4(w16[4 * v], w16[4 * v + 1], w16[4 * v + 2], w16[4 * v + 3]);
-                *reinterpret_cast<uint4*>(Xs + cm_off(r, o0 + 8 * v, SBO_X)) = wv;
-                if (node < n)
-                    *reinterpret_cast<uint4*>(hb + (size_t)node * HID + o0 + 8 * v) = wv;
+            for (int v = 0; v < HID / 16; ++v) {
+                const int o = 16 * v + 8 * (lane & 1);
+                float a[8];
+#pragma unroll
+                for (int k = -1; k < F_IN; ++k) {
+                    const float4* wk =
+                        reinterpret_cast<const float4*>(fl + (k < 0 ? HID * F_IN : k * HID) + o);
+                    const float4 wl = wk[0], wh = wk[1];
+                    const float wv[8] = {wl.x, wl.y, wl.z, wl.w, wh.x, wh.y, wh.z, wh.w};
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        if (k < 0) a[i] = wv[i];
+                        else a[i] += wv[i] * fi[k < 0 ? 0 : k];
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) a[i] = node < n ? fmaxf(a[i], 0.f) : 0.f;
+                *reinterpret_cast<uint4*>(Xs + x_off(r, o)) = pack8(a);
             }
         } else {
-            // [h; agg] rows, 8 nodes per pass: lane l owns row 16 w + l / 4 (+8) and the 16
-            // features [16 (l % 4), +16)
-            for (int pass = 0; pass < 2; ++pass) {
-                const int r = 16 * warp + (lane >> 2) + 8 * pass, f0 = 16 * (lane & 3),
-                          node = tb + r;
-                float acc16[16], pz[16];
+            // [h; agg] rows: eight lanes take four nodes, one after the other
+            const int r0 = 16 * warp + 4 * sub, nb0 = tb + r0, ka = tk0 & ~3;
+            const bool staged = spending;
 #pragma unroll
-                for (int q = 0; q < 16; ++q) acc16[q] = 0.f;
-                uint4 hv4[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
-                if (node < n) {
-                    const uint4* hp = reinterpret_cast<const uint4*>(hb + (size_t)node * HID + f0);
-                    const uint4* pp =
-                        reinterpret_cast<const uint4*>(pq_in + (size_t)node * 2 * HID + f0);
-#pragma unroll
-                    for (int v = 0; v < 2; ++v) {
-                        hv4[v] = hp[v];
-                        const uint4 pv = pp[v];
-                        const unsigned w4[4] = {pv.x, pv.y, pv.z, pv.w};
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const float2 f2 =
-                                __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w4[u]));
-                            pz[8 * v + 2 * u] = f2.x + cs[f0 + 8 * v + 2 * u];
-                            pz[8 * v + 2 * u + 1] = f2.y + cs[f0 + 8 * v + 2 * u + 1];
-                        }
-                    }
-                    const int k0 = ptr[node], k1 = ptr[node + 1];
-                    for (int k = k0; k < k1; ++k) {
-                        const int j = nbr[k];
-                        const float e0 = e[3 * (size_t)k], e1 = e[3 * (size_t)k + 1],
-                                    e2 = e[3 * (size_t)k + 2];
-                        const uint4* qp = reinterpret_cast<const uint4*>(
-                            pq_in + (size_t)j * 2 * HID + HID + f0);
-                        const uint4 qa = qp[0], qb = qp[1];
-                        const unsigned w8[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-#pragma unroll
-                        for (int u = 0; u < 8; ++u) {
-                            const float2 q2 = __bfloat1622float2(
-                                *reinterpret_cast<const __nv_bfloat162*>(&w8[u]));
-                            const int o = f0 + 2 * u;
-                            const float z0 = pz[2 * u] + q2.x +
-                                             (Cs[o * 3] * e0 + Cs[o * 3 + 1] * e1 + Cs[o * 3 + 2] * e2);
-                            const float z1 =
-                                pz[2 * u + 1] + q2.y +
-                                (Cs[o * 3 + 3] * e0 + Cs[o * 3 + 4] * e1 + Cs[o * 3 + 5] * e2);
-                            acc16[2 * u] += fmaxf(z0, 0.f);
-                            acc16[2 * u + 1] += fmaxf(z1, 0.f);
-                        }
-                    }
-                    const float inv = 1.f / (float)max(k1 - k0, 1);
-#pragma unroll
-                    for (int q = 0; q < 16; ++q) acc16[q] *= inv;
-                }
-#pragma unroll
-                for (int v = 0; v < 2; ++v) {
-                    *reinterpret_cast<uint4*>(Xs + cm_off(r, f0 + 8 * v, SBO_X)) = hv4[v];
-                    *reinterpret_cast<uint4*>(Xs + cm_off(r, HID + f0 + 8 * v, SBO_X)) =
-                        make_uint4(pack2(acc16[8 * v], acc16[8 * v + 1]),
-                                   pack2(acc16[8 * v + 2], acc16[8 * v + 3]),
-                                   pack2(acc16[8 * v + 4], acc16[8 * v + 5]),
-                                   pack2(acc16[8 * v + 6], acc16[8 * v + 7]));
+            for (int i = 0; i < 4; ++i) {
+                const bool in = nb0 + i < n;
+                cp_async16(xa + x_off(r0 + i, f0), hb + (in ? (size_t)(nb0 + i) * HID + f0 : 0),
+                           in ? 16 : 0);
+            }
+            const uint4* prow = reinterpret_cast<const uint4*>(pq_in + f0);
+            const uint4* qrow = reinterpret_cast<const uint4*>(pq_in + HID + f0);
+            uint4 pnext = nb0 < n ? prow[(size_t)nb0 * (2 * HID / 8)] : make_uint4(0u, 0u, 0u, 0u);
+            bool here = true;  // nothing is gathered by indices that did not arrive
+            if (staged) {
+                here = __all_sync(0xffffffffu, wait_parity(sbar, sphase & 1));
+                if (here) {
+                    spending = false;
+                    sphase += 1;
+                } else {
+                    atomicExch(err, (int)CFD_ERR_BARRIER);
+                    *abort_flag = 1;
                 }
             }
+            auto gather = [&](auto from_stage) {
+                constexpr bool STAGED = decltype(from_stage)::value;
+                int ke[5];  // the four nodes' first edges and the end of the last
+#pragma unroll
+                for (int i = 0; i < 5; ++i) ke[i] = __shfl_sync(0xffffffffu, pv, 4 * sub + i);
+                const int kn = ke[4];
+                int i = 0, k1 = ke[1], deg = ke[1] - ke[0];
+                f32x2 pz[4], acc[4];
+                auto open = [&]() {  // node i: z's part that its edges share, an empty sum
+                    const unsigned pw[4] = {pnext.x, pnext.y, pnext.z, pnext.w};
+                    if (i < 3 && nb0 + i + 1 < n) pnext = prow[(size_t)(nb0 + i + 1) * (2 * HID / 8)];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        pz[c] = add2(widen2(pw[c]), pair(cs[f0 + 2 * c], cs[f0 + 2 * c + 1]));
+                        acc[c] = 0ull;
+                    }
+                };
+                auto close = [&]() {  // the mean message of node i; on to the next
+                    const float inv = 1.f / (float)max(deg, 1);
+                    unsigned aw[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float2 m = unpair(acc[c]);
+                        aw[c] = pack2(m.x * inv, m.y * inv);
+                    }
+                    *reinterpret_cast<uint4*>(Xs + x_off(r0 + i, HID + f0)) =
+                        make_uint4(aw[0], aw[1], aw[2], aw[3]);
+                    i += 1;
+                    ke[1] = ke[2];
+                    ke[2] = ke[3];
+                    ke[3] = ke[4];
+                    deg = ke[1] - k1;
+                    k1 = ke[1];
+                };
+                auto fetch = [&](uint4(&q)[GB], int k) {
+#pragma unroll
+                    for (int u = 0; u < GB; ++u)
+                        if (k + u < kn) {
+                            const int j = STAGED ? sn[k - ka + u] : nbr[k + u];
+                            q[u] = qrow[(size_t)j * (2 * HID / 8)];
+                        }
+                };
+                auto use = [&](const uint4(&q)[GB], int k) {
+#pragma unroll
+                    for (int u = 0; u < GB; ++u)
+                        if (k + u < kn) {
+                            while (k + u == k1) {
+                                close();
+                                open();
+                            }
+                            const float* ep = STAGED ? se + 3 * (k - ka + u) : e + 3 * (size_t)(k + u);
+                            const f32x2 e0 = pair(ep[0], ep[0]), e1 = pair(ep[1], ep[1]),
+                                        e2 = pair(ep[2], ep[2]);
+                            const unsigned qw[4] = {q[u].x, q[u].y, q[u].z, q[u].w};
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) {
+                                // z = (p + c) + q + fma(C2, e2, fma(C0, e0, C1 e1))
+                                const float2 z = unpair(
+                                    add2(add2(pz[c], widen2(qw[c])),
+                                         fma2(C2[c], e2, fma2(C0[c], e0, mul2(C1[c], e1)))));
+                                acc[c] = add2(acc[c], pair(fmaxf(z.x, 0.f), fmaxf(z.y, 0.f)));
+                            }
+                        }
+                };
+                uint4 qa[GB], qb[GB];
+                fetch(qa, ke[0]);
+                open();
+                for (int k = ke[0]; k < kn; k += GB) {
+                    fetch(qb, k + GB);
+                    use(qa, k);
+                    k += GB;
+                    if (k >= kn) break;
+                    fetch(qa, k + GB);
+                    use(qb, k);
+                }
+                while (i < 4) {
+                    close();
+                    if (i < 4) open();
+                }
+            };
+            if (staged && here) gather(std::true_type{});
+            else if (here) gather(std::false_type{});
+            asm volatile("cp.async.wait_all;" ::: "memory");
         }
         fence_smem_async();
         fence_before();
@@ -1559,11 +1729,18 @@ __global__ void __launch_bounds__(NTHR, 2) k_infer_tc(
                 fence_after();
 #pragma unroll
                 for (int kk = 0; kk < 2 * HID / 16; ++kk)
-                    mma(tbase, sdesc(xa + kk * 2 * LBO, SBO_X), sdesc(ua + kk * 2 * LBO, SBO_U),
-                        idesc_bf16(TM, HID), kk > 0 ? 1u : 0u);
+                    mma(tbase, sdesc(xa + kk * 2 * LBO_X, SBO_X, LBO_X),
+                        sdesc(ua + kk * 2 * LBO, SBO_U, LBO), idesc_bf16(TM, HID), kk > 0 ? 1u : 0u);
                 commit(ubar);
             }
             pending = true;
+            // meanwhile the next tile's edges: every warp has read this one's
+            if (more) {
+                tk0 = nk0;
+                tk1 = nk1;
+                pv = nv;
+                stage();
+            }
             // the warp goes on only as a whole (tcgen05.ld is warp-collective)
             if (!__all_sync(0xffffffffu, wait_parity(ubar, phase & 1))) {
                 atomicExch(err, (int)CFD_ERR_BARRIER);
@@ -1573,38 +1750,20 @@ __global__ void __launch_bounds__(NTHR, 2) k_infer_tc(
                 phase += 1;
                 fence_after();
                 // h <- h + relu(v + u) on this thread's row, columns [32 half, +32)
-                const int node = tb + erow;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    float acc[8];
-                    if (c % 2 == 0) {
-                        float a16[16];
-                        tmem_ld16(tlane + 32 * half + 8 * c, a16);
+                for (int c = 0; c < 2; ++c) {
+                    float a16[16];
+                    tmem_ld16(tlane + 32 * half + 16 * c, a16);
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            acc[i] = a16[i];
-                            acc_hi[i] = a16[8 + i];
-                        }
-                    } else {
+                    for (int v = 0; v < 2; ++v) {
+                        const int k0 = 32 * half + 16 * c + 8 * v;
+                        uint4* xp = reinterpret_cast<uint4*>(Xs + x_off(erow, k0));
+                        float h[8];
+                        unpack8(*xp, h);
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) acc[i] = acc_hi[i];
+                        for (int i = 0; i < 8; ++i) h[i] = h[i] + fmaxf(a16[8 * v + i] + us[k0 + i], 0.f);
+                        *xp = pack8(h);
                     }
-                    const int k0 = 32 * half + 8 * c;
-                    uint4* xp = reinterpret_cast<uint4*>(Xs + cm_off(erow, k0, SBO_X));
-                    const uint4 hv = *xp;
-                    const unsigned hw[4] = {hv.x, hv.y, hv.z, hv.w};
-                    unsigned nw[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const float2 h2 =
-                            __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hw[u]));
-                        const int col = k0 + 2 * u;
-                        nw[u] = pack2(h2.x + fmaxf(acc[2 * u] + us[col], 0.f),
-                                      h2.y + fmaxf(acc[2 * u + 1] + us[col + 1], 0.f));
-                    }
-                    const uint4 nv = make_uint4(nw[0], nw[1], nw[2], nw[3]);
-                    *xp = nv;
-                    if (node < n) *reinterpret_cast<uint4*>(hb + (size_t)node * HID + k0) = nv;
                 }
             }
             fence_smem_async();
@@ -1618,62 +1777,79 @@ __global__ void __launch_bounds__(NTHR, 2) k_infer_tc(
                 fence_after();
 #pragma unroll
                 for (int kk = 0; kk < HID / 16; ++kk)
-                    mma(tbase, sdesc(xa + kk * 2 * LBO, SBO_X), sdesc(wa + kk * 2 * LBO, SBO_W),
-                        idesc_bf16(TM, 2 * HID), kk > 0 ? 1u : 0u);
+                    mma(tbase, sdesc(xa + kk * 2 * LBO_X, SBO_X, LBO_X),
+                        sdesc(wa + kk * 2 * LBO, SBO_W, LBO), idesc_bf16(TM, 2 * HID), kk > 0 ? 1u : 0u);
                 commit(ubar);
             }
             pending = true;
-            if (!__all_sync(0xffffffffu, wait_parity(ubar, phase & 1))) {
+            // meanwhile the tile's h rows go out, 4 rows per store (the last layer's h has no reader)
+            const int r0 = 32 * q4 + 16 * half;
+#pragma unroll
+            for (int it = 0; it < 4; ++it) {
+                const int r = r0 + 4 * it + sub;
+                if (tb + r < n)
+                    *reinterpret_cast<uint4*>(hb + (size_t)(tb + r) * HID + f0) =
+                        *reinterpret_cast<const uint4*>(Xs + x_off(r, f0));
+            }
+            const bool ok = __all_sync(0xffffffffu, wait_parity(ubar, phase & 1));
+            if (!ok) {
                 atomicExch(err, (int)CFD_ERR_BARRIER);
                 *abort_flag = 1;
             } else {
                 pending = false;
                 phase += 1;
                 fence_after();
-                const int node = tb + erow;
+            }
+            // P|Q rows into the tile's place (its MMAs are done; the pair of warps has read its h
+            // rows), then out, 2 rows per store
+            pair_sync(q4);
+            unsigned char* st = Xs + PQ_BLK * q4;
+            if (ok) {
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     float v[16];
                     tmem_ld16(tlane + 64 * half + 16 * c, v);
-                    if (node < n) {
-                        uint4* op = reinterpret_cast<uint4*>(pq_out + (size_t)node * 2 * HID +
-                                                             64 * half + 16 * c);
-                        op[0] = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]),
-                                           pack2(v[4], v[5]), pack2(v[6], v[7]));
-                        op[1] = make_uint4(pack2(v[8], v[9]), pack2(v[10], v[11]),
-                                           pack2(v[12], v[13]), pack2(v[14], v[15]));
-                    }
+                    uint4* op = reinterpret_cast<uint4*>(st + lane * PQ_ROW + 128 * half + 32 * c);
+                    op[0] = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]),
+                                       pack2(v[6], v[7]));
+                    op[1] = make_uint4(pack2(v[8], v[9]), pack2(v[10], v[11]), pack2(v[12], v[13]),
+                                       pack2(v[14], v[15]));
                 }
+            }
+            pair_sync(q4);
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+                const int r = 16 * half + 2 * it + (lane >> 4), node = tb + 32 * q4 + r;
+                if (node < n)
+                    *reinterpret_cast<uint4*>(pq_out + (size_t)node * 2 * HID + 8 * (lane & 15)) =
+                        *reinterpret_cast<const uint4*>(st + r * PQ_ROW + 16 * (lane & 15));
             }
         } else if (half == 0) {
             // decoder: y = W_out h + b_out on this thread's row
             const int node = tb + erow;
-            float hrow[HID];
+            float a[OUT];
 #pragma unroll
+            for (int o = 0; o < OUT; ++o) a[o] = wo[OUT * HID + o];
+#pragma unroll 2
             for (int c = 0; c < HID / 8; ++c) {
-                const uint4 hv = *reinterpret_cast<const uint4*>(Xs + cm_off(erow, 8 * c, SBO_X));
-                const unsigned hw[4] = {hv.x, hv.y, hv.z, hv.w};
+                float h[8];
+                unpack8(*reinterpret_cast<const uint4*>(Xs + x_off(erow, 8 * c)), h);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const float2 h2 =
-                        __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hw[u]));
-                    hrow[8 * c + 2 * u] = h2.x;
-                    hrow[8 * c + 2 * u + 1] = h2.y;
-                }
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int o = 0; o < OUT; ++o) a[o] += wo[o * HID + 8 * c + i] * h[i];
             }
             if (node < n)
-                for (int o = 0; o < OUT; ++o) {
-                    float a = wo[OUT * HID + o];
-                    for (int k = 0; k < HID; ++k) a += wo[o * HID + k] * hrow[k];
-                    y[(size_t)OUT * node + o] = a;
-                }
+#pragma unroll
+                for (int o = 0; o < OUT; ++o) y[(size_t)OUT * node + o] = a[o];
         }
         fence_before();
         __syncthreads();
         if (*abort_flag) break;
     }
-    // a commit that timed out may still land: wait for it (bounded) before the columns go
+    // what timed out or was left may still land: wait for it (bounded) before the memory goes
     if (tid == 0 && pending) wait_parity(ubar, phase & 1);
+    if (spending) wait_parity(sbar, sphase & 1);
     fence_before();
     __syncthreads();
     if (warp == 0) {

@@ -196,7 +196,8 @@ int graph_build(cfd_mpnn_graph** out, int npoin, const std::vector<int>& rowptr,
     };
     int rc;
     if ((rc = up(&g->ptr, ptr.data(), npoin + 1))) return rc;
-    if ((rc = up(&g->nbr, nbr.data(), m))) return rc;
+    nbr.resize(m + 4, 0);  // the inference pass reads nbr and e up to a 16-byte boundary
+    if ((rc = up(&g->nbr, nbr.data(), m + 4))) return rc;
     if ((rc = up(&g->src, src.data(), m))) return rc;
     if ((rc = up(&g->rev, rev.data(), m))) return rc;
     if ((rc = up(&g->kind, kind.data(), npoin))) return rc;
@@ -215,7 +216,7 @@ int graph_build(cfd_mpnn_graph** out, int npoin, const std::vector<int>& rowptr,
     if ((rc = dev_alloc(o, &g->G, 1))) return rc;
     const size_t n = npoin;
     if ((rc = dev_alloc(o, &g->f, n * F_IN))) return rc;
-    if ((rc = dev_alloc(o, &g->e, (size_t)m * E_F))) return rc;
+    if ((rc = dev_alloc(o, &g->e, (size_t)m * E_F + 4))) return rc;
     if (training) {
         if ((rc = dev_alloc(o, &g->target, n * OUT))) return rc;
         for (int l = 0; l <= LAYERS; ++l)
@@ -470,6 +471,8 @@ int cfd_mpnn_forward(cfd_mpnn* net, cfd_mpnn_graph* g, int bf16, double* ux, dou
     CFD_LAUNCH(k_guess, blocks_for(g->n, 256), 256, 0, g->stream, g->n, y, g->kind,
                (const double*)g->gnx, (const double*)g->gny, (const Globals*)g->G, g->ux, g->uy,
                (const int*)nullptr);
+    for (double* h : {ux, uy})
+        if (h) map_result(h, sizeof(double) * g->n);  // while the device works
     if (ux) CFD_CUDA(cudaMemcpyAsync(ux, g->ux, sizeof(double) * g->n, cudaMemcpyDeviceToHost, g->stream));
     if (uy) CFD_CUDA(cudaMemcpyAsync(uy, g->uy, sizeof(double) * g->n, cudaMemcpyDeviceToHost, g->stream));
     int tc_err = 0;

@@ -109,7 +109,7 @@ class Net:
         return loss.value
 
     def forward(self, graph, bf16=True):
-        ux, uy = np.zeros(graph.n), np.zeros(graph.n)
+        ux, uy = np.empty(graph.n), np.empty(graph.n)
         check(abi.lib().cfd_mpnn_forward(self.h, graph.h, int(bool(bf16)), dptr(ux), dptr(uy)),
               "cfd_mpnn_forward")
         return ux, uy

@@ -178,3 +178,34 @@ def test_trained_guess_beats_zero_guess(gpu_lib):
         tot0 += sum(r["iters_zero"])
         tot1 += sum(r["iters_net"])
     assert tot1 < 0.85 * tot0, (tot1, tot0)
+
+
+@pytest.mark.parametrize("hubs,arc,edges", [(0, 1, 384), (5, 67, 1024), (6, 54, 1026), (4, 249, 1868)])
+def test_inference_of_crowded_tiles_matches_mma_sync(gpu_lib, monkeypatch, hubs, arc, edges):
+    """A ring of 250 nodes around a centre, and `hubs` more nodes, the mesh's first, that each see
+    an arc of it: the first tile of 128 nodes has `edges` edges (1,024 are staged in shared
+    memory, more are read from global memory) and degrees between 3 and 250.  The two passes
+    differ in the order of the GEMMs' FP32 sums alone, and so by single BF16 roundings (2^-9) of
+    some activations."""
+    from types import SimpleNamespace
+    from cfd_gb300 import learned, solver
+    ring = hubs + 1 + np.arange(250, dtype=np.int32)
+    n = hubs + 251
+    inp = [(n, ring[k], ring[(k + 1) % 250]) for k in range(250)]
+    inp += [(h + 1, ring[(60 + k) % 250], ring[(61 + k) % 250]) for h in range(hubs) for k in range(arc)]
+    t = 2 * np.pi * np.arange(n) / n
+    case = SimpleNamespace(npoin=n, inpoel=np.array(inp, np.int32), x=np.cos(t) + 0.1 * np.sin(5 * t),
+                           y=0.8 * np.sin(t), i_m=ring[:16], ifm=ring[40:60])
+    p2 = solver.getPsup(case.inpoel, n)[1]
+    assert p2[min(n, 128)] - p2[0] == edges
+    G = learned.Graph(case)
+    rng = np.random.default_rng(arc)
+    G.set_bc(*(0.1 * rng.normal(size=(2, 36))))
+    net = learned.Net((learned.init_weights(3) + 0.02 * rng.normal(size=learned.n_params()))
+                      .astype(np.float32))
+    monkeypatch.setenv("CFD_MPNN_TC", "0")
+    m = np.stack(net.forward(G, bf16=True))
+    monkeypatch.delenv("CFD_MPNN_TC")
+    a, b = np.stack(net.forward(G, bf16=True)), np.stack(net.forward(G, bf16=True))
+    assert np.array_equal(a, b) and np.all(np.isfinite(a))
+    assert np.linalg.norm(a - m) <= 5e-3 * np.linalg.norm(m)
