@@ -80,6 +80,7 @@ struct Ctx {
     cudaEvent_t ev_side[4] = {};
     bool side_join = false;  // the branch still has to wait for ev_side[3]
     cudaEvent_t ev_scal = nullptr;
+    cudaEvent_t ev_tail = nullptr;  // the motion part of the step's k_motion_tail
     StepScal* h_scal = nullptr;  // pinned
     StepOut* h_out = nullptr;    // pinned step report
     StepOut* d_out = nullptr;
@@ -103,6 +104,9 @@ struct Ctx {
     unsigned char* d_bcflag = nullptr;
     double* d_bcval = nullptr;
     double2* d_nrm = nullptr;
+    // mixed form: the next step's, which normales writes beside the RK stages
+    unsigned char* d_bcflag_n = nullptr;
+    double2* d_nrm_n = nullptr;
     int *d_wnode = nullptr, *d_wptr = nullptr;
     int2 *d_wedge = nullptr, *d_walls = nullptr;
     int* d_set_ptr = nullptr;

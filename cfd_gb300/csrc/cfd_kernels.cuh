@@ -164,7 +164,6 @@ struct MotionTailArgs {
     double* part;  // [3 * nset][gridDim.x] per-block force sums
     double4_32a* fgeo; // null, or per set edge the step-start geometry (the motion part writes,
                    // the forces part reads: the mesh may have moved in between)
-    NormalsArgs nv;    // the forces part also runs normales (nv.nwn = 0: not)
     unsigned* count;
     StepScal* sc;
 };
@@ -230,19 +229,20 @@ int node_bulk_smem(const int* esup_ptr_host, int npoin);
 __global__ void k_elem_geometry(int nelem, const int4* elem, const double* X, const double* Y,
                                 int gcl, int literal, const float2* W, const float2* Wold,
                                 int put_area, double* area_old, double* area64, float* areaf,
-                                float4* geo, double* terms, NormalsArgs nv);
+                                float4* geo, double* terms);
 constexpr int kGeoNodeBlock = 128;  // block size of k_node_geometry
 __global__ void k_elem_grad64(int nelem, const int4* elem, const double* X, const double* Y,
                               const int* slot_pos, float2* k64);
 // k_node_geometry (block kGeoNodeBlock); row64 (relative tests): the Laplacian rows summed
-// from k64 (element-matrix rows as double-float pairs, written as valf + val_lo), not from geo
+// from k64 (element-matrix rows as double-float pairs, written as valf + val_lo), not from
+// geo; nv: normales of the same mesh, in blocks of their own after the grid's
 cudaError_t launch_node_geometry(bool row64, unsigned grid, cudaStream_t stream, int npoin,
                                  const int* esup_ptr, const int* esup_slot,
                                  const uchar4* lap_pos, const float4* geo, const double* terms,
                                  const double* dtp, int gcl, const int* rowptr, float* valf,
                                  double* invdiag, float* invdiagf, double* M, float* invM,
                                  const float2* W, float2* Wold, const float2* k64,
-                                 float* val_lo);
+                                 float* val_lo, NormalsArgs nv);
 __global__ void k_widen_geo(int nelem, const float4* geo, double* dN, double* area);
 __global__ void k_motion_update_mixed(int npoin, const double* xpos, const double* ypos,
                                       const StepScal* sc, double* X, double* Y, double* WX,

@@ -89,6 +89,7 @@ Ctx::~Ctx() {
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     if (ev_scal) cudaEventDestroy(ev_scal);
+    if (ev_tail) cudaEventDestroy(ev_tail);
     for (cudaEvent_t e : pool) cudaEventDestroy(e);
     for (auto& m : mark)
         if (m) cudaEventDestroy(m);
@@ -757,6 +758,7 @@ int Ctx::create(const cfd_mesh* m, const cfd_params* p, int precision_mode) {
     }
     CFD_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CFD_CUDA(cudaEventCreateWithFlags(&ev_scal, cudaEventDisableTiming));
+    CFD_CUDA(cudaEventCreateWithFlags(&ev_tail, cudaEventDisableTiming));
     CFD_CUDA(cudaEventCreateWithFlags(&ev_iters, cudaEventDisableTiming));
     CFD_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
     CFD_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
@@ -947,6 +949,8 @@ int Ctx::create(const cfd_mesh* m, const cfd_params* p, int precision_mode) {
         if ((st = dalloc(&d_WX_n, N))) return st;
         if ((st = dalloc(&d_WY_n, N))) return st;
         if ((st = dalloc(&d_Wf_n, N))) return st;
+        if ((st = dalloc(&d_bcflag_n, N))) return st;
+        if ((st = dalloc(&d_nrm_n, N))) return st;
         if ((st = dalloc(&d_fgeo, std::max<size_t>(1, bc.set_elem.size())))) return st;
         if ((st = dalloc(&d_tcount, 4))) return st;
         if ((st = dalloc(&d_node_err, 1))) return st;
@@ -974,8 +978,12 @@ int Ctx::create(const cfd_mesh* m, const cfd_params* p, int precision_mode) {
     // setup geometry: NORMALES, DERIV, MASAS, laplace (ns2DComp.ALE.f90:88-100)
     st = (prec == CFD_PREC_MIXED) ? geometry_mixed(true, true) : geometry(true, true);
     if (st) return st;
-    if (prec != CFD_PREC_MIXED)
+    if (prec != CFD_PREC_MIXED) {
         CFD_CUDA(cudaMemcpyAsync(d_area_old, d_area, sizeof(double) * E, cudaMemcpyDeviceToDevice, stream));
+    } else {  // normales rewrites the wall nodes' entries alone
+        CFD_CUDA(cudaMemcpyAsync(d_bcflag_n, d_bcflag, N, cudaMemcpyDeviceToDevice, stream));
+        CFD_CUDA(cudaMemcpyAsync(d_nrm_n, d_nrm, sizeof(double2) * N, cudaMemcpyDeviceToDevice, stream));
+    }
     CFD_CUDA(cudaStreamSynchronize(stream));
     return tcollect();
 }
@@ -1014,21 +1022,20 @@ int Ctx::geometry_mixed(bool setup, bool put_area, bool to_next, cudaStream_t sv
     const int TB = 256;
     const bool gcl = !setup && prm.mass_mode != CFD_MASS_MASAS;
     // to_next (the step's mesh-motion branch): the next step's geo8, 1/M, with W the next
-    // and W_old the current W (putW by the buffer swap); normales are left to the caller
-    // (the RK stages still read this step's).  Otherwise normales ride on the element pass
-    // (its own blocks after the elements').
+    // and W_old the current W (putW by the buffer swap).  normales ride on the node pass, in
+    // blocks of their own; beside the RK stages, which still read this step's, they write the
+    // next step's flags and normals.
     float4* geo8 = to_next ? d_geo8_n : d_geo8;
     float* invMf = to_next ? d_invMf_n : d_invMf;
     const float2* Wn = to_next ? d_Wf_n : d_Wf;
     const float2* Wo = to_next ? d_Wf : d_Wof;
     tstart(TM_DERIV);
-    const NormalsArgs nv{to_next ? 0 : nwn, d_wnode, d_wptr, d_wedge, d_walls, d_X, d_Y, d_bcflag,
-                         d_nrm};
-    CFD_LAUNCH(k_elem_geometry,
-               nv.nwn > 0 ? blocks_for(E, TB) + blocks_for(nv.nwn, TB) : branch_grid(E, TB, sv), TB,
-               0, stream, E, d_elem, d_X, d_Y, gcl ? 1 : 0,
-               prm.mass_mode == CFD_MASS_GCL_LITERAL ? 1 : 0, Wn, Wo,
-               (gcl || put_area) ? 1 : 0, d_area_old, d_area, d_areaf, geo8, d_gterms, nv);
+    const bool nrm_next = to_next && prm.motion_law != CFD_MOTION_NEWMARK;
+    const NormalsArgs nv{nwn, d_wnode, d_wptr, d_wedge, d_walls, d_X, d_Y,
+                         nrm_next ? d_bcflag_n : d_bcflag, nrm_next ? d_nrm_n : d_nrm};
+    CFD_LAUNCH(k_elem_geometry, branch_grid(E, TB, sv), TB, 0, stream, E, d_elem, d_X, d_Y,
+               gcl ? 1 : 0, prm.mass_mode == CFD_MASS_GCL_LITERAL ? 1 : 0, Wn, Wo,
+               (gcl || put_area) ? 1 : 0, d_area_old, d_area, d_areaf, geo8, d_gterms);
     area_put = gcl || put_area;
     tstop(TM_DERIV);
     tstart(TM_LAPLACE);
@@ -1039,7 +1046,7 @@ int Ctx::geometry_mixed(bool setup, bool put_area, bool to_next, cudaStream_t sv
                                   N, d_esup_ptr, d_esup_slot, d_lap_pos, geo8, d_gterms,
                                   &d_scal->dtmin, gcl ? 1 : 0, d_rowptr, d_valf, d_invdiag,
                                   d_invdiagf, d_M, invMf, Wn, to_next ? (float2*)nullptr : d_Wof,
-                                  (const float2*)d_k64, d_val_lo));
+                                  (const float2*)d_k64, d_val_lo, nv));
     tstop(TM_LAPLACE);
     return CFD_OK;
 }
@@ -1066,7 +1073,7 @@ int Ctx::enqueue_mixed(bool learned) {
     // The mesh motion of a prescribed law needs DTMIN and the step-start mesh only, and
     // what it produces (the moved mesh, W, the new geometry) is the next step's: it runs
     // on its own stream beside the RK stages, writing the next-step buffers (swapped after
-    // the step), and joins before FORCES.  The Newmark law needs this step's forces: its
+    // the step), and joins at its end.  The Newmark law needs this step's forces: its
     // motion follows them on the main stream.
     const bool structural = prm.motion_law == CFD_MOTION_NEWMARK;
     const bool fork = !timers_on && !structural;
@@ -1115,6 +1122,7 @@ int Ctx::enqueue_mixed(bool learned) {
         m.count = d_tcount + 1;
         tstart(TM_FORCES);
         CFD_LAUNCH(k_motion_tail, (unsigned)tail_blocks, 256, 0, s, m);
+        CFD_CUDA(cudaEventRecord(ev_tail, s));
         tstop(TM_FORCES);
         tstart(TM_GRAD);
         int st = run_pcg(2, learned, true, s);
@@ -1174,24 +1182,17 @@ int Ctx::enqueue_mixed(bool learned) {
     if (structural) {
         if ((st = motion(stream))) return st;
     } else {
-        // FORCES on the step's pressure and the step-start edge geometry
-        if (fork) CFD_CUDA(cudaStreamWaitEvent(stream, ev_join, 0));
+        // FORCES on the step's pressure and the step-start edge geometry, which the motion
+        // part has kept: beside the end of the mesh motion
+        if (fork) CFD_CUDA(cudaStreamWaitEvent(stream, ev_tail, 0));
         MotionTailArgs f = t;
         f.do_motion = 0;
         f.do_forces = 1;
         f.count = d_tcount + 2;
-        if (prm.moving == 1)  // normales of the moved mesh ride on this launch
-            f.nv = NormalsArgs{nwn, d_wnode, d_wptr, d_wedge, d_walls, d_X, d_Y, d_bcflag, d_nrm};
         tstart(TM_FORCES);
         CFD_LAUNCH(k_motion_tail, (unsigned)tail_blocks, 256, 0, stream, f);
         tstop(TM_FORCES);
-    }
-    if (prm.moving == 1 && structural) {  // normales of the moved mesh (the Newmark path)
-        tstart(TM_NORMALES);
-        if (nwn > 0)
-            CFD_LAUNCH(k_normales, blocks_for(nwn, TB), TB, 0, stream, nwn, d_wnode, d_wptr, d_wedge,
-                       d_walls, d_X, d_Y, d_bcflag, d_nrm);
-        tstop(TM_NORMALES);
+        if (fork) CFD_CUDA(cudaStreamWaitEvent(stream, ev_join, 0));
     }
     if (fv_each) {  // FORCE_VISC at the print block's point: moved mesh, this step's dNx
         st = force_visc_now();
@@ -1231,6 +1232,10 @@ void Ctx::swap_mixed_buffers() {
         area_put = prm.mass_mode != CFD_MASS_MASAS;  // also of a replayed step
         std::swap(d_geo8, d_geo8_n);
         std::swap(d_invMf, d_invMf_n);
+        if (prm.motion_law != CFD_MOTION_NEWMARK) {
+            std::swap(d_bcflag, d_bcflag_n);
+            std::swap(d_nrm, d_nrm_n);
+        }
     }
     buf ^= 1;
 }

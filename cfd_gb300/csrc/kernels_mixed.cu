@@ -764,17 +764,8 @@ __global__ void k_elem_geometry(int nelem, const int4* __restrict__ elem,
                                 const float2* __restrict__ Wold, int put_area,
                                 double* __restrict__ area_old, double* __restrict__ area64,
                                 float* __restrict__ areaf, float4* __restrict__ geo,
-                                double* __restrict__ terms, NormalsArgs nv) {
-    // the blocks after the elements' do normales (one wall node per thread)
-    const int eblocks = (nelem + blockDim.x - 1) / blockDim.x;
-    if (nv.nwn > 0 && (int)blockIdx.x >= eblocks) {
-        const int k = ((int)blockIdx.x - eblocks) * blockDim.x + threadIdx.x;
-        if (k < nv.nwn) normales_node(nv, k);
-        return;
-    }
-    // grid-stride over the elements (the normales blocks, when any, follow eblocks blocks)
-    const int estride = (nv.nwn > 0 ? eblocks : (int)gridDim.x) * blockDim.x;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nelem; e += estride) {
+                                double* __restrict__ terms) {
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nelem; e += gridDim.x * blockDim.x) {
     const int4 n = elem[e];
     const double X0 = X[n.x], Y0 = Y[n.x];
     const double dx1 = X[n.y] - X0, dy1 = Y[n.y] - Y0;
@@ -866,6 +857,20 @@ __device__ __forceinline__ DF df_of(double v) {
 // written as valf + val_lo (the pair's h and l); the FP32 geometry is then read only for
 // MASAS.
 constexpr int kLapRow = 16;
+// two float4 of a 32-byte aligned record in one load: half as many passes of the L1's tags
+// over a warp of scattered records
+__device__ __forceinline__ void load32(const float4* p, float4& a, float4& b) {
+    const double4_32a v = *reinterpret_cast<const double4_32a*>(p);
+    auto f = [](double d, float& x, float& y) {
+        const long long u = __double_as_longlong(d);
+        x = __int_as_float((int)u);
+        y = __int_as_float((int)(u >> 32));
+    };
+    f(v.x, a.x, a.y);
+    f(v.y, a.z, a.w);
+    f(v.z, b.x, b.y);
+    f(v.w, b.z, b.w);
+}
 constexpr int kGeoBatch = 2;  // slots per pass of k_node_geometry
 constexpr int kGeoBlock = kGeoNodeBlock;
 
@@ -879,26 +884,42 @@ k_node_geometry(int npoin, const int* __restrict__ esup_ptr, const int* __restri
                 double* __restrict__ invdiag, float* __restrict__ invdiagf,
                 double* __restrict__ M, float* __restrict__ invM,
                 const float2* __restrict__ W, float2* __restrict__ Wold,
-                const float2* __restrict__ k64, float* __restrict__ val_lo) {
-    __shared__ float row[ROW64 ? 1 : kGeoBlock][kLapRow + 1];
-    __shared__ float2 row64[ROW64 ? kGeoBlock : 1][kLapRow + 1];
+                const float2* __restrict__ k64, float* __restrict__ val_lo, NormalsArgs nv) {
+    __shared__ float row[kGeoBlock / 32][ROW64 ? 1 : 32 * kLapRow];
+    __shared__ float2 row64[kGeoBlock / 32][ROW64 ? 32 * kLapRow : 1];
     const bool need_geo = !ROW64 || !gcl;
-    // grid-stride (a smaller grid leaves room for kernels running beside it)
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npoin; p += gridDim.x * blockDim.x) {
-    float* acc = row[ROW64 ? 0 : threadIdx.x];
-    float2* acc64 = row64[ROW64 ? threadIdx.x : 0];
-    const int r0 = rowptr[p], r1 = rowptr[p + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // the last blocks do normales (one wall node per thread)
+    const int nblocks = (int)gridDim.x - (nv.nwn + kGeoBlock - 1) / kGeoBlock;
+    if ((int)blockIdx.x >= nblocks) {
+        const int k = ((int)blockIdx.x - nblocks) * kGeoBlock + threadIdx.x;
+        if (k < nv.nwn) normales_node(nv, k);
+        return;
+    }
+    // grid-stride (a smaller grid leaves room for kernels running beside it); a warp takes 32
+    // nodes, sums their rows, which are one run of the matrix, in shared memory and writes
+    // the run out in whole sectors
+    for (int pw = blockIdx.x * kGeoBlock + 32 * warp; pw < npoin; pw += nblocks * kGeoBlock) {
+    const int p = pw + lane;
+    const bool live = p < npoin;
+    const int r0 = rowptr[min(p, npoin)], r1 = rowptr[min(p + 1, npoin)];
+    const int base = __shfl_sync(0xffffffffu, r0, 0), total = __shfl_sync(0xffffffffu, r1, 31) - base;
     const int len = r1 - r0;
-    const bool in_smem = len <= kLapRow;
-    if (ROW64) {
-        if (in_smem)
-            for (int k = 0; k < len; ++k) acc64[k] = make_float2(0.f, 0.f);
-    } else if (in_smem) {
-#pragma unroll
-        for (int k = 0; k < kLapRow; ++k) acc[k] = 0.f;
-    } else {
+    const bool in_smem = total <= 32 * kLapRow;
+    float* run = row[warp];
+    float2* run64 = row64[warp];
+    float* acc = run + (ROW64 || !in_smem ? 0 : r0 - base);
+    float2* acc64 = run64 + (ROW64 && in_smem ? r0 - base : 0);
+    if (in_smem) {
+        for (int k = lane; k < total; k += 32) {
+            if (ROW64) run64[k] = make_float2(0.f, 0.f);
+            else run[k] = 0.f;
+        }
+        __syncwarp();
+    } else if (!ROW64) {
         for (int k = r0; k < r1; ++k) valf[k] = 0.f;
     }
+    if (live) {
     Acc m1;
     m1.init();
     double tot = 0.0;  // gcl: (tot1 + tot2) times 3
@@ -926,10 +947,7 @@ k_node_geometry(int npoin, const int* __restrict__ esup_ptr, const int* __restri
         for (int u = 0; u < kGeoBatch; ++u)
             if (sb + u < s1) {
                 const int e = slot[u] / 3;
-                if (need_geo) {
-                    ga[u] = geo[2 * (size_t)e];
-                    gb[u] = geo[2 * (size_t)e + 1];
-                }
+                if (need_geo) load32(geo + 2 * (size_t)e, ga[u], gb[u]);
                 if (gcl) tm[u] = terms[e];
             }
 #pragma unroll
@@ -966,10 +984,6 @@ k_node_geometry(int npoin, const int* __restrict__ esup_ptr, const int* __restri
     if (ROW64) {
         float diag;
         if (in_smem) {
-            for (int k = 0; k < len; ++k) {
-                valf[r0 + k] = acc64[k].x;
-                val_lo[r0 + k] = acc64[k].y;
-            }
             diag = acc64[0].x;
         } else {  // long rows (rare): one pass over the slots per entry
             diag = 0.f;
@@ -990,12 +1004,7 @@ k_node_geometry(int npoin, const int* __restrict__ esup_ptr, const int* __restri
         idf = 1.f / diag;  // the Jacobi scaling is FP32 in every pass
     } else {
         float diag;
-        if (in_smem) {
-            for (int k = 0; k < len; ++k) valf[r0 + k] = acc[k];
-            diag = acc[0];
-        } else {
-            diag = valf[r0];
-        }
+        diag = in_smem ? acc[0] : valf[r0];
         idf = 1.f / diag;
     }
     invdiagf[p] = idf;
@@ -1010,6 +1019,15 @@ k_node_geometry(int npoin, const int* __restrict__ esup_ptr, const int* __restri
     M[p] = m;
     invM[p] = 1.f / d2f_trunc(m);
     }
+    if (in_smem) {
+        __syncwarp();
+        for (int k = lane; k < total; k += 32) {
+            valf[base + k] = ROW64 ? run64[k].x : run[k];
+            if (ROW64) val_lo[base + k] = run64[k].y;
+        }
+        __syncwarp();
+    }
+    }
 }
 cudaError_t launch_node_geometry(bool row64, unsigned grid, cudaStream_t stream, int npoin,
                                  const int* esup_ptr, const int* esup_slot,
@@ -1017,15 +1035,16 @@ cudaError_t launch_node_geometry(bool row64, unsigned grid, cudaStream_t stream,
                                  const double* dtp, int gcl, const int* rowptr, float* valf,
                                  double* invdiag, float* invdiagf, double* M, float* invM,
                                  const float2* W, float2* Wold, const float2* k64,
-                                 float* val_lo) {
+                                 float* val_lo, NormalsArgs nv) {
+    grid += blocks_for(nv.nwn, kGeoBlock) * (nv.nwn > 0);
     if (row64)
         k_node_geometry<true><<<grid, kGeoBlock, 0, stream>>>(
             npoin, esup_ptr, esup_slot, lap_pos, geo, terms, dtp, gcl, rowptr, valf, invdiag,
-            invdiagf, M, invM, W, Wold, k64, val_lo);
+            invdiagf, M, invM, W, Wold, k64, val_lo, nv);
     else
         k_node_geometry<false><<<grid, kGeoBlock, 0, stream>>>(
             npoin, esup_ptr, esup_slot, lap_pos, geo, terms, dtp, gcl, rowptr, valf, invdiag,
-            invdiagf, M, invM, W, Wold, k64, val_lo);
+            invdiagf, M, invM, W, Wold, k64, val_lo, nv);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return cudaGetLastError();
 }
@@ -1208,8 +1227,6 @@ __global__ void __launch_bounds__(256) k_motion_tail(MotionTailArgs a) {
     const int gs = gridDim.x * blockDim.x;
     auto first = [&](int w0) { return ((t - w0) & 255) * (int)gridDim.x + (int)blockIdx.x; };
     if (a.do_motion && !structural) tail_transf(a, mv, first(0), first(64), gs);
-    if (a.do_forces)  // normales of the moved mesh, for the next step's wall condition
-        for (int k = first(128); k < a.nv.nwn; k += gs) normales_node(a.nv, k);
     if (a.do_motion && a.fgeo)  // the edge geometry FORCES will need, before the mesh moves
         for (int k = first(128); k < a.set_ptr[a.nset]; k += gs) {
             const int2 ed = a.set_edges[k];
