@@ -1209,18 +1209,14 @@ unsigned Ctx::branch_grid(long n, int threads, cudaStream_t s) const {
     return std::min<unsigned>(full, (unsigned)(branch_bpsm * nsm));
 }
 
-// Grid of the BiCG row kernels (256 threads) over nblk 256-row groups: beside the RK stages, 4
-// blocks per SM.  5, as the other branch kernels have, is more than stay resident with the
-// FP32 kernels' registers, so that every fifth block ran in a second wave of its own
-// (k_bicg_resid_mixed at 1M nodes alone: 49 us on 5, 35 on 4); whole steps on 3, 4, 6: 0.536,
-// 0.535, 0.534 ms at 1M nodes, 1.66, 1.61, 1.72 at 3.1M, 0.591, 0.566, 0.570 at 590k (host
-// coupled).  The relative tests' precise passes stay on branch_bpsm (6.03 against 5.93 ms per
-// 20 steps of 262,144 nodes): the grid is part of the order of their sums, and their long
-// solves amplify its last bit.
+// Grid of the BiCG row kernels (256 threads) over nblk 256-row groups: beside the RK stages,
+// branch_bpsm blocks per SM.  The grid is part of the order of the kernels' sums, and long solves
+// amplify a sum's last bit, so that it stays what it is; with batches of 3 the FP32 kernels need
+// 48 and 40 registers, and 5 blocks are resident (k_bicg_resid_mixed at 1M nodes alone: 49 us with
+// batches of 8 and a second wave of every fifth block, 35 us so, 38 us on 4 blocks per SM).
 unsigned Ctx::row_grid(long nblk, cudaStream_t s) const {
     if (!s || branch_bpsm <= 0) return (unsigned)nblk;
-    const int per_sm = prm.bicg_tol_mode == CFD_BICG_TOL_ABS ? 4 : branch_bpsm;
-    return (unsigned)std::min<long>(nblk, (long)per_sm * nsm);
+    return (unsigned)std::min<long>(nblk, (long)branch_bpsm * nsm);
 }
 
 // The next-step buffers become the current ones (after each mixed step)

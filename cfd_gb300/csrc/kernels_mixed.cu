@@ -871,6 +871,10 @@ __device__ __forceinline__ void load32(const float4* p, float4& a, float4& b) {
     f(v.z, b.x, b.y);
     f(v.w, b.z, b.w);
 }
+// Bound by the L1's passes over its scattered gathers: a record is one 256-bit load, and a warp's
+// 32 rows are summed in shared memory and written out as one run.  84 -> 69 us alone at
+// 1,048,576 nodes.  Batches of 2 slots: 3 and 4 need 72 and 95 registers, which the RK
+// kernels beside it miss (whole steps 515, 530, 540 us).
 constexpr int kGeoBatch = 2;  // slots per pass of k_node_geometry
 constexpr int kGeoBlock = kGeoNodeBlock;
 

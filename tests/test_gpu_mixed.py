@@ -181,3 +181,43 @@ def test_full_size_mixed_learned_matches_fp64(gpu_lib):
     f.close()
     m.close()
     net.close()
+
+
+def two_hubs(m):
+    """Two fans over one line of m points: the hubs are nodes 1 and 2, the line's points follow."""
+    from test_edge_cases import square
+    y = np.linspace(-1.0, 1.0, m)
+    t = np.pi * (np.arange(m) + 0.5) / m
+    x = np.concatenate([[-0.5, 0.5], 0.0 * y, -np.sin(t) - 0.1, np.sin(t) + 0.1])
+    y = np.concatenate([[0.0, 0.0], y, -np.cos(t), -np.cos(t)])
+    line, left, right = (3 + s * m + np.arange(m) for s in range(3))
+    tri = []
+    for hub, loop in ((1, np.concatenate([line, left[::-1]])), (2, np.concatenate([line[::-1], right]))):
+        tri += [(hub, a, b) for a, b in zip(loop, np.roll(loop, -1))]
+    k, _ = square(2, perturbed=False)
+    k.x, k.y, k.inpoel = x, y, np.array(tri, np.int32)
+    return k
+
+
+@pytest.mark.parametrize("m", [40, 89, 90, 125])
+@pytest.mark.parametrize("rel_test", [False, True])
+def test_laplacian_rows_of_hubs(gpu_lib, m, rel_test):
+    """The first 32 rows of the mesh-motion matrix hold 4 m + 153 entries (313 to 653): up to
+    512 a warp of the node pass sums them in shared memory.  An element matrix entry is q times
+    a product of gradients, with q and the gradients from an area that a sliver's edges cancel in
+    (aspect up to 100): 2^-24 of FP32 grows to ~1e-5 of a row, 2^-46 of the pairs to ~1e-11."""
+    from cfd_gb300 import abi, solver
+    from oracle import oracle as O
+    k = two_hubs(m)
+    if rel_test:
+        k.params.bicg_tol_mode = abi.CFD_BICG_TOL_REL
+    s = solver.Solver(k, precision=abi.CFD_PREC_MIXED)
+    v = s.laplace_values()
+    s.close()
+    g = O.deriv(k.x, k.y, k.inpoel)
+    assert g["area"].min() > 0
+    rp, idx = O.laplace_pattern(k.inpoel, k.npoin)
+    ref, _ = O.laplace(k.inpoel, g["dNx"], g["dNy"], k.x, k.y, rp, idx)
+    assert rp[32] == 4 * m + 153
+    scale = np.repeat(np.maximum.reduceat(np.abs(ref), rp[:-1]), np.diff(rp))
+    assert np.all(np.abs(v - ref) <= (1e-9 if rel_test else 1e-4) * scale)
