@@ -415,6 +415,7 @@ int cfd_ctx_upload_mesh(cfd_ctx* ctx, const double* X, const double* Y, const do
     if (!ctx) return arg_error("ctx");
     Ctx& c = ctx->impl;
     const size_t n8 = 8 * (size_t)c.npoin;
+    if (c.prec != CFD_PREC_MIXED) TRY(c.keep_put());
     if (X) CFD_CUDA(cudaMemcpyAsync(c.d_X, X, n8, cudaMemcpyHostToDevice, c.stream));
     if (Y) CFD_CUDA(cudaMemcpyAsync(c.d_Y, Y, n8, cudaMemcpyHostToDevice, c.stream));
     if (W_X) CFD_CUDA(cudaMemcpyAsync(c.d_WX, W_X, n8, cudaMemcpyHostToDevice, c.stream));
@@ -1083,7 +1084,8 @@ int cfd_gcl(double* M, const double* W_x, const double* W_y, const double* W_x_o
     TRY(s.alloc(&d_terms, E));
     TRY(m.check(s, inpoel, E, N));
     CFD_CUDA(launch_gcl(s.stream, N, E, m.el, m.ptr, m.slot, d_geo, d_a, d_ao, d_wx, d_wy, d_wxo,
-                        d_wyo, d_dt, mode == CFD_MASS_GCL_LITERAL ? 1 : 0, d_terms, d_M));
+                        d_wyo, d_dt, mode == CFD_MASS_GCL_LITERAL ? 1 : 0, d_terms, d_M,
+                        d_M));
     TRY(s.get(M, d_M, N));
     return s.sync();
 }

@@ -129,6 +129,12 @@ struct Ctx {
     double *d_WX = nullptr, *d_WY = nullptr, *d_M = nullptr, *d_Wxo = nullptr, *d_Wyo = nullptr;
     double *d_area = nullptr, *d_area_old = nullptr, *d_geo = nullptr, *d_DT = nullptr,
            *d_DTL = nullptr;
+    // FP64 form: what the mesh motion writes beside the RK stages, for the next step (the pointers
+    // are swapped); put_is_current: putW's and putArea's values are the current W and area,
+    // not yet copied to d_Wxo, d_Wyo, d_area_old
+    double *d_X_n = nullptr, *d_Y_n = nullptr, *d_M_n = nullptr, *d_area_n = nullptr, *d_geo_n = nullptr;
+    bool put_is_current = false;
+    cudaEvent_t ev_forces = nullptr;
     bool area_put = false;  // mixed form: the current area is in d_area_old (putArea), not d_area
     double *d_SHOC = nullptr, *d_TS1 = nullptr, *d_TS2 = nullptr, *d_TS3 = nullptr;
     double *d_contrib = nullptr, *d_contribF = nullptr;
@@ -233,7 +239,8 @@ struct Ctx {
 
     ~Ctx();
     int create(const cfd_mesh* m, const cfd_params* p, int precision_mode);
-    int geometry(bool masas, bool with_laplace);
+    int geometry(bool masas, bool with_laplace, bool to_next = false, cudaStream_t sv = nullptr);
+    int keep_put();
     int geometry_mixed(bool setup, bool put_area = false, bool to_next = false,
                        cudaStream_t sv = nullptr);
     void swap_mixed_buffers();

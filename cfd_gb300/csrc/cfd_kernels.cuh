@@ -266,7 +266,7 @@ cudaError_t launch_gcl(cudaStream_t st, int npoin, int nelem, const int4* elem,
                        const int* esup_ptr, const int* esup_slot, const double* geo,
                        const double* area, const double* area_old, const double* Wx,
                        const double* Wy, const double* Wxo, const double* Wyo, const double* dtp,
-                       int literal, double2* scratch, double* M);
+                       int literal, double2* scratch, const double* M, double* M_out);
 __global__ void k_deltat(int nelem, const int4* elem, const double* T, const double* VX,
                          const double* VY, const double* WX, const double* WY,
                          const double* area, double fsafe, Rcp t_inf, double* DT,
@@ -364,8 +364,8 @@ __global__ void k_transf(int nnmove, const int* fix_node, const int* fix_set, co
                          const double* Y, const double* xref, const double* yref, double ca,
                          double sa, double yposr, double* xfix_x, double* xfix_y);
 __global__ void k_motion_update(int npoin, const double* xpos, const double* ypos,
-                                const StepScal* sc, double* X, double* Y, double* WX,
-                                double* WY);
+                                const StepScal* sc, const double* X0, const double* Y0, double* X,
+                                double* Y, double* WX, double* WY);
 
 // ------------------------------------------------------------------ PCG
 struct PcgArgs {

@@ -90,6 +90,7 @@ Ctx::~Ctx() {
     if (ev_join) cudaEventDestroy(ev_join);
     if (ev_scal) cudaEventDestroy(ev_scal);
     if (ev_tail) cudaEventDestroy(ev_tail);
+    if (ev_forces) cudaEventDestroy(ev_forces);
     for (cudaEvent_t e : pool) cudaEventDestroy(e);
     for (auto& m : mark)
         if (m) cudaEventDestroy(m);
@@ -101,29 +102,45 @@ Ctx::~Ctx() {
 }
 
 // ------------------------------------------------------------------ geometry of the mesh
-int Ctx::geometry(bool masas, bool with_laplace) {
+// to_next (the step): into the next step's dN, area, M, on stream sv; normales are the caller's
+int Ctx::geometry(bool masas, bool with_laplace, bool to_next, cudaStream_t sv) {
+    const cudaStream_t stream = sv ? sv : this->stream;
     const int N = npoin, E = nelem;
     const int TB = 256;
-    tstart(TM_NORMALES);
-    if (nwn > 0)
-        CFD_LAUNCH(k_normales, blocks_for(nwn, TB), TB, 0, stream, nwn, d_wnode, d_wptr,
-                   d_wedge, d_walls, d_X, d_Y, d_bcflag, d_nrm);
-    tstop(TM_NORMALES);
+    double *geo = to_next ? d_geo_n : d_geo, *area = to_next ? d_area_n : d_area;
+    if (!to_next) {
+        tstart(TM_NORMALES);
+        if (nwn > 0)
+            CFD_LAUNCH(k_normales, blocks_for(nwn, TB), TB, 0, stream, nwn, d_wnode, d_wptr,
+                       d_wedge, d_walls, d_X, d_Y, d_bcflag, d_nrm);
+        tstop(TM_NORMALES);
+    }
     tstart(TM_DERIV);
-    CFD_LAUNCH(k_deriv, blocks_for(E, TB), TB, 0, stream, E, d_elem, d_X, d_Y, d_area, d_geo,
+    CFD_LAUNCH(k_deriv, blocks_for(E, TB), TB, 0, stream, E, d_elem, d_X, d_Y, area, geo,
                (double*)nullptr, (double*)nullptr, (double*)nullptr);
     tstop(TM_DERIV);
     if (masas) {
         tstart(TM_MASAS);
-        CFD_LAUNCH(k_mass, blocks_for(N, TB), TB, 0, stream, N, d_esup_ptr, d_esup_slot, d_area, d_M);
+        CFD_LAUNCH(k_mass, blocks_for(N, TB), TB, 0, stream, N, d_esup_ptr, d_esup_slot, area,
+                   to_next ? d_M_n : d_M);
         tstop(TM_MASAS);
     }
     if (with_laplace) {
         tstart(TM_LAPLACE);
-        CFD_CUDA(launch_laplace(stream, N, E, d_elem, d_esup_ptr, d_esup_slot, d_lap_pos, d_geo,
+        CFD_CUDA(launch_laplace(stream, N, E, d_elem, d_esup_ptr, d_esup_slot, d_lap_pos, geo,
                                 d_X, d_Y, d_rowptr, d_lapq, d_val, d_diag));
         tstop(TM_LAPLACE);
     }
+    return CFD_OK;
+}
+
+// Before the current W or area change other than by a step: putW's, putArea's copies
+int Ctx::keep_put() {
+    if (!put_is_current) return CFD_OK;
+    put_is_current = false;
+    CFD_CUDA(cudaMemcpyAsync(d_Wxo, d_WX, sizeof(double) * npoin, cudaMemcpyDeviceToDevice, stream));
+    CFD_CUDA(cudaMemcpyAsync(d_Wyo, d_WY, sizeof(double) * npoin, cudaMemcpyDeviceToDevice, stream));
+    CFD_CUDA(cudaMemcpyAsync(d_area_old, d_area, sizeof(double) * nelem, cudaMemcpyDeviceToDevice, stream));
     return CFD_OK;
 }
 
@@ -463,6 +480,7 @@ int Ctx::smooth(int* iters, double* min_quality, bool node_order) {
     if (prec == CFD_PREC_MIXED) {
         if ((st = geometry_mixed(true, true))) return st;
     } else {
+        if ((st = keep_put())) return st;
         if ((st = geometry(true, true))) return st;
         CFD_CUDA(cudaMemcpyAsync(d_area_old, d_area, sizeof(double) * nelem,
                                  cudaMemcpyDeviceToDevice, stream));
@@ -549,6 +567,14 @@ int Ctx::step_once() {
         dtl_arr = d_DTL;
     }
     const double* dtl_scalar = &d_scal->dtmin;
+    // The mesh motion of a prescribed law needs DTMIN and the step-start mesh only, and what it
+    // produces is the next step's: it runs on its own stream beside the RK stages and writes the
+    // next step's buffers, and FORCES, one block, runs on a third stream beside the next step's
+    // first passes.  Small meshes leave most of the GPU free (8,192 nodes: STEP8); at 1,048,576
+    // nodes the RK stages fill it and the gain is what the serial FORCES and the solves' waits
+    // took (STEP1M).
+    const bool smooth_now = smooth_every > 0 && iter % smooth_every == 0;
+    const bool fork = !timers_on && prm.motion_law != CFD_MOTION_NEWMARK && !smooth_now && !fv_each;
     // RK (subrutinas.f90:645-849): ESTAB once, then 4 stages of calcRHS+FUENTE and update
     tstart(TM_ESTAB);
     CFD_LAUNCH(k_estab, blocks_for(E, 128), 128, 0, stream, E, d_elem, d_U, d_T,
@@ -560,6 +586,7 @@ int Ctx::step_once() {
     GasConst gc{prm.fcv, prm.fk, prm.fmu, prm.gama, prm.t_inf, prm.cte, prm.fr};
     const bool viscous = prm.fmu > 2.2250738585072014e-308;
     const int NRK = 4;
+    CFD_CUDA(cudaStreamWaitEvent(stream, ev_forces, 0));  // the last step's FORCES reads P
     for (int irk = 1; irk <= NRK; ++irk) {
         const double rk_fact = 1.0 / (NRK + 1 - irk);
         // calcRHS and FUENTE see the step-start U in every stage (subrutinas.f90:685,
@@ -584,15 +611,24 @@ int Ctx::step_once() {
         CFD_CUDA(launch_node_stage(stream, irk, na));
         tstop(TM_UPDATE);
     }
+    // FORCES on the step's pressure and the step-start mesh
+    const cudaStream_t fs = fork ? stream3 : stream;
+    if (fork) {
+        CFD_CUDA(cudaEventRecord(ev_fork, stream));
+        CFD_CUDA(cudaStreamWaitEvent(fs, ev_fork, 0));
+    }
+    tstart(TM_FORCES);
+    CFD_LAUNCH(k_forces, 1, 256, 0, fs, bc.nset_numb, d_set_ptr, d_set_edges, d_P, d_X, d_Y,
+               d_xref, d_yref, d_scal);
+    tstop(TM_FORCES);
+    // the last step's FORCES, before this step's mesh takes the buffers that it reads
+    if (fork) CFD_CUDA(cudaStreamWaitEvent(stream2, ev_forces, 0));
+    if (fork) CFD_CUDA(cudaEventRecord(ev_forces, fs));
     // fluidStructure (meshMove.f90:28-142) needs TIME: the host reads DTMIN
     CFD_CUDA(cudaEventSynchronize(ev_scal));
     const double dtmin = h_scal->dtmin;
     time = time + dtmin;
     last_dtmin = dtmin;
-    tstart(TM_FORCES);
-    CFD_LAUNCH(k_forces, 1, 256, 0, stream, bc.nset_numb, d_set_ptr, d_set_edges, d_P, d_X, d_Y,
-               d_xref, d_yref, d_scal);
-    tstop(TM_FORCES);
     const double PI = std::acos(-1.0);
     double alphav = disn[1], yposrv = disn[0];
     if (prm.motion_law == CFD_MOTION_HARMONIC) {
@@ -616,46 +652,63 @@ int Ctx::step_once() {
     }
     const double alpha = disn[1] - alphav, yposr = disn[0] - yposrv;
     const double ca = std::cos(alpha), sa = std::sin(alpha);
+    // the mesh motion's stream; beside the RK stages it starts from DTMIN
+    const cudaStream_t b = fork ? stream2 : stream;
+    if (fork) CFD_CUDA(cudaStreamWaitEvent(b, ev_scal, 0));
     tstart(TM_TRANSF);
     if (nnmove > 0)
-        CFD_LAUNCH(k_transf, blocks_for(nnmove, TB), TB, 0, stream, nnmove, d_fix_node, d_fix_set,
+        CFD_LAUNCH(k_transf, blocks_for(nnmove, TB), TB, 0, b, nnmove, d_fix_node, d_fix_set,
                    d_X, d_Y, d_xref, d_yref, ca, sa, yposr, d_xfix[0], d_xfix[1]);
     tstop(TM_TRANSF);
     if (prm.guess_mode == CFD_GUESS_ZERO) {
-        CFD_CUDA(cudaMemsetAsync(d_pos[0], 0, sizeof(double) * N, stream));
-        CFD_CUDA(cudaMemsetAsync(d_pos[1], 0, sizeof(double) * N, stream));
+        CFD_CUDA(cudaMemsetAsync(d_pos[0], 0, sizeof(double) * N, b));
+        CFD_CUDA(cudaMemsetAsync(d_pos[1], 0, sizeof(double) * N, b));
     }
     tstart(TM_GRAD);
-    int st = run_pcg(2);
+    int st = run_pcg(2, false, false, b);
     if (st) return st;
     tstop(TM_GRAD);
-    CFD_LAUNCH(k_motion_update, blocks_for(N, TB), TB, 0, stream, N, d_pos[0], d_pos[1], d_scal,
-               d_X, d_Y, d_WX, d_WY);
-    if (smooth_every > 0 && iter % smooth_every == 0) {
-        st = smooth_in_step(stream, d_WX, d_WY, nullptr);
-        if (st) return st;
-    }
+    CFD_LAUNCH(k_motion_update, blocks_for(N, TB), TB, 0, b, N, d_pos[0], d_pos[1], d_scal,
+               d_X, d_Y, d_X_n, d_Y_n, d_WX_n, d_WY_n);
+    std::swap(d_X, d_X_n);
+    std::swap(d_Y, d_Y_n);
+    std::swap(d_WX, d_WX_n);
+    std::swap(d_WY, d_WY_n);
+    if (smooth_now && (st = smooth_in_step(b, d_WX, d_WY, nullptr))) return st;
     if (fv_each) {  // FORCE_VISC at the print block's point: moved mesh, previous dNx
         st = force_visc_now();
         if (st) return st;
     }
     if (prm.moving == 1) {  // ns2DComp.ALE.f90:259-275
-        st = geometry(prm.mass_mode == CFD_MASS_MASAS, false);
-        if (st) return st;
-        if (prm.mass_mode != CFD_MASS_MASAS) {  // gcl main, then putW/putArea
+        const bool masas = prm.mass_mode == CFD_MASS_MASAS;
+        if ((st = geometry(masas, false, true, b))) return st;
+        if (!masas) {  // gcl main, then putW/putArea: the swapped W and area
             tstart(TM_MASAS);
-            CFD_CUDA(launch_gcl(stream, N, E, d_elem, d_esup_ptr, d_esup_slot, d_geo, d_area,
-                                d_area_old, d_WX, d_WY, d_Wxo, d_Wyo, &d_scal->dtmin,
-                                prm.mass_mode == CFD_MASS_GCL_LITERAL ? 1 : 0, d_gcl64, d_M));
-            CFD_CUDA(cudaMemcpyAsync(d_Wxo, d_WX, sizeof(double) * N, cudaMemcpyDeviceToDevice, stream));
-            CFD_CUDA(cudaMemcpyAsync(d_Wyo, d_WY, sizeof(double) * N, cudaMemcpyDeviceToDevice, stream));
-            CFD_CUDA(cudaMemcpyAsync(d_area_old, d_area, sizeof(double) * E, cudaMemcpyDeviceToDevice, stream));
+            CFD_CUDA(launch_gcl(b, N, E, d_elem, d_esup_ptr, d_esup_slot, d_geo_n, d_area_n,
+                                put_is_current ? d_area : d_area_old, d_WX, d_WY,
+                                put_is_current ? d_WX_n : d_Wxo, put_is_current ? d_WY_n : d_Wyo,
+                                &d_scal->dtmin, prm.mass_mode == CFD_MASS_GCL_LITERAL ? 1 : 0,
+                                d_gcl64, d_M, d_M_n));
+            put_is_current = true;
             tstop(TM_MASAS);
         }
         tstart(TM_LAPLACE);
-        CFD_CUDA(launch_laplace(stream, N, E, d_elem, d_esup_ptr, d_esup_slot, d_lap_pos, d_geo,
+        CFD_CUDA(launch_laplace(b, N, E, d_elem, d_esup_ptr, d_esup_slot, d_lap_pos, d_geo_n,
                                 d_X, d_Y, d_rowptr, d_lapq, d_val, d_diag));
         tstop(TM_LAPLACE);
+        std::swap(d_geo, d_geo_n);
+        std::swap(d_area, d_area_n);
+        std::swap(d_M, d_M_n);
+    }
+    if (fork) {
+        CFD_CUDA(cudaEventRecord(ev_join, b));
+        CFD_CUDA(cudaStreamWaitEvent(stream, ev_join, 0));
+    }
+    if (prm.moving == 1 && nwn > 0) {  // the RK stages have read this step's flags and normals
+        tstart(TM_NORMALES);
+        CFD_LAUNCH(k_normales, blocks_for(nwn, TB), TB, 0, stream, nwn, d_wnode, d_wptr, d_wedge,
+                   d_walls, d_X, d_Y, d_bcflag, d_nrm);
+        tstop(TM_NORMALES);
     }
     std::swap(d_U, d_U1);  // U = U1 (:277-281)
     bandera_host += 1;
@@ -668,6 +721,7 @@ int Ctx::step(int nsteps, cfd_step_report* rep) {
         int st = (prec == CFD_PREC_MIXED) ? step_once_mixed() : step_once();
         if (st) return st;
     }
+    if (prec != CFD_PREC_MIXED) CFD_CUDA(cudaStreamWaitEvent(stream, ev_forces, 0));
     // the report: one gather on the device, one copy into pinned memory
     CFD_LAUNCH(k_pack_report, 1, 32, 0, stream, (const StepScal*)d_scal,
                (const MotionScal*)(d_motion ? d_motion + buf : nullptr), (const int*)d_pcg_iters, (const int*)d_pcg_conv,
@@ -759,6 +813,7 @@ int Ctx::create(const cfd_mesh* m, const cfd_params* p, int precision_mode) {
     CFD_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CFD_CUDA(cudaEventCreateWithFlags(&ev_scal, cudaEventDisableTiming));
     CFD_CUDA(cudaEventCreateWithFlags(&ev_tail, cudaEventDisableTiming));
+    CFD_CUDA(cudaEventCreateWithFlags(&ev_forces, cudaEventDisableTiming));
     CFD_CUDA(cudaEventCreateWithFlags(&ev_iters, cudaEventDisableTiming));
     CFD_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
     CFD_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
@@ -831,6 +886,12 @@ int Ctx::create(const cfd_mesh* m, const cfd_params* p, int precision_mode) {
     for (double** q : {&d_area, &d_area_old, &d_DT, &d_DTL, &d_SHOC, &d_TS1, &d_TS2, &d_TS3})
         if ((st = dalloc(q, E))) return st;
     if ((st = dalloc(&d_geo, 6 * (size_t)E))) return st;
+    if (prec == CFD_PREC_FP64) {
+        for (double** q : {&d_X_n, &d_Y_n, &d_WX_n, &d_WY_n, &d_M_n})
+            if ((st = dalloc(q, N))) return st;
+        if ((st = dalloc(&d_area_n, E))) return st;
+        if ((st = dalloc(&d_geo_n, 6 * (size_t)E))) return st;
+    }
     if ((st = dalloc(&d_contrib, 12 * (size_t)E))) return st;
     if ((st = dalloc(&d_contribF, 12 * (size_t)E))) return st;
     if (prec == CFD_PREC_FP64 && (st = dalloc(&d_einv, (size_t)kElemInvPlanes * E))) return st;

@@ -84,10 +84,11 @@ __global__ void k_gcl_terms(int nelem, const int4* __restrict__ elem,
     terms[e] = make_double2(div3(divW * area[e]), div3(divWo * area_old[e]));
 }
 
-// Per node: tot1, tot2 as the ordered sums over the elements around it, M += dt(t1 + t2)/2
+// Per node: tot1, tot2 as the ordered sums over the elements around it, M_out = M + dt(t1 + t2)/2
+// (M_out may be M)
 __global__ void k_gcl(int npoin, const int* __restrict__ esup_ptr,
                       const int* __restrict__ esup_slot, const double2* __restrict__ terms,
-                      const double* __restrict__ dtp, double* __restrict__ M) {
+                      const double* __restrict__ dtp, const double* M, double* M_out) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= npoin) return;
     double t1 = 0.0, t2 = 0.0;
@@ -96,17 +97,17 @@ __global__ void k_gcl(int npoin, const int* __restrict__ esup_ptr,
         t1 = t1 + tm.x;
         t2 = t2 + tm.y;
     }
-    M[p] = M[p] + (*dtp) * (t1 + t2) / 2.0;
+    M_out[p] = M[p] + (*dtp) * (t1 + t2) / 2.0;
 }
 
 cudaError_t launch_gcl(cudaStream_t st, int npoin, int nelem, const int4* elem,
                        const int* esup_ptr, const int* esup_slot, const double* geo,
                        const double* area, const double* area_old, const double* Wx,
                        const double* Wy, const double* Wxo, const double* Wyo, const double* dtp,
-                       int literal, double2* scratch, double* M) {
+                       int literal, double2* scratch, const double* M, double* M_out) {
     k_gcl_terms<<<blocks_for(nelem, 256), 256, 0, st>>>(nelem, elem, geo, area, area_old, Wx, Wy,
                                                         Wxo, Wyo, literal, scratch);
-    k_gcl<<<blocks_for(npoin, 256), 256, 0, st>>>(npoin, esup_ptr, esup_slot, scratch, dtp, M);
+    k_gcl<<<blocks_for(npoin, 256), 256, 0, st>>>(npoin, esup_ptr, esup_slot, scratch, dtp, M, M_out);
     g_launches.fetch_add(2, std::memory_order_relaxed);
     return cudaGetLastError();
 }
@@ -1105,18 +1106,19 @@ __global__ void k_transf(int nnmove, const int* __restrict__ fix_node, const int
     xfix_y[k] = dy;
 }
 
-// meshMove.f90:99-126: X += XPOS, W_X = XPOS/DTMIN (and y)
+// meshMove.f90:99-126: X += XPOS, W_X = XPOS/DTMIN (and y), into the next step's X, Y, W
 __global__ void k_motion_update(int npoin, const double* __restrict__ xpos, const double* __restrict__ ypos,
-                                const StepScal* __restrict__ sc, double* __restrict__ X,
+                                const StepScal* __restrict__ sc, const double* __restrict__ X0,
+                                const double* __restrict__ Y0, double* __restrict__ X,
                                 double* __restrict__ Y, double* __restrict__ WX,
                                 double* __restrict__ WY) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= npoin) return;
     const double dt = sc->dtmin;
     double xp = xpos[p], yp = ypos[p];
-    X[p] = X[p] + xp;
+    X[p] = X0[p] + xp;
     WX[p] = xp / dt;
-    Y[p] = Y[p] + yp;
+    Y[p] = Y0[p] + yp;
     WY[p] = yp / dt;
 }
 

@@ -292,3 +292,40 @@ def test_full_size_one_step_parity_and_properties(gpu_lib):
     eq(g2.state()["U"], st["U"], "determinism")
     g.close()
     g2.close()
+
+
+@pytest.mark.parametrize("mass_mode", [1, 2])
+@pytest.mark.parametrize("mesh_too", [False, True])
+def test_steps_around_an_upload_of_the_mesh(gpu_lib, mass_mode, mesh_too):
+    """putW's and putArea's values are the last step's W and area until the host replaces W or the
+    mesh, and stay theirs through the replacement: two steps, an upload (W, or W and the mesh),
+    one step, W again, two steps, against the oracle."""
+    from cfd_gb300 import solver
+    from oracle import oracle as O
+    k = small_case(3, scale=16, seed=9, moving=1, motion_law=1, heave_amp=0.02, motion_freq=0.5,
+                   mass_mode=mass_mode)
+    g, o = solver.Solver(k), O.OracleCase(k)
+    rng = np.random.default_rng(3)
+
+    def check(steps):
+        for _ in range(steps):
+            assert g.step(1).dtmin == o.step(1).dtmin
+        sg, so = g.state(), o.state()
+        for key in ("U", "T", "X", "Y"):
+            eq(sg[key], so[key], key)
+        gg, go = g.geometry(), o.geometry()
+        for key in gg:
+            eq(gg[key], go[key], key)
+
+    check(2)
+    w = 0.05 * rng.normal(size=(2, k.npoin))
+    s = o.state()
+    new = dict(X=s["X"] * (1 + 1e-6), Y=s["Y"] * (1 - 1e-6)) if mesh_too else {}
+    for side in (g, o):
+        side.set_mesh(W_X=w[0], W_Y=w[1], **new)
+    check(1)
+    for side in (g, o):
+        side.set_mesh(W_Y=w[0])
+    check(2)
+    g.close()
+    o.close()
