@@ -310,7 +310,7 @@ __global__ void k_edge_features(int m, const int* __restrict__ src, const int* _
 // keeps every vector load free of bank conflicts.  Each output sums its k in ascending order
 // from the bias.  49,794 nodes: 112-154 us per product with one output column and 32 rows
 // per thread and the weights re-read from global memory, 35-45 us with 8 x 4 outputs in
-// 64-row block tiles, 26-40 us now.
+// 64-row block tiles, 28-33 us now.
 constexpr int GR = 16;  // rows of a warp's group
 // what the product's epilogue does
 enum : int {
@@ -331,10 +331,10 @@ struct GemmShape {
     static_assert(8 * L == N && RT * RG == GR, "thread tile");
 };
 
-// Y[n][N] = X[n][K] . B.  TRANS: B[k][c] = W[c][k] (forward), else W[k][c] (backward).  X is
+// Y[n][N] = X[n][K] . W[K][N].  The weights come by cp.async while the warp loads its first rows.  X is
 // [X1 | X2] in 64-column halves when X2 is given (K = 128), and masked (X1 where gate > 0,
 // else 0) when gate is given.
-template <int K, int N, bool TRANS, int EPI>
+template <int K, int N, int EPI>
 __global__ void __launch_bounds__(32 * GemmShape<K, N>::WARPS, GemmShape<K, N>::PER_SM)
 k_gemm(int n, const float* __restrict__ X1, const float* __restrict__ X2,
        const float* __restrict__ gate, const float* __restrict__ W, const float* __restrict__ bias,
@@ -346,20 +346,11 @@ k_gemm(int n, const float* __restrict__ X1, const float* __restrict__ X2,
     constexpr int T = 32 * G::WARPS, RT = G::RT, KS = G::KS;
     const int tid = threadIdx.x, lane = tid & 31;
     float* Xs = gsm + K * N + (tid >> 5) * GR * KS;  // the warp's rows
-    if (TRANS) {
-        for (int q = tid; q < N * K / 4; q += T) {  // lanes over the columns: conflict-free
-            const int c = q % N, k = 4 * (q / N);
-            const float4 w = *reinterpret_cast<const float4*>(W + (size_t)c * K + k);
-            Bs[k * N + c] = w.x;
-            Bs[(k + 1) * N + c] = w.y;
-            Bs[(k + 2) * N + c] = w.z;
-            Bs[(k + 3) * N + c] = w.w;
-        }
-    } else {
-        for (int q = tid; q < K * N / 4; q += T)
-            reinterpret_cast<float4*>(Bs)[q] = reinterpret_cast<const float4*>(W)[q];
-    }
-    __syncthreads();
+    const unsigned bs = (unsigned)__cvta_generic_to_shared(Bs);
+#pragma unroll
+    for (int q = tid; q < K * N / 4; q += T)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(bs + 16 * q), "l"(W + 4 * q)
+                     : "memory");
     const int c0 = 4 * (lane % G::L), c1 = c0 + N / 2, rg = lane / G::L;
     float4 ba = make_float4(0.f, 0.f, 0.f, 0.f), bb = ba;
     if (bias) {
@@ -367,20 +358,25 @@ k_gemm(int n, const float* __restrict__ X1, const float* __restrict__ X2,
         bb = *reinterpret_cast<const float4*>(bias + c1);
     }
     const int ngroup = (n + GR - 1) / GR;
+    // each warp comes here once, before its first rows' products: a barrier of its own
+    auto weights_ready = [&]() {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory");
+    };
+    bool ready = false;
     // groups interleaved over the blocks, so that a last partial round spreads over all SMs
     for (int grp = (tid >> 5) * gridDim.x + blockIdx.x; grp < ngroup; grp += gridDim.x * G::WARPS) {
         const int base = grp * GR;
         __syncwarp();  // the previous group has been read
-#pragma unroll 8
+#pragma unroll 16
         for (int q = lane; q < GR * K / 4; q += 32) {
             const int r = q / (K / 4), k = 4 * (q - r * (K / 4)), row = base + r;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
             if (row < n) {
-                if (K == 128 && X2)
-                    v = k < 64 ? *reinterpret_cast<const float4*>(X1 + (size_t)row * 64 + k)
-                               : *reinterpret_cast<const float4*>(X2 + (size_t)row * 64 + (k - 64));
-                else
-                    v = *reinterpret_cast<const float4*>(X1 + (size_t)row * K + k);
+                // one address, not a load on either side of a branch: a group's loads go out together
+                const float* src = K == 128 && X2 ? (k < 64 ? X1 : X2 - 64) + (size_t)row * 64 + k
+                                                  : X1 + (size_t)row * K + k;
+                v = *reinterpret_cast<const float4*>(src);
                 if (gate) {
                     const float4 g = *reinterpret_cast<const float4*>(gate + (size_t)row * K + k);
                     v = make_float4(g.x > 0.f ? v.x : 0.f, g.y > 0.f ? v.y : 0.f,
@@ -388,6 +384,10 @@ k_gemm(int n, const float* __restrict__ X1, const float* __restrict__ X2,
                 }
             }
             *reinterpret_cast<float4*>(Xs + r * KS + k) = v;
+        }
+        if (!ready) {
+            weights_ready();
+            ready = true;
         }
         __syncwarp();
         float acc[RT][8];
@@ -456,9 +456,10 @@ k_gemm(int n, const float* __restrict__ X1, const float* __restrict__ X2,
             }
         }
     }
+    if (!ready) weights_ready();  // a warp without rows
 }
 
-template <int K, int N, bool TRANS, int EPI>
+template <int K, int N, int EPI>
 static int gemm(cudaStream_t st, int n, const float* X1, const float* X2, const float* gate,
                 const float* W, const float* bias, const int* ptr, const float* E, float* Y,
                 float* Y2) {
@@ -468,42 +469,59 @@ static int gemm(cudaStream_t st, int n, const float* X1, const float* X2, const 
     int dev = 0;
     CFD_CUDA(cudaGetDevice(&dev));
     if (dev > 63 || !(done.load(std::memory_order_relaxed) >> dev & 1ull)) {
-        CFD_CUDA(cudaFuncSetAttribute(k_gemm<K, N, TRANS, EPI>,
+        CFD_CUDA(cudaFuncSetAttribute(k_gemm<K, N, EPI>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM));
         if (dev <= 63) done.fetch_or(1ull << dev, std::memory_order_relaxed);
     }
     // the resident blocks of the 152 SMs (each loads the weights once), fewer for few rows
     const unsigned grid = std::min<unsigned>(blocks_for(n, GR * G::WARPS), kTrainChunks * G::PER_SM);
-    CFD_LAUNCH((k_gemm<K, N, TRANS, EPI>), grid, 32 * G::WARPS, G::SMEM, st, n, X1, X2, gate, W,
+    CFD_LAUNCH((k_gemm<K, N, EPI>), grid, 32 * G::WARPS, G::SMEM, st, n, X1, X2, gate, W,
                bias, ptr, E, Y, Y2);
     return CFD_OK;
 }
 
 int dense_pq(cudaStream_t st, int n, const float* h, const float* W, float* pq) {
-    return gemm<HID, 2 * HID, true, GE_PLAIN>(st, n, h, nullptr, nullptr, W, nullptr, nullptr,
+    return gemm<HID, 2 * HID, GE_PLAIN>(st, n, h, nullptr, nullptr, W, nullptr, nullptr,
                                               nullptr, pq, nullptr);
 }
 int dense_update(cudaStream_t st, int n, const float* h, const float* agg, const float* W,
                  const float* b, float* v, float* h1) {
-    return gemm<2 * HID, HID, true, GE_RESIDUAL>(st, n, h, agg, nullptr, W, b, nullptr, nullptr, v,
+    return gemm<2 * HID, HID, GE_RESIDUAL>(st, n, h, agg, nullptr, W, b, nullptr, nullptr, v,
                                                  h1);
 }
 int dense_update_bwd(cudaStream_t st, int n, const float* dh, const float* v, const float* W,
                      const int* ptr, float* dhc) {
-    return gemm<HID, 2 * HID, false, GE_SPLIT>(st, n, dh, nullptr, v, W, nullptr, ptr, nullptr,
+    return gemm<HID, 2 * HID, GE_SPLIT>(st, n, dh, nullptr, v, W, nullptr, ptr, nullptr,
                                                dhc, nullptr);
 }
 int dense_pq_bwd(cudaStream_t st, int n, const float* dpq, const float* W, const float* dhc,
                  float* dh) {
-    return gemm<2 * HID, HID, false, GE_ACCUM>(st, n, dpq, nullptr, nullptr, W, nullptr, nullptr,
+    return gemm<2 * HID, HID, GE_ACCUM>(st, n, dpq, nullptr, nullptr, W, nullptr, nullptr,
                                                dhc, dh, nullptr);
 }
 
-// h0 = relu(W_in f + b_in); h0 > 0 where the argument is, so it is its own backward mask
+// h0 = relu(W_in f + b_in); h0 > 0 where the argument is, so it is its own backward mask.  The
+// last kEncodeExtra blocks write the layers' dense weights transposed, [input][output] at the same
+// offsets of wt, for the forward products (the transposition by each block of each product
+// cost 4 to 10 us of 30 to 44).
 __global__ void __launch_bounds__(256) k_encode(int n, const float* __restrict__ f,
                                                 const float* __restrict__ w,
-                                                float* __restrict__ h) {
+                                                float* __restrict__ h, float* __restrict__ wt) {
     __shared__ float fs[64 * F_IN];
+    const int tb = (int)blockIdx.x - ((int)gridDim.x - kEncodeExtra);
+    if (tb >= 0) {
+        for (int q = tb * 256 + threadIdx.x; q < LAYERS * 4 * HID * HID; q += kEncodeExtra * 256) {
+            const int off = layer_off(q / (4 * HID * HID)), r = q % (4 * HID * HID);
+            if (r < 2 * HID * HID) {
+                const int k = r / (2 * HID), c = r % (2 * HID);
+                wt[off + L_A + r] = w[off + L_A + c * HID + k];
+            } else {
+                const int r2 = r - 2 * HID * HID, k = r2 / HID, c = r2 % HID;
+                wt[off + L_U + r2] = w[off + L_U + c * 2 * HID + k];
+            }
+        }
+        return;
+    }
     const int base = blockIdx.x * 64, o = threadIdx.x & 63;
     for (int q = threadIdx.x; q < 64 * F_IN; q += 256)
         fs[q] = base + q / F_IN < n ? f[(size_t)base * F_IN + q] : 0.f;
@@ -529,9 +547,10 @@ __global__ void __launch_bounds__(256) k_encode(int n, const float* __restrict__
 // dW[O][I] = sum_r dY[r][O] X[r][I] (and the bias sum_r dY[r][O]) for O x I = 64 x 128 or
 // 128 x 64: two groups of 256 threads take alternate rows of a 32-row tile, a thread forms
 // 8 x 4 outputs (3 vector loads for 32 FMAs), the next tile's values are loaded while this
-// one is summed.  49,794 nodes: 128 us + 54 us of fold before (2 shared loads per FMA, 64
-// rows per partial, 779 partials folded by one thread each), 26-33 us now.
-template <int O, int I>
+// one is summed; with BIAS (O = 64) the columns of dY are summed beside, four rows of a tile a
+// thread (by the products' threads they were a fifth of the FP32 operations).  49,794 nodes: 128 us + 54 us of fold before (2 shared loads per FMA, 64
+// rows per partial, 779 partials folded by one thread each), 25-32 us now.
+template <int O, int I, bool BIAS>
 __global__ void __launch_bounds__(512)
 k_wgrad(int n, const float* __restrict__ dY, const float* __restrict__ gate,
         const float* __restrict__ X1, const float* __restrict__ X2, float* __restrict__ part,
@@ -543,7 +562,9 @@ k_wgrad(int n, const float* __restrict__ dY, const float* __restrict__ gate,
     const int i0 = 4 * (t % IT), o0 = 8 * (t / IT);
     const int rows = (n + kTrainChunks - 1) / kTrainChunks;
     const int b0 = blockIdx.x * rows, b1 = min(n, b0 + rows);
-    float acc[8][4] = {}, bs[8] = {};
+    static_assert(!BIAS || O == 64, "64 columns by 8 groups of 4 rows");
+    const int bo = tid & 63, br = 4 * (tid >> 6);
+    float acc[8][4] = {}, bsum = 0.f;
     float4 pre[V];
     auto fetch = [&](int base) {
 #pragma unroll
@@ -564,10 +585,9 @@ k_wgrad(int n, const float* __restrict__ dY, const float* __restrict__ gate,
             } else {
                 const int p = q - R * O / 4, r = p / (I / 4), c = 4 * (p - r * (I / 4)),
                           row = base + r;
-                if (row < b1)
-                    w = (I == 64 || c < 64)
-                            ? *reinterpret_cast<const float4*>(X1 + (size_t)row * 64 + c)
-                            : *reinterpret_cast<const float4*>(X2 + (size_t)row * 64 + (c - 64));
+                if (row < b1)  // one address, not a load on either side of a branch
+                    w = *reinterpret_cast<const float4*>((I == 64 || c < 64 ? X1 : X2 - 64) +
+                                                         (size_t)row * 64 + c);
             }
             pre[v] = w;
         }
@@ -583,6 +603,9 @@ k_wgrad(int n, const float* __restrict__ dY, const float* __restrict__ gate,
         }
         __syncthreads();
         if (base + R < b1) fetch(base + R);
+        if (BIAS)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) bsum += ys[(br + u) * O + bo];
 #pragma unroll 4
         for (int r = grp; r < R; r += 2) {
             const float4 ya = *reinterpret_cast<const float4*>(ys + r * O + o0);
@@ -595,7 +618,6 @@ k_wgrad(int n, const float* __restrict__ dY, const float* __restrict__ gate,
                 acc[a][1] = fmaf(y[a], x.y, acc[a][1]);
                 acc[a][2] = fmaf(y[a], x.z, acc[a][2]);
                 acc[a][3] = fmaf(y[a], x.w, acc[a][3]);
-                bs[a] += y[a];
             }
         }
     }
@@ -622,25 +644,26 @@ k_wgrad(int n, const float* __restrict__ dY, const float* __restrict__ gate,
             }
         }
     }
-    if (bias_off >= 0 && i0 == 0) {
-        if (grp == 1)
+    if (BIAS) {  // ys has been read
+        ys[tid] = bsum;
+        __syncthreads();
+        if (tid < O) {
+            float s = 0.f;
 #pragma unroll
-            for (int a = 0; a < 8; ++a) ys[o0 + a] = bs[a];
+            for (int u = 0; u < 8; ++u) s += ys[64 * u + tid];
+            out[bias_off + tid] = s;
+        }
     }
-    __syncthreads();
-    if (bias_off >= 0 && i0 == 0 && grp == 0)
-#pragma unroll
-        for (int a = 0; a < 8; ++a) out[bias_off + o0 + a] = bs[a] + ys[o0 + a];
 }
 
 int wgrad_update(cudaStream_t st, int n, const float* dh, const float* v, const float* h,
                  const float* agg, float* part, int layer) {
-    CFD_LAUNCH((k_wgrad<HID, 2 * HID>), kTrainChunks, 512, 0, st, n, dh, v, h, agg, part,
+    CFD_LAUNCH((k_wgrad<HID, 2 * HID, true>), kTrainChunks, 512, 0, st, n, dh, v, h, agg, part,
                layer_off(layer) + L_U, layer_off(layer) + L_u);
     return CFD_OK;
 }
 int wgrad_pq(cudaStream_t st, int n, const float* dpq, const float* h, float* part, int layer) {
-    CFD_LAUNCH((k_wgrad<2 * HID, HID>), kTrainChunks, 512, 0, st, n, dpq, (const float*)nullptr, h,
+    CFD_LAUNCH((k_wgrad<2 * HID, HID, false>), kTrainChunks, 512, 0, st, n, dpq, (const float*)nullptr, h,
                (const float*)nullptr, part, layer_off(layer) + L_A, -1);
     return CFD_OK;
 }
@@ -691,14 +714,15 @@ __global__ void __launch_bounds__(512) k_wgrad_in(int n, const float* __restrict
     }
 }
 
-// out[q] = sum over the chunks c, in order, of part[c][q], in four interleaved sums so that
-// four loads are in flight
+// out[q] = sum over the chunks c, in order, of part[c][q], in four interleaved sums, sixteen
+// loads in flight
 __global__ void k_fold(int nq, const float* __restrict__ part, float* __restrict__ out,
                        float* __restrict__ loss) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nq) return;
     static_assert(kTrainChunks % 4 == 0, "four sums");
     float a[4] = {};
+#pragma unroll 4
     for (int c = 0; c < kTrainChunks; c += 4)
 #pragma unroll
         for (int u = 0; u < 4; ++u) a[u] += part[(size_t)(c + u) * nq + q];
@@ -712,13 +736,22 @@ __global__ void k_fold(int nq, const float* __restrict__ part, float* __restrict
 //     z = P_i + Q_j + C e_k + c,   agg_i = sum_k relu(z) / max(deg_i, 1);
 // z itself is not kept: the backward pass needs its signs only, 64 bits per edge (bit l of
 // plane b: channel 4 l + b), formed by four ballots.  Before, z was written and read back
-// per edge and channel (76 MB per layer at 49,794 nodes: 76 + 22 us against 33 us now).
+// per edge and channel (76 MB per layer at 49,794 nodes: 76 + 22 us against 28 us now).  A block
+// takes several groups of nodes: C and c are loaded once, and a group's first loads run beside
+// the edges of the group before (34 us with a block per 16 nodes).
+// A warp takes the nodes i and i + 2 (half_warp_node): structured triangulations alternate
+// nodes of 4 and 8 edges, and a warp is as slow as the longer of its two (backward
+// 27 us with i and i + 1, 23 so).
+__device__ __forceinline__ int half_warp_node(int half_warp) {
+    const int w = half_warp >> 1;
+    return 4 * (w >> 1) + (w & 1) + 2 * (half_warp & 1);
+}
 __global__ void __launch_bounds__(256)
 k_edge_fwd(int n, const int* __restrict__ ptr, const int* __restrict__ nbr,
            const float* __restrict__ PQ, const float* __restrict__ e, const float* __restrict__ C,
            const float* __restrict__ c, ushort4* __restrict__ mask, float* __restrict__ agg) {
-    const int i = (int)((blockIdx.x * 256u + threadIdx.x) >> 4), l = threadIdx.x & 15;
-    const int half = threadIdx.x & 16;
+    const int l = threadIdx.x & 15, half = threadIdx.x & 16;
+    const int at = half_warp_node(threadIdx.x >> 4), nblk = (n + 15) / 16;
     float cw[4][3], cb[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -726,11 +759,26 @@ k_edge_fwd(int n, const int* __restrict__ ptr, const int* __restrict__ nbr,
 #pragma unroll
         for (int u = 0; u < 3; ++u) cw[q][u] = C[(4 * l + q) * 3 + u];
     }
+    // a block's 16-node groups; the next group's row pointers and P row load beside this one's edges
+    int nk0 = 0, nk1 = 0;
+    float4 np = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto head = [&](int b) {
+        const int i = 16 * b + at;
+        if (b >= nblk || i >= n) {
+            nk0 = nk1 = 0;
+            return;
+        }
+        nk0 = ptr[i];
+        nk1 = ptr[i + 1];
+        np = *reinterpret_cast<const float4*>(PQ + (size_t)i * 2 * HID + 4 * l);
+    };
+    head(blockIdx.x);
+    for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
+    const int i = 16 * b + at;
     const bool live = i < n;
-    const int k0 = live ? ptr[i] : 0, k1 = live ? ptr[i + 1] : 0;
-    float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (live) p = *reinterpret_cast<const float4*>(PQ + (size_t)i * 2 * HID + 4 * l);
-    const float pv[4] = {p.x, p.y, p.z, p.w};
+    const int k0 = nk0, k1 = nk1;
+    const float pv[4] = {np.x, np.y, np.z, np.w};
+    head(b + gridDim.x);
     float s[4] = {};
     const int deg = k1 - k0, steps = max(deg, __shfl_xor_sync(0xffffffffu, deg, 16));
     constexpr int B = 4;  // edges whose gathers go out together
@@ -771,6 +819,7 @@ k_edge_fwd(int n, const int* __restrict__ ptr, const int* __restrict__ nbr,
         *reinterpret_cast<float4*>(agg + (size_t)i * HID + 4 * l) =
             make_float4(s[0] / d, s[1] / d, s[2] / d, s[3] / d);
     }
+    }
 }
 
 // Backward of the messages from g = d agg / deg (the second half of the dhc rows) and the
@@ -780,7 +829,7 @@ k_edge_fwd(int n, const int* __restrict__ ptr, const int* __restrict__ nbr,
 // so no per-edge gradient is stored.  kTrainChunks blocks, the nodes interleaved over their
 // half-warps; the block's dC, dc go to its row of `part`.  Before: 95 + 53 + 265 + 28 us per
 // layer (the edge gradients written, read by the weight gradient and the node sums, the
-// partials folded by one block); 26 us now.
+// partials folded by one block); 23 us now.
 __global__ void __launch_bounds__(1024)
 k_edge_bwd(int n, const int* __restrict__ ptr, const int* __restrict__ nbr,
            const int* __restrict__ rev, const ushort4* __restrict__ mask,
@@ -790,7 +839,7 @@ k_edge_bwd(int n, const int* __restrict__ ptr, const int* __restrict__ nbr,
     const int l = threadIdx.x & 15;
     float GC[4][3] = {}, Gc[4] = {};
     const int stride = gridDim.x * 64;
-    for (int i = blockIdx.x * 64 + (threadIdx.x >> 4); i < n; i += stride) {
+    for (int i = blockIdx.x * 64 + half_warp_node(threadIdx.x >> 4); i < n; i += stride) {
         const int k0 = ptr[i], k1 = ptr[i + 1];
         const float4 g4 = *reinterpret_cast<const float4*>(dhc + (size_t)i * 2 * HID + HID + 4 * l);
         const float g[4] = {g4.x, g4.y, g4.z, g4.w};

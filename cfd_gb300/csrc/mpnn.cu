@@ -63,6 +63,7 @@ struct cfd_mpnn_graph {
     float* v[LAYERS] = {};               // n x HID
     ushort4* mask[LAYERS] = {};          // m (the signs of the messages' 64 channels)
     float *pq = nullptr, *y = nullptr;   // n x 2HID, n x OUT
+    float* wt = nullptr;                 // the pass's dense weights, transposed
     // backward; part: kTrainChunks rows of every parameter's partial gradient and the loss
     float *dh = nullptr, *dhc = nullptr, *dpq = nullptr, *part = nullptr, *loss = nullptr;
     // inference (BF16)
@@ -93,13 +94,14 @@ int forward_fp32(cfd_mpnn& net, cfd_mpnn_graph& g, const float* target = nullptr
     cudaStream_t st = g.stream;
     const int n = g.n;
     int rc;
-    CFD_LAUNCH(k_encode, nb_of(n, 64), 256, 0, st, n, (const float*)g.f, (const float*)net.w, g.h[0]);
+    CFD_LAUNCH(k_encode, nb_of(n, 64) + kEncodeExtra, 256, 0, st, n, (const float*)g.f,
+               (const float*)net.w, g.h[0], g.wt);
     for (int l = 0; l < LAYERS; ++l) {
-        const float* W = net.w + layer_off(l);
-        if ((rc = dense_pq(st, n, g.h[l], W + L_A, g.pq))) return rc;
-        CFD_LAUNCH(k_edge_fwd, nb_of(n, 16), 256, 0, st, n, g.ptr, g.nbr, (const float*)g.pq,
+        const float *W = net.w + layer_off(l), *Wt = g.wt + layer_off(l);
+        if ((rc = dense_pq(st, n, g.h[l], Wt + L_A, g.pq))) return rc;
+        CFD_LAUNCH(k_edge_fwd, std::min(nb_of(n, 16), kEdgeBlocks), 256, 0, st, n, g.ptr, g.nbr, (const float*)g.pq,
                    (const float*)g.e, W + L_C, W + L_c, g.mask[l], g.agg[l]);
-        if ((rc = dense_update(st, n, g.h[l], g.agg[l], W + L_U, W + L_u, g.v[l], g.h[l + 1])))
+        if ((rc = dense_update(st, n, g.h[l], g.agg[l], Wt + L_U, W + L_u, g.v[l], g.h[l + 1])))
             return rc;
     }
     // with a target (training) the decoder also starts the backward pass
@@ -228,6 +230,7 @@ int graph_build(cfd_mpnn_graph** out, int npoin, const std::vector<int>& rowptr,
         }
         if ((rc = dev_alloc(o, &g->pq, n * 2 * HID))) return rc;
         if ((rc = dev_alloc(o, &g->y, n * OUT))) return rc;
+        if ((rc = dev_alloc(o, &g->wt, N_PARAMS))) return rc;
         if ((rc = dev_alloc(o, &g->dh, n * HID))) return rc;
         if ((rc = dev_alloc(o, &g->dhc, n * 2 * HID))) return rc;
         if ((rc = dev_alloc(o, &g->dpq, n * 2 * HID))) return rc;

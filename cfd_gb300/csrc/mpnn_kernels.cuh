@@ -25,7 +25,7 @@ __global__ void k_features(int n, const double* X, const double* Y, const int* k
 __global__ void k_edge_features(int m, const int* src, const int* nbr, const double* X,
                                 const double* Y, const Globals* G, float* e, const int* gate);
 // FP32 training passes (kernels_mpnn.cu): P|Q = [A; B] h; v = U [h; agg] + u and h1 = h +
-// relu(v); their backward products (dhc = [dh | dagg / deg], dh += its first half + dPQ [A; B])
+// relu(v), from the transposed weights that k_encode leaves in wt; their backward products (dhc = [dh | dagg / deg], dh += its first half + dPQ [A; B])
 int dense_pq(cudaStream_t st, int n, const float* h, const float* W, float* pq);
 int dense_update(cudaStream_t st, int n, const float* h, const float* agg, const float* W,
                  const float* b, float* v, float* h1);
@@ -37,7 +37,9 @@ int dense_pq_bwd(cudaStream_t st, int n, const float* dpq, const float* W, const
 int wgrad_update(cudaStream_t st, int n, const float* dh, const float* v, const float* h,
                  const float* agg, float* part, int layer);
 int wgrad_pq(cudaStream_t st, int n, const float* dpq, const float* h, float* part, int layer);
-__global__ void k_encode(int n, const float* f, const float* w, float* h);
+constexpr unsigned kEdgeBlocks = 152 * 6;  // blocks of k_edge_fwd at most (resident)
+constexpr int kEncodeExtra = 64;  // blocks of k_encode that transpose the weights
+__global__ void k_encode(int n, const float* f, const float* w, float* h, float* wt);
 __global__ void k_wgrad_in(int n, const float* dh, const float* h0, const float* f, float* part);
 __global__ void k_fold(int nq, const float* part, float* out, float* loss);
 __global__ void k_edge_fwd(int n, const int* ptr, const int* nbr, const float* PQ, const float* e,
