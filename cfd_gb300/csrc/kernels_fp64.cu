@@ -29,7 +29,7 @@ __global__ void k_deriv(int nelem, const int4* __restrict__ elem, const double* 
                 (xl[1] * yl[0] + xl[2] * yl[1] + xl[0] * yl[2])) / 2.0;
     area[e] = a;
     const size_t E = (size_t)nelem;
-    // FP64-pipe bound: the six quotients by one reciprocal (the same bits; 252 -> 200 us at
+    // FP64-pipe bound: the six quotients by one reciprocal (the same bits; 252 -> 191 us at
     // 1,048,576 nodes)
     const double a2 = 2.0 * a, y = 1.0 / a2, l = rcp_lo(a2, y);
     geo[e] = div_rcp2(yl[1] - yl[2], a2, y, l);
@@ -450,17 +450,19 @@ k_elem_rhs(int e0, int e1, int nelem, const int4* __restrict__ elem, const doubl
         const double w0 = WX[p[0]], w1 = WX[p[1]], w2 = WX[p[2]];
         const double y0 = WY[p[0]], y1 = WY[p[1]], y2 = WY[p[2]];
         // sp(:,1)=(.5,.5,0), sp(:,2)=(0,.5,.5), sp(:,3)=(.5,0,.5); zero terms dropped
-        const double wx[3] = {0.5 * w0 + 0.5 * w1, 0.5 * w1 + 0.5 * w2, 0.5 * w0 + 0.5 * w2};
-        const double wy[3] = {0.5 * y0 + 0.5 * y1, 0.5 * y1 + 0.5 * y2, 0.5 * y0 + 0.5 * y2};
+        // every half is exact: twice the velocities at the points, four times the sums
+        const double wx[3] = {w0 + w1, w1 + w2, w0 + w2};
+        const double wy[3] = {y0 + y1, y1 + y2, y0 + y2};
+        const double qAR = 0.25 * AR;
         double* of = contribF + 12 * (size_t)e;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const double q0 = Ux[q] * wx[0] + Uy[q] * wy[0];
             const double q1 = Ux[q] * wx[1] + Uy[q] * wy[1];
             const double q2 = Ux[q] * wx[2] + Uy[q] * wy[2];
-            of[q] = -(AR * (0.5 * q0 + 0.5 * q2));      // node 1: sp(1,:) = (.5, 0, .5)
-            of[4 + q] = -(AR * (0.5 * q0 + 0.5 * q1));  // node 2: sp(2,:) = (.5, .5, 0)
-            of[8 + q] = -(AR * (0.5 * q1 + 0.5 * q2));  // node 3: sp(3,:) = (0, .5, .5)
+            of[q] = -(qAR * (q0 + q2));      // node 1: sp(1,:) = (.5, 0, .5)
+            of[4 + q] = -(qAR * (q0 + q1));  // node 2: sp(2,:) = (.5, .5, 0)
+            of[8 + q] = -(qAR * (q1 + q2));  // node 3: sp(3,:) = (0, .5, .5)
         }
     }
 }
@@ -530,7 +532,7 @@ static_assert(kInvPlanes == kElemInvPlanes, "cache planes");
 // Both kernels are bound by the FP64 pipe (85% of it).  Kept out of it: the second product of
 // 0.5*a + 0.5*b (the halves are exact: 0.5*(a + b) has the same bits), the divisions by a
 // shared divisor (div_rcp2), and in the replay the prefix of each sum that no stage changes.
-// 1,048,576 nodes: the replay 1,669 us before, 1,514 now; k_elem_inv 3,912 and 3,875 us.
+// 1,048,576 nodes: the replay 1,669 us before, 1,514 now; k_elem_inv 3,912 and 3,808 us.
 
 template <bool VISCOUS>
 __global__ void __launch_bounds__(128)
@@ -696,17 +698,19 @@ k_elem_inv(int nelem, const int4* __restrict__ elem, const double* __restrict__ 
         const double AR = div3(ar * dtl);
         const double w0 = WX[p[0]], w1 = WX[p[1]], w2 = WX[p[2]];
         const double y0 = WY[p[0]], y1 = WY[p[1]], y2 = WY[p[2]];
-        const double wx[3] = {0.5 * w0 + 0.5 * w1, 0.5 * w1 + 0.5 * w2, 0.5 * w0 + 0.5 * w2};
-        const double wy[3] = {0.5 * y0 + 0.5 * y1, 0.5 * y1 + 0.5 * y2, 0.5 * y0 + 0.5 * y2};
+        // every half is exact: twice the velocities at the points, four times the sums
+        const double wx[3] = {w0 + w1, w1 + w2, w0 + w2};
+        const double wy[3] = {y0 + y1, y1 + y2, y0 + y2};
+        const double qAR = 0.25 * AR;
         double* of = contribF + 12 * (size_t)e;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const double q0 = Ux[q] * wx[0] + Uy[q] * wy[0];
             const double q1 = Ux[q] * wx[1] + Uy[q] * wy[1];
             const double q2 = Ux[q] * wx[2] + Uy[q] * wy[2];
-            of[q] = -(AR * (0.5 * q0 + 0.5 * q2));
-            of[4 + q] = -(AR * (0.5 * q0 + 0.5 * q1));
-            of[8 + q] = -(AR * (0.5 * q1 + 0.5 * q2));
+            of[q] = -(qAR * (q0 + q2));
+            of[4 + q] = -(qAR * (q0 + q1));
+            of[8 + q] = -(qAR * (q1 + q2));
         }
     }
 }
