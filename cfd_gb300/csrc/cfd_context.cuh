@@ -198,8 +198,13 @@ struct Ctx {
     // mixed form: one step (the network not run) captured as a CUDA graph and replayed;
     // off with the timers or CFD_GRAPHS=0, or when the capture fails
     bool graphs_on = false, capturing = false;
-    cudaGraph_t step_graph[2] = {nullptr, nullptr};   // per buffer parity (below)
-    cudaGraphExec_t step_exec[2] = {nullptr, nullptr};
+    // per buffer parity (below), and whether the step finds its DTMIN formed (2) and forms the
+    // next one's (1)
+    cudaGraph_t step_graph[2][4] = {};
+    cudaGraphExec_t step_exec[2][4] = {};
+    // within one cfd_step call: the last step has formed the coming step's DTMIN
+    bool dt_ahead = false;
+    cudaEvent_t ev_geo = nullptr;  // the next step's W and areas are there
     // mixed form: what the mesh-motion branch writes for the next step while the RK stages
     // read the current values; swapped after every step (parity `buf`)
     float4* d_geo8_n = nullptr;
@@ -264,8 +269,16 @@ struct Ctx {
                prm.guess_mode == CFD_GUESS_LEARNED_EXTRAPOLATED;
     }
     int guess_extrapolate(const PcgArgs& a, cudaStream_t s, unsigned grid);
-    int enqueue_mixed(bool learned);
-    int launch_step_graph(bool* launched);
+    int enqueue_mixed(bool learned, bool more);
+    int enqueue_dtmin(const float2* W);
+    // A step forms the next one's DTMIN where its passes leave SMs idle: up to 11,000 elements per
+    // SM (836,000 nodes).  20 steps of 262,144 nodes 4.46 -> 4.16 ms, 409,600 5.24 -> 4.82, 810,000
+    // 9.00 -> 8.51; from 921,600 on between 1.2% slower and 1.5% faster.
+    bool forms_ahead() const {
+        return !timers_on && prm.motion_law != CFD_MOTION_NEWMARK && !smoothing_now && !fv_each &&
+               nelem <= 11000L * nsm;
+    }
+    int launch_step_graph(bool* launched, bool more);
     int set_guess_net(cfd_mpnn* n, double gate);
     int force_visc_now();
     int smooth(int* iters, double* min_quality, bool node_order = false);
@@ -279,7 +292,7 @@ struct Ctx {
     bool smoothing_now = false;
     int set_force_visc_each_step(bool on);
     int step_once();
-    int step_once_mixed();
+    int step_once_mixed(bool more);
     int step(int nsteps, cfd_step_report* rep);
     int tstart(int slot);
     int tstop(int slot, int ncalls = 1);

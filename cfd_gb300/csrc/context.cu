@@ -90,6 +90,7 @@ Ctx::~Ctx() {
     if (ev_join) cudaEventDestroy(ev_join);
     if (ev_scal) cudaEventDestroy(ev_scal);
     if (ev_tail) cudaEventDestroy(ev_tail);
+    if (ev_geo) cudaEventDestroy(ev_geo);
     if (ev_forces) cudaEventDestroy(ev_forces);
     for (cudaEvent_t e : pool) cudaEventDestroy(e);
     for (auto& m : mark)
@@ -717,8 +718,9 @@ int Ctx::step_once() {
 
 int Ctx::step(int nsteps, cfd_step_report* rep) {
     if (nsteps < 0) return CFD_ERR_ARG;
+    dt_ahead = false;
     for (int s = 0; s < nsteps; ++s) {
-        int st = (prec == CFD_PREC_MIXED) ? step_once_mixed() : step_once();
+        int st = (prec == CFD_PREC_MIXED) ? step_once_mixed(s + 1 < nsteps) : step_once();
         if (st) return st;
     }
     if (prec != CFD_PREC_MIXED) CFD_CUDA(cudaStreamWaitEvent(stream, ev_forces, 0));
@@ -813,6 +815,7 @@ int Ctx::create(const cfd_mesh* m, const cfd_params* p, int precision_mode) {
     CFD_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CFD_CUDA(cudaEventCreateWithFlags(&ev_scal, cudaEventDisableTiming));
     CFD_CUDA(cudaEventCreateWithFlags(&ev_tail, cudaEventDisableTiming));
+    CFD_CUDA(cudaEventCreateWithFlags(&ev_geo, cudaEventDisableTiming));
     CFD_CUDA(cudaEventCreateWithFlags(&ev_forces, cudaEventDisableTiming));
     CFD_CUDA(cudaEventCreateWithFlags(&ev_iters, cudaEventDisableTiming));
     CFD_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
@@ -1097,6 +1100,7 @@ int Ctx::geometry_mixed(bool setup, bool put_area, bool to_next, cudaStream_t sv
     CFD_LAUNCH(k_elem_geometry, branch_grid(E, TB, sv), TB, 0, stream, E, d_elem, d_X, d_Y,
                gcl ? 1 : 0, prm.mass_mode == CFD_MASS_GCL_LITERAL ? 1 : 0, Wn, Wo,
                (gcl || put_area) ? 1 : 0, d_area_old, d_area, d_areaf, geo8, d_gterms);
+    if (to_next) CFD_CUDA(cudaEventRecord(ev_geo, stream));
     area_put = gcl || put_area;
     tstop(TM_DERIV);
     tstart(TM_LAPLACE);
@@ -1105,32 +1109,39 @@ int Ctx::geometry_mixed(bool setup, bool put_area, bool to_next, cudaStream_t sv
                    (const int*)d_slot_pos, d_k64);
     CFD_CUDA(launch_node_geometry(d_val_lo != nullptr, branch_grid(N, kGeoNodeBlock, sv), stream,
                                   N, d_esup_ptr, d_esup_slot, d_lap_pos, geo8, d_gterms,
-                                  &d_scal->dtmin, gcl ? 1 : 0, d_rowptr, d_valf, d_invdiag,
+                                  // the step's DTMIN: the next one's may be formed beside this pass
+                                  to_next ? &(d_motion + (buf ^ 1))->dtmin : &d_scal->dtmin,
+                                  gcl ? 1 : 0, d_rowptr, d_valf, d_invdiag,
                                   d_invdiagf, d_M, invMf, Wn, to_next ? (float2*)nullptr : d_Wof,
                                   (const float2*)d_k64, d_val_lo, nv));
     tstop(TM_LAPLACE);
     return CFD_OK;
 }
 
-// The device work of one mixed step, in order.  No host wait: DTMIN, the clock and the
-// motion increment stay on the device, so the sequence can be captured as a graph.
-int Ctx::enqueue_mixed(bool learned) {
-    const int N = npoin, E = nelem;
-    const int TB = 256;
-    // deltat alone (a light pass, so that the mesh motion forks early); the FP64 refinement
-    // of the elements near the FP32 minimum, whose last block forms DTMIN.  ESTAB is formed
-    // in the stage-1 element pass.
+// deltat alone (a light pass, so that the mesh motion forks early); the FP64 refinement of the
+// elements near the FP32 minimum, whose last block forms DTMIN.  ESTAB is formed in the stage-1
+// element pass.
+int Ctx::enqueue_dtmin(const float2* W) {
+    const int E = nelem, TB = 256, nchunk = (int)blocks_for(E, TB);
     tstart(TM_DELTAT);
     CFD_LAUNCH(k_deltat_mixed, blocks_for(E, TB), TB, 0, stream, E, d_elem, d_Tf, d_VXf, d_VYf,
-               d_Wf, d_areaf, (float)prm.t_inf, (float)prm.fsafe, &d_scal->dtmin32_bits,
+               W, d_areaf, (float)prm.t_inf, (float)prm.fsafe, &d_scal->dtmin32_bits,
                d_blockmin, d_dtef);
-    {
-        const int nchunk = (int)blocks_for(E, TB);
-        CFD_LAUNCH(k_deltat_refine, blocks_for(nchunk, TB), TB, 0, stream, E, d_elem, d_Tf, d_VXf,
-                   d_VYf, d_Wf, d_areaf, (const unsigned long long*)d_blockmin, nchunk,
-                   (float)prm.fsafe, (float)prm.t_inf, d_scal, d_tcount, prm.itlocal);
-    }
+    CFD_LAUNCH(k_deltat_refine, blocks_for(nchunk, TB), TB, 0, stream, E, d_elem, d_Tf, d_VXf,
+               d_VYf, W, d_areaf, (const unsigned long long*)d_blockmin, nchunk,
+               (float)prm.fsafe, (float)prm.t_inf, d_scal, d_tcount, prm.itlocal);
     tstop(TM_DELTAT);
+    return CFD_OK;
+}
+
+// The device work of one mixed step, in order.  No host wait: DTMIN, the clock and the
+// motion increment stay on the device, so the sequence can be captured as a graph.  `more`: the
+// same call goes on with another step.
+int Ctx::enqueue_mixed(bool learned, bool more) {
+    const int N = npoin, E = nelem;
+    const int TB = 256;
+    if (!dt_ahead)
+        if (int st = enqueue_dtmin(d_Wf)) return st;
     // The mesh motion of a prescribed law needs DTMIN and the step-start mesh only, and
     // what it produces (the moved mesh, W, the new geometry) is the next step's: it runs
     // on its own stream beside the RK stages, writing the next-step buffers (swapped after
@@ -1138,6 +1149,11 @@ int Ctx::enqueue_mixed(bool learned) {
     // motion follows them on the main stream.
     const bool structural = prm.motion_law == CFD_MOTION_NEWMARK;
     const bool fork = !timers_on && !structural;
+    // The next step's DTMIN needs the last RK stage, the new W and the new areas, not the node
+    // geometry that ends the mesh motion: where the call goes on it is formed beside that pass,
+    // with FORCES on a third stream (a step opens otherwise with 12 us, at 15,150 nodes, of a
+    // nearly idle GPU: 53 -> 50 us a step there).
+    const bool ahead = more && forms_ahead();
     MotionTailArgs t{};
     t.nset = bc.nset_numb;
     t.set_ptr = d_set_ptr;
@@ -1192,6 +1208,7 @@ int Ctx::enqueue_mixed(bool learned) {
         CFD_LAUNCH(k_motion_update_mixed, branch_grid(N, TB, s), TB, 0, s, N, d_pos[0], d_pos[1],
                    d_scal, d_X, d_Y, d_WX_n, d_WY_n, d_Wf_n);
         if (smoothing_now && (st = smooth_in_step(s, d_WX_n, d_WY_n, d_Wf_n))) return st;
+        if (prm.moving != 1) CFD_CUDA(cudaEventRecord(ev_geo, s));
         if (prm.moving == 1 && (st = geometry_mixed(false, false, true, s))) return st;
         if (side_join) {  // the fields' update on stream3 (it reads this step's solutions)
             CFD_CUDA(cudaStreamWaitEvent(s, ev_side[3], 0));
@@ -1244,15 +1261,26 @@ int Ctx::enqueue_mixed(bool learned) {
         if ((st = motion(stream))) return st;
     } else {
         // FORCES on the step's pressure and the step-start edge geometry, which the motion
-        // part has kept: beside the end of the mesh motion
-        if (fork) CFD_CUDA(cudaStreamWaitEvent(stream, ev_tail, 0));
+        // part has kept: beside the end of the mesh motion, and beside the next DTMIN
+        const cudaStream_t fs = ahead ? stream3 : stream;
+        if (ahead) {
+            CFD_CUDA(cudaEventRecord(ev_fork, stream));
+            CFD_CUDA(cudaStreamWaitEvent(fs, ev_fork, 0));
+        }
+        if (fork) CFD_CUDA(cudaStreamWaitEvent(fs, ev_tail, 0));
         MotionTailArgs f = t;
         f.do_motion = 0;
         f.do_forces = 1;
         f.count = d_tcount + 2;
         tstart(TM_FORCES);
-        CFD_LAUNCH(k_motion_tail, (unsigned)tail_blocks, 256, 0, stream, f);
+        CFD_LAUNCH(k_motion_tail, (unsigned)tail_blocks, 256, 0, fs, f);
         tstop(TM_FORCES);
+        if (ahead) {
+            CFD_CUDA(cudaEventRecord(ev_forces, fs));
+            CFD_CUDA(cudaStreamWaitEvent(stream, ev_geo, 0));
+            if ((st = enqueue_dtmin(d_Wf_n))) return st;
+            CFD_CUDA(cudaStreamWaitEvent(stream, ev_forces, 0));
+        }
         if (fork) CFD_CUDA(cudaStreamWaitEvent(stream, ev_join, 0));
     }
     if (fv_each) {  // FORCE_VISC at the print block's point: moved mesh, this step's dNx
@@ -1298,26 +1326,29 @@ void Ctx::swap_mixed_buffers() {
 }
 
 void Ctx::drop_graphs() {
-    for (int p = 0; p < 2; ++p) {
-        if (step_exec[p]) cudaGraphExecDestroy(step_exec[p]);
-        if (step_graph[p]) cudaGraphDestroy(step_graph[p]);
-        step_exec[p] = nullptr;
-        step_graph[p] = nullptr;
+    for (int p = 0; p < 8; ++p) {
+        cudaGraphExec_t& x = step_exec[p & 1][p >> 1];
+        cudaGraph_t& g = step_graph[p & 1][p >> 1];
+        if (x) cudaGraphExecDestroy(x);
+        if (g) cudaGraphDestroy(g);
+        x = nullptr;
+        g = nullptr;
     }
 }
 
 // Replay the captured step, capturing it first.  *launched = false when the capture is
 // not possible here (the caller then enqueues the step launch by launch, and stays so).
-int Ctx::launch_step_graph(bool* launched) {
+int Ctx::launch_step_graph(bool* launched, bool more) {
     *launched = false;
-    // one graph per buffer parity: the captured pointers are the parity's
-    cudaGraph_t& step_graph = this->step_graph[buf];
-    cudaGraphExec_t& step_exec = this->step_exec[buf];
+    // one graph per buffer parity (the captured pointers are the parity's) and place of DTMIN
+    const int at = (dt_ahead ? 2 : 0) + (more ? 1 : 0);
+    cudaGraph_t& step_graph = this->step_graph[buf][at];
+    cudaGraphExec_t& step_exec = this->step_exec[buf][at];
     if (!step_exec) {
         const long long k0 = g_launches.load();
         CFD_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         capturing = true;
-        const int st = enqueue_mixed(false);
+        const int st = enqueue_mixed(false, more);
         capturing = false;
         cudaGraph_t g = nullptr;
         const cudaError_t ce = cudaStreamEndCapture(stream, &g);
@@ -1348,7 +1379,7 @@ int Ctx::launch_step_graph(bool* launched) {
 // when guess_gate is 0): the host reads the previous solve's counts once they are in
 // pinned memory (mid previous step, while the device finishes its mesh update).  The
 // steps without the network replay a captured graph from the second step on.
-int Ctx::step_once_mixed() {
+int Ctx::step_once_mixed(bool more) {
     iter += 1;
     bool learned = false;
     if (learned_mode() && net && lgraph) {
@@ -1364,17 +1395,19 @@ int Ctx::step_once_mixed() {
     smoothing_now = smooth_every > 0 && iter % smooth_every == 0;
     if (graphs_on && !learned && !smoothing_now && mixed_steps > 0) {
         bool launched = false;
-        int st = launch_step_graph(&launched);
+        int st = launch_step_graph(&launched, more);
         if (st) return st;
         if (launched) {
             mixed_steps += 1;
+            dt_ahead = more && forms_ahead();
             swap_mixed_buffers();
             return CFD_OK;
         }
     }
-    int st = enqueue_mixed(learned);
+    int st = enqueue_mixed(learned, more);
     if (st) return st;
     mixed_steps += 1;
+    dt_ahead = more && forms_ahead();
     swap_mixed_buffers();
     return tcollect();
 }

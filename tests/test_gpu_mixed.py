@@ -221,3 +221,41 @@ def test_laplacian_rows_of_hubs(gpu_lib, m, rel_test):
     assert rp[32] == 4 * m + 153
     scale = np.repeat(np.maximum.reduceat(np.abs(ref), rp[:-1]), np.diff(rp))
     assert np.all(np.abs(v - ref) <= (1e-9 if rel_test else 1e-4) * scale)
+
+
+@pytest.mark.parametrize("over", [{}, dict(motion_law=0), dict(moving=0), dict(mass_mode=0),
+                                  dict(mass_mode=1), dict(itlocal=50), dict(guess_mode=2),
+                                  dict(bicg_tol_mode=1), dict(motion_law=2)])
+@pytest.mark.parametrize("graphs", ["1", "0"])
+def test_steps_of_one_call_equal_single_calls(gpu_lib, monkeypatch, over, graphs):
+    """Within a call a step forms the next one's DTMIN beside its node geometry; a single call
+    forms its own.  The state, the mesh, the geometry and the report are the same bit for bit,
+    also where a call follows another and where the host uploads the state between calls."""
+    from cfd_gb300 import abi, solver
+    monkeypatch.setenv("CFD_GRAPHS", graphs)
+    kw = dict(moving=1, motion_law=1, heave_amp=0.05, motion_freq=0.5, mass_mode=2)
+    kw.update(over)
+    k = small_case(3, scale=20, seed=4, **kw)
+    a = solver.Solver(k, precision=abi.CFD_PREC_MIXED)
+    b = solver.Solver(k, precision=abi.CFD_PREC_MIXED)
+    for n, upload in ((5, False), (1, False), (4, True), (2, False), (7, False)):
+        if upload:
+            s = a.state()
+            for side in (a, b):
+                side.set_state(s["U"] * (1 + 1e-6), s["T"])
+        ra = a.step(n)
+        for _ in range(n):
+            rb = b.step(1)
+        assert (ra.iter, ra.time, ra.dtmin) == (rb.iter, rb.time, rb.dtmin)
+        assert tuple(ra.bicg_iters) == tuple(rb.bicg_iters)
+        for i in range(ra.nset_numb):
+            assert (ra.fx[i], ra.fy[i], ra.rm[i]) == (rb.fx[i], rb.fy[i], rb.rm[i])
+        sa, sb = a.state(), b.state()
+        ga, gb = a.geometry(), b.geometry()
+        for key in sa:
+            assert np.array_equal(sa[key], sb[key]), key
+        for key in ga:
+            assert np.array_equal(ga[key], gb[key]), key
+    assert np.isfinite(sa["U"]).all()
+    a.close()
+    b.close()
