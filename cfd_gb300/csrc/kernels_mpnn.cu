@@ -299,6 +299,11 @@ __global__ void k_edge_features(int m, const int* __restrict__ src, const int* _
     }
 }
 
+// ------------------------------------------------------------------ FP32 training passes
+// The ~40 kernels of a loss and gradient run one after the other in one stream, 10 to 35 us each
+// at 49,794 nodes, and are launched as a chain (launch_chain): a kernel's blocks are placed while
+// the one ahead drains, 1.00 -> 0.92 ms of a pass.
+
 // ------------------------------------------------------------------ FP32 dense layers
 // The dense products of a training step, n x 64 or n x 128 rows against 64 x 128 weights: a
 // register-tiled FP32 GEMM, bound by the FP32 pipe.  A block holds the whole weight matrix in
@@ -346,6 +351,8 @@ k_gemm(int n, const float* __restrict__ X1, const float* __restrict__ X2,
     constexpr int T = 32 * G::WARPS, RT = G::RT, KS = G::KS;
     const int tid = threadIdx.x, lane = tid & 31;
     float* Xs = gsm + K * N + (tid >> 5) * GR * KS;  // the warp's rows
+    const int z = chain_wait();
+    W += z;
     const unsigned bs = (unsigned)__cvta_generic_to_shared(Bs);
 #pragma unroll
     for (int q = tid; q < K * N / 4; q += T)
@@ -366,7 +373,7 @@ k_gemm(int n, const float* __restrict__ X1, const float* __restrict__ X2,
     bool ready = false;
     // groups interleaved over the blocks, so that a last partial round spreads over all SMs
     for (int grp = (tid >> 5) * gridDim.x + blockIdx.x; grp < ngroup; grp += gridDim.x * G::WARPS) {
-        const int base = grp * GR;
+        const int base = grp * GR + z;
         __syncwarp();  // the previous group has been read
 #pragma unroll 16
         for (int q = lane; q < GR * K / 4; q += 32) {
@@ -475,8 +482,8 @@ static int gemm(cudaStream_t st, int n, const float* X1, const float* X2, const 
     }
     // the resident blocks of the 152 SMs (each loads the weights once), fewer for few rows
     const unsigned grid = std::min<unsigned>(blocks_for(n, GR * G::WARPS), kTrainChunks * G::PER_SM);
-    CFD_LAUNCH((k_gemm<K, N, EPI>), grid, 32 * G::WARPS, G::SMEM, st, n, X1, X2, gate, W,
-               bias, ptr, E, Y, Y2);
+    CFD_LAUNCH_CHAIN((k_gemm<K, N, EPI>), grid, 32 * G::WARPS, G::SMEM, st, n, X1, X2, gate, W,
+                     bias, ptr, E, Y, Y2);
     return CFD_OK;
 }
 
@@ -508,6 +515,7 @@ __global__ void __launch_bounds__(256) k_encode(int n, const float* __restrict__
                                                 const float* __restrict__ w,
                                                 float* __restrict__ h, float* __restrict__ wt) {
     __shared__ float fs[64 * F_IN];
+    w += chain_wait();
     const int tb = (int)blockIdx.x - ((int)gridDim.x - kEncodeExtra);
     if (tb >= 0) {
         for (int q = tb * 256 + threadIdx.x; q < LAYERS * 4 * HID * HID; q += kEncodeExtra * 256) {
@@ -561,7 +569,7 @@ k_wgrad(int n, const float* __restrict__ dY, const float* __restrict__ gate,
     constexpr int IT = I / 4;
     const int i0 = 4 * (t % IT), o0 = 8 * (t / IT);
     const int rows = (n + kTrainChunks - 1) / kTrainChunks;
-    const int b0 = blockIdx.x * rows, b1 = min(n, b0 + rows);
+    const int b0 = blockIdx.x * rows + chain_wait(), b1 = min(n, b0 + rows);
     static_assert(!BIAS || O == 64, "64 columns by 8 groups of 4 rows");
     const int bo = tid & 63, br = 4 * (tid >> 6);
     float acc[8][4] = {}, bsum = 0.f;
@@ -658,13 +666,14 @@ k_wgrad(int n, const float* __restrict__ dY, const float* __restrict__ gate,
 
 int wgrad_update(cudaStream_t st, int n, const float* dh, const float* v, const float* h,
                  const float* agg, float* part, int layer) {
-    CFD_LAUNCH((k_wgrad<HID, 2 * HID, true>), kTrainChunks, 512, 0, st, n, dh, v, h, agg, part,
-               layer_off(layer) + L_U, layer_off(layer) + L_u);
+    CFD_LAUNCH_CHAIN((k_wgrad<HID, 2 * HID, true>), kTrainChunks, 512, 0, st, n, dh, v, h, agg,
+                     part, layer_off(layer) + L_U, layer_off(layer) + L_u);
     return CFD_OK;
 }
 int wgrad_pq(cudaStream_t st, int n, const float* dpq, const float* h, float* part, int layer) {
-    CFD_LAUNCH((k_wgrad<2 * HID, HID, false>), kTrainChunks, 512, 0, st, n, dpq, (const float*)nullptr, h,
-               (const float*)nullptr, part, layer_off(layer) + L_A, -1);
+    CFD_LAUNCH_CHAIN((k_wgrad<2 * HID, HID, false>), kTrainChunks, 512, 0, st, n, dpq,
+                     (const float*)nullptr, h, (const float*)nullptr, part, layer_off(layer) + L_A,
+                     -1);
     return CFD_OK;
 }
 
@@ -679,7 +688,7 @@ __global__ void __launch_bounds__(512) k_wgrad_in(int n, const float* __restrict
     __shared__ float red[G][64 * (F_IN + 1)];
     const int o = threadIdx.x & 63, g = threadIdx.x >> 6;
     const int rows = (n + kTrainChunks - 1) / kTrainChunks;
-    const int b0 = blockIdx.x * rows, b1 = min(n, b0 + rows);
+    const int b0 = blockIdx.x * rows + chain_wait(), b1 = min(n, b0 + rows);
     float acc[F_IN + 1] = {};
     for (int base = b0; base < b1; base += R) {
         __syncthreads();
@@ -718,7 +727,7 @@ __global__ void __launch_bounds__(512) k_wgrad_in(int n, const float* __restrict
 // loads in flight
 __global__ void k_fold(int nq, const float* __restrict__ part, float* __restrict__ out,
                        float* __restrict__ loss) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x + chain_wait();
     if (q >= nq) return;
     static_assert(kTrainChunks % 4 == 0, "four sums");
     float a[4] = {};
@@ -750,8 +759,9 @@ __global__ void __launch_bounds__(256)
 k_edge_fwd(int n, const int* __restrict__ ptr, const int* __restrict__ nbr,
            const float* __restrict__ PQ, const float* __restrict__ e, const float* __restrict__ C,
            const float* __restrict__ c, ushort4* __restrict__ mask, float* __restrict__ agg) {
-    const int l = threadIdx.x & 15, half = threadIdx.x & 16;
-    const int at = half_warp_node(threadIdx.x >> 4), nblk = (n + 15) / 16;
+    const int z = chain_wait();
+    const int l = (threadIdx.x & 15) + z, half = threadIdx.x & 16;
+    const int at = half_warp_node(threadIdx.x >> 4) + z, nblk = (n + 15) / 16;
     float cw[4][3], cb[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -836,10 +846,11 @@ k_edge_bwd(int n, const int* __restrict__ ptr, const int* __restrict__ nbr,
            const float* __restrict__ dhc, const float* __restrict__ e, float* __restrict__ dPQ,
            float* __restrict__ part, int off) {
     __shared__ float red[16][4 * HID];
-    const int l = threadIdx.x & 15;
+    const int z = chain_wait();
+    const int l = (threadIdx.x & 15) + z;
     float GC[4][3] = {}, Gc[4] = {};
     const int stride = gridDim.x * 64;
-    for (int i = blockIdx.x * 64 + half_warp_node(threadIdx.x >> 4); i < n; i += stride) {
+    for (int i = blockIdx.x * 64 + half_warp_node(threadIdx.x >> 4) + z; i < n; i += stride) {
         const int k0 = ptr[i], k1 = ptr[i + 1];
         const float4 g4 = *reinterpret_cast<const float4*>(dhc + (size_t)i * 2 * HID + HID + 4 * l);
         const float g[4] = {g4.x, g4.y, g4.z, g4.w};
@@ -909,7 +920,7 @@ k_decode(int n, const float* __restrict__ h, const float* __restrict__ w, float*
          const float* __restrict__ target, const int* __restrict__ kind, float inv_nfree,
          float* __restrict__ dh, float* __restrict__ part) {
     __shared__ float red[8][(HID + 1) * OUT + 1];
-    const int l = threadIdx.x & 3;
+    const int z = chain_wait(), l = (threadIdx.x & 3) + z;
     float wo[OUT][16], GW[OUT][16] = {}, gb[OUT] = {}, loss = 0.f;
 #pragma unroll
     for (int o = 0; o < OUT; ++o)
@@ -917,7 +928,7 @@ k_decode(int n, const float* __restrict__ h, const float* __restrict__ w, float*
         for (int k = 0; k < 16; ++k) wo[o][k] = w[OFF_W_OUT + o * HID + 16 * l + k];
     const int stride = gridDim.x * 64;
     // whole warps walk the loop together (the shuffles below)
-    for (int i0 = blockIdx.x * 64 + 8 * (threadIdx.x >> 5); i0 < n; i0 += stride) {
+    for (int i0 = blockIdx.x * 64 + 8 * (threadIdx.x >> 5) + z; i0 < n; i0 += stride) {
         const int i = i0 + ((threadIdx.x & 31) >> 2);
         float hv[16];
 #pragma unroll

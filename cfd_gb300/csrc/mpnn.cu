@@ -99,14 +99,15 @@ int forward_fp32(cfd_mpnn& net, cfd_mpnn_graph& g, const float* target = nullptr
     for (int l = 0; l < LAYERS; ++l) {
         const float *W = net.w + layer_off(l), *Wt = g.wt + layer_off(l);
         if ((rc = dense_pq(st, n, g.h[l], Wt + L_A, g.pq))) return rc;
-        CFD_LAUNCH(k_edge_fwd, std::min(nb_of(n, 16), kEdgeBlocks), 256, 0, st, n, g.ptr, g.nbr, (const float*)g.pq,
-                   (const float*)g.e, W + L_C, W + L_c, g.mask[l], g.agg[l]);
+        CFD_LAUNCH_CHAIN(k_edge_fwd, std::min(nb_of(n, 16), kEdgeBlocks), 256, 0, st, n, g.ptr,
+                         g.nbr, (const float*)g.pq, (const float*)g.e, W + L_C, W + L_c, g.mask[l],
+                         g.agg[l]);
         if ((rc = dense_update(st, n, g.h[l], g.agg[l], Wt + L_U, W + L_u, g.v[l], g.h[l + 1])))
             return rc;
     }
     // with a target (training) the decoder also starts the backward pass
-    CFD_LAUNCH(k_decode, kTrainChunks, 256, 0, st, n, (const float*)g.h[LAYERS], (const float*)net.w,
-               g.y, target, g.kind, 1.f / (float)std::max(g.nfree, 1), g.dh, g.part);
+    CFD_LAUNCH_CHAIN(k_decode, kTrainChunks, 256, 0, st, n, (const float*)g.h[LAYERS],
+                     (const float*)net.w, g.y, target, g.kind, 1.f / (float)std::max(g.nfree, 1), g.dh, g.part);
     return CFD_OK;
 }
 
@@ -121,16 +122,16 @@ int backward_fp32(cfd_mpnn& net, cfd_mpnn_graph& g, float* loss_out) {
         if ((rc = wgrad_update(st, n, g.dh, g.v[l], g.h[l], g.agg[l], g.part, l))) return rc;
         if ((rc = dense_update_bwd(st, n, g.dh, g.v[l], W + L_U, g.ptr, g.dhc))) return rc;
         // agg_i = mean_j relu(z_ij)
-        CFD_LAUNCH(k_edge_bwd, kTrainChunks, 1024, 0, st, n, g.ptr, g.nbr, g.rev,
-                   (const ushort4*)g.mask[l], (const float*)g.dhc, (const float*)g.e, g.dpq, g.part,
-                   layer_off(l) + L_C);
+        CFD_LAUNCH_CHAIN(k_edge_bwd, kTrainChunks, 1024, 0, st, n, g.ptr, g.nbr, g.rev,
+                         (const ushort4*)g.mask[l], (const float*)g.dhc, (const float*)g.e, g.dpq,
+                         g.part, layer_off(l) + L_C);
         if ((rc = wgrad_pq(st, n, g.dpq, g.h[l], g.part, l))) return rc;
         if ((rc = dense_pq_bwd(st, n, g.dpq, W + L_A, g.dhc, g.dh))) return rc;
     }
-    CFD_LAUNCH(k_wgrad_in, kTrainChunks, 512, 0, st, n, (const float*)g.dh, (const float*)g.h[0],
-               (const float*)g.f, g.part);
-    CFD_LAUNCH(k_fold, nb_of(N_PARAMS + 1, 128), 128, 0, st, N_PARAMS + 1, (const float*)g.part,
-               net.g, g.loss);
+    CFD_LAUNCH_CHAIN(k_wgrad_in, kTrainChunks, 512, 0, st, n, (const float*)g.dh,
+                     (const float*)g.h[0], (const float*)g.f, g.part);
+    CFD_LAUNCH_CHAIN(k_fold, nb_of(N_PARAMS + 1, 128), 128, 0, st, N_PARAMS + 1,
+                     (const float*)g.part, net.g, g.loss);
     if (loss_out) {
         CFD_CUDA(cudaMemcpyAsync(loss_out, g.loss, sizeof(float), cudaMemcpyDeviceToHost, st));
         CFD_CUDA(cudaStreamSynchronize(st));
