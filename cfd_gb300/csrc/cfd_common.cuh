@@ -34,11 +34,12 @@ void set_last_cuda_error(cudaError_t e, const char* what, const char* file, int 
 // A kernel of a chain in one stream may be placed before the kernel ahead of it has ended
 // (programmatic dependent launch): its blocks take SMs as that one's last blocks leave them, and
 // wait in chain_wait().  Every thread of a kernel launched so calls chain_wait() before it reads
-// or writes global memory; only then may the next kernel be placed.  The result is 0 and goes into
-// the addresses of what is read afterwards: the compiler may move a load through a const
-// __restrict__ pointer above the wait otherwise.  Used for the training
-// passes; the FP64 step's RK stages got slower by it (2.33 -> 2.64 ms a 10-step march at 8,192
-// nodes, 5.58 -> 5.80 ms for 5 steps at 69,390).
+// or writes what a kernel of the chain writes; only then may the next kernel be placed, so the one
+// before the one ahead has ended too.  The chain's first kernel is launched plainly.  The result
+// is 0 and goes into the addresses of what is read afterwards: the compiler may move a load
+// through a const __restrict__ pointer above the wait otherwise.  Used for the network's passes;
+// the FP64 step's RK stages got slower by it (2.33 -> 2.64 ms for 10 steps at 8,192 nodes, 5.58 ->
+// 5.80 for 5 steps at 69,390).
 template <class... P, class... A>
 cudaError_t launch_chain(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
                          cudaStream_t stream, A... args) {
