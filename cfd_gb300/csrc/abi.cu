@@ -308,6 +308,24 @@ int cfd_selftest_waits(long long polls, int* barrier_status, int* mbarrier_statu
     return CFD_OK;
 }
 
+int cfd_selftest_solve_wait(long long polls, int* wait_status) {
+    if (polls < 1 || polls > (1LL << 24) || !wait_status)
+        return arg_error("polls in [1, 2^24] and a status pointer");
+    Scratch s;
+    TRY(s.init(4096));
+    GridBar* gb;
+    int *out, h = -1;
+    TRY(s.alloc(&gb, 1));
+    TRY(s.alloc(&out, 1));
+    CFD_CUDA(cudaMemsetAsync(gb, 0, sizeof(GridBar), s.stream));
+    CFD_CUDA(cudaMemsetAsync(out, 0xff, sizeof(int), s.stream));
+    CFD_LAUNCH(k_selftest_solve_wait, 1, 32, 0, s.stream, gb, out, polls);
+    TRY(s.get(&h, out, 1));
+    TRY(s.sync());
+    *wait_status = h;
+    return CFD_OK;
+}
+
 void* cfd_ctx_stream(cfd_ctx* ctx) { return ctx ? (void*)ctx->impl.stream : nullptr; }
 
 int cfd_ctx_mark(cfd_ctx* ctx, int slot) {

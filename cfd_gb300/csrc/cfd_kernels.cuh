@@ -431,6 +431,7 @@ struct PcgArgs {
 cudaError_t launch_pcg_fp64(cudaStream_t st, PcgArgs a);
 __global__ void k_pcg_mixed(PcgArgs a);
 __global__ void k_selftest_waits(GridBar* gb, int* out, long long limit);
+__global__ void k_selftest_solve_wait(GridBar* gb, int* out, long long limit);
 __global__ void k_bicg_fix_mixed(PcgArgs a);
 // first pass of a mixed solve (k_bicg_resid_mixed, the variant of a.tol_mode)
 cudaError_t launch_bicg_resid_mixed(unsigned grid, cudaStream_t stream, const PcgArgs& a);

@@ -40,10 +40,11 @@ constexpr int kGroup = 4;             // chunks a block takes between two barrie
 // ------------------------------------------------------------------ barrier of one launch
 // gb->arrive counts arrivals from zero; a waiter leaves when the count has reached `target`
 // (compared modulo 2^32).  One hop: the last arrival itself releases the waiters.  false: the
-// bounds ran out (gb->err is set).  The last block to leave a launch that did not fail clears
-// the count for the next one (gb->gen counts the leavers), so that no clearing stands before
-// each launch; after a failure the host clears it.
-__device__ __forceinline__ bool bar_arrive_wait(GridBar* gb, unsigned target) {
+// wait gave up after about `limit` polls or kWaitNs (gb->err is set).  The last block to leave a
+// launch that did not fail clears the count for the next one (gb->gen counts the leavers), so
+// that no clearing stands before each launch; after a failure the host clears it.
+__device__ __forceinline__ bool bar_arrive_wait(GridBar* gb, unsigned target,
+                                                long long limit = kSpinLimit) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&gb->arrive) : "memory");
     unsigned long long t0 = 0;
     for (long long spins = 0;; ++spins) {
@@ -53,7 +54,7 @@ __device__ __forceinline__ bool bar_arrive_wait(GridBar* gb, unsigned target) {
         if ((spins & 63) == 63) {
             const unsigned long long now = globaltimer_ns();
             if (t0 == 0) t0 = now;
-            if (now - t0 > kWaitNs || spins > kSpinLimit) {
+            if (now - t0 > kWaitNs || spins > limit) {
                 atomicExch(&gb->err, (int)CFD_ERR_BARRIER);
                 return false;
             }
@@ -603,10 +604,6 @@ cudaError_t launch_pcg_fp64(cudaStream_t st, PcgArgs a) {
     return e;
 }
 
-// Failure-detection self-test of the two bounded waits (one block): a grid barrier that
-// expects a second block that never comes, and an mbarrier nothing arrives on.  Both give
-// up after `limit` polls; out[0] = the barrier's error word, out[1] = CFD_ERR_BARRIER when
-// the mbarrier wait gave up (0 if it completed).
 // CFD_GUESS_EXTRAPOLATED: the solves start from the last two increments extrapolated to
 // this step.  A solve's unknown is the step's mesh increment, the mean mesh velocity over the
 // step times DTMIN; with that velocity linear in time through the last two steps' midpoints,
@@ -719,6 +716,10 @@ cudaError_t launch_selftest_divrcp(long long n, unsigned long long seed, unsigne
     return cudaGetLastError();
 }
 
+// Failure-detection self-test of the mixed solve's grid barrier and the mbarrier wait (one block):
+// a grid barrier that expects a second block that never comes, and an mbarrier nothing arrives
+// on.  Both give up after `limit` polls; out[0] = the barrier's error word, out[1] =
+// CFD_ERR_BARRIER when the mbarrier wait gave up (0 if it completed).
 __global__ void k_selftest_waits(GridBar* gb, int* out, long long limit) {
     __shared__ __align__(8) unsigned long long bar;
     grid_barrier(gb, 2u, limit);
@@ -729,6 +730,12 @@ __global__ void k_selftest_waits(GridBar* gb, int* out, long long limit) {
         out[1] = mbar_wait_bounded(ubar, 0u, limit) ? 0 : (int)CFD_ERR_BARRIER;
         out[0] = gb->err;
     }
+}
+
+// The same of the FP64 solve's barrier: *out = the barrier's error word when the wait for a second
+// arrival that never comes gave up, 0 if it did not.
+__global__ void k_selftest_solve_wait(GridBar* gb, int* out, long long limit) {
+    if (threadIdx.x == 0) *out = bar_arrive_wait(gb, 2u, limit) ? 0 : gb->err;
 }
 
 }  // namespace cfd

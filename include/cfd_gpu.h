@@ -485,13 +485,16 @@ int cfd_ctx_smoothing_stats(cfd_ctx* ctx, long long* out2);
 /* Number of kernels this library launched since process start (all contexts). */
 long long cfd_kernel_launches(void);
 
-/* Failure-detection self-test (no counterpart in the reference): runs, in one block, the
- * library's two bounded device waits on conditions that never come true (a grid barrier
- * that a second block never reaches; an mbarrier nothing arrives on), each giving up after
- * `polls` polls (1 .. 2^24; the library's kernels use 2^24) or 1 s on the GPU's global
- * timer, whichever comes first (every wait of the library has both bounds).  Both statuses
- * come back as CFD_ERR_BARRIER and the device stays usable. */
+/* Failure-detection self-test (no counterpart in the reference): runs, in one block, two of
+ * the library's bounded device waits on conditions that never come true (the mixed solve's
+ * grid barrier, which a second block never reaches; an mbarrier nothing arrives on), each
+ * giving up after `polls` polls (1 .. 2^24; the library's kernels use 2^24) or 1 s on the
+ * GPU's global timer, whichever comes first (every wait of the library has both bounds).
+ * Both statuses come back as CFD_ERR_BARRIER and the device stays usable. */
 int cfd_selftest_waits(long long polls, int* barrier_status, int* mbarrier_status);
+/* The same for the FP64 solve's grid barrier: a second arrival never comes, the wait gives up
+ * with CFD_ERR_BARRIER. */
+int cfd_selftest_solve_wait(long long polls, int* wait_status);
 
 /* Arithmetic self-test (no counterpart in the reference): the FP64 kernels divide by 3 with
  * a multiply and two FMAs (Markstein's correction of the quotient by the rounded reciprocal);

@@ -120,6 +120,25 @@ def test_bounded_waits_give_up_and_the_device_stays_usable(gpu_lib):
 
 
 @pytest.mark.gpu
+def test_fp64_solve_wait_gives_up(gpu_lib):
+    """The FP64 solve's own grid barrier: the wait for an arrival that never comes gives up with
+    CFD_ERR_BARRIER, and FP64 steps run afterwards in the same process."""
+    import ctypes as C
+    from cfd_gb300 import abi, solver
+    w = C.c_int(-1)
+    for polls in (1, 1000, 100000):
+        abi.check(abi.lib().cfd_selftest_solve_wait(polls, C.byref(w)), "selftest")
+        assert w.value == abi.CFD_ERR_BARRIER
+    for polls in (0, (1 << 24) + 1):
+        assert abi.lib().cfd_selftest_solve_wait(polls, C.byref(w)) == abi.CFD_ERR_ARG
+    k = small_case(3, scale=16, seed=3)
+    s = solver.Solver(k)
+    rep = s.step(2)
+    assert rep.iter == 2 and np.isfinite(s.state()["U"]).all()
+    s.close()
+
+
+@pytest.mark.gpu
 def test_div3_equals_the_division(gpu_lib):
     """The FP64 kernels' division by 3 (a multiply and two FMAs) gives the IEEE quotient
     x / 3.0 bit for bit over 2^32 inputs: raw bit patterns (every exponent, zeros,
