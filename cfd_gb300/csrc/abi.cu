@@ -326,6 +326,65 @@ int cfd_selftest_solve_wait(long long polls, int* wait_status) {
     return CFD_OK;
 }
 
+int cfd_selftest_failed_barrier(int* solve_status) {
+    if (!solve_status) return arg_error("status pointer");
+    Scratch s;
+    TRY(s.init(4096));
+    // 2 x = 4 from x = 3 on a barrier that gave up with one arrival counted
+    const GridBar failed{1u, 0u, (int)CFD_ERR_BARRIER, 0};
+    const int rowptr[2] = {0, 1}, zero = 0, none = -1;
+    const double two = 2.0, four = 4.0, x0 = 3.0;
+    GridBar* gb;
+    unsigned char* isfix;
+    int *rp, *col, *it, *cv;
+    double *val, *x, *b, *w, *rz;
+    TRY(s.put(&gb, &failed, 1));
+    TRY(s.put(&rp, rowptr, 2));
+    TRY(s.put(&col, &zero, 1));
+    TRY(s.put(&val, &two, 1));
+    TRY(s.put(&x, &x0, 1));
+    TRY(s.put(&b, &four, 1));
+    TRY(s.put(&it, &none, 1));
+    TRY(s.alloc(&isfix, 1));
+    CFD_CUDA(cudaMemsetAsync(isfix, 0, 1, s.stream));
+    TRY(s.alloc(&w, 5 + 6));  // r, z, y, p, 1/diag; the partials of one chunk
+    TRY(s.alloc(&rz, 1));
+    TRY(s.alloc(&cv, 1));
+    PcgArgs a{};
+    a.n = 1;
+    a.nsolve = 1;
+    a.rowptr = rp;
+    a.col = col;
+    a.val = a.diag = val;
+    a.isfix = isfix;
+    a.x[0] = a.x[1] = x;
+    a.b[0] = a.b[1] = b;
+    a.r[0] = a.r[1] = w;
+    a.z[0] = a.z[1] = w + 1;
+    a.y[0] = a.y[1] = w + 2;
+    a.p[0][0] = a.p[1][0] = w + 3;
+    a.rdiag = w + 4;
+    a.part = w + 5;
+    a.bar = gb;
+    a.tol = 1.0e-10;
+    a.maxit = 10;
+    a.iters_out = it;
+    a.rz_out = rz;
+    a.conv_out = cv;
+    CFD_CUDA(launch_pcg_fp64(s.stream, a));
+    double xe = 0.0;
+    int iters = 0;
+    GridBar after{};
+    TRY(s.get(&xe, x, 1));
+    TRY(s.get(&iters, it, 1));
+    TRY(s.get(&after, gb, 1));
+    TRY(s.sync());
+    const bool untouched = xe == x0 && iters == none && after.err == failed.err &&
+                           after.arrive == failed.arrive && after.gen == failed.gen;
+    *solve_status = untouched ? (int)CFD_ERR_BARRIER : 0;
+    return CFD_OK;
+}
+
 void* cfd_ctx_stream(cfd_ctx* ctx) { return ctx ? (void*)ctx->impl.stream : nullptr; }
 
 int cfd_ctx_mark(cfd_ctx* ctx, int slot) {

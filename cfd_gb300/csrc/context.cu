@@ -745,7 +745,8 @@ int Ctx::step(int nsteps, cfd_step_report* rep) {
         disn[1] = ms.disn1;
     }
     if (gb.err) {
-        // a barrier that gave up is left mid-count: the next solve starts from a fresh one
+        // a barrier that gave up is left mid-count and the call's later solves did nothing: the
+        // next call starts from a fresh one
         CFD_CUDA(cudaMemsetAsync(d_bar, 0, sizeof(GridBar), stream));
         set_last_message("a bounded device wait gave up (BiCG grid barrier or node-pass copy)");
         return CFD_ERR_BARRIER;

@@ -40,9 +40,10 @@ constexpr int kGroup = 4;             // chunks a block takes between two barrie
 // ------------------------------------------------------------------ barrier of one launch
 // gb->arrive counts arrivals from zero; a waiter leaves when the count has reached `target`
 // (compared modulo 2^32).  One hop: the last arrival itself releases the waiters.  false: the
-// wait gave up after about `limit` polls or kWaitNs (gb->err is set).  The last block to leave a
-// launch that did not fail clears the count for the next one (gb->gen counts the leavers), so
-// that no clearing stands before each launch; after a failure the host clears it.
+// wait gave up after about `limit` polls or kWaitNs, or another wait has (gb->err is set).  The
+// last block to leave a launch that did not fail clears the count for the next one (gb->gen
+// counts the leavers), so that no clearing stands before each launch.  A failure leaves the count
+// as it stood; launches that find err set do nothing, until the host has reported and cleared it.
 __device__ __forceinline__ bool bar_arrive_wait(GridBar* gb, unsigned target,
                                                 long long limit = kSpinLimit) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&gb->arrive) : "memory");
@@ -52,6 +53,7 @@ __device__ __forceinline__ bool bar_arrive_wait(GridBar* gb, unsigned target,
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&gb->arrive) : "memory");
         if ((int)(v - target) >= 0) return true;
         if ((spins & 63) == 63) {
+            if (*(volatile const int*)&gb->err) return false;
             const unsigned long long now = globaltimer_ns();
             if (t0 == 0) t0 = now;
             if (now - t0 > kWaitNs || spins > limit) {
@@ -180,6 +182,8 @@ __global__ void __launch_bounds__(kChunk, 1) k_pcg_fp64(PcgArgs a) {
     unsigned target = 0;
     const bool rel = a.tol_mode != CFD_BICG_TOL_ABS;   // r.r per iteration
     const bool relb = a.tol_mode == CFD_BICG_TOL_REL;  // ||b - A.x_D|| as reference
+    // after a barrier of an earlier launch gave up; one thread reads it, for the whole block
+    if (__syncthreads_or(t == 0 && *(volatile const int*)&a.bar->err != 0)) return;
     if (t == 0) s.fail = 0;
 
     auto leave = [&] {  // one thread; the block waits no more

@@ -495,6 +495,9 @@ int cfd_selftest_waits(long long polls, int* barrier_status, int* mbarrier_statu
 /* The same for the FP64 solve's grid barrier: a second arrival never comes, the wait gives up
  * with CFD_ERR_BARRIER. */
 int cfd_selftest_solve_wait(long long polls, int* wait_status);
+/* An FP64 solve (of one row) on a barrier that has given up: the solves after a failure do
+ * nothing until the call has reported it (solve_status CFD_ERR_BARRIER; 0: the solve ran). */
+int cfd_selftest_failed_barrier(int* solve_status);
 
 /* Arithmetic self-test (no counterpart in the reference): the FP64 kernels divide by 3 with
  * a multiply and two FMAs (Markstein's correction of the quotient by the rounded reciprocal);

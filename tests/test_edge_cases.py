@@ -139,6 +139,18 @@ def test_fp64_solve_wait_gives_up(gpu_lib):
 
 
 @pytest.mark.gpu
+def test_fp64_solve_after_a_failure_does_nothing(gpu_lib):
+    """A give-up leaves the FP64 solve's barrier with arrivals counted, on which the next solve's
+    blocks would pass it early: a solve that finds the error set leaves x, its report and the
+    barrier as they are."""
+    import ctypes as C
+    from cfd_gb300 import abi
+    v = C.c_int(-1)
+    abi.check(abi.lib().cfd_selftest_failed_barrier(C.byref(v)), "selftest")
+    assert v.value == abi.CFD_ERR_BARRIER
+
+
+@pytest.mark.gpu
 def test_div3_equals_the_division(gpu_lib):
     """The FP64 kernels' division by 3 (a multiply and two FMAs) gives the IEEE quotient
     x / 3.0 bit for bit over 2^32 inputs: raw bit patterns (every exponent, zeros,
