@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(kChunk, 1) k_pcg_fp64(PcgArgs a) {
             int ok = 1;
             if (lane == 0) ok = bar_arrive_wait(a.bar, target) ? 1 : 0;
             ok = __shfl_sync(0xffffffffu, ok, 0);
+            __syncwarp();  // lane 0's acquire comes before every lane's reads (a shuffle orders none)
             if (ok) {
                 const int q = slot_at(code, wp);
                 const double v = chunk_fold(a.part + q * nc, nc);
