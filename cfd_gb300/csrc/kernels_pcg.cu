@@ -251,7 +251,8 @@ __global__ void __launch_bounds__(kChunk, 1) k_pcg_fp64(PcgArgs a) {
     if (ON_CHIP) {
         const long i = (long)blockIdx.x * kChunk + t;
         int key = 0;
-        if (i < n && !a.isfix[i]) key = min(a.rowptr[i + 1] - a.rowptr[i], kSortLen - 1);
+        if (i < n && !a.isfix[i])  // row pointers that descend: an empty row, as in the row loops
+            key = max(0, min(a.rowptr[i + 1] - a.rowptr[i], kSortLen - 1));
         if (t < kSortLen) s.hist[t] = 0;
         __syncthreads();
         if (i < n) atomicAdd(&s.hist[key], 1);

@@ -356,3 +356,27 @@ def test_gpu_solve_at_chunk_edges(gpu_lib, oracle, n, mode):
     xg, ig = solver.biCG(vals, idx, rp, diag, x0, b, data, fix, tol=1e-8, maxit=25, tol_mode=tm)
     assert (ig.iters, ig.converged, ig.rz, ig.relres) == (io.iters, io.converged, io.rz, io.relres)
     assert np.array_equal(xg, xo)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["abs", "rel"])
+def test_gpu_solve_with_descending_row_pointers(gpu_lib, oracle, mode):
+    """A row whose pointers descend is an empty row, as in the oracle's loops: two or three entries
+    back at every 97th row, and all the way from the last entry at three rows, one of them
+    the first of a 1024-row chunk."""
+    from cfd_gb300 import abi, solver
+    n = 3000
+    vals, idx, rp, diag = _graph_matrix(n, 7)
+    for k in range(50, n - 2, 97):
+        rp[k] = rp[k + 1] + 2 + k % 2
+    rp[[700, 1024, 2900]] = rp[n]
+    assert rp.min() == 0 and rp.max() == rp[n] and (np.diff(rp) < 0).sum() > 30
+    rng = np.random.default_rng(8)
+    fix = np.arange(1, n, 500, dtype=np.int32)
+    data, x0, b = rng.normal(size=len(fix)), 0.1 * rng.normal(size=n), rng.normal(size=n)
+    tm = abi.CFD_BICG_TOL_ABS if mode == "abs" else abi.CFD_BICG_TOL_REL
+    xo, io = oracle.bicg(vals, idx, rp, diag, x0, b, data, fix, tol=1e-8, maxit=4, tol_mode=tm)
+    xg, ig = solver.biCG(vals, idx, rp, diag, x0, b, data, fix, tol=1e-8, maxit=4, tol_mode=tm)
+    assert np.isfinite(xo).all()
+    assert (ig.iters, ig.converged, ig.rz, ig.relres) == (io.iters, io.converged, io.rz, io.relres)
+    assert np.array_equal(xg, xo)
