@@ -202,6 +202,7 @@ struct Ctx {
     // next one's (1)
     cudaGraph_t step_graph[2][4] = {};
     cudaGraphExec_t step_exec[2][4] = {};
+    long long step_kernels[2][4] = {};  // kernels of one replay of each
     // within one cfd_step call: the last step has formed the coming step's DTMIN
     bool dt_ahead = false;
     cudaEvent_t ev_geo = nullptr;  // the next step's W and areas are there
@@ -213,7 +214,7 @@ struct Ctx {
     float2* d_Wf_n = nullptr;
     double4_32a* d_fgeo = nullptr;  // per force-set edge: the step-start edge geometry
     int buf = 0;
-    long long graph_kernels = 0;  // kernels of one replay
+    long long graph_kernels = 0;  // kernels of the last replay
     long long mixed_steps = 0;    // steps of this context (the first runs uncaptured)
     long long graph_replays = 0;
     int* d_slot_pos = nullptr;

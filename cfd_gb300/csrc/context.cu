@@ -1360,7 +1360,7 @@ int Ctx::launch_step_graph(bool* launched, bool more) {
             cudaGraphInstantiate(&ex, g, 0) == cudaSuccess) {
             step_graph = g;
             step_exec = ex;
-            graph_kernels = nk;
+            step_kernels[buf][at] = nk;
         } else {
             if (g) cudaGraphDestroy(g);
             (void)cudaGetLastError();
@@ -1369,6 +1369,7 @@ int Ctx::launch_step_graph(bool* launched, bool more) {
         }
     }
     CFD_CUDA(cudaGraphLaunch(step_exec, stream));
+    graph_kernels = step_kernels[buf][at];
     g_launches.fetch_add(graph_kernels, std::memory_order_relaxed);
     graph_replays += 1;
     *launched = true;

@@ -311,7 +311,7 @@ class Solver:
         return fvx[:n], fvy[:n], skin[:ne]
 
     def graph_state(self):
-        """(1 if steps replay a captured CUDA graph, replays so far, kernels per replay)."""
+        """(1 if steps replay a captured CUDA graph, replays so far, kernels in the last replay)."""
         out = (C.c_longlong * 3)()
         check(abi.lib().cfd_ctx_graph_state(self.h, out), "cfd_ctx_graph_state")
         return tuple(int(v) for v in out)

@@ -451,7 +451,8 @@ int cfd_ctx_set_force_visc(cfd_ctx* ctx, int each_step);
 int cfd_ctx_force_visc(cfd_ctx* ctx, double* F_VX, double* F_VY, double* skin);
 
 /* Mixed form: out3 = (1 if steps replay a captured CUDA graph, steps replayed so far,
- * kernels in one replay).  The first step of a context, and steps that run the learned
+ * kernels in the last replay: the first, the inner and the last steps of a call can differ in
+ * where DTMIN is formed).  The first step of a context, and steps that run the learned
  * guess, are enqueued launch by launch; CFD_GRAPHS=0 or CFD_TIMERS=1 at create turn the
  * graph off.  No counterpart in the reference (its time loop calls the routines of
  * ns2DComp.ALE.f90:114-283 one by one). */

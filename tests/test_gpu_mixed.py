@@ -259,3 +259,28 @@ def test_steps_of_one_call_equal_single_calls(gpu_lib, monkeypatch, over, graphs
     assert np.isfinite(sa["U"]).all()
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("over", [{}, dict(motion_law=2), dict(moving=0)])
+def test_launch_counts_with_and_without_graphs(gpu_lib, monkeypatch, over):
+    """cfd_kernel_launches counts the kernels that ran: calls of one, two, three and 20 steps
+    launch as many with the steps replayed from captured graphs (which differ by the place of
+    the next DTMIN) as enqueued launch by launch."""
+    from cfd_gb300 import abi, solver
+    kw = dict(moving=1, motion_law=1, heave_amp=0.05, motion_freq=0.5, mass_mode=2)
+    kw.update(over)
+    counts = []
+    for graphs in ("0", "1"):
+        monkeypatch.setenv("CFD_GRAPHS", graphs)
+        s = solver.Solver(small_case(3, scale=20, seed=4, **kw), precision=abi.CFD_PREC_MIXED)
+        seen = []
+        for n in (1, 3, 1, 20, 1, 1, 2, 20):
+            before = abi.lib().cfd_kernel_launches()
+            s.step(n)
+            seen.append(abi.lib().cfd_kernel_launches() - before)
+        counts.append(seen)
+        if graphs == "1":
+            s.step(1)  # a step by itself: its kernels and the report's
+            assert s.graph_state()[2] == seen[4] - 1
+        s.close()
+    assert counts[0] == counts[1]
