@@ -142,6 +142,7 @@ SIGNATURES = {
     "cfd_ctx_set_guess_refine": (C.c_int, [_P, C.c_int]),
     "cfd_ctx_guess_stats_ex": (C.c_int, [_P, C.POINTER(C.c_longlong)]),
     "cfd_ctx_graph_state": (C.c_int, [_P, C.POINTER(C.c_longlong)]),
+    "cfd_ctx_graph_count": (C.c_int, [_P, _ip]),
     "cfd_ctx_set_force_visc": (C.c_int, [_P, C.c_int]),
     "cfd_ctx_smooth": (C.c_int, [_P, _ip, _dp]),
     "cfd_ctx_smooth_ex": (C.c_int, [_P, C.c_int, _ip, _dp]),

@@ -639,6 +639,14 @@ int cfd_ctx_graph_state(cfd_ctx* ctx, long long* out3) {
     return CFD_OK;
 }
 
+int cfd_ctx_graph_count(cfd_ctx* ctx, int* graphs) {
+    if (!ctx || !graphs) return arg_error("ctx/graphs");
+    *graphs = 0;
+    for (const auto& parity : ctx->impl.step_exec)
+        for (const cudaGraphExec_t x : parity) *graphs += x != nullptr;
+    return CFD_OK;
+}
+
 int cfd_step(cfd_ctx* ctx, int nsteps, cfd_step_report* rep) {
     if (!ctx) return arg_error("ctx");
     return ctx->impl.step(nsteps, rep);

@@ -270,7 +270,7 @@ struct Ctx {
                prm.guess_mode == CFD_GUESS_LEARNED_EXTRAPOLATED;
     }
     int guess_extrapolate(const PcgArgs& a, cudaStream_t s, unsigned grid);
-    int enqueue_mixed(bool learned, bool more);
+    int enqueue_mixed(bool learned, bool ahead);
     int enqueue_dtmin(const float2* W);
     // A step forms the next one's DTMIN where its passes leave SMs idle: up to 11,000 elements per
     // SM (836,000 nodes).  20 steps of 262,144 nodes 4.46 -> 4.16 ms, 409,600 5.24 -> 4.82, 810,000
@@ -279,7 +279,7 @@ struct Ctx {
         return !timers_on && prm.motion_law != CFD_MOTION_NEWMARK && !smoothing_now && !fv_each &&
                nelem <= 11000L * nsm;
     }
-    int launch_step_graph(bool* launched, bool more);
+    int launch_step_graph(bool* launched, bool ahead);
     int set_guess_net(cfd_mpnn* n, double gate);
     int force_visc_now();
     int smooth(int* iters, double* min_quality, bool node_order = false);

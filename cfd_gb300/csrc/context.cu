@@ -1136,9 +1136,9 @@ int Ctx::enqueue_dtmin(const float2* W) {
 }
 
 // The device work of one mixed step, in order.  No host wait: DTMIN, the clock and the
-// motion increment stay on the device, so the sequence can be captured as a graph.  `more`: the
-// same call goes on with another step.
-int Ctx::enqueue_mixed(bool learned, bool more) {
+// motion increment stay on the device, so the sequence can be captured as a graph.  `ahead`: the
+// same call goes on with another step, whose DTMIN this one forms (forms_ahead()).
+int Ctx::enqueue_mixed(bool learned, bool ahead) {
     const int N = npoin, E = nelem;
     const int TB = 256;
     if (!dt_ahead)
@@ -1154,7 +1154,6 @@ int Ctx::enqueue_mixed(bool learned, bool more) {
     // geometry that ends the mesh motion: where the call goes on it is formed beside that pass,
     // with FORCES on a third stream (a step opens otherwise with 12 us, at 15,150 nodes, of a
     // nearly idle GPU: 53 -> 50 us a step there).
-    const bool ahead = more && forms_ahead();
     MotionTailArgs t{};
     t.nset = bc.nset_numb;
     t.set_ptr = d_set_ptr;
@@ -1339,17 +1338,17 @@ void Ctx::drop_graphs() {
 
 // Replay the captured step, capturing it first.  *launched = false when the capture is
 // not possible here (the caller then enqueues the step launch by launch, and stays so).
-int Ctx::launch_step_graph(bool* launched, bool more) {
+int Ctx::launch_step_graph(bool* launched, bool ahead) {
     *launched = false;
     // one graph per buffer parity (the captured pointers are the parity's) and place of DTMIN
-    const int at = (dt_ahead ? 2 : 0) + (more ? 1 : 0);
+    const int at = (dt_ahead ? 2 : 0) + (ahead ? 1 : 0);
     cudaGraph_t& step_graph = this->step_graph[buf][at];
     cudaGraphExec_t& step_exec = this->step_exec[buf][at];
     if (!step_exec) {
         const long long k0 = g_launches.load();
         CFD_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         capturing = true;
-        const int st = enqueue_mixed(false, more);
+        const int st = enqueue_mixed(false, ahead);
         capturing = false;
         cudaGraph_t g = nullptr;
         const cudaError_t ce = cudaStreamEndCapture(stream, &g);
@@ -1395,21 +1394,22 @@ int Ctx::step_once_mixed(bool more) {
     // a step that smooths its moved mesh waits on the host for the sweeps' convergence
     // flags: it is enqueued launch by launch
     smoothing_now = smooth_every > 0 && iter % smooth_every == 0;
+    const bool ahead = more && forms_ahead();
     if (graphs_on && !learned && !smoothing_now && mixed_steps > 0) {
         bool launched = false;
-        int st = launch_step_graph(&launched, more);
+        int st = launch_step_graph(&launched, ahead);
         if (st) return st;
         if (launched) {
             mixed_steps += 1;
-            dt_ahead = more && forms_ahead();
+            dt_ahead = ahead;
             swap_mixed_buffers();
             return CFD_OK;
         }
     }
-    int st = enqueue_mixed(learned, more);
+    int st = enqueue_mixed(learned, ahead);
     if (st) return st;
     mixed_steps += 1;
-    dt_ahead = more && forms_ahead();
+    dt_ahead = ahead;
     swap_mixed_buffers();
     return tcollect();
 }

@@ -316,6 +316,12 @@ class Solver:
         check(abi.lib().cfd_ctx_graph_state(self.h, out), "cfd_ctx_graph_state")
         return tuple(int(v) for v in out)
 
+    def graph_count(self):
+        """Captured step graphs that the context holds."""
+        n = C.c_int()
+        check(abi.lib().cfd_ctx_graph_count(self.h, C.byref(n)), "cfd_ctx_graph_count")
+        return n.value
+
     def step(self, n=1):
         rep = abi.CfdStepReport()
         check(abi.lib().cfd_step(self.h, int(n), C.byref(rep)), "cfd_step")

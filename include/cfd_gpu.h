@@ -457,6 +457,8 @@ int cfd_ctx_force_visc(cfd_ctx* ctx, double* F_VX, double* F_VY, double* skin);
  * graph off.  No counterpart in the reference (its time loop calls the routines of
  * ns2DComp.ALE.f90:114-283 one by one). */
 int cfd_ctx_graph_state(cfd_ctx* ctx, long long* out3);
+/* Mixed form: the captured step graphs that the context holds. */
+int cfd_ctx_graph_count(cfd_ctx* ctx, int* graphs);
 
 /* Smooth the context's mesh as the reference does at setup (ns2DComp.ALE.f90:62-72,
  * smoothing.f90; the mesh-motion boundary nodes stay), then recompute its geometry (normals,

@@ -284,3 +284,19 @@ def test_launch_counts_with_and_without_graphs(gpu_lib, monkeypatch, over):
             assert s.graph_state()[2] == seen[4] - 1
         s.close()
     assert counts[0] == counts[1]
+
+
+@pytest.mark.parametrize("case", ["newmark", "force_visc"])
+def test_two_graphs_where_no_step_forms_the_next_dtmin(gpu_lib, case):
+    """Where a step does not form the next one's DTMIN, its place in a call changes nothing: the
+    context holds one graph per buffer parity, whatever the lengths of the calls."""
+    from cfd_gb300 import abi, solver
+    k = small_case(3, scale=20, seed=4, moving=1, motion_law=2 if case == "newmark" else 1,
+                   heave_amp=0.05, motion_freq=0.5, mass_mode=2)
+    s = solver.Solver(k, precision=abi.CFD_PREC_MIXED)
+    if case == "force_visc":
+        s.set_force_visc(True)
+    for n in (1, 3, 1, 20, 1, 2):
+        s.step(n)
+    assert s.graph_count() == 2
+    s.close()
