@@ -279,7 +279,9 @@ struct Ctx {
         return !timers_on && prm.motion_law != CFD_MOTION_NEWMARK && !smoothing_now && !fv_each &&
                nelem <= 11000L * nsm;
     }
+    int capture_step(int at);
     int launch_step_graph(bool* launched, bool ahead);
+    void capture_ahead();
     int set_guess_net(cfd_mpnn* n, double gate);
     int force_visc_now();
     int smooth(int* iters, double* min_quality, bool node_order = false);

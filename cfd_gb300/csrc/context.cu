@@ -729,6 +729,7 @@ int Ctx::step(int nsteps, cfd_step_report* rep) {
                (const MotionScal*)(d_motion ? d_motion + buf : nullptr), (const int*)d_pcg_iters, (const int*)d_pcg_conv,
                (const double*)d_pcg_rz, (const GridBar*)d_bar, (const int*)d_node_err, d_out);
     CFD_CUDA(cudaMemcpyAsync(h_out, d_out, sizeof(StepOut), cudaMemcpyDeviceToHost, stream));
+    if (prec == CFD_PREC_MIXED && nsteps > 0) capture_ahead();
     CFD_CUDA(cudaStreamSynchronize(stream));
     *h_scal = h_out->sc;
     const MotionScal ms = h_out->ms;
@@ -1336,43 +1337,73 @@ void Ctx::drop_graphs() {
     }
 }
 
+// Capture the step of the current parity in place `at` of a call (step_exec); a capture that is
+// not possible here turns the graphs off.
+int Ctx::capture_step(int at) {
+    cudaGraphExec_t ex = nullptr;
+    cudaGraph_t g = nullptr;
+    const long long k0 = g_launches.load();
+    CFD_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+    const bool was_ahead = dt_ahead;
+    dt_ahead = (at & 2) != 0;
+    capturing = true;
+    const int st = enqueue_mixed(false, (at & 1) != 0);
+    capturing = false;
+    dt_ahead = was_ahead;
+    const cudaError_t ce = cudaStreamEndCapture(stream, &g);
+    const long long nk = g_launches.load() - k0;
+    g_launches.fetch_sub(nk);  // captured, not run
+    if (st == CFD_OK && ce == cudaSuccess && g && cudaGraphInstantiate(&ex, g, 0) == cudaSuccess) {
+        step_graph[buf][at] = g;
+        step_exec[buf][at] = ex;
+        step_kernels[buf][at] = nk;
+    } else {
+        if (g) cudaGraphDestroy(g);
+        (void)cudaGetLastError();
+        graphs_on = false;
+    }
+    return CFD_OK;
+}
+
 // Replay the captured step, capturing it first.  *launched = false when the capture is
 // not possible here (the caller then enqueues the step launch by launch, and stays so).
 int Ctx::launch_step_graph(bool* launched, bool ahead) {
     *launched = false;
     // one graph per buffer parity (the captured pointers are the parity's) and place of DTMIN
     const int at = (dt_ahead ? 2 : 0) + (ahead ? 1 : 0);
-    cudaGraph_t& step_graph = this->step_graph[buf][at];
-    cudaGraphExec_t& step_exec = this->step_exec[buf][at];
-    if (!step_exec) {
-        const long long k0 = g_launches.load();
-        CFD_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        capturing = true;
-        const int st = enqueue_mixed(false, ahead);
-        capturing = false;
-        cudaGraph_t g = nullptr;
-        const cudaError_t ce = cudaStreamEndCapture(stream, &g);
-        const long long nk = g_launches.load() - k0;
-        g_launches.fetch_sub(nk);  // captured, not run
-        cudaGraphExec_t ex = nullptr;
-        if (st == CFD_OK && ce == cudaSuccess && g &&
-            cudaGraphInstantiate(&ex, g, 0) == cudaSuccess) {
-            step_graph = g;
-            step_exec = ex;
-            step_kernels[buf][at] = nk;
-        } else {
-            if (g) cudaGraphDestroy(g);
-            (void)cudaGetLastError();
-            graphs_on = false;
-            return CFD_OK;
-        }
+    if (!step_exec[buf][at]) {
+        const int st = capture_step(at);
+        if (st || !graphs_on) return st;
     }
-    CFD_CUDA(cudaGraphLaunch(step_exec, stream));
+    CFD_CUDA(cudaGraphLaunch(step_exec[buf][at], stream));
     graph_kernels = step_kernels[buf][at];
     g_launches.fetch_add(graph_kernels, std::memory_order_relaxed);
     graph_replays += 1;
     *launched = true;
     return CFD_OK;
+}
+
+// The graphs that the coming calls may need are captured while the device still works on this
+// one's steps (a capture takes 40-80 us of a host that would wait), those first that a call
+// opens with: the steps of a context's first call, whose solves start cold, leave time for all.
+// The first two single steps after a call of three: 133 and 125 us at 15,150 nodes with every
+// graph captured at its first use, 87 and 86 so; 434 and 423 us at 589,824, 367 and 351 so.
+void Ctx::capture_ahead() {
+    const bool always_net = learned_mode() && net && lgraph && (guess_first || guess_gate <= 0.0);
+    if (!graphs_on || mixed_steps == 0 || always_net) return;
+    smoothing_now = false;  // the steps that smooth are not replayed
+    const bool put = area_put;
+    for (const int at : {0, 1, 3, 2}) {
+        if (at && !forms_ahead()) break;
+        for (int parity = 0; parity < 2; ++parity) {
+            if (graphs_on && !step_exec[buf][at] && cudaStreamQuery(stream) == cudaErrorNotReady &&
+                capture_step(at) != CFD_OK)
+                graphs_on = false;
+            swap_mixed_buffers();  // the other parity's pointers, then this one's again
+        }
+    }
+    area_put = put;
+    (void)cudaGetLastError();  // "not ready" is no error
 }
 
 // One mixed step.  The learned guess runs on the first solve after the network was

@@ -300,3 +300,33 @@ def test_two_graphs_where_no_step_forms_the_next_dtmin(gpu_lib, case):
         s.step(n)
     assert s.graph_count() == 2
     s.close()
+
+
+def test_graphs_are_captured_while_the_first_call_runs(gpu_lib):
+    """The cold solve of a context's first step takes longer than the captures: all eight
+    graphs (two parities, four places of the DTMIN passes) are there when the call returns, none
+    is captured by the calls that follow, and those give the bits of steps without graphs."""
+    import os
+    from cfd_gb300 import abi, case as cs, solver
+    p = cs.flow_params(0.8, 5000.0, fsafe=0.25, moving=1, motion_law=1, heave_amp=0.05,
+                       motion_freq=0.1, mass_mode=2)
+    p.estab_mode, p.bicg_tol_mode, p.bicg_maxit = 2, abi.CFD_BICG_TOL_REL, 20000
+    k = cs.ogrid_case("ellipse", 384, 384, p, "ellipse", incidence_deg=2.0, r_out=30.0, seed=1)
+    a = solver.Solver(k, precision=abi.CFD_PREC_MIXED)
+    os.environ["CFD_GRAPHS"] = "0"
+    try:
+        b = solver.Solver(k, precision=abi.CFD_PREC_MIXED)
+    finally:
+        del os.environ["CFD_GRAPHS"]
+    ra, rb = a.step(1), b.step(1)
+    assert ra.bicg_iters[1] > 500  # tens of milliseconds
+    assert a.graph_count() == 8 and b.graph_count() == 0
+    for n in (1, 1, 3, 2, 5):
+        ra, rb = a.step(n), b.step(n)
+        assert (ra.time, ra.dtmin, ra.iter) == (rb.time, rb.dtmin, rb.iter)
+    sa, sb = a.state(), b.state()
+    for key in sa:
+        assert np.array_equal(sa[key], sb[key]), key
+    assert a.graph_count() == 8 and a.graph_state()[1] == 12
+    a.close()
+    b.close()
