@@ -276,7 +276,7 @@ __global__ void k_dtl(int nelem, double* DT, double* DTL, const StepScal* sc, do
 // ESTAB's launch constants: what is the same for every element is formed once on the host
 // (GAMM(1:3) averaged when uniform, times FR; the divisors with their reciprocals)
 struct EstabArgs {
-    double gm, gmfr, fr;
+    double gmfr, fr;
     Rcp rho_inf, t_inf;
     int mode;
     double eps, dirx, diry;
@@ -284,7 +284,7 @@ struct EstabArgs {
 inline EstabArgs estab_args(double gamm, double fr, double rho_inf, double t_inf, int mode,
                             double eps, double dirx, double diry) {
     const double gm = (gamm + gamm + gamm) / 3.0;
-    return EstabArgs{gm, gm * fr, fr, make_rcp(rho_inf), make_rcp(t_inf), mode, eps, dirx, diry};
+    return EstabArgs{gm * fr, fr, make_rcp(rho_inf), make_rcp(t_inf), mode, eps, dirx, diry};
 }
 __global__ void k_estab(int nelem, const int4* elem, const double* U, const double* T,
                         const double* GAMM, const double* VX, const double* VY, const double* WX,
@@ -376,7 +376,7 @@ struct PcgArgs {
     const double* val;
     const double* diag;
     double* rdiag;               // FP64 form: RN(1/diag), formed by the first pass and used
-                                 // for the iterations' quotients (null: the division)
+                                 // for the iterations' quotients
     const unsigned char* isfix;  // per node: Dirichlet row
     int nfix;                    // unique fixed nodes (last entry of the reference list)
     const int* fix_node;
@@ -387,8 +387,8 @@ struct PcgArgs {
     double* r[2];
     double* z[2];
     double* y[2];
-    double* p[2][2];             // ping-pong search directions
-    double* part;                // [2 phases][2 solves][nchunks] chunk partial sums
+    double* p[2][2];             // search directions (ping-pong in the mixed form, p[s][0] in the FP64 one)
+    double* part;                // [3 sums][2 solves][nchunks] chunk partials (absolute test: 2 sums)
     // mixed form only: FP32 matrix values, 1/diag, FP32 shadows of p (ping-pong) and z
     const float* valf;
     const float* val_lo;         // relative tests: valf + val_lo = the FP64-assembled matrix

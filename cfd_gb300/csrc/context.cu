@@ -901,8 +901,9 @@ int Ctx::create(const cfd_mesh* m, const cfd_params* p, int precision_mode) {
     if ((st = dalloc(&d_contribF, 12 * (size_t)E))) return st;
     if (prec == CFD_PREC_FP64 && (st = dalloc(&d_einv, (size_t)kElemInvPlanes * E))) return st;
     for (int s = 0; s < 2; ++s) {
-        for (double** q : {&d_pos[s], &d_r[s], &d_z[s], &d_y[s], &d_p[s][0], &d_p[s][1]})
+        for (double** q : {&d_pos[s], &d_r[s], &d_z[s], &d_y[s], &d_p[s][0]})
             if ((st = dalloc(q, N))) return st;
+        if (prec == CFD_PREC_MIXED && (st = dalloc(&d_p[s][1], N))) return st;
         if ((st = dalloc(&d_xfix[s], nnmove))) return st;
         CFD_CUDA(cudaMemsetAsync(d_pos[s], 0, sizeof(double) * N, stream));
         CFD_CUDA(cudaMemsetAsync(d_xfix[s], 0, sizeof(double) * (nnmove ? nnmove : 1), stream));
@@ -934,14 +935,16 @@ int Ctx::create(const cfd_mesh* m, const cfd_params* p, int precision_mode) {
     std::memcpy(h_scal, &sc0, sizeof(sc0));
     CFD_CUDA(cudaMemcpyAsync(d_scal, h_scal, sizeof(StepScal), cudaMemcpyHostToDevice, stream));
     CFD_CUDA(cudaStreamSynchronize(stream));
-    // persistent mixed BiCG grid: co-resident blocks only
-    int dev = 0, per_sm = 0;
+    int dev = 0;
     CFD_CUDA(cudaGetDevice(&dev));
     CFD_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    CFD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_mixed, 256, 0));
-    long g = (long)nsm * (per_sm > 0 ? per_sm : 1);
-    if (g > nc) g = nc;
-    pcg_grid = (int)(g > 0 ? g : 1);
+    if (prec == CFD_PREC_MIXED) {  // persistent mixed BiCG grid: co-resident blocks only
+        int per_sm = 0;
+        CFD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_mixed, 256, 0));
+        long g = (long)nsm * (per_sm > 0 ? per_sm : 1);
+        if (g > nc) g = nc;
+        pcg_grid = (int)(g > 0 ? g : 1);
+    }
     // RESTART: freestream (ns2DComp.ALE.f90:59-60, :404-420)
     std::vector<double> U(4 * (size_t)N), T(N), VX(N), VY(N), zero(N, 0.0);
     for (int i = 0; i < N; ++i) {

@@ -598,7 +598,6 @@ cudaError_t launch_pcg_fp64(cudaStream_t st, PcgArgs a) {
     if (e != cudaSuccess) return e;
     const long nc = ((long)a.n + kChunk - 1) / kChunk;
     const bool chip = nc <= nsm;
-    if (!chip && !a.rdiag) return cudaErrorInvalidValue;
     const int smem = chip ? (int)sizeof(PcgShared<1>) + kEll * kChunk * 12 : (int)sizeof(PcgShared<kGroup>);
     const void* fn = chip ? (const void*)k_pcg_fp64<true> : (const void*)k_pcg_fp64<false>;
     if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)

@@ -20,9 +20,10 @@
 namespace cfd {
 namespace {
 
-// Work space: r, z, y and the two search directions (5 vectors of npoin doubles), the
-// chunk partial sums of the dots (4 x npoin/1024), then a 256-byte control block with the
-// grid barrier and the solve's outputs.
+// Work space: r, z, y, the search direction and 1/diag (5 vectors of npoin doubles; a solve of
+// no more 1024-row chunks than SMs keeps all but the direction on chip), the chunk partial sums of
+// the dots (4 x npoin/1024), then a 256-byte control block with the grid barrier and the
+// solve's outputs.
 constexpr int kNoallocMaxN = CFD_NOALLOC_MAX_NPOIN;
 constexpr long kVecBytes = 5L * kNoallocMaxN * 8;
 constexpr long kPartBytes = 4L * ((kNoallocMaxN + kChunk - 1) / kChunk) * 8;
@@ -100,7 +101,7 @@ extern "C" int cfd_bicg_device_noalloc(const double* spMtx, const int* col, cons
     a.z[0] = a.z[1] = v + N;
     a.y[0] = a.y[1] = v + 2 * N;
     a.p[0][0] = a.p[1][0] = v + 3 * N;
-    a.p[0][1] = a.p[1][1] = v + 4 * N;
+    a.rdiag = v + 4 * N;
     a.part = (double*)(base + kVecBytes);
     a.bar = &ctl->bar;
     a.tol = tol;
