@@ -674,11 +674,12 @@ __global__ void k_guess_extrapolate_hist(const double* __restrict__ dtn_p,
     if (blockIdx.x == 0 && threadIdx.x == 0) guess_history(*dtn_p, hist);
 }
 
-// div_rcp and div_rcp2 against the division x / d over n input pairs: a third raw 64-bit patterns for
-// both (splitmix64: every exponent and sign, zeros, subnormals, infinities, NaNs), a third
-// with both of magnitude 2^-60 .. 2^60, a third with x = d * m for a random significand m
-// moved by up to +-2^12 ulps (quotients next to binade edges and to halfway cases).  Counts
-// the pairs whose results differ in any bit (NaNs count as equal).
+// div_rcp and div_rcp2 against the division x / d over n input pairs, a quarter of each kind: raw
+// 64-bit patterns for both (splitmix64: every exponent and sign, subnormals, infinities, NaNs);
+// both of magnitude 2^-60 .. 2^60; x = d * m for a random significand m moved by up to +-2^12
+// ulps (quotients next to binade edges and to halfway cases); the ends of the range that the
+// short forms take (exponents 200 and 1800, 800 apart, one more and one less) and x = +-0.
+// Counts the pairs whose results differ in any bit (NaNs count as equal).
 __device__ __forceinline__ unsigned long long splitmix(unsigned long long z) {
     z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
     z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
@@ -692,7 +693,7 @@ __global__ void k_selftest_divrcp(long long n, unsigned long long seed,
         const unsigned long long z1 = splitmix(seed + (unsigned long long)i * 0x9e3779b97f4a7c15ull);
         const unsigned long long z2 = splitmix(z1 + 0x632be59bd9b4e019ull);
         unsigned long long bx = z1, bd = z2;
-        const int kind = (int)(i % 3);
+        const int kind = (int)(i % 4);
         if (kind == 1) {
             bx = (z1 & 0x800fffffffffffffull) | ((963ull + (z1 >> 52) % 121ull) << 52);
             bd = (z2 & 0x800fffffffffffffull) | ((963ull + (z2 >> 52) % 121ull) << 52);
@@ -702,6 +703,14 @@ __global__ void k_selftest_divrcp(long long n, unsigned long long seed,
                                                               (1023ull << 52)));
             const long long b = __double_as_longlong(__longlong_as_double((long long)bd) * m);
             bx = (unsigned long long)(b + ((long long)(z1 >> 52 & 0x1fffull) - 4096));
+        } else if (kind == 3) {
+            const int end[8] = {0, 199, 200, 201, 1023, 1799, 1800, 1801};
+            const int apart[8] = {-801, -800, -799, 0, 799, 800, 801, 0};
+            const int ed = end[z2 >> 52 & 7], k = (int)(z1 >> 52 & 7);
+            const int ex = k == 3 ? end[z1 >> 55 & 7] : min(max(ed + apart[k], 0), 2046);
+            bd = (z2 & 0x800fffffffffffffull) | ((unsigned long long)ed << 52);
+            bx = z1 & 0x8000000000000000ull;
+            if (k < 7) bx = (z1 & 0x800fffffffffffffull) | ((unsigned long long)ex << 52);
         }
         const double x = __longlong_as_double((long long)bx), d = __longlong_as_double((long long)bd);
         const double y = 1.0 / d;

@@ -508,9 +508,11 @@ int cfd_selftest_failed_barrier(int* solve_status);
  * patterns from `seed`, values in 2^-40 .. 2^40, and values next to 3 * 2^k) and returns
  * the number whose bits differ. */
 int cfd_selftest_div3(long long n, unsigned long long seed, unsigned long long* mismatches);
-/* The same for the FP64 BiCG's quotients r/diag: a multiply by RN(1/diag) and four FMAs
- * (two Markstein corrections) against the division, over n pairs from `seed` (raw bit
- * patterns, magnitudes 2^-60 .. 2^60, quotients next to binade edges and halfway cases). */
+/* The same for the FP64 form's quotients by a divisor whose reciprocal is at hand (the BiCG's
+ * r/diag, a shared divisor's): a multiply and a few FMAs (Markstein corrections) against the
+ * division, over n pairs from `seed` (raw bit patterns, magnitudes 2^-60 .. 2^60, quotients
+ * next to binade edges and halfway cases, the ends of the exponent range that takes the short
+ * form, zeros of both signs). */
 int cfd_selftest_div_rcp(long long n, unsigned long long seed, unsigned long long* mismatches);
 
 const char* cfd_strerror(int status);
