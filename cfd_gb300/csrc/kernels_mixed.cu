@@ -766,39 +766,39 @@ __global__ void k_elem_geometry(int nelem, const int4* __restrict__ elem,
                                 float* __restrict__ areaf, float4* __restrict__ geo,
                                 double* __restrict__ terms) {
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nelem; e += gridDim.x * blockDim.x) {
-    const int4 n = elem[e];
-    const double X0 = X[n.x], Y0 = Y[n.x];
-    const double dx1 = X[n.y] - X0, dy1 = Y[n.y] - Y0;
-    const double dx2 = X[n.z] - X0, dy2 = Y[n.z] - Y0;
-    // 2a = x1*y2 - x2*y1 (the reference's signed area from differences to node 1), FP64
-    const double a64 = 0.5 * (dx1 * dy2 - dx2 * dy1);
-    const float x1 = d2f_trunc(dx1), y1 = d2f_trunc(dy1);
-    const float x2 = d2f_trunc(dx2), y2 = d2f_trunc(dy2);
-    const float a2f = fmaf(x1, y2, -(x2 * y1));
-    const float area = 0.5f * a2f;
-    const float ia = fdiv(1.f, a2f);
-    const float gx[3] = {(y1 - y2) * ia, y2 * ia, -y1 * ia};  // (y_2 - y_3)/(2a), ... with y_1 = 0
-    const float gy[3] = {(x2 - x1) * ia, -x2 * ia, x1 * ia};
-    const float s2 = gx[0] * gx[0] + gy[0] * gy[0] + gx[1] * gx[1] + gy[1] * gy[1] +
-                     gx[2] * gx[2] + gy[2] * gy[2];
-    const float am = area * s2;
-    const float q = am * am * (1.f / 3.f);
-    geo[2 * (size_t)e] = make_float4(gx[0], gx[1], gx[2], gy[0]);
-    geo[2 * (size_t)e + 1] = make_float4(gy[1], gy[2], area, q);
-    areaf[e] = area;
-    if (gcl) {
-        const int nn[3] = {n.x, n.y, n.z};
-        float divW = 0.f, divWo = 0.f;
+        const int4 n = elem[e];
+        const double X0 = X[n.x], Y0 = Y[n.x];
+        const double dx1 = X[n.y] - X0, dy1 = Y[n.y] - Y0;
+        const double dx2 = X[n.z] - X0, dy2 = Y[n.z] - Y0;
+        // 2a = x1*y2 - x2*y1 (the reference's signed area from differences to node 1), FP64
+        const double a64 = 0.5 * (dx1 * dy2 - dx2 * dy1);
+        const float x1 = d2f_trunc(dx1), y1 = d2f_trunc(dy1);
+        const float x2 = d2f_trunc(dx2), y2 = d2f_trunc(dy2);
+        const float a2f = fmaf(x1, y2, -(x2 * y1));
+        const float area = 0.5f * a2f;
+        const float ia = fdiv(1.f, a2f);
+        const float gx[3] = {(y1 - y2) * ia, y2 * ia, -y1 * ia};  // (y_2 - y_3)/(2a), ... with y_1 = 0
+        const float gy[3] = {(x2 - x1) * ia, -x2 * ia, x1 * ia};
+        const float s2 = gx[0] * gx[0] + gy[0] * gy[0] + gx[1] * gx[1] + gy[1] * gy[1] +
+                         gx[2] * gx[2] + gy[2] * gy[2];
+        const float am = area * s2;
+        const float q = am * am * (1.f / 3.f);
+        geo[2 * (size_t)e] = make_float4(gx[0], gx[1], gx[2], gy[0]);
+        geo[2 * (size_t)e + 1] = make_float4(gy[1], gy[2], area, q);
+        areaf[e] = area;
+        if (gcl) {
+            const int nn[3] = {n.x, n.y, n.z};
+            float divW = 0.f, divWo = 0.f;
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const float2 w = W[nn[i]], wo = Wold[nn[i]];
-            divW += gx[i] * w.x + gy[i] * (literal ? w.x : w.y);
-            divWo += gx[i] * wo.x + gy[i] * (literal ? wo.x : wo.y);
+            for (int i = 0; i < 3; ++i) {
+                const float2 w = W[nn[i]], wo = Wold[nn[i]];
+                divW += gx[i] * w.x + gy[i] * (literal ? w.x : w.y);
+                divWo += gx[i] * wo.x + gy[i] * (literal ? wo.x : wo.y);
+            }
+            terms[e] = f2d_bits(divW) * a64 + f2d_bits(divWo) * area_old[e];
         }
-        terms[e] = f2d_bits(divW) * a64 + f2d_bits(divWo) * area_old[e];
-    }
-    if (put_area) area_old[e] = a64;  // putArea; then also the area a download reads
-    else area64[e] = a64;
+        if (put_area) area_old[e] = a64;  // putArea; then also the area a download reads
+        else area64[e] = a64;
     }
 }
 
@@ -904,133 +904,133 @@ k_node_geometry(int npoin, const int* __restrict__ esup_ptr, const int* __restri
     // nodes, sums their rows, which are one run of the matrix, in shared memory and writes
     // the run out in whole sectors
     for (int pw = blockIdx.x * kGeoBlock + 32 * warp; pw < npoin; pw += nblocks * kGeoBlock) {
-    const int p = pw + lane;
-    const bool live = p < npoin;
-    const int r0 = rowptr[min(p, npoin)], r1 = rowptr[min(p + 1, npoin)];
-    const int base = __shfl_sync(0xffffffffu, r0, 0), total = __shfl_sync(0xffffffffu, r1, 31) - base;
-    const int len = r1 - r0;
-    const bool in_smem = total <= 32 * kLapRow;
-    float* run = row[warp];
-    float2* run64 = row64[warp];
-    float* acc = run + (ROW64 || !in_smem ? 0 : r0 - base);
-    float2* acc64 = run64 + (ROW64 && in_smem ? r0 - base : 0);
-    if (in_smem) {
-        for (int k = lane; k < total; k += 32) {
-            if (ROW64) run64[k] = make_float2(0.f, 0.f);
-            else run[k] = 0.f;
-        }
-        __syncwarp();
-    } else if (!ROW64) {
-        for (int k = r0; k < r1; ++k) valf[k] = 0.f;
-    }
-    if (live) {
-    Acc m1;
-    m1.init();
-    double tot = 0.0;  // gcl: (tot1 + tot2) times 3
-    // kGeoBatch slots per pass: their loads go out together, the sums stay in slot order
-    const int s0 = esup_ptr[p], s1 = esup_ptr[p + 1];
-    for (int sb = s0; sb < s1; sb += kGeoBatch) {
-        int slot[kGeoBatch];
-        uchar4 pos[kGeoBatch];
-        float4 ga[kGeoBatch], gb[kGeoBatch];
-        double tm[kGeoBatch];
-        float2 kr[kGeoBatch][3];
-#pragma unroll
-        for (int u = 0; u < kGeoBatch; ++u)
-            if (sb + u < s1) {
-                slot[u] = esup_slot[sb + u];
-                pos[u] = lap_pos[sb + u];
-                if (ROW64) {
-                    const float2* k = k64 + 3 * (size_t)(sb + u);
-                    kr[u][0] = k[0];
-                    kr[u][1] = k[1];
-                    kr[u][2] = k[2];
-                }
-            }
-#pragma unroll
-        for (int u = 0; u < kGeoBatch; ++u)
-            if (sb + u < s1) {
-                const int e = slot[u] / 3;
-                if (need_geo) load32(geo + 2 * (size_t)e, ga[u], gb[u]);
-                if (gcl) tm[u] = terms[e];
-            }
-#pragma unroll
-        for (int u = 0; u < kGeoBatch; ++u) {
-            if (sb + u >= s1) break;
-            if (gcl) {
-                tot = tot + tm[u];
-            } else {
-                m1.add(gb[u].z);
-            }
-            if (ROW64) {
-                if (in_smem) {
-                    df_acc(acc64[pos[u].x], kr[u][0]);
-                    df_acc(acc64[pos[u].y], kr[u][1]);
-                    df_acc(acc64[pos[u].z], kr[u][2]);
-                }
-                continue;
-            }
-            const int i = slot[u] - 3 * (slot[u] / 3);
-            const float gx[3] = {ga[u].x, ga[u].y, ga[u].z}, gy[3] = {ga[u].w, gb[u].x, gb[u].y};
-            const float q = gb[u].w;
-            const float dxi = (i == 0) ? gx[0] : (i == 1 ? gx[1] : gx[2]);
-            const float dyi = (i == 0) ? gy[0] : (i == 1 ? gy[1] : gy[2]);
-            const unsigned char pj[3] = {pos[u].x, pos[u].y, pos[u].z};
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const float v = (dxi * gx[j] + dyi * gy[j]) * q;
-                if (in_smem) acc[pj[j]] += v;
-                else valf[r0 + pj[j]] += v;  // long rows (rare)
-            }
-        }
-    }
-    float idf;
-    if (ROW64) {
-        float diag;
+        const int p = pw + lane;
+        const bool live = p < npoin;
+        const int r0 = rowptr[min(p, npoin)], r1 = rowptr[min(p + 1, npoin)];
+        const int base = __shfl_sync(0xffffffffu, r0, 0), total = __shfl_sync(0xffffffffu, r1, 31) - base;
+        const int len = r1 - r0;
+        const bool in_smem = total <= 32 * kLapRow;
+        float* run = row[warp];
+        float2* run64 = row64[warp];
+        float* acc = run + (ROW64 || !in_smem ? 0 : r0 - base);
+        float2* acc64 = run64 + (ROW64 && in_smem ? r0 - base : 0);
         if (in_smem) {
-            diag = acc64[0].x;
-        } else {  // long rows (rare): one pass over the slots per entry
-            diag = 0.f;
-            for (int kk = 0; kk < len; ++kk) {
-                float2 one = make_float2(0.f, 0.f);
-                for (int sl = s0; sl < s1; ++sl) {
-                    const float2* k = k64 + 3 * (size_t)sl;
-                    const uchar4 ps = lap_pos[sl];
-                    if (ps.x == kk) df_acc(one, k[0]);
-                    if (ps.y == kk) df_acc(one, k[1]);
-                    if (ps.z == kk) df_acc(one, k[2]);
-                }
-                valf[r0 + kk] = one.x;
-                val_lo[r0 + kk] = one.y;
-                if (kk == 0) diag = one.x;
+            for (int k = lane; k < total; k += 32) {
+                if (ROW64) run64[k] = make_float2(0.f, 0.f);
+                else run[k] = 0.f;
             }
+            __syncwarp();
+        } else if (!ROW64) {
+            for (int k = r0; k < r1; ++k) valf[k] = 0.f;
         }
-        idf = 1.f / diag;  // the Jacobi scaling is FP32 in every pass
-    } else {
-        float diag;
-        diag = in_smem ? acc[0] : valf[r0];
-        idf = 1.f / diag;
-    }
-    invdiagf[p] = idf;
-    invdiag[p] = f2d_bits(idf);
-    double m;
-    if (gcl) {
-        m = M[p] + (*dtp) * (tot * (1.0 / 6.0));
-        if (Wold) Wold[p] = W[p];  // putW (null: the caller swaps W buffers instead)
-    } else {
-        m = f2d_bits(m1.value()) * (1.0 / 3.0);
-    }
-    M[p] = m;
-    invM[p] = 1.f / d2f_trunc(m);
-    }
-    if (in_smem) {
-        __syncwarp();
-        for (int k = lane; k < total; k += 32) {
-            valf[base + k] = ROW64 ? run64[k].x : run[k];
-            if (ROW64) val_lo[base + k] = run64[k].y;
+        if (live) {
+            Acc m1;
+            m1.init();
+            double tot = 0.0;  // gcl: (tot1 + tot2) times 3
+            // kGeoBatch slots per pass: their loads go out together, the sums stay in slot order
+            const int s0 = esup_ptr[p], s1 = esup_ptr[p + 1];
+            for (int sb = s0; sb < s1; sb += kGeoBatch) {
+                int slot[kGeoBatch];
+                uchar4 pos[kGeoBatch];
+                float4 ga[kGeoBatch], gb[kGeoBatch];
+                double tm[kGeoBatch];
+                float2 kr[kGeoBatch][3];
+#pragma unroll
+                for (int u = 0; u < kGeoBatch; ++u)
+                    if (sb + u < s1) {
+                        slot[u] = esup_slot[sb + u];
+                        pos[u] = lap_pos[sb + u];
+                        if (ROW64) {
+                            const float2* k = k64 + 3 * (size_t)(sb + u);
+                            kr[u][0] = k[0];
+                            kr[u][1] = k[1];
+                            kr[u][2] = k[2];
+                        }
+                    }
+#pragma unroll
+                for (int u = 0; u < kGeoBatch; ++u)
+                    if (sb + u < s1) {
+                        const int e = slot[u] / 3;
+                        if (need_geo) load32(geo + 2 * (size_t)e, ga[u], gb[u]);
+                        if (gcl) tm[u] = terms[e];
+                    }
+#pragma unroll
+                for (int u = 0; u < kGeoBatch; ++u) {
+                    if (sb + u >= s1) break;
+                    if (gcl) {
+                        tot = tot + tm[u];
+                    } else {
+                        m1.add(gb[u].z);
+                    }
+                    if (ROW64) {
+                        if (in_smem) {
+                            df_acc(acc64[pos[u].x], kr[u][0]);
+                            df_acc(acc64[pos[u].y], kr[u][1]);
+                            df_acc(acc64[pos[u].z], kr[u][2]);
+                        }
+                        continue;
+                    }
+                    const int i = slot[u] - 3 * (slot[u] / 3);
+                    const float gx[3] = {ga[u].x, ga[u].y, ga[u].z}, gy[3] = {ga[u].w, gb[u].x, gb[u].y};
+                    const float q = gb[u].w;
+                    const float dxi = (i == 0) ? gx[0] : (i == 1 ? gx[1] : gx[2]);
+                    const float dyi = (i == 0) ? gy[0] : (i == 1 ? gy[1] : gy[2]);
+                    const unsigned char pj[3] = {pos[u].x, pos[u].y, pos[u].z};
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        const float v = (dxi * gx[j] + dyi * gy[j]) * q;
+                        if (in_smem) acc[pj[j]] += v;
+                        else valf[r0 + pj[j]] += v;  // long rows (rare)
+                    }
+                }
+            }
+            float idf;
+            if (ROW64) {
+                float diag;
+                if (in_smem) {
+                    diag = acc64[0].x;
+                } else {  // long rows (rare): one pass over the slots per entry
+                    diag = 0.f;
+                    for (int kk = 0; kk < len; ++kk) {
+                        float2 one = make_float2(0.f, 0.f);
+                        for (int sl = s0; sl < s1; ++sl) {
+                            const float2* k = k64 + 3 * (size_t)sl;
+                            const uchar4 ps = lap_pos[sl];
+                            if (ps.x == kk) df_acc(one, k[0]);
+                            if (ps.y == kk) df_acc(one, k[1]);
+                            if (ps.z == kk) df_acc(one, k[2]);
+                        }
+                        valf[r0 + kk] = one.x;
+                        val_lo[r0 + kk] = one.y;
+                        if (kk == 0) diag = one.x;
+                    }
+                }
+                idf = 1.f / diag;  // the Jacobi scaling is FP32 in every pass
+            } else {
+                float diag;
+                diag = in_smem ? acc[0] : valf[r0];
+                idf = 1.f / diag;
+            }
+            invdiagf[p] = idf;
+            invdiag[p] = f2d_bits(idf);
+            double m;
+            if (gcl) {
+                m = M[p] + (*dtp) * (tot * (1.0 / 6.0));
+                if (Wold) Wold[p] = W[p];  // putW (null: the caller swaps W buffers instead)
+            } else {
+                m = f2d_bits(m1.value()) * (1.0 / 3.0);
+            }
+            M[p] = m;
+            invM[p] = 1.f / d2f_trunc(m);
         }
-        __syncwarp();
-    }
+        if (in_smem) {
+            __syncwarp();
+            for (int k = lane; k < total; k += 32) {
+                valf[base + k] = ROW64 ? run64[k].x : run[k];
+                if (ROW64) val_lo[base + k] = run64[k].y;
+            }
+            __syncwarp();
+        }
     }
 }
 cudaError_t launch_node_geometry(bool row64, unsigned grid, cudaStream_t stream, int npoin,

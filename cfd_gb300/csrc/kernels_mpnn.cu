@@ -784,51 +784,51 @@ k_edge_fwd(int n, const int* __restrict__ ptr, const int* __restrict__ nbr,
     };
     head(blockIdx.x);
     for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
-    const int i = 16 * b + at;
-    const bool live = i < n;
-    const int k0 = nk0, k1 = nk1;
-    const float pv[4] = {np.x, np.y, np.z, np.w};
-    head(b + gridDim.x);
-    float s[4] = {};
-    const int deg = k1 - k0, steps = max(deg, __shfl_xor_sync(0xffffffffu, deg, 16));
-    constexpr int B = 4;  // edges whose gathers go out together
-    for (int t0 = 0; t0 < steps; t0 += B) {
-        float4 qv[B];
-        float ev[B][3];
+        const int i = 16 * b + at;
+        const bool live = i < n;
+        const int k0 = nk0, k1 = nk1;
+        const float pv[4] = {np.x, np.y, np.z, np.w};
+        head(b + gridDim.x);
+        float s[4] = {};
+        const int deg = k1 - k0, steps = max(deg, __shfl_xor_sync(0xffffffffu, deg, 16));
+        constexpr int B = 4;  // edges whose gathers go out together
+        for (int t0 = 0; t0 < steps; t0 += B) {
+            float4 qv[B];
+            float ev[B][3];
 #pragma unroll
-        for (int u = 0; u < B; ++u) {
-            const int k = k0 + t0 + u;
-            qv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            ev[u][0] = ev[u][1] = ev[u][2] = 0.f;
-            if (k < k1) {
-                qv[u] = *reinterpret_cast<const float4*>(PQ + (size_t)nbr[k] * 2 * HID + HID + 4 * l);
+            for (int u = 0; u < B; ++u) {
+                const int k = k0 + t0 + u;
+                qv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                ev[u][0] = ev[u][1] = ev[u][2] = 0.f;
+                if (k < k1) {
+                    qv[u] = *reinterpret_cast<const float4*>(PQ + (size_t)nbr[k] * 2 * HID + HID + 4 * l);
 #pragma unroll
-                for (int q = 0; q < 3; ++q) ev[u][q] = e[3 * (size_t)k + q];
+                    for (int q = 0; q < 3; ++q) ev[u][q] = e[3 * (size_t)k + q];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                if (t0 + u >= steps) break;  // the same in the whole warp
+                const int k = k0 + t0 + u;
+                const float qq[4] = {qv[u].x, qv[u].y, qv[u].z, qv[u].w};
+                unsigned short bits[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float z = pv[q] + qq[q] +
+                                    (cw[q][0] * ev[u][0] + cw[q][1] * ev[u][1] + cw[q][2] * ev[u][2]) +
+                                    cb[q];
+                    const bool on = k < k1 && z > 0.f;
+                    s[q] += on ? z : 0.f;
+                    bits[q] = (unsigned short)(__ballot_sync(0xffffffffu, on) >> half);
+                }
+                if (l == 0 && k < k1) mask[k] = make_ushort4(bits[0], bits[1], bits[2], bits[3]);
             }
         }
-#pragma unroll
-        for (int u = 0; u < B; ++u) {
-            if (t0 + u >= steps) break;  // the same in the whole warp
-            const int k = k0 + t0 + u;
-            const float qq[4] = {qv[u].x, qv[u].y, qv[u].z, qv[u].w};
-            unsigned short bits[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const float z = pv[q] + qq[q] +
-                                (cw[q][0] * ev[u][0] + cw[q][1] * ev[u][1] + cw[q][2] * ev[u][2]) +
-                                cb[q];
-                const bool on = k < k1 && z > 0.f;
-                s[q] += on ? z : 0.f;
-                bits[q] = (unsigned short)(__ballot_sync(0xffffffffu, on) >> half);
-            }
-            if (l == 0 && k < k1) mask[k] = make_ushort4(bits[0], bits[1], bits[2], bits[3]);
+        if (live) {
+            const float d = (float)max(deg, 1);
+            *reinterpret_cast<float4*>(agg + (size_t)i * HID + 4 * l) =
+                make_float4(s[0] / d, s[1] / d, s[2] / d, s[3] / d);
         }
-    }
-    if (live) {
-        const float d = (float)max(deg, 1);
-        *reinterpret_cast<float4*>(agg + (size_t)i * HID + 4 * l) =
-            make_float4(s[0] / d, s[1] / d, s[2] / d, s[3] / d);
-    }
     }
 }
 
