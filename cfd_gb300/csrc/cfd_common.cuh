@@ -273,7 +273,9 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 }
 
 // Sense-free generation barrier for cooperative launches.  A block that waits longer than
-// the bounds above sets *err = CFD_ERR_BARRIER and leaves; callers check err.
+// the bounds above, or finds that another has, sets *err = CFD_ERR_BARRIER and leaves; callers
+// check err after each barrier, so that a launch after a failure, which left its counts standing,
+// ends at its first barrier.
 
 struct GridBar {
     unsigned int arrive;
@@ -299,7 +301,8 @@ __device__ __forceinline__ void grid_barrier(GridBar* gb, unsigned nblocks,
             const unsigned long long t0 = globaltimer_ns();
             while (*vgen == g) {
                 if (++spins > limit ||
-                    ((spins & 63) == 0 && globaltimer_ns() - t0 > kWaitNs)) {
+                    ((spins & 63) == 0 &&
+                     (*(volatile int*)&gb->err || globaltimer_ns() - t0 > kWaitNs))) {
                     atomicExch(&gb->err, (int)CFD_ERR_BARRIER);
                     break;
                 }

@@ -44,6 +44,16 @@ constexpr int kGroup = 4;             // chunks a block takes between two barrie
 // last block to leave a launch that did not fail clears the count for the next one (gb->gen
 // counts the leavers), so that no clearing stands before each launch.  A failure leaves the count
 // as it stood; launches that find err set do nothing, until the host has reported and cleared it.
+// bar_clock, every 64 polls: when the wait began (0 before), or ~0 to give up; one copy, out of
+// the iterations' instructions.
+__device__ __noinline__ unsigned long long bar_clock(GridBar* gb, unsigned long long t0, bool over) {
+    if (*(volatile const int*)&gb->err) return ~0ull;
+    const unsigned long long now = globaltimer_ns();
+    if (t0 == 0) t0 = now;
+    if (!over && now - t0 <= kWaitNs) return t0;
+    atomicExch(&gb->err, (int)CFD_ERR_BARRIER);
+    return ~0ull;
+}
 __device__ __forceinline__ bool bar_arrive_wait(GridBar* gb, unsigned target,
                                                 long long limit = kSpinLimit) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&gb->arrive) : "memory");
@@ -52,15 +62,7 @@ __device__ __forceinline__ bool bar_arrive_wait(GridBar* gb, unsigned target,
         unsigned v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&gb->arrive) : "memory");
         if ((int)(v - target) >= 0) return true;
-        if ((spins & 63) == 63) {
-            if (*(volatile const int*)&gb->err) return false;
-            const unsigned long long now = globaltimer_ns();
-            if (t0 == 0) t0 = now;
-            if (now - t0 > kWaitNs || spins > limit) {
-                atomicExch(&gb->err, (int)CFD_ERR_BARRIER);
-                return false;
-            }
-        }
+        if ((spins & 63) == 63 && (t0 = bar_clock(gb, t0, spins > limit)) == ~0ull) return false;
     }
 }
 

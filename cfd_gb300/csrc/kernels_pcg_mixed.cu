@@ -533,7 +533,6 @@ __global__ void __launch_bounds__(256, 2) k_pcg_mixed(PcgArgs a) {
     __shared__ double sh[4][256];
     __shared__ double res[4];
     __shared__ double s_thr[2], s_ref2[2];  // relative modes: threshold on r.r, ref.ref
-    __shared__ bool s_failed;  // a barrier of an earlier launch gave up and left its counts standing
     const int t = threadIdx.x;
     const int n = a.n;
     const int ns = a.nsolve;
@@ -558,9 +557,7 @@ __global__ void __launch_bounds__(256, 2) k_pcg_mixed(PcgArgs a) {
         s_ref2[t] = a.bscal[8 * t + 4];
         s_thr[t] = a.bscal[8 * t + 5];
     }
-    if (t == 2) s_failed = bar_failed_m(a.bar);
     __syncthreads();
-    if (s_failed) return;
     int prev[2] = {0, 0};  // a second pass: the first pass's iterations
 #pragma unroll
     for (int s = 0; s < 2; ++s)
