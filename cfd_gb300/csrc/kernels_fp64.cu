@@ -450,7 +450,8 @@ k_elem_rhs(int e0, int e1, int nelem, const int4* __restrict__ elem, const doubl
         const double w0 = WX[p[0]], w1 = WX[p[1]], w2 = WX[p[2]];
         const double y0 = WY[p[0]], y1 = WY[p[1]], y2 = WY[p[2]];
         // sp(:,1)=(.5,.5,0), sp(:,2)=(0,.5,.5), sp(:,3)=(.5,0,.5); zero terms dropped
-        // every half is exact: twice the velocities at the points, four times the sums
+        // the halves folded: twice the velocities at the points, four times the sums (the same
+        // bits for normal values whose doubles do not overflow)
         const double wx[3] = {w0 + w1, w1 + w2, w0 + w2};
         const double wy[3] = {y0 + y1, y1 + y2, y0 + y2};
         const double qAR = 0.25 * AR;
@@ -530,7 +531,8 @@ static_assert(kInvPlanes == kElemInvPlanes, "cache planes");
 // 8 Cv*rho, 9 P22, 10 P23a, 11 P23b, 12 3*Uy(2)*v1, 13 Uy(3)*v2
 //
 // Both kernels are bound by the FP64 pipe (85% of it).  Kept out of it: the second product of
-// 0.5*a + 0.5*b (the halves are exact: 0.5*(a + b) has the same bits), the divisions by a
+// 0.5*a + 0.5*b (0.5*(a + b) has the same bits, but where a half is subnormal, whose last bit
+// can differ, or a + b overflows), the divisions by a
 // shared divisor (div_rcp2), and in the replay the prefix of each sum that no stage changes.
 // 1,048,576 nodes: the replay 1,669 us before, 1,514 now; k_elem_inv 3,912 and 3,808 us.
 
@@ -698,7 +700,8 @@ k_elem_inv(int nelem, const int4* __restrict__ elem, const double* __restrict__ 
         const double AR = div3(ar * dtl);
         const double w0 = WX[p[0]], w1 = WX[p[1]], w2 = WX[p[2]];
         const double y0 = WY[p[0]], y1 = WY[p[1]], y2 = WY[p[2]];
-        // every half is exact: twice the velocities at the points, four times the sums
+        // the halves folded: twice the velocities at the points, four times the sums (the same
+        // bits for normal values whose doubles do not overflow)
         const double wx[3] = {w0 + w1, w1 + w2, w0 + w2};
         const double wy[3] = {y0 + y1, y1 + y2, y0 + y2};
         const double qAR = 0.25 * AR;

@@ -23,7 +23,8 @@ static_assert((N_PARAMS + 1) % 4 == 0 && L_SIZE % 4 == 0 && LAYER0 % 4 == 0 && L
 // fit g = t + M d, d = p - c, over the body nodes: since sum d = 0, t = mean g and each row
 // of M solves [Sxx Sxy; Sxy Syy] m = [sum g d_x; sum g d_y].  A launch is latency: a
 // dependent FP64 add waits 64 clocks, so the sums of a pass are formed side by side
-// (block_trees) and a thread's nodes are loaded four at a time (34 us beside a 262,144-node step with one tree after the other, 21 us now).
+// (block_trees) and a thread's nodes are loaded four at a time (34 us beside a 262,144-node step
+// with one tree after the other, 21 us now).
 __global__ void k_globals(int nb, const int* __restrict__ bnode, const int* __restrict__ bkind,
                           const double* __restrict__ gx, const double* __restrict__ gy,
                           const double* __restrict__ X, const double* __restrict__ Y,
@@ -556,8 +557,9 @@ __global__ void __launch_bounds__(256) k_encode(int n, const float* __restrict__
 // 128 x 64: two groups of 256 threads take alternate rows of a 32-row tile, a thread forms
 // 8 x 4 outputs (3 vector loads for 32 FMAs), the next tile's values are loaded while this
 // one is summed; with BIAS (O = 64) the columns of dY are summed beside, four rows of a tile a
-// thread (by the products' threads they were a fifth of the FP32 operations).  49,794 nodes: 128 us + 54 us of fold before (2 shared loads per FMA, 64
-// rows per partial, 779 partials folded by one thread each), 25-32 us now.
+// thread (by the products' threads they were a fifth of the FP32 operations).  49,794 nodes:
+// 128 us + 54 us of fold before (2 shared loads per FMA, 64 rows per partial, 779 partials
+// folded by one thread each), 25-32 us now.
 template <int O, int I, bool BIAS>
 __global__ void __launch_bounds__(512)
 k_wgrad(int n, const float* __restrict__ dY, const float* __restrict__ gate,
@@ -750,7 +752,7 @@ __global__ void k_fold(int nq, const float* __restrict__ part, float* __restrict
 // the edges of the group before (34 us with a block per 16 nodes).
 // A warp takes the nodes i and i + 2 (half_warp_node): structured triangulations alternate
 // nodes of 4 and 8 edges, and a warp is as slow as the longer of its two (backward
-// 27 us with i and i + 1, 23 so).
+// 27 us with i and i + 1, 23 so, on such a mesh; on others one pairing is as good as another).
 __device__ __forceinline__ int half_warp_node(int half_warp) {
     const int w = half_warp >> 1;
     return 4 * (w >> 1) + (w & 1) + 2 * (half_warp & 1);

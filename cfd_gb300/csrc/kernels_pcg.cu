@@ -26,8 +26,8 @@
 // three barriers with two folds, which one warp per sum does alone: the chunk's products and
 // the partials go from memory straight into the fixed tree, and the scalars' divisions are
 // made once per block.  With 256-thread blocks (four rows per thread, vectors and matrix
-// re-read, every thread dividing the scalars) an iteration took 34.1 us at 147,456 rows,
-// 49.7 at 262,144 and 173 at 1,048,576; now 21.2, 42.5 and 132 us.
+// re-read, every thread dividing the scalars) an iteration took 32.1 us at 147,456 rows,
+// 46.0 at 262,144 and 167 at 1,048,576; now 21.8, 43.9 and 145 us.
 #include "cfd_kernels.cuh"
 
 namespace cfd {
@@ -84,8 +84,8 @@ __device__ __noinline__ double chunk_sum(const double* q, int cnt) {
     });
 }
 
-// The nc chunk partials -> their fold (256 lanes with stride 256, then the tree), by one warp; the loads are
-// clamped, not branched over, so that a lane's eight go out together
+// The nc chunk partials -> their fold (256 lanes with stride 256, then the tree), by one warp; the
+// loads are clamped, not branched over, so that a lane's eight go out together
 __device__ __noinline__ double chunk_fold(const double* part, long nc) {
     const int lane = threadIdx.x & 31, t = 32 * (lane >> 2) + (lane & 3);
     double acc[8];

@@ -25,7 +25,8 @@ __global__ void k_features(int n, const double* X, const double* Y, const int* k
 __global__ void k_edge_features(int m, const int* src, const int* nbr, const double* X,
                                 const double* Y, const Globals* G, float* e, const int* gate);
 // FP32 training passes (kernels_mpnn.cu): P|Q = [A; B] h; v = U [h; agg] + u and h1 = h +
-// relu(v), from the transposed weights that k_encode leaves in wt; their backward products (dhc = [dh | dagg / deg], dh += its first half + dPQ [A; B])
+// relu(v), from the transposed weights that k_encode leaves in wt; their backward products
+// (dhc = [dh | dagg / deg], dh += its first half + dPQ [A; B])
 int dense_pq(cudaStream_t st, int n, const float* h, const float* W, float* pq);
 int dense_update(cudaStream_t st, int n, const float* h, const float* agg, const float* W,
                  const float* b, float* v, float* h1);
