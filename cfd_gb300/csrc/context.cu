@@ -1340,6 +1340,19 @@ void Ctx::drop_graphs() {
     }
 }
 
+static long long kernel_nodes(cudaGraph_t g) {
+    size_t n = 0;
+    if (cudaGraphGetNodes(g, nullptr, &n) != cudaSuccess) return 0;
+    std::vector<cudaGraphNode_t> node(n);
+    if (n && cudaGraphGetNodes(g, node.data(), &n) != cudaSuccess) return 0;
+    long long k = 0;
+    for (const cudaGraphNode_t q : node) {
+        cudaGraphNodeType t;
+        k += cudaGraphNodeGetType(q, &t) == cudaSuccess && t == cudaGraphNodeTypeKernel;
+    }
+    return k;
+}
+
 // Capture the step of the current parity in place `at` of a call (step_exec); a capture that is
 // not possible here turns the graphs off.
 int Ctx::capture_step(int at) {
@@ -1354,8 +1367,9 @@ int Ctx::capture_step(int at) {
     capturing = false;
     dt_ahead = was_ahead;
     const cudaError_t ce = cudaStreamEndCapture(stream, &g);
-    const long long nk = g_launches.load() - k0;
-    g_launches.fetch_sub(nk);  // captured, not run
+    // captured, not run; counted in the graph, since other threads launch at the same time
+    const long long nk = g ? kernel_nodes(g) : g_launches.load() - k0;
+    g_launches.fetch_sub(nk);
     if (st == CFD_OK && ce == cudaSuccess && g && cudaGraphInstantiate(&ex, g, 0) == cudaSuccess) {
         step_graph[buf][at] = g;
         step_exec[buf][at] = ex;

@@ -330,3 +330,34 @@ def test_graphs_are_captured_while_the_first_call_runs(gpu_lib):
     assert a.graph_count() == 8 and a.graph_state()[1] == 12
     a.close()
     b.close()
+
+
+def test_launch_counts_of_two_threads(gpu_lib):
+    """Contexts that two threads step at the same time (each captures its graphs while the other
+    launches) add to cfd_kernel_launches what they add one after the other."""
+    import threading
+    from cfd_gb300 import abi, solver
+    kw = dict(moving=1, motion_law=1, heave_amp=0.05, motion_freq=0.5, mass_mode=2)
+    cases = [small_case(3, scale=20, seed=s, **kw) for s in (4, 5)]
+
+    def march(k):
+        for _ in range(6):
+            s = solver.Solver(k, precision=abi.CFD_PREC_MIXED)
+            for n in (1, 3, 1, 8, 1):
+                s.step(n)
+            s.close()
+
+    def launches(run):
+        before = abi.lib().cfd_kernel_launches()
+        run()
+        return abi.lib().cfd_kernel_launches() - before
+
+    def together():
+        t = [threading.Thread(target=march, args=(k,)) for k in cases]
+        for q in t:
+            q.start()
+        for q in t:
+            q.join()
+
+    alone = launches(lambda: [march(k) for k in cases])
+    assert launches(together) == alone
