@@ -284,6 +284,10 @@ struct GridBar {
     int pad;
 };
 
+// every 64 polls: out of time, or another block has given up (out of the barrier's own instructions)
+static __device__ __noinline__ bool grid_bar_over(GridBar* gb, unsigned long long t0) {
+    return *(volatile int*)&gb->err || globaltimer_ns() - t0 > kWaitNs;
+}
 __device__ __forceinline__ void grid_barrier(GridBar* gb, unsigned nblocks,
                                              long long limit = kSpinLimit) {
     __syncthreads();
@@ -300,9 +304,7 @@ __device__ __forceinline__ void grid_barrier(GridBar* gb, unsigned nblocks,
             long long spins = 0;
             const unsigned long long t0 = globaltimer_ns();
             while (*vgen == g) {
-                if (++spins > limit ||
-                    ((spins & 63) == 0 &&
-                     (*(volatile int*)&gb->err || globaltimer_ns() - t0 > kWaitNs))) {
+                if (++spins > limit || ((spins & 63) == 0 && grid_bar_over(gb, t0))) {
                     atomicExch(&gb->err, (int)CFD_ERR_BARRIER);
                     break;
                 }
